@@ -125,9 +125,8 @@ __device__ __noinline__ void near_fp64(const double* __restrict__ x, const doubl
         PairP0 p;
         pair_setup(s, x[0], x[1], x[2], p);
         if (TK) {
-            TMoments m;
-            t_moments(s, nrm, p, m);
-            t_block(m, nrm, c, s.eps2, blk);
+            src_normal(s, nrm);
+            t_pair(s, nrm, p, t_coef(c), blk);
         } else {
             UMoments m;
             u_moments(s, p, m);

@@ -462,9 +462,8 @@ near_eval_kernel(NearEvalArgs a) {
         pair_setup(src, a.x_field[3 * f], a.x_field[3 * f + 1], a.x_field[3 * f + 2], p);
         if (TKERNEL) {
             const double* nrm = a.normals + 3 * s;
-            TMoments m;
-            t_moments(src, nrm, p, m);
-            t_block(m, nrm, a.c, src.eps2, blk);
+            src_normal(src, nrm);
+            t_pair(src, nrm, p, t_coef(a.c), blk);
         } else {
             UMoments m;
             u_moments(src, p, m);
@@ -1202,11 +1201,10 @@ __global__ void __launch_bounds__(DR_THREADS) disp_readout_kernel(DispReadoutArg
                 if (!g.ok) continue;
                 PairP0 p;
                 pair_setup(g, ox, oy, oz, p);
-                TMoments m;
                 const double* n = a.normals + 3 * s;
-                t_moments(g, n, p, m);
+                src_normal(g, n);
                 double blk[3][3];
-                t_block(m, n, a.c, g.eps2, blk);
+                t_pair(g, n, p, t_coef(a.c), blk);
                 const double* d = a.density + 3 * s;
 #pragma unroll
                 for (int r = 0; r < 3; r++) acc[r] += blk[r][0] * d[0] + blk[r][1] * d[1] + blk[r][2] * d[2];

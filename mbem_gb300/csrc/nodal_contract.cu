@@ -6,15 +6,17 @@
 // block: a few observers still fill the part, each partial sum has one owner
 // and the sums are added in slice, then rank order through distributed shared
 // memory (deterministic, no workspace). Bound by the FP64 pipe: the stress of a
-// 16 x 16 P2 fault at 2,000 observers went from 266 to 16.7 ms.
+// 16 x 16 P2 fault at 2,000 observers went from 266 to 15.9 ms.
 #include <cooperative_groups.h>
 
+#include "contract_split.cuh"
 #include "nodal_launch.cuh"
 
 namespace mbem {
 
 namespace cg = cooperative_groups;
 
+constexpr int NC_TILE = 16;                           // source records in shared memory at a time
 constexpr int NC_T = 0, NC_U = 1, NC_STRESS = 2;      // kinds: T, U, 2 + MBEM_STRESS_*
 
 template <int P>
@@ -46,7 +48,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a,
     const int slices = ND_THREADS / ob;
     const int lane = threadIdx.x % ob, slice = threadIdx.x / ob;
     const int64_t f = (int64_t)(blockIdx.x / ranks) * ob + lane;
-    const bool active = f < a.n_field_pts;
+    const bool active = f < a.n_field_pts && slice < slices;
     double x[3] = {0.0, 0.0, 0.0};
     if (active) {
         x[0] = a.x_field[3 * f];
@@ -189,16 +191,12 @@ int nodal_contract(int kind, const double* x, int64_t nf, const double* tv, cons
     a.which = kind >= NC_STRESS ? kind - NC_STRESS : 0;
     a.alpha = alpha; a.accumulate = accumulate; a.out = out;
     if (nf == 0) return MBEM_OK;
-    // three rounds of resident blocks: first the cluster splits the sources
-    // (each source's record is still made once per observer group), then the
-    // block's slices do, down to four observers a block
-    int ranks = 1, ob = ND_THREADS;
-    while (ranks < 8 && 16 * ranks < ns && ceil_div(nf, ob) * ranks < 3 * ND_SLOTS) ranks *= 2;
-    while (ob > 4 && (ND_THREADS / ob) * ranks < ns && ceil_div(nf, ob) * ranks < 3 * ND_SLOTS) ob /= 2;
+    const ConSplit sp = contract_split(nf, ns, ND_THREADS, NC_TILE, order == 1 ? 1200.0 : 2200.0, 600.0);
+    const int ob = sp.ob, ranks = sp.ranks;
     const int64_t grid = ceil_div(nf, ob) * ranks;
     MBEM_REQUIRE(grid < (int64_t)1 << 31, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)nf);
-    const cudaError_t ce = order == 1 ? launch_nodal_contract<1>(kind, a, (unsigned)grid, ranks, ob, 16, (cudaStream_t)stream)
-                                      : launch_nodal_contract<2>(kind, a, (unsigned)grid, ranks, ob, 16, (cudaStream_t)stream);
+    const cudaError_t ce = order == 1 ? launch_nodal_contract<1>(kind, a, (unsigned)grid, ranks, ob, NC_TILE, (cudaStream_t)stream)
+                                      : launch_nodal_contract<2>(kind, a, (unsigned)grid, ranks, ob, NC_TILE, (cudaStream_t)stream);
     if (ce != cudaSuccess) return set_error(MBEM_ERR_CUDA, "nodal_contract_kernel: %s", cudaGetErrorString(ce));
     return launch_status("nodal_contract_kernel");
 }

@@ -35,14 +35,16 @@
 
 namespace mbem {
 
-enum NodalFam { NF_T, NF_U, NF_H, NF_E, NF_S };   // T, U, DD stress, eigenstress, Kelvin stress
+// T, U, DD stress, eigenstress, Kelvin stress; TG and HG: T and DD for any source
+// normal. For the frame's normal the trace identities |d|^2 = R^2 - eps^2 leave T
+// with n = 5 to degree 2 (3 in general) and DD with n = 7 to degree 3 (4).
+enum NodalFam { NF_T, NF_U, NF_H, NF_E, NF_S, NF_TG, NF_HG };
 
 constexpr int ND_MAXK = 6;
 constexpr double ND_D_STAR = 10.0;
 
 __host__ __device__ constexpr int nd_nodes(int p) { return (p + 1) * (p + 2) / 2; }
 __host__ __device__ constexpr int nd_max(int a, int b) { return a > b ? a : b; }
-__host__ __device__ constexpr int nd_tri(int a, int b) { return (a + b) * (a + b + 1) / 2 + b; }
 __host__ __device__ constexpr int nd_len(int d) { return d < 0 ? 1 : (d + 1) * (d + 2) / 2; }
 __host__ __device__ constexpr int nd_edge(int d) { return d < 0 ? -1 : nd_max(d - 1, 0); }
 
@@ -50,10 +52,11 @@ __host__ __device__ constexpr int nd_edge(int d) { return d < 0 ? -1 : nd_max(d 
 // closure under the recursion and its seeds), and the edge degrees they need.
 template <int P, int F>
 struct NDeg {
-    static constexpr int d7 = F == NF_H ? 4 + P : F == NF_E ? P : -1;
-    static constexpr int d5 = F == NF_H ? 2 + P : F == NF_E ? 0 : F == NF_U ? -1 : 3 + P;
-    static constexpr int d3 = F == NF_H ? P : F == NF_E ? 0 : F == NF_U ? 2 + P : 1 + P;
-    static constexpr int d1 = F == NF_H ? (P >= 2 ? P - 2 : -1) : F == NF_E ? -1 : F == NF_U ? P : P - 1;
+    static constexpr bool H = F == NF_H || F == NF_HG;
+    static constexpr int d7 = F == NF_H ? 3 + P : F == NF_HG ? 4 + P : F == NF_E ? P : -1;
+    static constexpr int d5 = H ? 2 + P : F == NF_E ? 0 : F == NF_U ? -1 : F == NF_T ? 2 + P : 3 + P;
+    static constexpr int d3 = H ? P : F == NF_E ? 0 : F == NF_U ? 2 + P : 1 + P;
+    static constexpr int d1 = H ? (P >= 2 ? P - 2 : -1) : F == NF_E ? -1 : F == NF_U ? P : P - 1;
     static constexpr int dm1 = (F == NF_U && P == 2) ? 0 : -1;
     static constexpr int e5 = nd_edge(d7);
     static constexpr int e3 = nd_max(nd_edge(d5), d5 >= 0 ? 0 : -1);
@@ -543,10 +546,10 @@ __device__ __noinline__ void node_tables(const NodalRec& g, const double* x, Nod
         if constexpr (F == NF_U) {
             weight_moments<P, 0>(M.m1, C, &W.w1[k]);
             weight_moments<P, 2>(M.m3, C, W.w3[k]);
-        } else if constexpr (F == NF_T || F == NF_S) {
+        } else if constexpr (F == NF_TG || F == NF_S) {
             weight_moments<P, 1>(M.m3, C, W.w3[k]);
             weight_moments<P, 3>(M.m5, C, W.w5[k]);
-        } else if constexpr (F == NF_H) {
+        } else if constexpr (F == NF_HG) {
             weight_moments<P, 0>(M.m3, C, W.w3[k]);
             weight_moments<P, 2>(M.m5, C, W.w5[k]);
             weight_moments<P, 4>(M.m7, C, W.w7[k]);
@@ -561,78 +564,14 @@ __device__ __forceinline__ bool node_by_node(const NodalRec& g) { return P == 2 
 // ---------------------------------------------------------------------------
 // local forms (source frame)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void rotate_full(const NodalRec& g, const double B[3][3], double G[3][3]) {
-    double Y[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) Y[a][j] = B[a][0] * g.ex[j] + B[a][1] * g.ey[j] + B[a][2] * g.nh[j];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) G[i][j] = g.ex[i] * Y[0][j] + g.ey[i] * Y[1][j] + g.nh[i] * Y[2][j];
-}
-// symmetric L (00 11 22 01 02 12) to the global frame, same layout
-__device__ __forceinline__ void rotate_six(const NodalRec& g, const double L[6], double G[6]) {
-    const int ix[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-    double Y[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            Y[a][j] = L[ix[a][0]] * g.ex[j] + L[ix[a][1]] * g.ey[j] + L[ix[a][2]] * g.nh[j];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = i; j < 3; j++) G[ix[i][j]] = g.ex[i] * Y[0][j] + g.ey[i] * Y[1][j] + g.nh[i] * Y[2][j];
-}
-__device__ __forceinline__ void to_frame(const NodalRec& g, const double* v, double l[3]) {
-    l[0] = v[0] * g.ex[0] + v[1] * g.ex[1] + v[2] * g.ex[2];
-    l[1] = v[0] * g.ey[0] + v[1] * g.ey[1] + v[2] * g.ey[2];
-    l[2] = v[0] * g.nh[0] + v[1] * g.nh[1] + v[2] * g.nh[2];
-}
-
-// coefficients of the combined T block: out = n_j alpha_i + n_i beta_j - 6 c5 W_ij + d_ij n.beta
-struct TCoef {
-    double ca, c1m3, ce3, cb, ce6, w6;   // ce3, ce6 without eps^2
-};
-__host__ __device__ __forceinline__ TCoef t_coef(const double c[6]) {
-    TCoef t;
-    t.ca = c[0] + 4.0 * c[1] + 2.0 * c[4];
-    t.c1m3 = -3.0 * c[1];
-    t.ce3 = c[2];
-    t.cb = c[3] + c[4];
-    t.ce6 = c[5];
-    t.w6 = -6.0 * c[4];
-    return t;
-}
-
-// The T block (source frame, normal +e3) of the moments shifted by (SA, SB).
+// The T block (source frame, normal s e3) of the moments shifted by (SA, SB).
 template <int SA, int SB>
 __device__ __forceinline__ void t_local_shift(const double* m3, const double* m5, double z, double eps2,
-                                              const TCoef& c, double B[3][3]) {
+                                              const TCoef& c, double s, double B[3][3]) {
 #define M3_(a, b) m3[nd_tri((a) + SA, (b) + SB)]
 #define M5_(a, b) m5[nd_tri((a) + SA, (b) + SB)]
-    const double z2 = z * z, zi3 = z * M3_(0, 0), zi5 = z * M5_(0, 0);
-    const double q0 = z2 * M5_(1, 0), q1 = z2 * M5_(0, 1), q2 = z2 * zi5;     // -T022, -T122, T222
-    const double w00 = z * M5_(2, 0), w11 = z * M5_(0, 2), w01 = z * M5_(1, 1);
-    const double t0 = -(M5_(3, 0) + M5_(1, 2)) - q0, t1 = -(M5_(2, 1) + M5_(0, 3)) - q1, t2 = (w00 + w11) + q2;
-    const double ce3 = c.ce3 * eps2, ce6 = c.ce6 * eps2;
-    const double al0 = c.c1m3 * t0 - (c.ca * M3_(1, 0) + ce3 * M5_(1, 0));
-    const double al1 = c.c1m3 * t1 - (c.ca * M3_(0, 1) + ce3 * M5_(0, 1));
-    const double al2 = c.c1m3 * t2 + (c.ca * zi3 + ce3 * zi5);
-    const double be0 = -(c.cb * M3_(1, 0) + ce6 * M5_(1, 0));
-    const double be1 = -(c.cb * M3_(0, 1) + ce6 * M5_(0, 1));
-    const double be2 = c.cb * zi3 + ce6 * zi5;
-    B[0][0] = c.w6 * w00 + be2;
-    B[1][1] = c.w6 * w11 + be2;
-    B[0][1] = B[1][0] = c.w6 * w01;
-    const double v0 = -c.w6 * q0, v1 = -c.w6 * q1;
-    B[0][2] = v0 + al0;
-    B[1][2] = v1 + al1;
-    B[2][0] = v0 + be0;
-    B[2][1] = v1 + be1;
-    B[2][2] = c.w6 * q2 + al2 + 2.0 * be2;
+    t_local(M3_(0, 0), M3_(1, 0), M3_(0, 1), M5_(0, 0), M5_(1, 0), M5_(0, 1), M5_(2, 0), M5_(1, 1), M5_(0, 2), z, eps2,
+            c, s, B);
 #undef M3_
 #undef M5_
 }
@@ -648,8 +587,7 @@ __device__ __forceinline__ void t_local_col(const double* m3, const double* m5, 
                  T011 = -m5[nd_tri(1, 2)], T012 = z * m5[nd_tri(1, 1)], T022 = -z2 * m5[nd_tri(1, 0)],
                  T111 = -m5[nd_tri(0, 3)], T112 = z * m5[nd_tri(0, 2)], T122 = -z2 * m5[nd_tri(0, 1)],
                  T222 = z2 * z * m5[0];
-    const double tl[3] = {T000 + T011 + T022, T001 + T111 + T122, T002 + T112 + T222};
-    const double ce3 = c.ce3 * eps2, ce6 = c.ce6 * eps2;
+    const double c5 = c.c5 * eps2, ce6 = c.ce6 * eps2;
     // T3[i][J][.] . nl
     double W[3];
     if (J == 0) {
@@ -671,118 +609,9 @@ __device__ __forceinline__ void t_local_col(const double* m3, const double* m5, 
     const double gam = nl[0] * be[0] + nl[1] * be[1] + nl[2] * be[2];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        const double al = c.ca * V3[i] + c.c1m3 * tl[i] + ce3 * V5[i];
+        const double al = c.c3 * V3[i] + c5 * V5[i];
         out[i] += nl[J] * al + nl[i] * be[J] + c.w6 * W[i] + (i == J ? gam : 0.0);
     }
-}
-
-// material constants of the stress forms
-struct SMat {
-    double mu, lam, C1, c34;
-    double k3a;        // 3 c34 - 9
-    double x1;         // 3 c34 - 18
-    double blob;       // 2 (1 - nu), times eps^2: cblob
-    double phi;        // 15 / (8 pi), times eps^4
-};
-__host__ __device__ inline SMat stress_mat(double mu, double lam) {
-    SMat m;
-    const double nu = lam / (2.0 * (lam + mu));
-    m.mu = mu;
-    m.lam = lam;
-    m.C1 = 1.0 / (16.0 * MBEM_PI * mu * (1.0 - nu));
-    m.c34 = 3.0 - 4.0 * nu;
-    m.k3a = 3.0 * m.c34 - 9.0;
-    m.x1 = 3.0 * m.c34 - 18.0;
-    m.blob = 2.0 * (1.0 - nu);
-    m.phi = 15.0 / (8.0 * MBEM_PI);
-    return m;
-}
-
-// Stress (00 11 22 01 02 12, source frame, normal +e3) of slip along e_K with
-// the moment set (m3[0]; m5 to degree 2; m7 to degree 4), times w and added:
-// the DD stress of tri_kernels.py:900-964 for that normal and slip, and with
-// EIG the eigenstress (tri_kernels.py:1206-1214) taken off.
-template <int K>
-__device__ __forceinline__ void dd_unit(const double* m3, const double* m5, const double* m7, double z, double eps2,
-                                        const SMat& m, bool eig, double w, double out[6]) {
-#define A5(a, b) m5[nd_tri(a, b)]
-#define A7(a, b) m7[nd_tri(a, b)]
-    const double cb = m.blob * eps2;
-    const double z2 = z * z;
-    const double I3 = m3[0], I5 = A5(0, 0), I7 = A7(0, 0);
-    const double phi = eig ? m.phi * eps2 * eps2 * I7 : 0.0;
-    if (K < 2) {
-        // u: the slip axis, v: the other in-plane axis; d = (-xi, z)
-#define U5(a, b) (K == 0 ? A5(a, b) : A5(b, a))
-#define U7(a, b) (K == 0 ? A7(a, b) : A7(b, a))
-        const double T5u3 = -z * U5(1, 0), T5v3 = -z * U5(0, 1), T533 = z2 * I5;
-        const double zu = -z * U7(1, 0), zv = -z * U7(0, 1), z33 = z2 * I7;
-        const double c15 = 15.0 * cb;
-        const double Fu3 = m.k3a * T5u3 + c15 * zu;
-        const double Fv3 = m.k3a * T5v3 + c15 * zv;
-        const double Fuv = m.k3a * U5(1, 1) + c15 * U7(1, 1);
-        const double Fuu33 = m.k3a * (U5(2, 0) + T533) + c15 * (U7(2, 0) + z33);
-        const double q0 = -z * U7(3, 0), q1 = -z * U7(1, 2), q2 = z2 * zu;        // T4 uuu3, vvu3, 33u3
-        const double q3 = -z * U7(2, 1), q4 = z2 * U7(2, 0), q5 = z2 * U7(1, 1);  // uvu3, u3u3, v3u3
-        const double tr = 2.0 * Fu3 - 18.0 * T5u3 + 30.0 * ((q0 + q1) + q2);
-        const double g = -m.C1 * m.mu * w;
-        const double t = m.lam * tr;
-        const double base = -12.0 * T5u3;
-        const double sA = 2.0 * ((1.0 - m.c34) * I3 - 3.0 * cb * I5);
-        const double suu = t + m.mu * (base + 2.0 * Fu3 + 60.0 * q0);
-        const double svv = t + m.mu * (base + 60.0 * q1);
-        const double s33 = t + m.mu * (base + 2.0 * Fu3 + 60.0 * q2);
-        const double suv = Fv3 + 60.0 * q3, su3 = sA + Fuu33 + 60.0 * q4, sv3 = Fuv + 60.0 * q5;
-        const double gn = -m.C1 * w;
-        // sigma = -C1 mu (lam tr delta + mu (Y + Y^T))
-        const double gm = gn * m.mu;
-        out[K] += gm * suu;
-        out[1 - K] += gm * svv;
-        out[2] += gm * s33;
-        const double g2 = g * m.mu;
-        out[3] += g2 * suv;
-        out[K == 0 ? 4 : 5] += g2 * su3 - (m.mu * w) * phi;
-        out[K == 0 ? 5 : 4] += g2 * sv3;
-#undef U5
-#undef U7
-    } else {
-        const double T00 = A5(2, 0), T11 = A5(0, 2), T01 = A5(1, 1), T02 = -z * A5(1, 0), T12 = -z * A5(0, 1),
-                     T22 = z2 * I5;
-        const double S00 = A7(2, 0), S11 = A7(0, 2), S01 = A7(1, 1), S02 = -z * A7(1, 0), S12 = -z * A7(0, 1),
-                     S22 = z2 * I7;
-        const double trT = (T00 + T11) + T22, trS = (S00 + S11) + S22;
-        // T4_rt33 and t4c_rt = T4_rt11 + T4_rt22 + T4_rt33
-        const double Q00 = z2 * S00, Q11 = z2 * S11, Q01 = z2 * S01, Q02 = z2 * S02, Q12 = z2 * S12, Q22 = z2 * S22;
-        const double C00 = (A7(4, 0) + A7(2, 2)) + Q00, C11 = (A7(2, 2) + A7(0, 4)) + Q11,
-                     C01 = (A7(3, 1) + A7(1, 3)) + Q01, C02 = Q02 - z * (A7(3, 0) + A7(1, 2)),
-                     C12 = Q12 - z * (A7(2, 1) + A7(0, 3)), C22 = (Q00 + Q11) + Q22;
-        const double c15 = 15.0 * cb;
-        const double I3c = I3;
-        const double xd = (4.0 - m.c34) * I3c - 3.0 * trT - 3.0 * cb * I5;
-        const double trX = 3.0 * xd + m.x1 * trT + 15.0 * ((C00 + C11) + C22) + c15 * trS;
-        const double F02 = m.k3a * T02 + c15 * S02, F12 = m.k3a * T12 + c15 * S12, F22 = m.k3a * T22 + c15 * S22;
-        const double A = (1.0 - m.c34) * I3 - 3.0 * cb * I5;
-        const double trY = 2.0 * A + 6.0 * I3 + 2.0 * F22 - 18.0 * T22 - 6.0 * trT + 30.0 * C22;
-        const double trB = m.lam * trX + m.mu * trY;
-        const double yd = 4.0 * I3 - 12.0 * T22;
-        // X = xd delta + x1 T + 15 C + c15 S ; Y + Y^T = yd delta - 12 T + 60 Q + (e3, F terms) + 4 A e3 e3
-        const double l2 = 2.0 * m.lam, mu = m.mu;
-        const double diag = m.lam * trB + mu * (l2 * xd + mu * yd);
-        const double gw = -m.C1 * w;
-        const double ep = phi * w;
-        out[0] += gw * (diag + mu * (l2 * (m.x1 * T00 + 15.0 * C00 + c15 * S00) + mu * (60.0 * Q00 - 12.0 * T00))) -
-                  ep * m.lam;
-        out[1] += gw * (diag + mu * (l2 * (m.x1 * T11 + 15.0 * C11 + c15 * S11) + mu * (60.0 * Q11 - 12.0 * T11))) -
-                  ep * m.lam;
-        out[2] += gw * (diag + mu * (l2 * (m.x1 * T22 + 15.0 * C22 + c15 * S22) +
-                                     mu * (60.0 * Q22 - 12.0 * T22 + 4.0 * (F22 + A)))) -
-                  ep * (m.lam + 2.0 * mu);
-        out[3] += gw * mu * (l2 * (m.x1 * T01 + 15.0 * C01 + c15 * S01) + mu * (60.0 * Q01 - 12.0 * T01));
-        out[4] += gw * mu * (l2 * (m.x1 * T02 + 15.0 * C02 + c15 * S02) + mu * (60.0 * Q02 - 12.0 * T02 + 2.0 * F02));
-        out[5] += gw * mu * (l2 * (m.x1 * T12 + 15.0 * C12 + c15 * S12) + mu * (60.0 * Q12 - 12.0 * T12 + 2.0 * F12));
-    }
-#undef A5
-#undef A7
 }
 
 // the same for any normal nl and a slip sl (source frame) through the general
@@ -869,14 +698,13 @@ __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x,
             for (int i = 0; i < 3; i++)
 #pragma unroll
                 for (int j = 0; j < 3; j++) acc[k][i][j] = 0.0;
-        const double ce3 = c.ce3 * g.eps2, ce6 = c.ce6 * g.eps2;
+        const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
         const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
         far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double, double, double R2, double w,
                                                       double l0, double l1, double l2) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = w * iR * iR2, b = a * iR2;
-            const double r2 = R2 - g.eps2;
-            const double pa = c.ca * a + (ce3 + c.c1m3 * r2) * b, pb = c.cb * a + ce6 * b;
+            const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
             const double d0 = -xi1, d1 = -xi2;
             const double dn = d0 * n0 + d1 * n1 + z * n2;
             const double wn = c.w6 * b * dn, gam = pb * dn;
@@ -912,7 +740,7 @@ __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x,
     }
     if (!g.aligned || node_by_node<P>(g)) {
         NodeTab<P> W;
-        node_tables<P, NF_T>(g, x, W);
+        node_tables<P, NF_TG>(g, x, W);
 #pragma unroll 1
         for (int k = 0; k < K; k++) {
             double col[3][3], T[3][3], G[3][3];
@@ -939,9 +767,7 @@ __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x,
 #define MBEM_ND_SHIFT(sa, sb)                                                                        \
 {                                                                                                \
     double T[3][3];                                                                              \
-    t_local_shift<sa, sb>(M.m3, M.m5, z, g.eps2, c, T);                                          \
-    _Pragma("unroll") for (int i = 0; i < 3; i++)                                                \
-        _Pragma("unroll") for (int j = 0; j < 3; j++) T[i][j] *= g.s;                            \
+    t_local_shift<sa, sb>(M.m3, M.m5, z, g.eps2, c, g.s, T);                                     \
     rotate_full(g, T, B[nd_tri(sa, sb)]);                                                        \
 }
     MBEM_ND_SHIFT(0, 0)
@@ -1004,8 +830,8 @@ __device__ __forceinline__ void pair_t_basis(const NodalRec& g, const double* x,
                 }
         });
     } else {
-        NMom<P, NF_T> M;
-        nodal_moments<P, NF_T>(g, o, M);
+        NMom<P, NF_TG> M;
+        nodal_moments<P, NF_TG>(g, o, M);
         double l[3];
         lam_at_foot(g, o, l);
 #pragma unroll
@@ -1168,7 +994,7 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
     const double z = o.z;
     double v[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        const double ce3 = c.ce3 * g.eps2, ce6 = c.ce6 * g.eps2;
+        const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
         const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
         far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double e1, double e2, double R2,
                                                       double w, double, double, double) {
@@ -1176,8 +1002,7 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
                          u2 = den_value<P>(D.f[2], e1, e2);
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = w * iR * iR2, b = a * iR2;
-            const double r2 = R2 - g.eps2;
-            const double pa = c.ca * a + (ce3 + c.c1m3 * r2) * b, pb = c.cb * a + ce6 * b;
+            const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
             const double d0 = -xi1, d1 = -xi2;
             const double dn = d0 * n0 + d1 * n1 + z * n2, du = d0 * u0 + d1 * u1 + z * u2;
             const double un = u0 * n0 + u1 * n1 + u2 * n2;
@@ -1187,9 +1012,9 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
             v[1] += s * d1 + t * n1 + q * u1;
             v[2] += s * z + t * n2 + q * u2;
         });
-    } else if (node_by_node<P>(g)) {
+    } else if (!g.aligned || node_by_node<P>(g)) {
         NodeTab<P> W;
-        node_tables<P, NF_T>(g, x, W);
+        node_tables<P, NF_TG>(g, x, W);
 #pragma unroll 1
         for (int k = 0; k < nd_nodes(P); k++) {
             double q[3][3];
@@ -1207,11 +1032,14 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
         nodal_moments<P, NF_T>(g, o, M);
 #define MBEM_ND_COL(j)                                                \
     {                                                                 \
-        double C[nd_nodes(P)], W3[3], W5[10];                         \
+        double C[nd_nodes(P)], W3[3], W5[6], B[3][3];                 \
         den_at_foot<P>(D.f[j], o.X1, o.X2, C);                        \
         weight_moments<P, 1>(M.m3, C, W3);                            \
-        weight_moments<P, 3>(M.m5, C, W5);                            \
-        t_local_col<j>(W3, W5, z, g.eps2, c, g.nl, v);                \
+        weight_moments<P, 2>(M.m5, C, W5);                            \
+        t_local_shift<0, 0>(W3, W5, z, g.eps2, c, g.s, B);            \
+        v[0] += B[0][j];                                              \
+        v[1] += B[1][j];                                              \
+        v[2] += B[2][j];                                              \
     }
         MBEM_ND_COL(0)
         MBEM_ND_COL(1)
@@ -1363,7 +1191,7 @@ __device__ __forceinline__ void pair_dd_contract(const NodalRec& g, const NodalD
     } else {
         if (!g.aligned || node_by_node<P>(g)) {
             NodeTab<P> W;
-            node_tables<P, NF_H>(g, x, W);
+            node_tables<P, NF_HG>(g, x, W);
 #pragma unroll 1
             for (int k = 0; k < nd_nodes(P); k++) {
                 const double* sl = D.node[k];
@@ -1376,11 +1204,11 @@ __device__ __forceinline__ void pair_dd_contract(const NodalRec& g, const NodalD
             nodal_moments<P, NF_H>(g, o, M);
 #define MBEM_ND_COL(j)                                              \
     {                                                               \
-        double C[nd_nodes(P)], W3[1], W5[6], W7[15];                \
+        double C[nd_nodes(P)], W3[1], W5[6], W7[10];                \
         den_at_foot<P>(D.f[j], o.X1, o.X2, C);                      \
         weight_moments<P, 0>(M.m3, C, W3);                          \
         weight_moments<P, 2>(M.m5, C, W5);                          \
-        weight_moments<P, 4>(M.m7, C, W7);                          \
+        weight_moments<P, 3>(M.m7, C, W7);                          \
         I7[j] = W7[0];                                              \
         dd_unit<j>(W3, W5, W7, z, e2, m, eig, g.s, v);              \
     }
@@ -1526,7 +1354,7 @@ __device__ __forceinline__ void pair_kelvin_contract(const NodalRec& g, const No
 // ---------------------------------------------------------------------------
 enum { TR_SLIP = 0, TR_FORCE = 1, TR_EIGEN = 2, TR_TOTAL = 3 };
 
-template <int P, int F>
+template <int F>
 __device__ __forceinline__ void traction_block(const NodalRec& g, double z, const SMat& m, bool eig,
                                                const double nf[3], const double* W3, const double* W5,
                                                const double* W7, double T[3][3]) {
@@ -1548,7 +1376,7 @@ __device__ __forceinline__ void traction_block(const NodalRec& g, double z, cons
             v[3] = ph * m.mu * (sl[0] * g.nl[1] + g.nl[0] * sl[1]);                                              \
             v[4] = ph * m.mu * (sl[0] * g.nl[2] + g.nl[0] * sl[2]);                                              \
             v[5] = ph * m.mu * (sl[1] * g.nl[2] + g.nl[1] * sl[2]);                                              \
-        } else if (g.aligned) {                                                                                  \
+        } else if (F == NF_H) {                                                                                  \
             dd_unit<j>(W3, W5, W7, z, g.eps2, m, eig, g.s, v);                                                   \
         } else {                                                                                                 \
             dd_general(W3, W5, W7, z, g.eps2, m, g.nl, sl, eig, v);                                              \
@@ -1563,14 +1391,15 @@ __device__ __forceinline__ void traction_block(const NodalRec& g, double z, cons
     rotate_full(g, L, T);
 }
 
+// F as in NodalFam: NF_H for a source normal along the frame's, NF_HG for any
 template <int P, int F, class Put>
-__device__ __forceinline__ void pair_traction(const NodalRec& g, const double* x, const double* nfg, const SMat& m,
-                                              bool eig, Put&& put) {
+__device__ __forceinline__ void pair_traction_fam(const NodalRec& g, const double* x, const double* nfg, const SMat& m,
+                                                  bool eig, Put&& put) {
     constexpr int K = nd_nodes(P);
     const NodalObs o = nodal_obs(g, x);
     double nf[3];
     to_frame(g, nfg, nf);
-    constexpr int D3 = F == NF_S ? 1 : 0, D5 = F == NF_S ? 3 : 2, D7 = 4;
+    constexpr int D3 = F == NF_S ? 1 : 0, D5 = F == NF_S ? 3 : 2, D7 = F == NF_E ? 0 : F == NF_H ? 3 : 4;
     if (nodal_is_far(g, o)) {
         double W3[K][3], W5[K][10], W7[K][15];
 #pragma unroll
@@ -1600,21 +1429,24 @@ __device__ __forceinline__ void pair_traction(const NodalRec& g, const double* x
             for (int k = 0; k < K; k++) {
                 const double na = N[k] * a, nb = N[k] * b, nc = N[k] * c;
                 if (F != NF_E) {
+                    W3[k][0] += na;
 #pragma unroll
-                    for (int t = 0; t < nd_len(D3); t++) W3[k][t] += na * p[t];
+                    for (int t = 1; t < nd_len(D3); t++) W3[k][t] += na * p[t];
+                    W5[k][0] += nb;
 #pragma unroll
-                    for (int t = 0; t < nd_len(D5); t++) W5[k][t] += nb * p[t];
+                    for (int t = 1; t < nd_len(D5); t++) W5[k][t] += nb * p[t];
                 }
                 if (F != NF_S) {
+                    W7[k][0] += nc;
 #pragma unroll
-                    for (int t = 0; t < (F == NF_E ? 1 : nd_len(D7)); t++) W7[k][t] += nc * p[t];
+                    for (int t = 1; t < nd_len(D7); t++) W7[k][t] += nc * p[t];
                 }
             }
         });
 #pragma unroll 1
         for (int k = 0; k < K; k++) {
             double T[3][3];
-            traction_block<P, F>(g, o.z, m, eig, nf, W3[k], W5[k], W7[k], T);
+            traction_block<F>(g, o.z, m, eig, nf, W3[k], W5[k], W7[k], T);
             put(k, T);
         }
         return;
@@ -1627,15 +1459,25 @@ __device__ __forceinline__ void pair_traction(const NodalRec& g, const double* x
     for (int k = 0; k < K; k++) {
         double C[K], W3[3], W5[10], W7[15], T[3][3];
         shape_about_foot<P>(g, l, k, C);
-        if (F != NF_E) {
+        if constexpr (F != NF_E) {
             weight_moments<P, D3>(M.m3, C, W3);
             weight_moments<P, D5>(M.m5, C, W5);
         }
-        if (F == NF_E) weight_moments<P, 0>(M.m7, C, W7);
-        else if (F == NF_H) weight_moments<P, (F == NF_H ? D7 : 0)>(M.m7, C, W7);
-        traction_block<P, F>(g, o.z, m, eig, nf, W3, W5, W7, T);
+        if constexpr (F != NF_S) weight_moments<P, D7>(M.m7, C, W7);
+        traction_block<F>(g, o.z, m, eig, nf, W3, W5, W7, T);
         put(k, T);
     }
+}
+template <int P, class Put>
+static __device__ __noinline__ void pair_traction_general(const NodalRec& g, const double* x, const double* nfg,
+                                                          const SMat& m, bool eig, Put&& put) {
+    pair_traction_fam<P, NF_HG>(g, x, nfg, m, eig, put);
+}
+template <int P, int F, class Put>
+__device__ __forceinline__ void pair_traction(const NodalRec& g, const double* x, const double* nfg, const SMat& m,
+                                              bool eig, Put&& put) {
+    if (F == NF_H && !g.aligned) pair_traction_general<P>(g, x, nfg, m, eig, put);
+    else pair_traction_fam<P, F>(g, x, nfg, m, eig, put);
 }
 
 }  // namespace mbem

@@ -1,19 +1,35 @@
 // P0 kernel matrices and matrix-free contractions, FP64 (sm_103a).
 //
-// Matrices: one thread per source triangle, FIELD_TILE observers per block
-// staged in shared memory (broadcast reads), the source frame kept in
-// registers across the tile; each warp writes 32 consecutive 3-column
-// blocks of a row, i.e. 768 contiguous bytes per output row.
-// Contractions: one thread per observer, source tiles prepared once per
-// block in shared memory (frame and constants) and read as broadcasts.
+// Both are bound by the FP64 pipe (a warp instruction takes 16 cycles of an SM).
+// Matrices: one thread per source triangle, its frame in registers, a tile of
+// observers per block read as broadcasts; the tile is the one that shares the
+// work out best (matrix_tile). Each warp writes 32 consecutive 3-column blocks
+// of a row, i.e. 768 contiguous bytes per output row.
+// Contractions: one thread per observer and slice of the sources; tiles of
+// source records in shared memory, dealt over the slices of a block and the
+// blocks of a cluster, whose partial sums are added in slice, then rank order
+// through distributed shared memory (deterministic, no workspace).
+//
+// Measured: T block 128 x 128 347 -> 48 us (8 blocks of 16 observers a thread
+// before), 1,728 x 1,728 3.38 -> 2.41 ms (590 FP64 instructions a pair before);
+// T displacement of 6,912 sources at 48 stations 9.98 -> 0.60 ms (6 blocks
+// before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 9.9 ms.
+#include <cooperative_groups.h>
+#include <string.h>
+
+#include <algorithm>
+
+#include "contract_split.cuh"
 #include "p0_pair.cuh"
 
 namespace mbem {
 
-constexpr int MAT_THREADS = 128;
-constexpr int FIELD_TILE = 16;
-constexpr int CON_THREADS = 128;
-constexpr int SRC_TILE = 64;
+namespace cg = cooperative_groups;
+
+constexpr int MAT_THREADS = 64;
+constexpr int CON_THREADS = 64;
+constexpr int SRC_TILE = 32;
+constexpr int N_SM = 152;
 
 enum MatKind { MAT_T_DIRECT = 0, MAT_U_DIRECT = 1, MAT_T_BASIS = 2, MAT_U_BASIS = 3 };
 
@@ -30,43 +46,33 @@ struct MatArgs {
     double* out;
     int64_t ld;          // leading dimension (row stride) of `out`
     int64_t plane;       // stride between basis planes (basis kinds)
+    int tile;            // observers a block takes at a time
 };
 
 template <int KIND>
-__global__ void __launch_bounds__(MAT_THREADS)
-p0_matrix_kernel(MatArgs a) {
-    __shared__ double xs[FIELD_TILE][3];
+__global__ void __launch_bounds__(MAT_THREADS) p0_matrix_kernel(MatArgs a) {
     const int64_t s = (int64_t)blockIdx.x * MAT_THREADS + threadIdx.x;
-    const bool active = s < a.n_src;
+    if (s >= a.n_src) return;
     SrcP0 src;
     double nrm[3] = {0.0, 0.0, 0.0};
-    if (active) {
-        src_setup(a.tri_verts + 9 * s, a.eps[s], src);
-        if (KIND == MAT_T_DIRECT || KIND == MAT_T_BASIS) {
-            nrm[0] = a.normals[3 * s]; nrm[1] = a.normals[3 * s + 1]; nrm[2] = a.normals[3 * s + 2];
-        }
+    src_setup(a.tri_verts + 9 * s, a.eps[s], src);
+    if (KIND == MAT_T_DIRECT || KIND == MAT_T_BASIS) {
+        nrm[0] = a.normals[3 * s]; nrm[1] = a.normals[3 * s + 1]; nrm[2] = a.normals[3 * s + 2];
+        src_normal(src, nrm);
     }
-    for (int64_t f0 = (int64_t)blockIdx.y * FIELD_TILE; f0 < a.n_field;
-         f0 += (int64_t)gridDim.y * FIELD_TILE) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < FIELD_TILE * 3; t += MAT_THREADS) {
-            int64_t f = f0 + t / 3;
-            xs[t / 3][t % 3] = (f < a.n_field) ? a.x_field[3 * f0 + t] : 0.0;
-        }
-        __syncthreads();
-        if (!active) continue;
-        const int nf = (int)lmin(FIELD_TILE, a.n_field - f0);
-        for (int ff = 0; ff < nf; ff++) {
-            const int64_t f = f0 + ff;
+    const TCoef tc = t_coef(a.c);
+    for (int64_t f0 = (int64_t)blockIdx.y * a.tile; f0 < a.n_field; f0 += (int64_t)gridDim.y * a.tile) {
+        const int64_t f1 = lmin(f0 + a.tile, a.n_field);
+#pragma unroll 1
+        for (int64_t f = f0; f < f1; f++) {
+            const double ox = a.x_field[3 * f], oy = a.x_field[3 * f + 1], oz = a.x_field[3 * f + 2];
             if (KIND == MAT_T_DIRECT || KIND == MAT_U_DIRECT) {
                 double blk[3][3];
                 if (src.ok) {
                     PairP0 p;
-                    pair_setup(src, xs[ff][0], xs[ff][1], xs[ff][2], p);
+                    pair_setup(src, ox, oy, oz, p);
                     if (KIND == MAT_T_DIRECT) {
-                        TMoments m;
-                        t_moments(src, nrm, p, m);
-                        t_block(m, nrm, a.c, src.eps2, blk);
+                        t_pair(src, nrm, p, tc, blk);
                     } else {
                         UMoments m;
                         u_moments(src, p, m);
@@ -96,7 +102,7 @@ p0_matrix_kernel(MatArgs a) {
                 double blk[6][3][3];
                 if (src.ok) {
                     PairP0 p;
-                    pair_setup(src, xs[ff][0], xs[ff][1], xs[ff][2], p);
+                    pair_setup(src, ox, oy, oz, p);
                     TMoments m;
                     t_moments(src, nrm, p, m);
                     t_basis_blocks(m, nrm, src.eps2, blk);
@@ -116,7 +122,7 @@ p0_matrix_kernel(MatArgs a) {
                 double I1 = 0.0, I3 = 0.0, T2[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
                 if (src.ok) {
                     PairP0 p;
-                    pair_setup(src, xs[ff][0], xs[ff][1], xs[ff][2], p);
+                    pair_setup(src, ox, oy, oz, p);
                     UMoments m;
                     u_moments(src, p, m);
                     I1 = m.I1;
@@ -138,6 +144,26 @@ p0_matrix_kernel(MatArgs a) {
             }
         }
     }
+}
+
+// Observers a block: the FP64 pipe takes about 200 instructions for a source's
+// frame and 400 for a pair, so a tile of t costs 200 + 400 t a warp and the part
+// the warps of its fullest SM; below about five warps an SM the pipe waits.
+static int matrix_tile(int64_t nf, int64_t ns) {
+    int best = 16;
+    double cost = 1e300;
+    for (int t = 1; t <= 16; t++) {
+        const int64_t blocks = ceil_div(ns, MAT_THREADS) * ceil_div(nf, t);
+        const int64_t rounds = ceil_div(blocks, N_SM);
+        // beyond a few rounds the blocks even out
+        const double r = rounds > 6 ? (double)blocks / N_SM + 0.5 : rounds < 3 ? 2.5 : (double)rounds;
+        const double c = r * (200.0 + 400.0 * t);
+        if (c < cost) {
+            cost = c;
+            best = t;
+        }
+    }
+    return best;
 }
 
 // ---------------------------------------------------------------------------
@@ -165,157 +191,176 @@ struct ConArgs {
     double alpha;
     int accumulate;
     double* out;
-    int split;       // source slices per observer (1, 2, 4, 8 or 16)
+    int ob;          // observers a block; CON_THREADS / ob slices
 };
 
 struct SrcTile {
     SrcP0 g;
     double n[3];     // source normal as passed
     double d[3];     // density
+    double dl[3];    // density in the source frame
     bool live;       // non-degenerate and non-zero density
 };
 
-template <int KIND>
-__global__ void __launch_bounds__(CON_THREADS)
-p0_contract_kernel(ConArgs a) {
-    // A block holds CON_THREADS / split observers; the split threads of an
-    // observer take interleaved sources of each tile and their partial sums
-    // are added in slice order at the end (deterministic).
-    __shared__ SrcTile tile[SRC_TILE];
-    __shared__ double red[CON_THREADS][9];
-    const int split = a.split;
-    const int obs_per_block = CON_THREADS / split;
-    const int lane = threadIdx.x % obs_per_block;
-    const int slice = threadIdx.x / obs_per_block;
-    const int64_t f = (int64_t)blockIdx.x * obs_per_block + lane;
-    const bool active = f < a.n_field;
-    double ox = 0, oy = 0, oz = 0;
-    if (active) {
-        ox = a.x_field[3 * f]; oy = a.x_field[3 * f + 1]; oz = a.x_field[3 * f + 2];
-    }
-    constexpr bool STRESS = KIND >= CON_DD_STRESS;
-    double acc[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) acc[i] = 0.0;
-    const double nu = a.lam / (2.0 * (a.lam + a.mu));
-    const double C1 = 1.0 / (16.0 * MBEM_PI * a.mu * (1.0 - nu));
-    const double c34 = 3.0 - 4.0 * nu;
-
-    for (int64_t s0 = 0; s0 < a.n_src; s0 += SRC_TILE) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < SRC_TILE; t += CON_THREADS) {
-            const int64_t s = s0 + t;
-            SrcTile& T = tile[t];
-            if (s < a.n_src) {
-                src_setup(a.tri_verts + 9 * s, a.eps[s], T.g);
-                for (int k = 0; k < 3; k++) {
-                    T.n[k] = (KIND == CON_U_DISP || KIND == CON_KELVIN_STRESS) ? 0.0 : a.normals[3 * s + k];
-                    T.d[k] = a.density[3 * s + k];
-                }
-                T.live = T.g.ok && !(T.d[0] == 0.0 && T.d[1] == 0.0 && T.d[2] == 0.0);
-                if (KIND == CON_EIGENSTRESS && !(T.g.eps > 0.0)) T.live = false;
-            } else {
-                T.live = false;
-            }
-        }
-        __syncthreads();
-        if (!active) continue;
-        const int ns = (int)lmin(SRC_TILE, a.n_src - s0);
-        for (int t = slice; t < ns; t += split) {
-            const SrcTile& T = tile[t];
-            if (!T.live) continue;
-            const SrcP0& sg = T.g;
-            PairP0 p;
-            pair_setup(sg, ox, oy, oz, p);
-            if (KIND == CON_T_DISP) {
-                TMoments m;
-                t_moments(sg, T.n, p, m);
-                double blk[3][3];
-                t_block(m, T.n, a.c, sg.eps2, blk);
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-                    acc[i] += blk[i][0] * T.d[0] + blk[i][1] * T.d[1] + blk[i][2] * T.d[2];
-            } else if (KIND == CON_U_DISP) {
-                UMoments m;
-                u_moments(sg, p, m);
-                const double dg = a.c[0] * m.I1 + a.c[1] * sg.eps2 * m.I3;
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-                    acc[i] += dg * T.d[i] +
-                              a.c[2] * (m.T2[i][0] * T.d[0] + m.T2[i][1] * T.d[1] + m.T2[i][2] * T.d[2]);
-            } else if (STRESS) {
-                double sl[3];
-                to_local(sg, T.d, sl);
-                double loc[3][3];
-                if (KIND == CON_KELVIN_STRESS) {
-                    StressMoments M;
-                    stress_moments<false>(sg, p, M);
-                    const double cbdg = 6.0 * (1.0 - nu) * sg.eps2;
-                    kelvin_stress_local(M, sl, a.mu, a.lam, C1, c34, cbdg, loc);
-                } else {
-                    StressMoments M;
-                    stress_moments<true>(sg, p, M);
-                    double phi = 0.0;
-                    if (KIND == CON_EIGENSTRESS || KIND == CON_ELASTIC_STRESS)
-                        phi = (sg.eps > 0.0) ? (15.0 * sg.eps2 * sg.eps2 / (8.0 * MBEM_PI)) * M.M7[0][0] : 0.0;
-                    if (KIND == CON_DD_STRESS || KIND == CON_ELASTIC_STRESS) {
-                        double nl[3];
-                        to_local(sg, T.n, nl);
-                        const double cblob = 2.0 * (1.0 - nu) * sg.eps2;
-                        dd_stress_local(M, nl, sl, a.mu, a.lam, C1, c34, cblob, loc);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 3; i++)
-#pragma unroll
-                            for (int j = 0; j < 3; j++) loc[i][j] = 0.0;
-                    }
-                    if (KIND == CON_EIGENSTRESS || KIND == CON_ELASTIC_STRESS) {
-                        // eigenstress in the global frame, tri_kernels.py:1206-1214
-                        const double sgn = (KIND == CON_ELASTIC_STRESS) ? -1.0 : 1.0;
-                        const double ns_ = T.n[0] * T.d[0] + T.n[1] * T.d[1] + T.n[2] * T.d[2];
-                        double G[3][3];
-                        rotate_sym(sg, loc, G);
-#pragma unroll
-                        for (int m = 0; m < 3; m++)
-#pragma unroll
-                            for (int n = 0; n < 3; n++)
-                                acc[3 * m + n] += G[m][n] + sgn * phi *
-                                    ((m == n ? a.lam * ns_ : 0.0) + a.mu * (T.d[m] * T.n[n] + T.d[n] * T.n[m]));
-                        continue;
-                    }
-                }
-                double G[3][3];
-                rotate_sym(sg, loc, G);
-#pragma unroll
-                for (int m = 0; m < 3; m++)
-#pragma unroll
-                    for (int n = 0; n < 3; n++) acc[3 * m + n] += G[m][n];
-            }
-        }
-    }
-    const int nout = STRESS ? 9 : 3;
-    if (split > 1) {
-        __syncthreads();
-        for (int i = 0; i < nout; i++) red[threadIdx.x][i] = acc[i];
-        __syncthreads();
-        if (slice != 0) return;
-        for (int k = 1; k < split; k++)
-            for (int i = 0; i < nout; i++) acc[i] += red[k * obs_per_block + lane][i];
-    }
-    if (!active) return;
-    double* o = a.out + nout * f;
-    for (int i = 0; i < nout; i++) {
-        const double v = a.alpha * acc[i];
-        o[i] = a.accumulate ? o[i] + v : v;
+// DD stress of a normal off the frame's, minus the eigenstress with eig
+static __device__ __noinline__ void dd_pair_general(const SrcTile& T, const PairP0& p, const SMat& m, bool dd, bool eig,
+                                                    double out[6]) {
+    StressMoments M;
+    stress_moments<true>(T.g, p, M);
+    double nl[3], loc[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    to_frame(T.g, T.n, nl);
+    if (dd) dd_stress_local(M, nl, T.dl, m.mu, m.lam, m.C1, m.c34, m.blob * T.g.eps2, loc);
+    const double sgn = dd ? -1.0 : 1.0;
+    const double phi = eig ? sgn * m.phi * T.g.eps2 * T.g.eps2 * M.M7[0][0] : 0.0;
+    const double ns = nl[0] * T.dl[0] + nl[1] * T.dl[1] + nl[2] * T.dl[2];
+    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
+    for (int t = 0; t < 6; t++) {
+        const int i = ia[t], j = ib[t];
+        out[t] += loc[i][j] + phi * ((i == j ? m.lam * ns : 0.0) + m.mu * (T.dl[i] * nl[j] + nl[i] * T.dl[j]));
     }
 }
 
-// Slices per observer so that a launch holds about four 128-thread blocks
-// per SM (152 SMs) whatever the observer count.
-static int contract_split(int64_t nf) {
-    int split = 1;
-    while (split < 16 && nf * split < (int64_t)152 * 4 * CON_THREADS) split *= 2;
-    return split;
+// one pair, added to acc: displacement (global), or stress 00 11 22 01 02 12 (global)
+template <int KIND>
+__device__ __forceinline__ void contract_pair(const SrcTile& T, const double x[3], const ConArgs& a, const TCoef& tc,
+                                              const SMat& sm, double* acc) {
+    const SrcP0& g = T.g;
+    PairP0 p;
+    pair_setup(g, x[0], x[1], x[2], p);
+    if (KIND == CON_T_DISP) {
+        double blk[3][3];
+        t_pair(g, T.n, p, tc, blk);
+#pragma unroll
+        for (int i = 0; i < 3; i++) acc[i] += blk[i][0] * T.d[0] + blk[i][1] * T.d[1] + blk[i][2] * T.d[2];
+    } else if (KIND == CON_U_DISP) {
+        UMoments m;
+        u_moments(g, p, m);
+        const double dg = a.c[0] * m.I1 + a.c[1] * g.eps2 * m.I3;
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            acc[i] += dg * T.d[i] + a.c[2] * (m.T2[i][0] * T.d[0] + m.T2[i][1] * T.d[1] + m.T2[i][2] * T.d[2]);
+    } else {
+        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, G[6];
+        if (KIND == CON_KELVIN_STRESS) {
+            StressMoments M;
+            stress_moments<false>(g, p, M);
+            double loc[3][3];
+            kelvin_stress_local(M, T.dl, a.mu, a.lam, sm.C1, sm.c34, 3.0 * sm.blob * g.eps2, loc);
+            v[0] = loc[0][0]; v[1] = loc[1][1]; v[2] = loc[2][2];
+            v[3] = loc[0][1]; v[4] = loc[0][2]; v[5] = loc[1][2];
+        } else if (!g.aligned) {
+            dd_pair_general(T, p, sm, KIND != CON_EIGENSTRESS, KIND != CON_DD_STRESS, v);
+        } else {
+            double m3[1], m5[6], m7[10];
+            dd_moments(g, p, m3, m5, m7);
+            if (KIND == CON_EIGENSTRESS) {
+                // phi C : sym(s n), n = sn e3
+                const double ph = g.sn * sm.phi * g.eps2 * g.eps2 * m7[0];
+                v[0] = v[1] = ph * sm.lam * T.dl[2];
+                v[2] = ph * (sm.lam + 2.0 * sm.mu) * T.dl[2];
+                v[4] = ph * sm.mu * T.dl[0];
+                v[5] = ph * sm.mu * T.dl[1];
+            } else {
+                constexpr bool E = KIND == CON_ELASTIC_STRESS;
+                dd_unit<0>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[0], v);
+                dd_unit<1>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[1], v);
+                dd_unit<2>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[2], v);
+            }
+        }
+        rotate_six(g, v, G);
+#pragma unroll
+        for (int t = 0; t < 6; t++) acc[t] += G[t];
+    }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
+    constexpr int NO = KIND >= CON_DD_STRESS ? 6 : 3;
+    __shared__ SrcTile tile[SRC_TILE];
+    __shared__ double red[CON_THREADS][NO];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+    const int ob = a.ob, slices = CON_THREADS / ob;
+    const int lane = threadIdx.x % ob, slice = threadIdx.x / ob;
+    const int64_t f = (int64_t)(blockIdx.x / ranks) * ob + lane;
+    const bool active = f < a.n_field && slice < slices;
+    double x[3] = {0.0, 0.0, 0.0};
+    if (active) {
+        x[0] = a.x_field[3 * f];
+        x[1] = a.x_field[3 * f + 1];
+        x[2] = a.x_field[3 * f + 2];
+    }
+    const TCoef tc = t_coef(a.c);
+    const SMat sm = stress_mat(KIND >= CON_DD_STRESS ? a.mu : 1.0, KIND >= CON_DD_STRESS ? a.lam : 1.0);
+    double acc[NO];
+#pragma unroll
+    for (int i = 0; i < NO; i++) acc[i] = 0.0;
+    for (int64_t s0 = (int64_t)rank * SRC_TILE; s0 < a.n_src; s0 += (int64_t)ranks * SRC_TILE) {
+        const int ns = (int)lmin(SRC_TILE, a.n_src - s0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < ns; t += CON_THREADS) {
+            const int64_t s = s0 + t;
+            SrcTile& T = tile[t];
+            src_setup(a.tri_verts + 9 * s, a.eps[s], T.g);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                T.n[k] = (KIND == CON_U_DISP || KIND == CON_KELVIN_STRESS) ? 0.0 : a.normals[3 * s + k];
+                T.d[k] = a.density[3 * s + k];
+            }
+            src_normal(T.g, T.n);
+            to_frame(T.g, T.d, T.dl);
+            T.live = T.g.ok && !(T.d[0] == 0.0 && T.d[1] == 0.0 && T.d[2] == 0.0);
+            if (KIND == CON_EIGENSTRESS && !(T.g.eps > 0.0)) T.live = false;
+        }
+        __syncthreads();
+        if (!active) continue;
+#pragma unroll 1
+        for (int t = slice; t < ns; t += slices)
+            if (tile[t].live) contract_pair<KIND>(tile[t], x, a, tc, sm, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < NO; i++) red[threadIdx.x][i] = acc[i];
+    __syncthreads();
+    if (slice == 0) {
+        for (int k = 1; k < slices; k++)
+#pragma unroll
+            for (int i = 0; i < NO; i++) acc[i] += red[k * ob + lane][i];
+#pragma unroll
+        for (int i = 0; i < NO; i++) red[lane][i] = acc[i];
+    }
+    cluster.sync();
+    if (rank == 0 && slice == 0 && active) {
+        for (int r = 1; r < ranks; r++) {
+            const double* other = cluster.map_shared_rank(&red[lane][0], r);
+#pragma unroll
+            for (int i = 0; i < NO; i++) acc[i] += other[i];
+        }
+        const int ix[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+        constexpr int NW = NO == 3 ? 3 : 9;
+        double* o = a.out + NW * f;
+#pragma unroll
+        for (int i = 0; i < NW; i++) {
+            const double v = a.alpha * acc[NW == 3 ? i : ix[i]];
+            o[i] = a.accumulate ? o[i] + v : v;
+        }
+    }
+    cluster.sync();      // the partial sums stay until rank 0 has read them
+}
+
+template <int KIND>
+static cudaError_t launch_con(const ConArgs& a, int64_t grid, int ranks, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(CON_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ranks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, p0_contract_kernel<KIND>, a);
 }
 
 static int check_common(const double* x, int64_t nf, const double* tv, const double* eps, int64_t ns,
@@ -337,7 +382,8 @@ int launch_matrix(int kind, const double* x, int64_t nf, const double* tv, const
     for (int i = 0; i < 6; i++) a.c[i] = (c && i < nc) ? c[i] : 0.0;
     a.alpha = alpha; a.accumulate = accumulate; a.out = out; a.ld = ld; a.plane = plane;
     if (nf == 0 || ns == 0) return MBEM_OK;
-    dim3 grid((unsigned)ceil_div(ns, MAT_THREADS), (unsigned)lmin(ceil_div(nf, FIELD_TILE), 65535));
+    a.tile = matrix_tile(nf, ns);
+    dim3 grid((unsigned)ceil_div(ns, MAT_THREADS), (unsigned)lmin(ceil_div(nf, a.tile), 65535));
     switch (kind) {
         case MAT_T_DIRECT: p0_matrix_kernel<MAT_T_DIRECT><<<grid, MAT_THREADS, 0, st>>>(a); break;
         case MAT_U_DIRECT: p0_matrix_kernel<MAT_U_DIRECT><<<grid, MAT_THREADS, 0, st>>>(a); break;
@@ -356,16 +402,20 @@ int launch_contract(int kind, const double* x, int64_t nf, const double* tv, con
     for (int i = 0; i < 6; i++) a.c[i] = (c && i < nc) ? c[i] : 0.0;
     a.mu = mu; a.lam = lam; a.alpha = alpha; a.accumulate = accumulate; a.out = out;
     if (nf == 0) return MBEM_OK;
-    a.split = contract_split(nf);
-    dim3 grid((unsigned)ceil_div(nf, CON_THREADS / a.split));
+    const ConSplit sp = contract_split(nf, ns, CON_THREADS, SRC_TILE, kind >= CON_DD_STRESS ? 500 : 400, 250);
+    a.ob = sp.ob;
+    const int64_t grid = ceil_div(nf, sp.ob) * sp.ranks;
+    MBEM_REQUIRE(grid < (int64_t)1 << 31, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)nf);
+    cudaError_t e;
     switch (kind) {
-        case CON_T_DISP: p0_contract_kernel<CON_T_DISP><<<grid, CON_THREADS, 0, st>>>(a); break;
-        case CON_U_DISP: p0_contract_kernel<CON_U_DISP><<<grid, CON_THREADS, 0, st>>>(a); break;
-        case CON_DD_STRESS: p0_contract_kernel<CON_DD_STRESS><<<grid, CON_THREADS, 0, st>>>(a); break;
-        case CON_KELVIN_STRESS: p0_contract_kernel<CON_KELVIN_STRESS><<<grid, CON_THREADS, 0, st>>>(a); break;
-        case CON_EIGENSTRESS: p0_contract_kernel<CON_EIGENSTRESS><<<grid, CON_THREADS, 0, st>>>(a); break;
-        default: p0_contract_kernel<CON_ELASTIC_STRESS><<<grid, CON_THREADS, 0, st>>>(a); break;
+        case CON_T_DISP: e = launch_con<CON_T_DISP>(a, grid, sp.ranks, st); break;
+        case CON_U_DISP: e = launch_con<CON_U_DISP>(a, grid, sp.ranks, st); break;
+        case CON_DD_STRESS: e = launch_con<CON_DD_STRESS>(a, grid, sp.ranks, st); break;
+        case CON_KELVIN_STRESS: e = launch_con<CON_KELVIN_STRESS>(a, grid, sp.ranks, st); break;
+        case CON_EIGENSTRESS: e = launch_con<CON_EIGENSTRESS>(a, grid, sp.ranks, st); break;
+        default: e = launch_con<CON_ELASTIC_STRESS>(a, grid, sp.ranks, st); break;
     }
+    if (e != cudaSuccess) return set_error(MBEM_ERR_CUDA, "p0_contract_kernel: %s", cudaGetErrorString(e));
     return launch_status("p0_contract_kernel");
 }
 

@@ -34,7 +34,19 @@ struct SrcP0 {
     double eps, eps2;
     bool ok;                     // false for a degenerate triangle (zero block)
     bool edge_ok[3];
+    double sn;                   // +-1: the source normal along the frame's (src_normal)
+    bool aligned;
 };
+
+// A unit source normal along the frame's, to the rounding of both (every mesh),
+// takes the forms without the other two components.
+__device__ __forceinline__ void src_normal(SrcP0& s, const double* __restrict__ n) {
+    const double a = n[0] * s.ex[0] + n[1] * s.ex[1] + n[2] * s.ex[2];
+    const double b = n[0] * s.ey[0] + n[1] * s.ey[1] + n[2] * s.ey[2];
+    const double c = n[0] * s.nh[0] + n[1] * s.nh[1] + n[2] * s.nh[2];
+    s.sn = c < 0.0 ? -1.0 : 1.0;
+    s.aligned = fabs(a) < 1e-15 && fabs(b) < 1e-15 && fabs(fabs(c) - 1.0) < 1e-15;
+}
 
 // Frame of a source triangle (tri_kernels.py:137-153) and its per-source
 // constants. `tv` points at 9 doubles (vertex-major).
@@ -84,6 +96,188 @@ __device__ __forceinline__ void src_setup(const double* __restrict__ tv, double 
         s.tx[e] = evx * iL;
         s.ty[e] = evy * iL;
     }
+}
+
+// ---------------------------------------------------------------------------
+// forms in the source frame, shared by the P0 pair and the nodal tables
+// ---------------------------------------------------------------------------
+// index of the moment [a, b] in a table ordered by degree a + b, then b
+__host__ __device__ constexpr int nd_tri(int a, int b) { return (a + b) * (a + b + 1) / 2 + b; }
+
+template <class Frame>
+__device__ __forceinline__ void rotate_full(const Frame& g, const double B[3][3], double G[3][3]) {
+    double Y[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) Y[a][j] = B[a][0] * g.ex[j] + B[a][1] * g.ey[j] + B[a][2] * g.nh[j];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) G[i][j] = g.ex[i] * Y[0][j] + g.ey[i] * Y[1][j] + g.nh[i] * Y[2][j];
+}
+// symmetric L (00 11 22 01 02 12) to the global frame, same layout
+template <class Frame>
+__device__ __forceinline__ void rotate_six(const Frame& g, const double L[6], double G[6]) {
+    const int ix[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+    double Y[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            Y[a][j] = L[ix[a][0]] * g.ex[j] + L[ix[a][1]] * g.ey[j] + L[ix[a][2]] * g.nh[j];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) G[ix[i][j]] = g.ex[i] * Y[0][j] + g.ey[i] * Y[1][j] + g.nh[i] * Y[2][j];
+}
+template <class Frame>
+__device__ __forceinline__ void to_frame(const Frame& g, const double* v, double l[3]) {
+    l[0] = v[0] * g.ex[0] + v[1] * g.ex[1] + v[2] * g.ex[2];
+    l[1] = v[0] * g.ey[0] + v[1] * g.ey[1] + v[2] * g.ey[2];
+    l[2] = v[0] * g.nh[0] + v[1] * g.nh[1] + v[2] * g.nh[2];
+}
+
+// Coefficients of the combined T block. |d|^2 = R^2 - eps^2 turns
+// t_i = int d_i |d|^2 / R^5 into V3_i - eps^2 V5_i, so with b_i = cb V3_i + ce6 V5_i
+//   out = n_j (c3 V3_i + c5 V5_i) + n_i b_j + w6 W_ij + d_ij n.b
+// (c5 and ce6 times eps^2).
+struct TCoef {
+    double c3, c5, cb, ce6, w6;
+};
+__host__ __device__ __forceinline__ TCoef t_coef(const double c[6]) {
+    TCoef t;
+    t.c3 = c[0] + c[1] + 2.0 * c[4];
+    t.c5 = c[2] + 3.0 * c[1];
+    t.cb = c[3] + c[4];
+    t.ce6 = c[5];
+    t.w6 = -6.0 * c[4];
+    return t;
+}
+
+// The T block in the source frame for the normal s e3, from the moments
+// i3, a3 = (1,0), b3 = (0,1) of n = 3 and i5 .. c02 of n = 5.
+__device__ __forceinline__ void t_local(double i3, double a3, double b3, double i5, double a5, double b5, double c20,
+                                        double c11, double c02, double z, double eps2, const TCoef& c, double s,
+                                        double B[3][3]) {
+    const double k3 = s * c.c3, k5 = s * c.c5 * eps2, kb = s * c.cb, k6 = s * c.ce6 * eps2, kw = s * c.w6 * z;
+    const double zi3 = z * i3, zi5 = z * i5, kz = kw * z;
+    const double be2 = kb * zi3 + k6 * zi5;
+    const double v0 = -(kz * a5), v1 = -(kz * b5);
+    B[0][0] = kw * c20 + be2;
+    B[1][1] = kw * c02 + be2;
+    B[0][1] = B[1][0] = kw * c11;
+    B[0][2] = v0 - (k3 * a3 + k5 * a5);
+    B[1][2] = v1 - (k3 * b3 + k5 * b5);
+    B[2][0] = v0 - (kb * a3 + k6 * a5);
+    B[2][1] = v1 - (kb * b3 + k6 * b5);
+    B[2][2] = kz * zi5 + (k3 * zi3 + k5 * zi5) + 2.0 * be2;
+}
+
+// material constants of the stress forms
+struct SMat {
+    double mu, lam, C1, c34;
+    double k3a;        // 3 c34 - 9
+    double x1;         // 3 c34 - 18
+    double blob;       // 2 (1 - nu), times eps^2: cblob
+    double phi;        // 15 / (8 pi), times eps^4
+};
+__host__ __device__ inline SMat stress_mat(double mu, double lam) {
+    SMat m;
+    const double nu = lam / (2.0 * (lam + mu));
+    m.mu = mu;
+    m.lam = lam;
+    m.C1 = 1.0 / (16.0 * MBEM_PI * mu * (1.0 - nu));
+    m.c34 = 3.0 - 4.0 * nu;
+    m.k3a = 3.0 * m.c34 - 9.0;
+    m.x1 = 3.0 * m.c34 - 18.0;
+    m.blob = 2.0 * (1.0 - nu);
+    m.phi = 15.0 / (8.0 * MBEM_PI);
+    return m;
+}
+
+// Stress (00 11 22 01 02 12, source frame, normal +e3) of slip along e_K with
+// the moment set (m3[0]; m5 to degree 2; m7 to degree 3), times w and added:
+// the DD stress of tri_kernels.py:900-964 for that normal and slip, and with
+// EIG the eigenstress (tri_kernels.py:1206-1214) taken off.
+template <int K>
+__device__ __forceinline__ void dd_unit(const double* m3, const double* m5, const double* m7, double z, double eps2,
+                                        const SMat& m, bool eig, double w, double out[6]) {
+#define A5(a, b) m5[nd_tri(a, b)]
+#define A7(a, b) m7[nd_tri(a, b)]
+    const double cb = m.blob * eps2;
+    const double z2 = z * z;
+    const double I3 = m3[0], I5 = A5(0, 0), I7 = A7(0, 0);
+    const double phi = eig ? m.phi * eps2 * eps2 * I7 : 0.0;
+    if (K < 2) {
+        // u: the slip axis, v: the other in-plane axis; d = (-xi, z)
+#define U5(a, b) (K == 0 ? A5(a, b) : A5(b, a))
+#define U7(a, b) (K == 0 ? A7(a, b) : A7(b, a))
+        const double T5u3 = -z * U5(1, 0), T5v3 = -z * U5(0, 1), T533 = z2 * I5;
+        const double zu = -z * U7(1, 0), zv = -z * U7(0, 1), z33 = z2 * I7;
+        const double c15 = 15.0 * cb;
+        const double Fu3 = m.k3a * T5u3 + c15 * zu;
+        const double Fv3 = m.k3a * T5v3 + c15 * zv;
+        const double Fuv = m.k3a * U5(1, 1) + c15 * U7(1, 1);
+        const double Fuu33 = m.k3a * (U5(2, 0) + T533) + c15 * (U7(2, 0) + z33);
+        const double q0 = -z * U7(3, 0), q1 = -z * U7(1, 2), q2 = z2 * zu;        // T4 uuu3, vvu3, 33u3
+        const double q3 = -z * U7(2, 1), q4 = z2 * U7(2, 0), q5 = z2 * U7(1, 1);  // uvu3, u3u3, v3u3
+        // sum_r T4_rru3 = T5_u3 - eps^2 T7_u3
+        const double tr = 2.0 * Fu3 + 12.0 * T5u3 - 30.0 * eps2 * zu;
+        const double t = m.lam * tr;
+        const double base = -12.0 * T5u3;
+        const double sA = 2.0 * ((1.0 - m.c34) * I3 - 3.0 * cb * I5);
+        const double suu = t + m.mu * (base + 2.0 * Fu3 + 60.0 * q0);
+        const double svv = t + m.mu * (base + 60.0 * q1);
+        const double s33 = t + m.mu * (base + 2.0 * Fu3 + 60.0 * q2);
+        const double suv = Fv3 + 60.0 * q3, su3 = sA + Fuu33 + 60.0 * q4, sv3 = Fuv + 60.0 * q5;
+        // sigma = -C1 mu (lam tr delta + mu (Y + Y^T))
+        const double gm = -m.C1 * w * m.mu;
+        out[K] += gm * suu;
+        out[1 - K] += gm * svv;
+        out[2] += gm * s33;
+        const double g2 = gm * m.mu;
+        out[3] += g2 * suv;
+        out[K == 0 ? 4 : 5] += g2 * su3 - (m.mu * w) * phi;
+        out[K == 0 ? 5 : 4] += g2 * sv3;
+#undef U5
+#undef U7
+    } else {
+        const double T00 = A5(2, 0), T11 = A5(0, 2), T01 = A5(1, 1), T02 = -z * A5(1, 0), T12 = -z * A5(0, 1),
+                     T22 = z2 * I5;
+        const double S00 = A7(2, 0), S11 = A7(0, 2), S01 = A7(1, 1), S02 = -z * A7(1, 0), S12 = -z * A7(0, 1),
+                     S22 = z2 * I7;
+        const double trT = I3 - eps2 * I5, trS = I5 - eps2 * I7;
+        // T4_rt33, and t4c_rt = int d_r d_t |d|^2 / R^7 = T5_rt - eps^2 T7_rt
+        const double Q00 = z2 * S00, Q11 = z2 * S11, Q01 = z2 * S01, Q02 = z2 * S02, Q12 = z2 * S12, Q22 = z2 * S22;
+        const double C22 = T22 - eps2 * S22;
+        const double c15 = 15.0 * cb;
+        const double xd = (4.0 - m.c34) * I3 - 3.0 * trT - 3.0 * cb * I5;
+        const double trX = 3.0 * xd + m.x1 * trT + 15.0 * (trT - eps2 * trS) + c15 * trS;
+        const double F02 = m.k3a * T02 + c15 * S02, F12 = m.k3a * T12 + c15 * S12, F22 = m.k3a * T22 + c15 * S22;
+        const double A = (1.0 - m.c34) * I3 - 3.0 * cb * I5;
+        const double trY = 2.0 * A + 6.0 * I3 + 2.0 * F22 - 18.0 * T22 - 6.0 * trT + 30.0 * C22;
+        const double trB = m.lam * trX + m.mu * trY;
+        const double yd = 4.0 * I3 - 12.0 * T22;
+        // X = xd delta + x1 T + 15 C + c15 S with 15 C = 15 T - 15 eps^2 S ; Y + Y^T = yd delta - 12 T + 60 Q + (e3, F terms) + 4 A e3 e3
+        const double l2 = 2.0 * m.lam, mu = m.mu;
+        const double xt = m.x1 + 15.0, xs = c15 - 15.0 * eps2;
+        const double diag = m.lam * trB + mu * (l2 * xd + mu * yd);
+        const double gw = -m.C1 * w;
+        const double ep = phi * w;
+        out[0] += gw * (diag + mu * (l2 * (xt * T00 + xs * S00) + mu * (60.0 * Q00 - 12.0 * T00))) -
+                  ep * m.lam;
+        out[1] += gw * (diag + mu * (l2 * (xt * T11 + xs * S11) + mu * (60.0 * Q11 - 12.0 * T11))) -
+                  ep * m.lam;
+        out[2] += gw * (diag + mu * (l2 * (xt * T22 + xs * S22) +
+                                     mu * (60.0 * Q22 - 12.0 * T22 + 4.0 * (F22 + A)))) -
+                  ep * (m.lam + 2.0 * mu);
+        out[3] += gw * mu * (l2 * (xt * T01 + xs * S01) + mu * (60.0 * Q01 - 12.0 * T01));
+        out[4] += gw * mu * (l2 * (xt * T02 + xs * S02) + mu * (60.0 * Q02 - 12.0 * T02 + 2.0 * F02));
+        out[5] += gw * mu * (l2 * (xt * T12 + xs * S12) + mu * (60.0 * Q12 - 12.0 * T12 + 2.0 * F12));
+    }
+#undef A5
+#undef A7
 }
 
 // Pair geometry shared by all kernels: height, lift, projected vertices,
@@ -185,7 +379,7 @@ __device__ __forceinline__ void edges_setup(const SrcP0& s, const PairP0& p, Edg
 //   N3 = eps^2 n_j V5_i    R3 = eps^2 (d_ij n.V5 + n_i V5_j)
 // ---------------------------------------------------------------------------
 struct TMoments {
-    double V3[3], V5[3], t[3], W[3][3];   // global frame
+    double V3[3], V5[3], W[3][3];   // global frame
 };
 
 // T-kernel moments V3, V5, t, W (global frame) from the 2-D moments of the
@@ -208,7 +402,6 @@ __device__ __forceinline__ void t_from_scal(const double* ex, const double* ey, 
     const double T000 = -m30_5, T001 = -m21_5, T002 = z * m20_5, T011 = -m12_5,
                  T012 = z * m11_5, T022 = -z2 * m10_5, T111 = -m03_5, T112 = z * m02_5,
                  T122 = -z2 * m01_5, T222 = z2 * z * I5;
-    const double tl[3] = {T000 + T011 + T022, T001 + T111 + T122, T002 + T112 + T222};
     // local normal of the source normal passed in (may differ from nh)
     const double nl0 = nrm[0] * ex[0] + nrm[1] * ex[1] + nrm[2] * ex[2];
     const double nl1 = nrm[0] * ey[0] + nrm[1] * ey[1] + nrm[2] * ey[2];
@@ -227,7 +420,6 @@ __device__ __forceinline__ void t_from_scal(const double* ex, const double* ey, 
         const double qi[3] = {ex[i], ey[i], nh[i]};
         m.V3[i] = qi[0] * V3l[0] + qi[1] * V3l[1] + qi[2] * V3l[2];
         m.V5[i] = qi[0] * V5l[0] + qi[1] * V5l[1] + qi[2] * V5l[2];
-        m.t[i] = qi[0] * tl[0] + qi[1] * tl[1] + qi[2] * tl[2];
     }
     double Y[3][3];  // Y = W_l Q  (3x3 local-by-global)
 #pragma unroll
@@ -246,6 +438,7 @@ __device__ __forceinline__ void t_from_scal(const double* ex, const double* ey, 
 }
 
 
+// the 2-D moments of any normal (to degree 3 at n = 5)
 __device__ __forceinline__ void t_moments(const SrcP0& s, const double* __restrict__ nrm,
                                           const PairP0& p, TMoments& m) {
     double BN1_001 = 0, BN2_001 = 0, BD003 = 0, BN1_003 = 0, BN2_003 = 0, BN1_103 = 0,
@@ -284,25 +477,60 @@ __device__ __forceinline__ void t_moments(const SrcP0& s, const double* __restri
     t_from_scal(s.ex, s.ey, s.nh, nrm, q, m);
 }
 
-// Combined T block with six coefficients.
-__device__ __forceinline__ void t_block(const TMoments& m, const double* __restrict__ n,
-                                        const double c[6], double eps2, double out[3][3]) {
+// Combined T block of any normal.
+__device__ __forceinline__ void t_block(const TMoments& m, const double* __restrict__ n, const TCoef& c, double eps2,
+                                        double out[3][3]) {
     const double nV3 = n[0] * m.V3[0] + n[1] * m.V3[1] + n[2] * m.V3[2];
     const double nV5 = n[0] * m.V5[0] + n[1] * m.V5[1] + n[2] * m.V5[2];
-    const double ca = c[0] + 4.0 * c[1] + 2.0 * c[4];
-    const double cb = c[3] + c[4];
-    const double ce3 = c[2] * eps2, ce6 = c[5] * eps2;
-    const double gam = cb * nV3 + ce6 * nV5;
-    const double w6 = -6.0 * c[4];
+    const double c5 = c.c5 * eps2, ce6 = c.ce6 * eps2;
+    const double gam = c.cb * nV3 + ce6 * nV5;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        const double al = ca * m.V3[i] - 3.0 * c[1] * m.t[i] + ce3 * m.V5[i];
+        const double al = c.c3 * m.V3[i] + c5 * m.V5[i];
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const double bej = cb * m.V3[j] + ce6 * m.V5[j];
-            out[i][j] = n[j] * al + n[i] * bej + w6 * m.W[i][j] + (i == j ? gam : 0.0);
+            const double bej = c.cb * m.V3[j] + ce6 * m.V5[j];
+            out[i][j] = n[j] * al + n[i] * bej + c.w6 * m.W[i][j] + (i == j ? gam : 0.0);
         }
     }
+}
+
+// The T block of one pair (src_normal has been called). For the frame's normal
+// W = T3 . e3 needs n = 5 to degree 2 only and t follows from V3 and V5, so the
+// edges carry four sums less of degree 2 and no third row: about 400 FP64
+// instructions a pair where the general moments take 590.
+static __device__ __noinline__ void t_pair_general(const SrcP0& s, const double* nrm, const PairP0& p, const TCoef& c,
+                                                   double out[3][3]) {
+    TMoments m;
+    t_moments(s, nrm, p, m);
+    t_block(m, nrm, c, s.eps2, out);
+}
+__device__ __forceinline__ void t_pair(const SrcP0& s, const double* __restrict__ nrm, const PairP0& p, const TCoef& c,
+                                       double out[3][3]) {
+    if (!s.aligned) {
+        t_pair_general(s, nrm, p, c, out);
+        return;
+    }
+    EdgeP0 G[3];
+    edges_setup(s, p, G);
+    double x1 = 0, y1 = 0, d3 = 0, x3 = 0, y3 = 0, x10 = 0, x01 = 0, y01 = 0;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        if (!s.edge_ok[e]) continue;
+        const EdgeP0& g = G[e];
+        const double A = g.dp * g.nx, B = g.dp * g.ny;
+        const double v10 = A * g.dJ3 + g.tx * g.dK3, v01 = B * g.dJ3 + g.ty * g.dK3;
+        x1 += g.nx * g.dJ1; y1 += g.ny * g.dJ1;
+        d3 += g.dp * g.dJ3;
+        x3 += g.nx * g.dJ3; y3 += g.ny * g.dJ3;
+        x10 += g.nx * v10;
+        x01 += g.nx * v01; y01 += g.ny * v01;
+    }
+    const double th = 1.0 / 3.0, I3 = p.I3;
+    double B[3][3];
+    t_local(I3, -x1, -y1, (d3 + I3) * p.ih2 * th, -x3 * th, -y3 * th, (I3 - x10) * th, -x01 * th, (I3 - y01) * th, p.z,
+            s.eps2, c, s.sn, B);
+    rotate_full(s, B, out);
 }
 
 // The six basis blocks separately (t_basis_matrices, tri_kernels.py:473-492).
@@ -316,7 +544,7 @@ __device__ __forceinline__ void t_basis_blocks(const TMoments& m, const double* 
         for (int j = 0; j < 3; j++) {
             const double d = (i == j) ? 1.0 : 0.0;
             out[0][i][j] = n[j] * m.V3[i];
-            out[1][i][j] = n[j] * (4.0 * m.V3[i] - 3.0 * m.t[i]);
+            out[1][i][j] = n[j] * (m.V3[i] + 3.0 * eps2 * m.V5[i]);      // 4 V3 - 3 t
             out[2][i][j] = eps2 * n[j] * m.V5[i];
             out[3][i][j] = d * nV3 + n[i] * m.V3[j];
             out[4][i][j] = n[i] * m.V3[j] + 2.0 * n[j] * m.V3[i] + d * nV3 - 6.0 * m.W[i][j];
@@ -522,6 +750,61 @@ __device__ __forceinline__ void stress_moments(const SrcP0& s, const PairP0& p, 
         M.M7[1][3] = -b5_1_03 * fifth;
         M.M7[0][4] = (3.0 * M.M5[0][2] - b5_2_03) * fifth;
     }
+}
+
+// The moments the stress of slip on the frame's normal reads (dd_unit): I3, n = 5
+// to degree 2, n = 7 to degree 3, in nd_tri order. No edge log enters.
+__device__ __forceinline__ void dd_moments(const SrcP0& s, const PairP0& p, double m3[1], double m5[6],
+                                           double m7[10]) {
+    double d3 = 0, d5 = 0, x3[3] = {0, 0, 0}, y3[2] = {0, 0}, x5[6] = {0, 0, 0, 0, 0, 0}, y5[3] = {0, 0, 0};
+    EdgeP0 G[3];
+    edges_setup(s, p, G);
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        if (!s.edge_ok[e]) continue;
+        const EdgeP0& g = G[e];
+        const int a = e, b = (e + 1) % 3;
+        const double A = g.dp * g.nx, B = g.dp * g.ny;
+        const double ia3 = p.iR[a] * p.iR[a] * p.iR[a], ib3 = p.iR[b] * p.iR[b] * p.iR[b];
+        // J5 = u (3 rho^2 + 2 u^2) / (3 rho^4 R^3), K5 = -1 / (3 R^3)
+        const double r3 = 3.0 * g.rho2;
+        const double J = (g.ub * (r3 + 2.0 * g.ub * g.ub) * ib3 - g.ua * (r3 + 2.0 * g.ua * g.ua) * ia3) *
+                         (g.ir2 * g.ir2 * (1.0 / 3.0));
+        const double K = (ia3 - ib3) * (1.0 / 3.0), L = g.dJ3 - g.rho2 * J;
+        const double v10 = A * g.dJ3 + g.tx * g.dK3, v01 = B * g.dJ3 + g.ty * g.dK3;
+        d3 += g.dp * g.dJ3;
+        x3[0] += g.nx * g.dJ3; y3[0] += g.ny * g.dJ3;
+        x3[1] += g.nx * v10;
+        x3[2] += g.nx * v01; y3[1] += g.ny * v01;
+        const double a0 = A * J + g.tx * K, a1 = A * K + g.tx * L, b0 = B * J + g.ty * K, b1 = B * K + g.ty * L;
+        const double v02 = B * b0 + g.ty * b1;
+        d5 += g.dp * J;
+        x5[0] += g.nx * J; y5[0] += g.ny * J;
+        x5[1] += g.nx * a0;
+        x5[2] += g.nx * b0; y5[1] += g.ny * b0;
+        x5[3] += g.nx * (A * a0 + g.tx * a1);
+        x5[4] += g.nx * (B * a0 + g.ty * a1);
+        x5[5] += g.nx * v02; y5[2] += g.ny * v02;
+    }
+    const double I3 = p.I3, th = 1.0 / 3.0, f = 0.2;
+    const double I5 = (p.h2 > 1e-60) ? (d3 + I3) * p.ih2 * th : 0.0;
+    m3[0] = I3;
+    m5[0] = I5;
+    m5[1] = -x3[0] * th;
+    m5[2] = -y3[0] * th;
+    m5[3] = (I3 - x3[1]) * th;
+    m5[4] = -x3[2] * th;
+    m5[5] = (I3 - y3[1]) * th;
+    m7[0] = (p.h2 > 1e-60) ? (d5 + 3.0 * I5) * p.ih2 * f : 0.0;
+    m7[1] = -x5[0] * f;
+    m7[2] = -y5[0] * f;
+    m7[3] = (I5 - x5[1]) * f;
+    m7[4] = -x5[2] * f;
+    m7[5] = (I5 - y5[1]) * f;
+    m7[6] = (2.0 * m5[1] - x5[3]) * f;
+    m7[7] = (m5[2] - x5[4]) * f;
+    m7[8] = -x5[5] * f;
+    m7[9] = (2.0 * m5[2] - y5[2]) * f;
 }
 
 // Local-frame moment tensors of d = (-xi1, -xi2, z): component c counts
