@@ -18,15 +18,15 @@ struct ConSplit {
 // ones whole blocks of observers, whose records are made least often. Fewer than
 // about five warps an SM leave the pipe waiting for results; beyond a few blocks
 // an SM the scheduler evens them out.
-inline ConSplit contract_split(int64_t nf, int64_t ns, int threads, int tile, double pair, double setup) {
+inline ConSplit contract_split(int64_t nf, int64_t ns, int threads, int max_ob, int tile, double pair, double setup) {
     constexpr int sms = 152;
     static const int obs[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
-    ConSplit best = {64, 1};
+    ConSplit best = {max_ob, 1};
     double cost = 1e300;
     for (int ranks = 1; ranks <= 8; ranks *= 2) {
         if (ranks > 1 && (int64_t)tile * (ranks / 2) >= ns) break;      // a rank would have no source
         for (int ob : obs) {
-            if (ob > threads || (ob > 1 && ob / 2 >= nf)) continue;
+            if (ob > max_ob || (ob > 1 && ob / 2 >= nf)) continue;
             const int slices = threads / ob;
             const int64_t blocks = ceil_div(nf, ob) * ranks;
             const double tiles = (double)ceil_div(ceil_div(ns, tile), ranks);

@@ -5,8 +5,8 @@
 //
 // Bound by the FP64 pipe. Against one thread per pair with run-time degrees and
 // tables in local memory (the 32-term series and about 12 KB a thread before),
-// the 8-per-face cube's P1 T block (1.77e6 pairs) went from 63.2 to 4.7 ms,
-// a ragged P2 U block (1,001 x 333) from 26.9 to 3.7 ms.
+// the 8-per-face cube's P1 T block (1.77e6 pairs) went from 63.2 to 4.6 ms,
+// a ragged P2 U block (1,001 x 333) from 26.9 to 2.4 ms.
 #include "nodal_launch.cuh"
 
 namespace mbem {
@@ -16,6 +16,7 @@ enum { ND_T = 0, ND_U = 1, ND_TBASIS = 2, ND_UBASIS = 3 };
 template <int P, int KIND>
 __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, int sb, int fb) {
     extern __shared__ __align__(16) unsigned char nd_smem[];
+    __shared__ PairQueue queue;
     NodalRec* recs = reinterpret_cast<NodalRec*>(nd_smem);
     constexpr int K = nd_nodes(P);
     const int64_t s0 = (int64_t)blockIdx.x * sb;
@@ -24,9 +25,15 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
     __syncthreads();
     const TCoef tc = t_coef(a.c);
     for (int64_t f0 = (int64_t)blockIdx.y * fb; f0 < a.n_field_pts; f0 += (int64_t)gridDim.y * fb) {
-        const int nf = (int)lmin(fb, a.n_field_pts - f0);
+        const int nf = (int)lmin(fb, a.n_field_pts - f0), total = ns * nf;
+        queue_pairs(queue, total, [&](int p) {
+            const int t = p / nf;
+            return pair_class<P>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
+        });
+        int p;
 #pragma unroll 1
-        for (int p = threadIdx.x; p < ns * nf; p += ND_THREADS) {
+        while (queue_next(queue, total, p)) {
+            if (p < 0) continue;
             const int t = p / nf;
             const int64_t f = f0 + (p - t * nf), s = s0 + t;
             const NodalRec& g = recs[t];
@@ -93,6 +100,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
                     for (int k = 0; k < K; k++) put(k, 0.0, 0.0, zero);
             }
         }
+        __syncthreads();      // the queue is read until every warp is here
     }
 }
 

@@ -6,7 +6,7 @@
 // block: a few observers still fill the part, each partial sum has one owner
 // and the sums are added in slice, then rank order through distributed shared
 // memory (deterministic, no workspace). Bound by the FP64 pipe: the stress of a
-// 16 x 16 P2 fault at 2,000 observers went from 266 to 15.9 ms.
+// 16 x 16 P2 fault at 2,000 observers went from 266 to 10.7 ms.
 #include <cooperative_groups.h>
 
 #include "contract_split.cuh"
@@ -16,7 +16,7 @@ namespace mbem {
 
 namespace cg = cooperative_groups;
 
-constexpr int NC_TILE = 16;                           // source records in shared memory at a time
+constexpr int NC_TILE = 32, NC_OBS = 16;              // sources a tile, most observers a block
 constexpr int NC_T = 0, NC_U = 1, NC_STRESS = 2;      // kinds: T, U, 2 + MBEM_STRESS_*
 
 template <int P>
@@ -35,34 +35,29 @@ __device__ __forceinline__ void contract_pair(const NodalTile<P>& t, const doubl
     else pair_dd_contract<P>(t.g, t.d, x, m, a.which == MBEM_STRESS_ELASTIC, acc, nullptr);
 }
 
-// ob observers a block, ND_THREADS / ob slices of each tile of st sources, the
-// tiles dealt over the cluster's blocks
+// ob observers a block, the source tiles dealt over the cluster's blocks. A
+// tile's pairs are evaluated in the queue's order, each into its own place, and
+// added to their observers in source order.
 template <int P, int KIND>
-__global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a, int ob, int st) {
+__global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a, int ob) {
     extern __shared__ __align__(16) unsigned char nd_smem[];
     constexpr int NO = KIND <= NC_U ? 3 : 6;
-    __shared__ double red[ND_THREADS][NO];
+    __shared__ PairQueue queue;
+    __shared__ double sum[NC_OBS * NO];
+    __shared__ double xs[NC_OBS][3];
     NodalTile<P>* tile = reinterpret_cast<NodalTile<P>*>(nd_smem);
+    double* val = reinterpret_cast<double*>(nd_smem + NC_TILE * sizeof(NodalTile<P>));     // (pair, NO)
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
-    const int slices = ND_THREADS / ob;
-    const int lane = threadIdx.x % ob, slice = threadIdx.x / ob;
-    const int64_t f = (int64_t)(blockIdx.x / ranks) * ob + lane;
-    const bool active = f < a.n_field_pts && slice < slices;
-    double x[3] = {0.0, 0.0, 0.0};
-    if (active) {
-        x[0] = a.x_field[3 * f];
-        x[1] = a.x_field[3 * f + 1];
-        x[2] = a.x_field[3 * f + 2];
-    }
+    const int64_t f0 = (int64_t)(blockIdx.x / ranks) * ob;
+    const int nf = (int)lmin(ob, a.n_field_pts - f0);
+    for (int i = threadIdx.x; i < 3 * nf; i += ND_THREADS) xs[i / 3][i % 3] = a.x_field[3 * f0 + i];
+    for (int i = threadIdx.x; i < nf * NO; i += ND_THREADS) sum[i] = 0.0;
     const TCoef tc = t_coef(a.c);
     const SMat m = stress_mat(a.mu, a.lam);
-    double acc[NO];
-#pragma unroll
-    for (int i = 0; i < NO; i++) acc[i] = 0.0;
     constexpr int K = nd_nodes(P);
-    for (int64_t s0 = (int64_t)rank * st; s0 < a.n_src; s0 += (int64_t)ranks * st) {
-        const int ns = (int)lmin(st, a.n_src - s0);
+    for (int64_t s0 = (int64_t)rank * NC_TILE; s0 < a.n_src; s0 += (int64_t)ranks * NC_TILE) {
+        const int ns = (int)lmin(NC_TILE, a.n_src - s0), total = ns * nf;
         __syncthreads();
         for (int t = threadIdx.x; t < ns; t += ND_THREADS) {
             const int64_t s = s0 + t;
@@ -70,35 +65,40 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a,
             nodal_den<P>(tile[t].g, a.density + 3 * K * s, tile[t].d);
         }
         __syncthreads();
-        if (!active) continue;
+        queue_pairs(queue, total, [&](int p) { return pair_class<P>(tile[p / nf].g, xs[p % nf]); });
+        int p;
 #pragma unroll 1
-        for (int t = slice; t < ns; t += slices)
-            if (tile[t].g.ok && !tile[t].d.zero) contract_pair<P, KIND>(tile[t], x, a, tc, m, acc);
-    }
+        while (queue_next(queue, total, p)) {
+            if (p < 0) continue;
+            const NodalTile<P>& T = tile[p / nf];
+            double acc[NO];
 #pragma unroll
-    for (int i = 0; i < NO; i++) red[threadIdx.x][i] = acc[i];
-    __syncthreads();
-    if (slice == 0) {
-        for (int k = 1; k < slices; k++)
+            for (int i = 0; i < NO; i++) acc[i] = 0.0;
+            if (T.g.ok && !T.d.zero) contract_pair<P, KIND>(T, xs[p % nf], a, tc, m, acc);
 #pragma unroll
-            for (int i = 0; i < NO; i++) acc[i] += red[k * ob + lane][i];
-#pragma unroll
-        for (int i = 0; i < NO; i++) red[lane][i] = acc[i];
+            for (int i = 0; i < NO; i++) val[p * NO + i] = acc[i];
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < nf * NO; i += ND_THREADS) {
+            double v = sum[i];
+            for (int t = 0; t < ns; t++) v += val[t * nf * NO + i];
+            sum[i] = v;
+        }
     }
     cluster.sync();
-    if (rank == 0 && slice == 0 && active) {
-        for (int r = 1; r < ranks; r++) {
-            const double* other = cluster.map_shared_rank(&red[lane][0], r);
-#pragma unroll
-            for (int i = 0; i < NO; i++) acc[i] += other[i];
-        }
+    if (rank == 0) {
         const int ix[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
         constexpr int NW = KIND <= NC_U ? 3 : 9;
-        double* o = a.out + NW * f;
-#pragma unroll
-        for (int i = 0; i < NW; i++) {
-            const double v = a.alpha * acc[NW == 3 ? i : ix[i]];
-            o[i] = a.accumulate ? o[i] + v : v;
+        for (int i = threadIdx.x; i < nf * NO; i += ND_THREADS) {
+            double v = sum[i];
+            for (int r = 1; r < ranks; r++) v += *cluster.map_shared_rank(&sum[i], r);
+            sum[i] = v;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < nf * NW; i += ND_THREADS) {
+            double* o = a.out + NW * f0 + i;
+            const double v = a.alpha * sum[(i / NW) * NO + (NW == 3 ? i % NW : ix[i % NW])];
+            *o = a.accumulate ? *o + v : v;
         }
     }
     cluster.sync();      // the partial sums stay until rank 0 has read them
@@ -148,14 +148,21 @@ int nodal_pairs_stress(const double* x, const double* tv, const double* normals,
     return launch_status("nodal_pairs_stress_kernel");
 }
 
+template <typename Kernel>
+static cudaError_t launch_contract_kernel(const cudaLaunchConfig_t& cfg, Kernel k, const NodalArgs& a, int ob) {
+    // up to 47 KB of dynamic beside 3 KB of static shared memory (P2): four blocks an SM
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+    return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k, a, ob);
+}
+
 template <int P>
-static cudaError_t launch_nodal_contract(int kind, const NodalArgs& a, unsigned grid, int ranks, int ob, int tile,
+static cudaError_t launch_nodal_contract(int kind, const NodalArgs& a, unsigned grid, int ranks, int ob,
                                          cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(ND_THREADS);
-    cfg.dynamicSmemBytes = (size_t)tile * sizeof(NodalTile<P>);
+    cfg.dynamicSmemBytes = NC_TILE * (sizeof(NodalTile<P>) + (size_t)ob * (kind <= NC_U ? 3 : 6) * sizeof(double));
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -163,15 +170,16 @@ static cudaError_t launch_nodal_contract(int kind, const NodalArgs& a, unsigned 
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    static_assert(NC_TILE * NC_OBS <= ND_TILE_PAIRS, "a tile's pairs fit its queue");
     switch (kind) {
-        case NC_T: return cudaLaunchKernelEx(&cfg, nodal_contract_kernel<P, NC_T>, a, ob, tile);
-        case NC_U: return cudaLaunchKernelEx(&cfg, nodal_contract_kernel<P, NC_U>, a, ob, tile);
+        case NC_T: return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_T>, a, ob);
+        case NC_U: return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_U>, a, ob);
         case NC_STRESS + MBEM_STRESS_KELVIN:
-            return cudaLaunchKernelEx(&cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_KELVIN>, a, ob, tile);
+            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_KELVIN>, a, ob);
         case NC_STRESS + MBEM_STRESS_EIGEN:
-            return cudaLaunchKernelEx(&cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_EIGEN>, a, ob, tile);
+            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_EIGEN>, a, ob);
         default:
-            return cudaLaunchKernelEx(&cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_DD>, a, ob, tile);
+            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_DD>, a, ob);
     }
 }
 
@@ -191,12 +199,12 @@ int nodal_contract(int kind, const double* x, int64_t nf, const double* tv, cons
     a.which = kind >= NC_STRESS ? kind - NC_STRESS : 0;
     a.alpha = alpha; a.accumulate = accumulate; a.out = out;
     if (nf == 0) return MBEM_OK;
-    const ConSplit sp = contract_split(nf, ns, ND_THREADS, NC_TILE, order == 1 ? 1200.0 : 2200.0, 600.0);
+    const ConSplit sp = contract_split(nf, ns, ND_THREADS, NC_OBS, NC_TILE, order == 1 ? 1200.0 : 2200.0, 600.0);
     const int ob = sp.ob, ranks = sp.ranks;
     const int64_t grid = ceil_div(nf, ob) * ranks;
     MBEM_REQUIRE(grid < (int64_t)1 << 31, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)nf);
-    const cudaError_t ce = order == 1 ? launch_nodal_contract<1>(kind, a, (unsigned)grid, ranks, ob, NC_TILE, (cudaStream_t)stream)
-                                      : launch_nodal_contract<2>(kind, a, (unsigned)grid, ranks, ob, NC_TILE, (cudaStream_t)stream);
+    const cudaError_t ce = order == 1 ? launch_nodal_contract<1>(kind, a, (unsigned)grid, ranks, ob, (cudaStream_t)stream)
+                                      : launch_nodal_contract<2>(kind, a, (unsigned)grid, ranks, ob, (cudaStream_t)stream);
     if (ce != cudaSuccess) return set_error(MBEM_ERR_CUDA, "nodal_contract_kernel: %s", cudaGetErrorString(ce));
     return launch_status("nodal_contract_kernel");
 }

@@ -104,15 +104,15 @@ struct NodalArgs {
     int64_t n_pairs;
 };
 
-// Blocks of sb sources x fb field points, their pairs dealt to the threads
-// with the field point running fastest (a warp reads one or two sources'
-// records). A block is as large as leaves four rounds of resident blocks, so
-// that the last round is short and each source's record is made few times.
+// Blocks of sb sources x fb field points. A block is as large as leaves four
+// rounds of resident blocks, so that the last round is short and each source's
+// record is made few times.
 struct PairTiles {
     int sb, fb;
     dim3 grid;
     size_t smem;
 };
+constexpr int ND_TILE_PAIRS = 1024;      // most pairs a tile holds
 static inline PairTiles pair_tiles(int64_t nf, int64_t ns) {
     PairTiles t;
     t.fb = (int)std::min<int64_t>(nf, ND_THREADS);
@@ -130,6 +130,63 @@ __device__ __forceinline__ void load_recs(const NodalArgs& a, int64_t s0, int ns
         const int64_t s = s0 + t;
         nodal_rec(a.tri_verts + 9 * s, a.normals ? a.normals + 3 * s : nullptr, a.eps[s], recs[t]);
     }
+}
+
+// A tile's pairs ordered by what they cost: beside the element, near, and the
+// far rules. A warp that mixes closed forms and quadratures runs both (45 to 69 %
+// of the lanes were at work in the P2 and traction kernels), so the block lists
+// its pairs by class and its warps take 32 at a time, whichever is free next.
+constexpr int ND_CLASSES = 5;
+struct PairQueue {
+    int count[ND_CLASSES], next;
+    uint16_t list[ND_TILE_PAIRS];
+};
+template <int P>
+__device__ __forceinline__ int pair_class(const NodalRec& g, const double* x) {
+    const double dx = x[0] - g.c[0], dy = x[1] - g.c[1], dz = x[2] - g.c[2];
+    const float q = (float)(dx * dx + dy * dy + dz * dz + g.eps2) / (float)g.L2;      // a hint: the pair decides again
+    if (q <= 4.0f) return 0;
+    if (q <= (float)(ND_D_STAR * ND_D_STAR)) return 1;
+    return 9 - nd_far_n<P>(q, 1.0);      // n = 7 .. 5 (and 4 with 5)
+}
+// queues `total` pairs (at most ND_TILE_PAIRS); cls(p) is called once a pair.
+// All threads of the block call it; it ends with a barrier.
+template <class Cls>
+__device__ __forceinline__ void queue_pairs(PairQueue& q, int total, Cls&& cls) {
+    if (threadIdx.x < ND_CLASSES) q.count[threadIdx.x] = 0;
+    if (threadIdx.x == 0) q.next = 0;
+    __syncthreads();
+    uint64_t kept = 0;                   // 3 bits a pair, ND_TILE_PAIRS / ND_THREADS = 16 pairs
+    int i = 0;
+    for (int p = threadIdx.x; p < total; p += ND_THREADS, i++) {
+        const int c = min(cls(p), ND_CLASSES - 1);
+        kept |= (uint64_t)c << (3 * i);
+        atomicAdd(&q.count[c], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int run = 0;
+        for (int c = ND_CLASSES - 1; c >= 0; c--) {      // the dearest first
+            const int n = q.count[c];
+            q.count[c] = run;
+            run += n;
+        }
+    }
+    __syncthreads();
+    i = 0;
+    for (int p = threadIdx.x; p < total; p += ND_THREADS, i++)
+        q.list[atomicAdd(&q.count[(kept >> (3 * i)) & 7], 1)] = (uint16_t)p;
+    __syncthreads();
+}
+// the next pair of this lane's warp's 32, or -1; ends when all are taken. The
+// whole warp calls it together.
+__device__ __forceinline__ bool queue_next(PairQueue& q, int total, int& p) {
+    int base = 0;
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) base = atomicAdd(&q.next, 32);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    p = base + lane < total ? (int)q.list[base + lane] : -1;
+    return base < total;
 }
 
 // field point of listed pair q

@@ -6,7 +6,7 @@
 // does not depend on the order of the adds).
 //
 // Bound by the FP64 pipe. 288 points x 6,144 P0 sources ("slip"): 70.2 ms with
-// run-time tables in local memory and 144 / 64 far points, 7.5 ms now.
+// run-time tables in local memory and 144 / 64 far points, 5.5 ms now.
 #include "nodal_launch.cuh"
 
 namespace mbem {
@@ -30,6 +30,7 @@ __device__ __forceinline__ void traction_pair(const NodalArgs& a, const NodalRec
 template <int P, int F>
 __global__ void __launch_bounds__(ND_THREADS) nodal_traction_kernel(NodalArgs a, int sb, int fb) {
     extern __shared__ __align__(16) unsigned char nd_smem[];
+    __shared__ PairQueue queue;
     NodalRec* recs = reinterpret_cast<NodalRec*>(nd_smem);
     const int64_t s0 = (int64_t)blockIdx.x * sb;
     const int ns = (int)lmin(sb, a.n_src - s0);
@@ -37,12 +38,19 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_traction_kernel(NodalArgs a,
     __syncthreads();
     const SMat m = stress_mat(a.mu, a.lam);
     for (int64_t f0 = (int64_t)blockIdx.y * fb; f0 < a.n_field_pts; f0 += (int64_t)gridDim.y * fb) {
-        const int nf = (int)lmin(fb, a.n_field_pts - f0);
+        const int nf = (int)lmin(fb, a.n_field_pts - f0), total = ns * nf;
+        queue_pairs(queue, total, [&](int p) {
+            const int t = p / nf;
+            return pair_class<P>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
+        });
+        int p;
 #pragma unroll 1
-        for (int p = threadIdx.x; p < ns * nf; p += ND_THREADS) {
+        while (queue_next(queue, total, p)) {
+            if (p < 0) continue;
             const int t = p / nf;
             traction_pair<P, F>(a, recs[t], f0 + (p - t * nf), s0 + t, m, a.which == TR_SLIP);
         }
+        __syncthreads();      // the queue is read until every warp is here
     }
 }
 

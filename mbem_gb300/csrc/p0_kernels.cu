@@ -402,7 +402,7 @@ int launch_contract(int kind, const double* x, int64_t nf, const double* tv, con
     for (int i = 0; i < 6; i++) a.c[i] = (c && i < nc) ? c[i] : 0.0;
     a.mu = mu; a.lam = lam; a.alpha = alpha; a.accumulate = accumulate; a.out = out;
     if (nf == 0) return MBEM_OK;
-    const ConSplit sp = contract_split(nf, ns, CON_THREADS, SRC_TILE, kind >= CON_DD_STRESS ? 500 : 400, 250);
+    const ConSplit sp = contract_split(nf, ns, CON_THREADS, CON_THREADS, SRC_TILE, kind >= CON_DD_STRESS ? 500 : 400, 250);
     a.ob = sp.ob;
     const int64_t grid = ceil_div(nf, sp.ob) * sp.ranks;
     MBEM_REQUIRE(grid < (int64_t)1 << 31, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)nf);
