@@ -41,26 +41,66 @@ static inline void nd_gauss_legendre(int n, double* x, double* w) {
     }
 }
 
+// Fully symmetric rules on the triangle, one line an orbit: points, weight (of a
+// unit sum), and two barycentric coordinates of a point of it. Degrees 6, 8, 9 and
+// 10 with 12, 16, 19 and 25 points, the orbit counts of Dunavant, Int. J. Numer.
+// Meth. Eng. 21 (1985); the values solve the moment equations (invariants
+// e2^i e3^j of the barycentric coordinates) by Newton's method in 50 digits.
+struct NdOrbit {
+    int n;
+    double w, a, b;
+};
+static const NdOrbit ND_ORBITS[4][6] = {
+    {{3, 0.1167862757263793660252896, 0.2492867451709104212916386, 0.2492867451709104212916386},
+     {3, 0.05084490637020681692093681, 0.0630890144915022283403316, 0.0630890144915022283403316},
+     {6, 0.08285107561837357519355346, 0.6365024991213986472301426, 0.05314504984481694735324967}},
+    {{1, 0.1443156076777871682510911, 1.0 / 3.0, 1.0 / 3.0},
+     {3, 0.03245849762319808031092593, 0.05054722831703097545842355, 0.05054722831703097545842355},
+     {3, 0.0950916342672846247938961, 0.4592925882927231560288155, 0.4592925882927231560288155},
+     {3, 0.1032173705347182502817916, 0.1705693077517602066222935, 0.1705693077517602066222935},
+     {6, 0.02723031417443499426484469, 0.008394777409957605337213835, 0.2631128296346381134217858}},
+    {{1, 0.09713579628279883381924198, 1.0 / 3.0, 1.0 / 3.0},
+     {3, 0.07782754100477427931673936, 0.4370895914929366372699304, 0.4370895914929366372699304},
+     {3, 0.0255776756586980312616788, 0.04472951339445270986510659, 0.04472951339445270986510659},
+     {3, 0.03133470022713907053685483, 0.4896825191987376277837069, 0.4896825191987376277837069},
+     {3, 0.07964773892721025303289177, 0.1882035356190327302409613, 0.1882035356190327302409613},
+     {6, 0.04328353937728937728937729, 0.7411985987844980206900799, 0.2219629891607656956751025}},
+    {{1, 0.08174332914628596642811868, 1.0 / 3.0, 1.0 / 3.0},
+     {3, 0.04595796360474472801378791, 0.1421611010565643850921621, 0.1421611010565643850921621},
+     {3, 0.01335296881314956627557298, 0.03205537321694351293098459, 0.03205537321694351293098459},
+     {6, 0.06390490639642404543289873, 0.1481328857838205504978068, 0.5300541189273440282770957},
+     {6, 0.03418464816295942862869158, 0.02961988948872976763383627, 0.3691467818278109869114208},
+     {6, 0.02529775770728838438904279, 0.8079306009228790650799499, 0.02836766533993843925043576}}};
+
 static inline NodalRules nd_make_rules() {
     NodalRules r;
     int k = 0;
-    for (int n : {8, 10, 12, 16}) {
+    for (int n : {7, 8, 9, 10, 12, 16}) {
         double x[16], w[16];
         nd_gauss_legendre(n, x, w);
-        for (int i = 0; i < n / 2; i++, k++) {     // decreasing nodes: the positive half first
+        for (int i = 0; i < n; i++, k++) {
+            if (2 * i + 1 == n) x[i] = 0.0;
             r.ex[k] = x[i];
-            r.ew[k] = w[i];
+            double f = w[i];
+            for (int p = 0; p < 6; p++, f *= x[i]) r.ew[k][p] = f;
         }
     }
     k = 0;
-    for (int n = 4; n <= 7; n++) {
-        double x[7], w[7];
-        nd_gauss_legendre(n, x, w);
-        for (int i = 0; i < n; i++, k++) {
-            r.fx[k] = 0.5 * (x[i] + 1.0);
-            r.fw[k] = 0.5 * w[i];
+    for (int d = 0; d < 4; d++)
+        for (const NdOrbit& o : ND_ORBITS[d]) {
+            const double c = 1.0 - o.a - o.b;
+            const double p[6][2] = {{o.a, o.b}, {c, o.a}, {o.b, c}, {o.b, o.a}, {o.a, c}, {c, o.b}};
+            for (int i = 0; i < o.n; i++, k++) {
+                const double l1 = p[i][0], l2 = p[i][1], l0 = 1.0 - l1 - l2, w = 0.5 * o.w;
+                r.fl[k][0] = l1; r.fl[k][1] = l2; r.fl[k][2] = w;
+                const double l[3] = {l0, l1, l2};
+                for (int v = 0; v < 3; v++) {
+                    r.fn[k][v] = w * l[v];
+                    r.fn[k][3 + v] = w * l[v] * (2.0 * l[v] - 1.0);
+                    r.fn[k][6 + v] = 4.0 * w * l[v] * l[(v + 1) % 3];
+                }
+            }
         }
-    }
     return r;
 }
 
@@ -136,7 +176,7 @@ __device__ __forceinline__ void load_recs(const NodalArgs& a, int64_t s0, int ns
 // far rules. A warp that mixes closed forms and quadratures runs both (45 to 69 %
 // of the lanes were at work in the P2 and traction kernels), so the block lists
 // its pairs by class and its warps take 32 at a time, whichever is free next.
-constexpr int ND_CLASSES = 5;
+constexpr int ND_CLASSES = 6;
 struct PairQueue {
     int count[ND_CLASSES], next;
     uint16_t list[ND_TILE_PAIRS];
@@ -147,7 +187,7 @@ __device__ __forceinline__ int pair_class(const NodalRec& g, const double* x) {
     const float q = (float)(dx * dx + dy * dy + dz * dz + g.eps2) / (float)g.L2;      // a hint: the pair decides again
     if (q <= 4.0f) return 0;
     if (q <= (float)(ND_D_STAR * ND_D_STAR)) return 1;
-    return 9 - nd_far_n<P>(q, 1.0);      // n = 7 .. 5 (and 4 with 5)
+    return 2 + nd_far_rule<P>(q, 1.0);
 }
 // queues `total` pairs (at most ND_TILE_PAIRS); cls(p) is called once a pair.
 // All threads of the block call it; it ends with a barrier.
@@ -159,14 +199,14 @@ __device__ __forceinline__ void queue_pairs(PairQueue& q, int total, Cls&& cls) 
     uint64_t kept = 0;                   // 3 bits a pair, ND_TILE_PAIRS / ND_THREADS = 16 pairs
     int i = 0;
     for (int p = threadIdx.x; p < total; p += ND_THREADS, i++) {
-        const int c = min(cls(p), ND_CLASSES - 1);
+        const int c = cls(p);
         kept |= (uint64_t)c << (3 * i);
         atomicAdd(&q.count[c], 1);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         int run = 0;
-        for (int c = ND_CLASSES - 1; c >= 0; c--) {      // the dearest first
+        for (int c = 0; c < ND_CLASSES; c++) {
             const int n = q.count[c];
             q.count[c] = run;
             run += n;

@@ -15,15 +15,20 @@
 //  * everything that depends on the source alone is in one record per source;
 //  * an edge evaluates one row of primitives, int u^k / R^m for the highest m,
 //    by an n-point Gauss rule whose n follows from the ellipse on which the
-//    integrand is analytic (a = (R_a + R_b) / L_e is its semi-axis; n = 8 at
-//    a >= 12, 10 at 6, 12 at 3.9, 16 at 2.2 keep the truncation below 1e-16 of
-//    int |u|^k / R^m), and the lower rows from it by additions of like-signed
-//    terms (R^2 = u^2 + rho^2). The rule has no cancellation, so it replaces
+//    integrand is analytic (a = (R_a + R_b) / L_e is its semi-axis; n = 7 at
+//    a >= 26, 8 at 15, 9 at 9.3, 10 at 6.6, 12 at 3.9, 16 at 2.2 keep the
+//    truncation below 1e-16 of int |u|^k / R^m), and the lower rows from it
+//    (R^2 is a polynomial in u). The rule has no cancellation, so it replaces
 //    both 32-term series (small |u| always has a >= 2.23) and, away from the
 //    edge, the closed form; a large-|u| interval with a < 2.2 is summed in
 //    pieces of ratio 2.5. Only what is left, an edge the observer is beside at
-//    less than about its length, takes the closed form;
+//    less than about its length, takes the closed form. The powers are of the
+//    rule's own abscissa (tabulated with its weights), the edge's midpoint the
+//    origin of the chain below;
 //  * (A + t u)^a (B + t' u)^b integrates by a chain of two-term combinations;
+//  * the far quadratures are fully symmetric rules of 12 to 25 points (degrees 6,
+//    8, 9, 10), as accurate from 10 longest edges on as 49 to 16 collapsed
+//    Gauss-Legendre points;
 //  * a nodal matrix block is assembled from the blocks of the shifted moments
 //    (one per monomial of the shape functions) instead of from one table per
 //    node, and a contraction folds the density's polynomial into the moments;
@@ -69,29 +74,34 @@ struct NDeg {
     static constexpr int ktop = top == 5 ? k5 : top == 3 ? k3 : k1;
 };
 
-// Gauss-Legendre tables: the positive nodes and weights of the edge rules
-// (n = 8, 10, 12, 16), and the rules on [0, 1] of the far quadrature (n = 4..7).
+// The edge rules (n = 7, 8, 9, 10, 12, 16): abscissae and weights times their
+// powers 0 .. 5; the last one's plain form also sums pieces. The far rules
+// (19, 16, 12 and 25 points): barycentric l1, l2, the weight (sum 1/2) and the
+// weight times the shape functions of P1 (3) and P2 (6).
+constexpr int ND_EDGE_Q = 7 + 8 + 9 + 10 + 12 + 16;
+constexpr int ND_FAR_Q = 12 + 16 + 19 + 25;
 struct NodalRules {
-    double ex[23], ew[23];
-    double fx[22], fw[22];
+    double ex[ND_EDGE_Q], ew[ND_EDGE_Q][6];
+    double fl[ND_FAR_Q][3], fn[ND_FAR_Q][9];
 };
 #ifndef MBEM_ND_RULES
 static __constant__ NodalRules c_nd;       // one copy per translation unit (nodal_rules_ready)
 #define MBEM_ND_RULES c_nd
 #endif
 
-// far rule n: its truncation is below 5e-16 of the pair's largest entry from
-// D / L = 10 on (n x n collapsed points against 16 x 16 over random triangles
-// and directions, T, U and stress kernels: P0 n = 5 from 17 and 4 from 52, P1
-// n = 6 from 11 and 5 from 27, P2 n = 6 from 15 and 5 from 48)
+// The far rule, 0 .. 3 for 25, 19, 16, 12 points: its truncation is below 5e-16 of
+// the pair's largest entry (against 256 points over random triangles and
+// directions, T, U and stress kernels; 4e-15 for the P2 stress between 10 and 11
+// longest edges, where the closed form on the other side is off by 1e-13)
 template <int P>
-__device__ __forceinline__ int nd_far_n(double D2, double L2) {
-    if (P == 0) return D2 > (52.0 * 52.0) * L2 ? 4 : D2 > (17.0 * 17.0) * L2 ? 5 : 6;
-    if (P == 1) return D2 > (27.0 * 27.0) * L2 ? 5 : D2 > (11.0 * 11.0) * L2 ? 6 : 7;
-    return D2 > (48.0 * 48.0) * L2 ? 5 : D2 > (15.0 * 15.0) * L2 ? 6 : 7;
+__device__ __forceinline__ int nd_far_rule(double D2, double L2) {
+    if (P == 0) return D2 > (42.0 * 42.0) * L2 ? 3 : D2 > (18.0 * 18.0) * L2 ? 2 : D2 > (11.0 * 11.0) * L2 ? 1 : 0;
+    if (P == 1) return D2 > (90.0 * 90.0) * L2 ? 3 : D2 > (30.0 * 30.0) * L2 ? 2 : D2 > (17.0 * 17.0) * L2 ? 1 : 0;
+    return D2 > (55.0 * 55.0) * L2 ? 2 : D2 > (26.0 * 26.0) * L2 ? 1 : 0;
 }
-// its offset in NodalRules::fx
-__device__ __forceinline__ int nd_far_off(int n) { return n * (n - 1) / 2 - 6; }
+// first and last + 1 point of rule r
+__device__ __forceinline__ int nd_far_first(int r) { return r == 0 ? 47 : r == 1 ? 28 : r == 2 ? 12 : 0; }
+__device__ __forceinline__ int nd_far_last(int r) { return r == 0 ? 72 : r == 1 ? 47 : r == 2 ? 28 : 12; }
 
 // ---------------------------------------------------------------------------
 // per-source record
@@ -187,38 +197,46 @@ __device__ __forceinline__ bool nodal_is_far(const NodalRec& g, const NodalObs& 
 template <int P, int F>
 struct EdgePrim {
     typedef NDeg<P, F> G;
+    // int v^k / R^m dv with u = off + step v, step included on use
     double p5[nd_max(G::k5, 0) + 1], p3[nd_max(G::k3, 0) + 1], p1[nd_max(G::k1, 0) + 1], pm1[nd_max(G::em1, 0) + 1];
+    double off, step;
 };
 
-// acc[k] += hl sum_q w_q u_q^k / R^TOP over the n-point rule on centre uc, half-length hl
+// s[k] = sum_q w_q x_q^k / R^TOP at u_q = uc + hl x_q
 template <int TOP, int KT>
-__device__ __forceinline__ void edge_gauss(double uc, double hl, double rho2, int q0, int q1, double acc[KT + 1]) {
-    double s[KT + 1];
+__device__ __forceinline__ void edge_gauss(double uc, double hl, double rho2, int q0, int q1, double s[KT + 1]) {
 #pragma unroll
     for (int k = 0; k <= KT; k++) s[k] = 0.0;
-#pragma unroll 1
+#pragma unroll 2
     for (int q = q0; q < q1; q++) {
-        const double dx = hl * MBEM_ND_RULES.ex[q], w = MBEM_ND_RULES.ew[q];
+        const double u = uc + hl * MBEM_ND_RULES.ex[q];
+        const double iR = rsqrt(u * u + rho2);
+        double f = iR;
+        if (TOP >= 3) {
+            const double iR2 = iR * iR;
+            f *= iR2;
+            if (TOP >= 5) f *= iR2;
+        }
 #pragma unroll
-        for (int sg = 0; sg < 2; sg++) {
-            const double u = sg ? uc + dx : uc - dx;
-            const double iR = rsqrt(u * u + rho2);
-            double f = w * iR;
-            if (TOP >= 3) {
-                const double iR2 = iR * iR;
-                f *= iR2;
-                if (TOP >= 5) f *= iR2;
-            }
-            s[0] += f;
+        for (int k = 0; k <= KT; k++) s[k] += f * MBEM_ND_RULES.ew[q][k];
+    }
+}
+// acc[k] += int u^k / R^TOP over a piece of the edge (n = 16)
+template <int TOP, int KT>
+__device__ __noinline__ void edge_piece(double uc, double hl, double rho2, double acc[KT + 1]) {
+#pragma unroll 1
+    for (int q = ND_EDGE_Q - 16; q < ND_EDGE_Q; q++) {
+        const double u = uc + hl * MBEM_ND_RULES.ex[q];
+        const double iR = rsqrt(u * u + rho2);
+        double f = hl * MBEM_ND_RULES.ew[q][0] * iR;
+        for (int m = 1; m < TOP; m += 2) f *= iR * iR;
+        acc[0] += f;
 #pragma unroll
-            for (int k = 1; k <= KT; k++) {
-                f *= u;
-                s[k] += f;
-            }
+        for (int k = 1; k <= KT; k++) {
+            f *= u;
+            acc[k] += f;
         }
     }
-#pragma unroll
-    for (int k = 0; k <= KT; k++) acc[k] += hl * s[k];
 }
 
 // conjugate closed-form differences (tri_nodal.py:346-382) and the upward
@@ -274,6 +292,37 @@ __device__ __noinline__ void edge_closed(double ua, double ub, double Le, double
     }
 }
 
+// |u| from umin >= 2 rho up, in pieces of ratio 2.5; an odd power keeps the sign of u
+template <int P, int F>
+__device__ __noinline__ void edge_pieces(double ua, double ub, double rho2, EdgePrim<P, F>& E) {
+    typedef NDeg<P, F> G;
+    double t[G::ktop + 1];
+#pragma unroll
+    for (int k = 0; k <= G::ktop; k++) t[k] = 0.0;
+    const double b = fmax(fabs(ua), fabs(ub));
+    double t0 = fmin(fabs(ua), fabs(ub));
+#pragma unroll 1
+    while (t0 < b) {
+        double t1 = 2.5 * t0;
+        if (!(t1 < b)) t1 = b;
+        edge_piece<G::top, G::ktop>(0.5 * (t0 + t1), 0.5 * (t1 - t0), rho2, t);
+        t0 = t1;
+    }
+    if (ua < 0.0)
+#pragma unroll
+        for (int k = 1; k <= G::ktop; k += 2) t[k] = -t[k];
+    // lower rows: u^k / R^(m-2) = u^(k+2) / R^m + rho^2 u^k / R^m
+#pragma unroll
+    for (int k = 0; k <= G::k5; k++) E.p5[k] = t[k];
+#pragma unroll
+    for (int k = 0; k <= G::k3; k++) E.p3[k] = G::top == 5 ? t[k + 2 <= G::ktop ? k + 2 : 0] + rho2 * t[k] : t[k];
+#pragma unroll
+    for (int k = 0; k <= G::k1; k++)
+        E.p1[k] = G::top > 1 ? E.p3[k + 2 <= G::k3 ? k + 2 : 0] + rho2 * E.p3[k <= G::k3 ? k : 0] : t[k];
+#pragma unroll
+    for (int k = 0; k <= G::em1; k++) E.pm1[k] = E.p1[k + 2 <= G::k1 ? k + 2 : 0] + rho2 * E.p1[k];
+}
+
 // The primitives of one edge, u in [ua, ub] (ub - ua = Le), rho^2 = R^2 - u^2.
 template <int P, int F>
 __device__ __forceinline__ void edge_primitives(double ua, double ub, double Le, double iLe, double RaRb_sum,
@@ -281,40 +330,37 @@ __device__ __forceinline__ void edge_primitives(double ua, double ub, double Le,
     typedef NDeg<P, F> G;
     const double a = RaRb_sum * iLe;
     const double umin = fmin(fabs(ua), fabs(ub));
-    const bool single = a >= 2.2;
-    if (single || (ua * ub > 0.0 && umin * umin >= 4.0 * rho2)) {
+    if (a >= 2.2) {
+        const double uc = 0.5 * (ua + ub), hl = 0.5 * Le;
+        // offsets 0, 7, 15, 24, 34, 46 of n = 7, 8, 9, 10, 12, 16
+        const int q0 = a >= 26.0 ? 0 : a >= 15.0 ? 7 : a >= 9.3 ? 15 : a >= 6.6 ? 24 : a >= 3.9 ? 34 : 46;
+        const int q1 = a >= 26.0 ? 7 : a >= 15.0 ? 15 : a >= 9.3 ? 24 : a >= 6.6 ? 34 : a >= 3.9 ? 46 : 62;
         double t[G::ktop + 1];
-#pragma unroll
-        for (int k = 0; k <= G::ktop; k++) t[k] = 0.0;
-        if (single) {
-            const int q0 = a >= 12.0 ? 0 : a >= 6.0 ? 4 : a >= 3.9 ? 9 : 15;
-            const int q1 = a >= 12.0 ? 4 : a >= 6.0 ? 9 : a >= 3.9 ? 15 : 23;
-            edge_gauss<G::top, G::ktop>(0.5 * (ua + ub), 0.5 * Le, rho2, q0, q1, t);
-        } else {
-            // |u| in [t0, b], pieces of ratio 2.5; an odd power keeps the sign of u
-            const double sg = ua < 0.0 ? -1.0 : 1.0;
-            const double b = fmax(fabs(ua), fabs(ub));
-            double t0 = umin;
-#pragma unroll 1
-            while (t0 < b) {
-                double t1 = 2.5 * t0;
-                if (!(t1 < b)) t1 = b;
-                edge_gauss<G::top, G::ktop>(0.5 * (t0 + t1), 0.5 * (t1 - t0), rho2, 15, 23, t);
-                t0 = t1;
-            }
-#pragma unroll
-            for (int k = 1; k <= G::ktop; k += 2) t[k] *= sg;
-        }
-        // lower rows: u^k / R^(m-2) = u^(k+2) / R^m + rho^2 u^k / R^m
+        edge_gauss<G::top, G::ktop>(uc, hl, rho2, q0, q1, t);
+        E.off = uc;
+        E.step = hl;
+        // lower rows: R^2 = hl^2 x^2 + 2 uc hl x + (uc^2 + rho^2)
+        const double r0 = uc * uc + rho2, r1 = Le * uc, r2 = hl * hl;
 #pragma unroll
         for (int k = 0; k <= G::k5; k++) E.p5[k] = t[k];
 #pragma unroll
-        for (int k = 0; k <= G::k3; k++) E.p3[k] = G::top == 5 ? t[k + 2 <= G::ktop ? k + 2 : 0] + rho2 * t[k] : t[k];
+        for (int k = 0; k <= G::k3; k++)
+            E.p3[k] = G::top == 5 ? (r0 * t[k] + r1 * t[k + 1 <= G::ktop ? k + 1 : 0]) + r2 * t[k + 2 <= G::ktop ? k + 2 : 0]
+                                  : t[k];
 #pragma unroll
         for (int k = 0; k <= G::k1; k++)
-            E.p1[k] = G::top > 1 ? E.p3[k + 2 <= G::k3 ? k + 2 : 0] + rho2 * E.p3[k <= G::k3 ? k : 0] : t[k];
+            E.p1[k] = G::top > 1 ? (r0 * E.p3[k <= G::k3 ? k : 0] + r1 * E.p3[k + 1 <= G::k3 ? k + 1 : 0]) +
+                                       r2 * E.p3[k + 2 <= G::k3 ? k + 2 : 0]
+                                 : t[k];
 #pragma unroll
-        for (int k = 0; k <= G::em1; k++) E.pm1[k] = E.p1[k + 2 <= G::k1 ? k + 2 : 0] + rho2 * E.p1[k];
+        for (int k = 0; k <= G::em1; k++)
+            E.pm1[k] = (r0 * E.p1[k] + r1 * E.p1[k + 1 <= G::k1 ? k + 1 : 0]) + r2 * E.p1[k + 2 <= G::k1 ? k + 2 : 0];
+        return;
+    }
+    E.off = 0.0;
+    E.step = 1.0;
+    if (ua * ub > 0.0 && umin * umin >= 4.0 * rho2) {
+        edge_pieces<P, F>(ua, ub, rho2, E);
     } else {
         edge_closed<P, F>(ua, ub, Le, rho2, E);
     }
@@ -426,22 +472,25 @@ __device__ __forceinline__ void nodal_moments(const NodalRec& g, const NodalObs&
         const double rho2 = dp * dp + h2;
         EdgePrim<P, F> E;
         edge_primitives<P, F>(ua, ub, g.Le[e], g.iLe[e], Rs, rho2, E);
-        const double A = dp * n1, B = dp * n2;
+        // the point of the edge at v: (A + sx v, B + sy v)
+        const double A = dp * n1 + E.off * tx, B = dp * n2 + E.off * ty;
+        const double sx = E.step * tx, sy = E.step * ty;
+        const double m1 = E.step * n1, m2 = E.step * n2, ds = E.step * dp;
         if (e5 >= 0) {
-            bd5 += dp * E.p5[0];
-            if (G::d7 >= 1) edge_chain<nd_max(e5, 0)>(E.p5, A, B, tx, ty, n1, n2, b5, c5);
+            bd5 += ds * E.p5[0];
+            if (G::d7 >= 1) edge_chain<nd_max(e5, 0)>(E.p5, A, B, sx, sy, m1, m2, b5, c5);
         }
         if (e3 >= 0) {
-            bd3 += dp * E.p3[0];
-            if (G::d5 >= 1) edge_chain<nd_max(e3, 0)>(E.p3, A, B, tx, ty, n1, n2, b3, c3);
+            bd3 += ds * E.p3[0];
+            if (G::d5 >= 1) edge_chain<nd_max(e3, 0)>(E.p3, A, B, sx, sy, m1, m2, b3, c3);
         }
         if (e1 >= 0) {
-            bd1 += dp * E.p1[0];
-            if (G::d3 >= 1) edge_chain<nd_max(e1, 0)>(E.p1, A, B, tx, ty, n1, n2, b1, c1v);
+            bd1 += ds * E.p1[0];
+            if (G::d3 >= 1) edge_chain<nd_max(e1, 0)>(E.p1, A, B, sx, sy, m1, m2, b1, c1v);
         }
         if (em1 >= 0) {
-            bdm += dp * E.pm1[0];
-            if (G::d1 >= 1) edge_chain<nd_max(em1, 0)>(E.pm1, A, B, tx, ty, n1, n2, bm, cm);
+            bdm += ds * E.pm1[0];
+            if (G::d1 >= 1) edge_chain<nd_max(em1, 0)>(E.pm1, A, B, sx, sy, m1, m2, bm, cm);
         }
     }
     const double ih2 = ih * ih;
@@ -494,19 +543,6 @@ __device__ __forceinline__ void lam_at_foot(const NodalRec& g, const NodalObs& o
 #pragma unroll
     for (int i = 0; i < 3; i++) l[i] = (g.abc[i][0] + o.X1 * g.abc[i][1]) + o.X2 * g.abc[i][2];
 }
-template <int P>
-__device__ __forceinline__ void shape_values(double l0, double l1, double l2, double N[nd_nodes(P)]) {
-    if (P == 0) {
-        N[0] = 1.0;
-    } else if (P == 1) {
-        N[0] = l0; N[1] = l1; N[2] = l2;
-    } else {
-        N[0] = l0 * (2.0 * l0 - 1.0); N[1] = l1 * (2.0 * l1 - 1.0); N[2] = l2 * (2.0 * l2 - 1.0);
-        const double q = 4.0 * l1;
-        N[3] = q * l0; N[4] = q * l2; N[5] = 4.0 * l2 * l0;
-    }
-}
-
 // W[a,b] (a + b <= D) = sum over monomials C[ap,bp] M[a + ap, b + bp]
 template <int P, int D>
 __device__ __forceinline__ void weight_moments(const double* M, const double* C, double* W) {
@@ -657,83 +693,110 @@ __device__ __forceinline__ void kelvin_six(const double* m3, const double* m5, d
 }
 
 // ---------------------------------------------------------------------------
-// far quadrature: fn(xi1, xi2, eta1, eta2, R^2, w, lam) at every point
+// far quadrature: fn(xi1, xi2, R^2, q) at every point q; sums are times 2 area
 // ---------------------------------------------------------------------------
 template <class Fn>
-__device__ __forceinline__ void far_points(const NodalRec& g, const NodalObs& o, int n, Fn&& fn) {
-    const int off = nd_far_off(n);
+__device__ __forceinline__ void far_points(const NodalRec& g, const NodalObs& o, int rule, Fn&& fn) {
     const double e1x = g.p2[1][0] - g.p2[0][0], e1y = g.p2[1][1] - g.p2[0][1];
     const double e2x = g.p2[2][0] - g.p2[0][0], e2y = g.p2[2][1] - g.p2[0][1];
+    const double ox = g.p2[0][0] - o.X1, oy = g.p2[0][1] - o.X2;
+    const int q1 = nd_far_last(rule);
 #pragma unroll 1
-    for (int i = 0; i < n; i++) {
-        const double gi = MBEM_ND_RULES.fx[off + i], r = 1.0 - gi;
-        const double wi = MBEM_ND_RULES.fw[off + i] * r * g.area2;
-        const double ax = g.p2[0][0] + gi * e1x, ay = g.p2[0][1] + gi * e1y;
-        const double bx = r * e2x, by = r * e2y;
-#pragma unroll 1
-        for (int j = 0; j < n; j++) {
-            const double gj = MBEM_ND_RULES.fx[off + j];
-            const double eta1 = ax + gj * bx, eta2 = ay + gj * by;
-            const double xi1 = eta1 - o.X1, xi2 = eta2 - o.X2;
-            const double R2 = xi1 * xi1 + xi2 * xi2 + o.h2;
-            const double l2 = gj * r;
-            fn(xi1, xi2, eta1, eta2, R2, wi * MBEM_ND_RULES.fw[off + j], r - l2, gi, l2);
-        }
+    for (int q = nd_far_first(rule); q < q1; q++) {
+        const double l1 = MBEM_ND_RULES.fl[q][0], l2 = MBEM_ND_RULES.fl[q][1];
+        const double xi1 = ox + l1 * e1x + l2 * e2x, xi2 = oy + l1 * e1y + l2 * e2y;
+        fn(xi1, xi2, xi1 * xi1 + xi2 * xi2 + o.h2, q);
     }
+}
+// weight of point q, and times the shape function of node k
+__device__ __forceinline__ double far_w(int q) { return MBEM_ND_RULES.fl[q][2]; }
+template <int P>
+__device__ __forceinline__ double far_wn(int q, int k) {
+    return P == 0 ? MBEM_ND_RULES.fl[q][2] : MBEM_ND_RULES.fn[q][(P == 2 ? 3 : 0) + k];
 }
 
 // ---------------------------------------------------------------------------
 // matrix blocks: put(k, G) receives node k's 3 x 3 block (global frame)
 // ---------------------------------------------------------------------------
+// T block (source frame) of one moment set and any normal
+__device__ __forceinline__ void t_general(const double* W3, const double* W5, double z, const NodalRec& g,
+                                          const TCoef& c, double T[3][3]) {
+    double col[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) col[j][0] = col[j][1] = col[j][2] = 0.0;
+    t_local_col<0>(W3, W5, z, g.eps2, c, g.nl, col[0]);
+    t_local_col<1>(W3, W5, z, g.eps2, c, g.nl, col[1]);
+    t_local_col<2>(W3, W5, z, g.eps2, c, g.nl, col[2]);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) T[i][j] = col[j][i];
+}
+
+// The far T blocks of a normal off the frame's.
+template <int P, class Put>
+__device__ __noinline__ void far_t_general(const NodalRec& g, const double* x, const TCoef& c, Put&& put) {
+    constexpr int K = nd_nodes(P);
+    const NodalObs o = nodal_obs(g, x);
+    double W3[K][3], W5[K][10];
+    for (int k = 0; k < K; k++) {
+        for (int t = 0; t < 3; t++) W3[k][t] = 0.0;
+        for (int t = 0; t < 10; t++) W5[k][t] = 0.0;
+    }
+    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        const double iR = rsqrt(R2), iR2 = iR * iR;
+        const double a = iR * iR2, b = a * iR2;
+        const double x11 = xi1 * xi1, x22 = xi2 * xi2;
+        const double p[10] = {1.0, xi1, xi2, x11, xi1 * xi2, x22, x11 * xi1, x11 * xi2, x22 * xi1, x22 * xi2};
+        for (int k = 0; k < K; k++) {
+            const double w = g.area2 * far_wn<P>(q, k), wa = w * a, wb = w * b;
+            for (int t = 0; t < 3; t++) W3[k][t] += wa * p[t];
+            for (int t = 0; t < 10; t++) W5[k][t] += wb * p[t];
+        }
+    });
+    for (int k = 0; k < K; k++) {
+        double T[3][3], G[3][3];
+        t_general(W3[k], W5[k], o.z, g, c, T);
+        rotate_full(g, T, G);
+        put(k, G);
+    }
+}
+
 template <int P, class Put>
 __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x, const TCoef& c, Put&& put) {
     constexpr int K = nd_nodes(P);
     const NodalObs o = nodal_obs(g, x);
     const double z = o.z;
     if (nodal_is_far(g, o)) {
-        double acc[K][3][3];
+        if (!g.aligned) {
+            far_t_general<P>(g, x, c, put);
+            return;
+        }
+        // per node: n = 3 and n = 5 to degree 2 but (0, 2), which (2, 0) leaves of I3 - h^2 I5
+        double acc[K][8];
 #pragma unroll
         for (int k = 0; k < K; k++)
 #pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) acc[k][i][j] = 0.0;
-        const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
-        const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double, double, double R2, double w,
-                                                      double l0, double l1, double l2) {
+            for (int t = 0; t < 8; t++) acc[k][t] = 0.0;
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double a = w * iR * iR2, b = a * iR2;
-            const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
-            const double d0 = -xi1, d1 = -xi2;
-            const double dn = d0 * n0 + d1 * n1 + z * n2;
-            const double wn = c.w6 * b * dn, gam = pb * dn;
-            const double w0 = wn * d0, w1 = wn * d1, wz = wn * z;
-            const double a0 = pa * d0, a1 = pa * d1, az = pa * z, b0 = pb * d0, b1 = pb * d1, bz = pb * z;
-            double B[3][3];
-            B[0][0] = w0 * d0 + gam + n0 * (a0 + b0);
-            B[1][1] = w1 * d1 + gam + n1 * (a1 + b1);
-            B[2][2] = wz * z + gam + n2 * (az + bz);
-            const double w01 = w0 * d1, w02 = w0 * z, w12 = w1 * z;
-            B[0][1] = w01 + n1 * a0 + n0 * b1;
-            B[1][0] = w01 + n0 * a1 + n1 * b0;
-            B[0][2] = w02 + n2 * a0 + n0 * bz;
-            B[2][0] = w02 + n0 * az + n2 * b0;
-            B[1][2] = w12 + n2 * a1 + n1 * bz;
-            B[2][1] = w12 + n1 * az + n2 * b1;
-            double N[K];
-            shape_values<P>(l0, l1, l2, N);
+            const double a = iR * iR2, b = a * iR2;
+            const double b1 = b * xi1, b2 = b * xi2;
+            const double p[8] = {a, a * xi1, a * xi2, b, b1, b2, b1 * xi1, b1 * xi2};
 #pragma unroll
-            for (int k = 0; k < K; k++)
+            for (int k = 0; k < K; k++) {
+                const double w = far_wn<P>(q, k);
 #pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int j = 0; j < 3; j++) acc[k][i][j] += N[k] * B[i][j];
+                for (int t = 0; t < 8; t++) acc[k][t] += w * p[t];
+            }
         });
 #pragma unroll
         for (int k = 0; k < K; k++) {
-            double G[3][3];
-            rotate_full(g, acc[k], G);
+            const double* m = acc[k];
+            double T[3][3], G[3][3];
+            t_local(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[0] - o.h2 * m[3] - m[6], z, g.eps2, c,
+                    g.s * g.area2, T);
+            rotate_full(g, T, G);
             put(k, G);
         }
         return;
@@ -743,16 +806,8 @@ __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x,
         node_tables<P, NF_TG>(g, x, W);
 #pragma unroll 1
         for (int k = 0; k < K; k++) {
-            double col[3][3], T[3][3], G[3][3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) col[j][0] = col[j][1] = col[j][2] = 0.0;
-            t_local_col<0>(W.w3[k], W.w5[k], z, g.eps2, c, g.nl, col[0]);
-            t_local_col<1>(W.w3[k], W.w5[k], z, g.eps2, c, g.nl, col[1]);
-            t_local_col<2>(W.w3[k], W.w5[k], z, g.eps2, c, g.nl, col[2]);
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) T[i][j] = col[j][i];
+            double T[3][3], G[3][3];
+            t_general(W.w3[k], W.w5[k], z, g, c, T);
             rotate_full(g, T, G);
             put(k, G);
         }
@@ -809,25 +864,16 @@ __device__ __forceinline__ void pair_t_basis(const NodalRec& g, const double* x,
             for (int t = 0; t < 3; t++) W3[k][t] = 0.0;
             for (int t = 0; t < 10; t++) W5[k][t] = 0.0;
         }
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double, double, double R2, double w,
-                                                      double l0, double l1, double l2) {
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double a = w * iR * iR2, b = a * iR2;
-            double N[K], x1p[4], x2p[4];
-            shape_values<P>(l0, l1, l2, N);
-            x1p[0] = x2p[0] = 1.0;
-            for (int t = 1; t < 4; t++) {
-                x1p[t] = x1p[t - 1] * xi1;
-                x2p[t] = x2p[t - 1] * xi2;
+            const double a = iR * iR2, b = a * iR2;
+            const double x11 = xi1 * xi1, x22 = xi2 * xi2;
+            const double p[10] = {1.0, xi1, xi2, x11, xi1 * xi2, x22, x11 * xi1, x11 * xi2, x22 * xi1, x22 * xi2};
+            for (int k = 0; k < K; k++) {
+                const double w = g.area2 * far_wn<P>(q, k), wa = w * a, wb = w * b;
+                for (int t = 0; t < 3; t++) W3[k][t] += wa * p[t];
+                for (int t = 0; t < 10; t++) W5[k][t] += wb * p[t];
             }
-            for (int q = 0; q <= 3; q++)
-                for (int t = 0; t <= q; t++) {
-                    const double f = b * x1p[q - t] * x2p[t], f3 = a * x1p[q - t] * x2p[t];
-                    for (int k = 0; k < K; k++) {
-                        W5[k][nd_tri(q - t, t)] += f * N[k];
-                        if (q <= 1) W3[k][nd_tri(q - t, t)] += f3 * N[k];
-                    }
-                }
         });
     } else {
         NMom<P, NF_TG> M;
@@ -871,26 +917,28 @@ __device__ __forceinline__ void pair_u(const NodalRec& g, const double* x, doubl
         for (int k = 0; k < K; k++)
 #pragma unroll
             for (int t = 0; t < 8; t++) A[k][t] = 0.0;
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double, double, double R2, double w,
-                                                      double l0, double l1, double l2) {
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double f = w * iR, a = f * iR2;
+            const double a = iR * iR2;
             const double v0 = a * xi1, v1 = a * xi2;
-            const double p[7] = {f, a, v0, v1, v0 * xi1, v0 * xi2, v1 * xi2};
-            double N[K];
-            shape_values<P>(l0, l1, l2, N);
+            // (0, 2) is what (2, 0) leaves of I1 - h^2 I3
+            const double p[6] = {iR, a, v0, v1, v0 * xi1, v0 * xi2};
 #pragma unroll
-            for (int k = 0; k < K; k++)
+            for (int k = 0; k < K; k++) {
+                const double w = far_wn<P>(q, k);
 #pragma unroll
-                for (int t = 0; t < 7; t++) A[k][t] += N[k] * p[t];
+                for (int t = 0; t < 6; t++) A[k][t] += w * p[t];
+            }
         });
+        const double f = c2 * g.area2;
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const double* p = A[k];
-            const double L[6] = {c2 * p[4], c2 * p[6], c2 * (z * z) * p[1], c2 * p[5], -c2 * z * p[2], -c2 * z * p[3]};
+            const double L[6] = {f * p[4], f * (p[0] - o.h2 * p[1] - p[4]), f * (z * z) * p[1],
+                                 f * p[5], -f * z * p[2],                    -f * z * p[3]};
             double G[6];
             rotate_six(g, L, G);
-            put(k, p[0], p[1], G);
+            put(k, g.area2 * p[0], g.area2 * p[1], G);
         }
         return;
     }
@@ -986,6 +1034,31 @@ __device__ __forceinline__ double den_value(const double* f, double e1, double e
     return f[0] + e1 * (f[1] + f[3] * e1 + f[4] * e2) + e2 * (f[2] + f[5] * e2);
 }
 
+// far displacement of a slip density on a normal off the frame's (source frame)
+template <int P>
+__device__ __noinline__ void far_t_contract_general(const NodalRec& g, const NodalDen<P>& D, const double* x,
+                                                    const TCoef& c, double v[3]) {
+    const NodalObs o = nodal_obs(g, x);
+    const double z = o.z, c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
+    const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
+    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
+        const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
+                     u2 = den_value<P>(D.f[2], e1, e2);
+        const double iR = rsqrt(R2), iR2 = iR * iR;
+        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2;
+        const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
+        const double d0 = -xi1, d1 = -xi2;
+        const double dn = d0 * n0 + d1 * n1 + z * n2, du = d0 * u0 + d1 * u1 + z * u2;
+        const double un = u0 * n0 + u1 * n1 + u2 * n2;
+        // (n.u) pa d + n pb (d.u) - 6 c5 b (d.n)(d.u) d + pb (d.n) u
+        const double s = un * pa + c.w6 * b * dn * du, t = pb * du, r = pb * dn;
+        v[0] += s * d0 + t * n0 + r * u0;
+        v[1] += s * d1 + t * n1 + r * u1;
+        v[2] += s * z + t * n2 + r * u2;
+    });
+}
+
 // displacement of a slip density, added to acc (global)
 template <int P>
 __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDen<P>& D, const double* x,
@@ -994,24 +1067,34 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
     const double z = o.z;
     double v[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
-        const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double e1, double e2, double R2,
-                                                      double w, double, double, double) {
-            const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
-                         u2 = den_value<P>(D.f[2], e1, e2);
-            const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double a = w * iR * iR2, b = a * iR2;
-            const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
-            const double d0 = -xi1, d1 = -xi2;
-            const double dn = d0 * n0 + d1 * n1 + z * n2, du = d0 * u0 + d1 * u1 + z * u2;
-            const double un = u0 * n0 + u1 * n1 + u2 * n2;
-            // (n.u) pa d + n pb (d.u) - 6 c5 b (d.n)(d.u) d + pb (d.n) u
-            const double s = un * pa + c.w6 * b * dn * du, t = pb * du, q = pb * dn;
-            v[0] += s * d0 + t * n0 + q * u0;
-            v[1] += s * d1 + t * n1 + q * u1;
-            v[2] += s * z + t * n2 + q * u2;
-        });
+        if (!g.aligned) {
+            far_t_contract_general<P>(g, D, x, c, v);
+        } else {
+            // normal s e3: s [ q d + pb z u + e3 sum pb (d.u) ], q = pa u3 + w6 z b (d.u)
+            const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2, wz = c.w6 * z;
+            double s0 = 0.0, s1 = 0.0, sq = 0.0, sd = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
+            far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+                const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
+                const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
+                             u2 = den_value<P>(D.f[2], e1, e2);
+                const double iR = rsqrt(R2), iR2 = iR * iR;
+                const double a = far_w(q) * iR * iR2, b = a * iR2;
+                const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
+                const double du = z * u2 - (xi1 * u0 + xi2 * u1);
+                const double r = pa * u2 + (wz * b) * du;
+                s0 += r * xi1;
+                s1 += r * xi2;
+                sq += r;
+                sd += pb * du;
+                t0 += pb * u0;
+                t1 += pb * u1;
+                t2 += pb * u2;
+            });
+            const double sa = g.s * g.area2;
+            v[0] = sa * (z * t0 - s0);
+            v[1] = sa * (z * t1 - s1);
+            v[2] = sa * (z * (t2 + sq) + sd);
+        }
     } else if (!g.aligned || node_by_node<P>(g)) {
         NodeTab<P> W;
         node_tables<P, NF_TG>(g, x, W);
@@ -1059,18 +1142,19 @@ __device__ __forceinline__ void pair_u_contract(const NodalRec& g, const NodalDe
     const double ce = c[1] * g.eps2;
     double v[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double e1, double e2, double R2,
-                                                      double w, double, double, double) {
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+            const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
             const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
                          u2 = den_value<P>(D.f[2], e1, e2);
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double f = w * iR, a = f * iR2;
-            const double d0 = -xi1, d1 = -xi2;
-            const double dg = c[0] * f + ce * a, s = c[2] * a * (d0 * u0 + d1 * u1 + z * u2);
-            v[0] += dg * u0 + s * d0;
-            v[1] += dg * u1 + s * d1;
-            v[2] += dg * u2 + s * z;
+            const double f = far_w(q) * iR, a = f * iR2;
+            const double dg = c[0] * f + ce * a, s = a * (z * u2 - (xi1 * u0 + xi2 * u1));
+            v[0] += dg * u0 - (c[2] * s) * xi1;
+            v[1] += dg * u1 - (c[2] * s) * xi2;
+            v[2] += dg * u2 + (c[2] * s) * z;
         });
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i] *= g.area2;
     } else if (node_by_node<P>(g)) {
         NodeTab<P> W;
         node_tables<P, NF_U>(g, x, W);
@@ -1103,6 +1187,144 @@ __device__ __forceinline__ void pair_u_contract(const NodalRec& g, const NodalDe
     for (int i = 0; i < 3; i++) acc[i] += g.ex[i] * v[0] + g.ey[i] * v[1] + g.nh[i] * v[2];
 }
 
+// eigenstress phi C : sym(s n) of I7 = int s / R^7 (source frame)
+__device__ __forceinline__ void eig_six(const SMat& m, double eps2, const double nl[3], const double I7[3],
+                                        double e[6]) {
+    const double phi = m.phi * eps2 * eps2;
+    const double un = nl[0] * I7[0] + nl[1] * I7[1] + nl[2] * I7[2];
+    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int t = 0; t < 6; t++) {
+        const int i = ia[t], j = ib[t];
+        e[t] = phi * ((i == j ? m.lam * un : 0.0) + m.mu * (I7[i] * nl[j] + nl[i] * I7[j]));
+    }
+}
+
+// Far DD stress and I7 = int u / R^7 for the normal s e3 (source frame): with a,
+// b, c = w / R^3, 5, 7, d = (-xi, z) and |d|^2 = R^2 - eps^2 every term is one of
+// f d d (f as below), G (z u + (d.u) e3) d, A u, and scalars in u3 and d.u, so the
+// sums are of those and the stress is formed once.
+template <int P>
+__device__ __forceinline__ void far_dd_frame(const NodalRec& g, const NodalDen<P>& D, const NodalObs& o, const SMat& m,
+                                             double v[6], double I7[3]) {
+    const double z = o.z, e = g.eps2, cb = m.blob * e, c15 = 15.0 * cb, ce = 15.0 * (cb - e);
+    const double lam = m.lam, mu = m.mu, xt = m.x1 + 15.0;
+    // f = u3 (kb b + kc c) + kd c (d.u)
+    const double kb = 2.0 * lam * xt - 12.0 * mu, kc = 2.0 * lam * ce, kd = 60.0 * mu * z;
+    double S00 = 0, S01 = 0, S11 = 0, f0s = 0, f1s = 0, fs = 0, au[3] = {0, 0, 0}, bu[3] = {0, 0, 0}, cu[3] = {0, 0, 0};
+    double bd = 0, cd = 0, V0 = 0, V1 = 0, W0[3] = {0, 0, 0}, W1[3] = {0, 0, 0};
+    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
+        const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
+        const double iR = rsqrt(R2), iR2 = iR * iR;
+        const double a = far_w(q) * iR * iR2, b = a * iR2, c = b * iR2;
+        const double du = z * u[2] - (xi1 * u[0] + xi2 * u[1]);
+        const double bq = b * du, cq = c * du;
+        const double f = u[2] * (kb * b + kc * c) + kd * cq;
+        const double f0 = f * xi1, f1 = f * xi2;
+        S00 += f0 * xi1;
+        S01 += f0 * xi2;
+        S11 += f1 * xi2;
+        f0s += f0;
+        f1s += f1;
+        fs += f;
+        bd += bq;
+        cd += cq;
+        const double ge = m.k3a * bq + c15 * cq, G = m.k3a * b + c15 * c;
+        V0 += ge * xi1;
+        V1 += ge * xi2;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            au[i] += a * u[i];
+            bu[i] += b * u[i];
+            cu[i] += c * u[i];
+            const double gu = G * u[i];
+            W0[i] += gu * xi1;
+            W1[i] += gu * xi2;
+        }
+    });
+    const double A0 = 1.0 - m.c34, B0 = 3.0 * (e - cb), l2 = 2.0 * lam, m2 = 2.0 * mu;
+    // lam tr Bs + the delta part of Bs + Bs^T, over C1
+    const double ka = lam * lam * (3.0 * A0 + xt) + 2.0 * lam * mu * A0 + mu * (l2 * A0 + 2.0 * m2);
+    const double kb3 = lam * lam * (3.0 * B0 - e * xt + ce) + lam * mu * 6.0 * (e - cb) + mu * l2 * B0;
+    const double kc3 = -lam * lam * e * ce;
+    const double pb = lam * mu * (12.0 + 2.0 * m.k3a) - 6.0 * mu * m2, pc = 2.0 * lam * mu * ce;
+    const double su = ka * au[2] + kb3 * bu[2] + kc3 * cu[2] + z * (pb * bd + pc * cd);
+    // Q = A u; W[j] = sum G d_j u (times z below), V = sum G (d.u) d
+    double Q[3], W2[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        Q[i] = A0 * au[i] - 3.0 * cb * bu[i];
+        W2[i] = z * (m.k3a * bu[i] + c15 * cu[i]);
+        W0[i] = -W0[i];
+        W1[i] = -W1[i];
+    }
+    const double V2 = z * (m.k3a * bd + c15 * cd);
+    const double s = -m.C1 * g.s * g.area2;
+    v[0] = s * (mu * (S00 + mu * (2.0 * z * W0[0])) + su);
+    v[1] = s * (mu * (S11 + mu * (2.0 * z * W1[1])) + su);
+    v[2] = s * (mu * (z * z * fs + mu * (4.0 * Q[2] + 2.0 * (z * W2[2] + V2))) + su);
+    v[3] = s * mu * (S01 + mu * z * (W0[1] + W1[0]));
+    v[4] = s * mu * (mu * (2.0 * Q[0] + z * (W0[2] + W2[0]) - V0) - z * f0s);
+    v[5] = s * mu * (mu * (2.0 * Q[1] + z * (W1[2] + W2[1]) - V1) - z * f1s);
+#pragma unroll
+    for (int i = 0; i < 3; i++) I7[i] = g.area2 * cu[i];
+}
+
+// the same for any normal
+template <int P>
+__device__ __noinline__ void far_dd_general(const NodalRec& g, const NodalDen<P>& D, const double* x, const SMat& m,
+                                            double v[6], double I7[3]) {
+    const NodalObs o = nodal_obs(g, x);
+    const double z = o.z, e2 = g.eps2;
+    const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
+    const double cb = m.blob * e2;
+    // sums of the point form: DD = e d d + g (w d + d w) + a (u n + n u) + delta s
+    double S[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, V[3] = {0.0, 0.0, 0.0}, su = 0.0, Q[3] = {0.0, 0.0, 0.0};
+    double W[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    const double l2 = 2.0 * m.lam, mu2 = 2.0 * m.mu;
+    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
+        const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
+        const double iR = rsqrt(R2), iR2 = iR * iR;
+        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2, c = b * iR2;
+        const double dd = R2 - e2;
+        const double d[3] = {-xi1, -xi2, z};
+        const double dn = d[0] * n0 + d[1] * n1 + z * n2, du = d[0] * u[0] + d[1] * u[1] + z * u[2];
+        const double un = u[0] * n0 + u[1] * n1 + u[2] * n2;
+        const double db = dd + cb;
+        const double X0 = (4.0 - m.c34) * a - 3.0 * db * b;
+        const double X1 = m.x1 * b + 15.0 * db * c;
+        const double A1 = (1.0 - m.c34) * a - 3.0 * cb * b;
+        const double p = du * dn;
+        const double S0 = 2.0 * un * a - 6.0 * p * b;
+        const double G = m.k3a * b + 15.0 * cb * c;
+        const double E = 30.0 * p * c - 6.0 * un * b;
+        const double ux = un * X1;
+        // Bs + Bs^T = delta (l2 un X0 + mu2 S0) + (l2 un X1 + mu2 E) d d + mu (2 A1 sym + G (w d + d w)), w = dn u + du n
+        const double f = l2 * ux + mu2 * E;
+        S[0] += f * d[0] * d[0]; S[1] += f * d[1] * d[1]; S[2] += f * z * z;
+        S[3] += f * d[0] * d[1]; S[4] += f * d[0] * z; S[5] += f * d[1] * z;
+        const double trX = 3.0 * (un * X0) + ux * dd;
+        const double trS = 2.0 * (A1 * un) + 3.0 * S0 + 2.0 * (G * p) + E * dd;
+        su += m.lam * (m.lam * trX + m.mu * trS) + m.mu * (l2 * (un * X0) + mu2 * S0);
+        for (int i = 0; i < 3; i++) {
+            Q[i] += A1 * u[i];
+            V[i] += G * du * d[i];
+            I7[i] += c * u[i];
+            for (int j = 0; j < 3; j++) W[i][j] += G * dn * d[i] * u[j];
+        }
+    });
+    const double nl[3] = {n0, n1, n2};
+    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
+    for (int t = 0; t < 6; t++) {
+        const int i = ia[t], j = ib[t];
+        const double sym = Q[i] * nl[j] + nl[i] * Q[j];
+        const double wd = W[i][j] + W[j][i] + V[i] * nl[j] + nl[i] * V[j];
+        v[t] = -m.C1 * (m.mu * (S[t] + m.mu * (2.0 * sym + wd)) + (i == j ? su : 0.0));
+    }
+}
+
 // stress of a slip density (DD, minus the eigenstress with EIG) added to acc (00 11 22 01 02 12, global); with
 // acc_e the eigenstress alone is added there
 template <int P>
@@ -1114,79 +1336,14 @@ __device__ __forceinline__ void pair_dd_contract(const NodalRec& g, const NodalD
     double I7[3] = {0.0, 0.0, 0.0};          // int u / R^7
     const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
     if (nodal_is_far(g, o)) {
-        const double cb = m.blob * e2;
-        const double xg = 3.0 * m.c34 - 9.0;
-        // sums of the point form: DD = e d d + g (w d + d w) + a (u n + n u) + delta s
-        double S[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, V[3] = {0.0, 0.0, 0.0}, su = 0.0;
-        double Q[3] = {0.0, 0.0, 0.0};
-        const double l2 = 2.0 * m.lam, mu2 = 2.0 * m.mu;
-        double W[3][3];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) W[i][j] = 0.0;
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double y1, double y2, double R2,
-                                                      double w, double, double, double) {
-            const double u0 = den_value<P>(D.f[0], y1, y2), u1 = den_value<P>(D.f[1], y1, y2),
-                         u2 = den_value<P>(D.f[2], y1, y2);
-            const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double a = w * iR * iR2, b = a * iR2, c = b * iR2;
-            const double dd = R2 - e2;
-            const double d0 = -xi1, d1 = -xi2;
-            const double dn = d0 * n0 + d1 * n1 + z * n2, du = d0 * u0 + d1 * u1 + z * u2;
-            const double un = u0 * n0 + u1 * n1 + u2 * n2;
-            const double db = dd + cb;
-            const double X0 = (4.0 - m.c34) * a - 3.0 * db * b;
-            const double X1 = m.x1 * b + 15.0 * db * c;
-            const double A1 = (1.0 - m.c34) * a - 3.0 * cb * b;
-            const double p = du * dn;
-            const double S0 = 2.0 * un * a - 6.0 * p * b;
-            const double G = xg * b + 15.0 * cb * c;
-            const double E = 30.0 * p * c - 6.0 * un * b;
-            const double ux = un * X1;
-            // Bs + Bs^T = delta (l2 un X0 + mu2 S0) + (l2 un X1 + mu2 E) d d + mu (2 A1 sym + G (w d + d w))
-            const double f = l2 * ux + mu2 * E;
-            const double f0 = f * d0, f1 = f * d1;
-            S[0] += f0 * d0; S[1] += f1 * d1; S[2] += (f * z) * z;
-            S[3] += f0 * d1; S[4] += f0 * z; S[5] += f1 * z;
-            // trace of Bs, and the delta part of Bs + Bs^T
-            const double trX = 3.0 * (un * X0) + ux * dd;
-            const double trS = 2.0 * (A1 * un) + 3.0 * S0 + 2.0 * (G * p) + E * dd;
-            su += m.lam * (m.lam * trX + m.mu * trS) + m.mu * (l2 * (un * X0) + mu2 * S0);
-            Q[0] += A1 * u0; Q[1] += A1 * u1; Q[2] += A1 * u2;
-            // G w d with w = dn u + du n
-            const double gd = G * dn, ge = G * du;
-            V[0] += ge * d0; V[1] += ge * d1; V[2] += ge * z;
-            const double g0 = gd * d0, g1 = gd * d1, g2 = gd * z;
-            W[0][0] += g0 * u0; W[0][1] += g0 * u1; W[0][2] += g0 * u2;
-            W[1][0] += g1 * u0; W[1][1] += g1 * u1; W[1][2] += g1 * u2;
-            W[2][0] += g2 * u0; W[2][1] += g2 * u1; W[2][2] += g2 * u2;
-            I7[0] += c * u0; I7[1] += c * u1; I7[2] += c * u2;
-        });
-        const double nl[3] = {n0, n1, n2};
-        const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-#pragma unroll
-        for (int t = 0; t < 6; t++) {
-            const int i = ia[t], j = ib[t];
-            const double sym = Q[i] * nl[j] + nl[i] * Q[j];
-            const double wd = W[i][j] + W[j][i] + V[i] * nl[j] + nl[i] * V[j];
-            v[t] = -m.C1 * (m.mu * (S[t] + m.mu * (2.0 * sym + wd)) + (i == j ? su : 0.0));
-        }
-        if (eig || acc_e) {
-            const double phi = m.phi * e2 * e2;
-            const double un = n0 * I7[0] + n1 * I7[1] + n2 * I7[2];
+        if (g.aligned) far_dd_frame<P>(g, D, o, m, v, I7);
+        else far_dd_general<P>(g, D, x, m, v, I7);
+        if (eig) {
+            const double nl[3] = {n0, n1, n2};
             double e[6];
+            eig_six(m, e2, nl, I7, e);
 #pragma unroll
-            for (int t = 0; t < 6; t++) {
-                const int i = ia[t], j = ib[t];
-                e[t] = phi * ((i == j ? m.lam * un : 0.0) + m.mu * (I7[i] * nl[j] + nl[i] * I7[j]));
-                if (eig) v[t] -= e[t];
-            }
-            if (acc_e) {
-                double G[6];
-                rotate_six(g, e, G);
-                for (int t = 0; t < 6; t++) acc_e[t] += G[t];
-            }
+            for (int t = 0; t < 6; t++) v[t] -= e[t];
         }
     } else {
         if (!g.aligned || node_by_node<P>(g)) {
@@ -1217,19 +1374,13 @@ __device__ __forceinline__ void pair_dd_contract(const NodalRec& g, const NodalD
             MBEM_ND_COL(2)
 #undef MBEM_ND_COL
         }
-        if (acc_e) {
-            const double nl[3] = {n0, n1, n2};
-            const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-            const double phi = m.phi * e2 * e2;
-            const double un = n0 * I7[0] + n1 * I7[1] + n2 * I7[2];
-            double e[6], G[6];
-            for (int t = 0; t < 6; t++) {
-                const int i = ia[t], j = ib[t];
-                e[t] = phi * ((i == j ? m.lam * un : 0.0) + m.mu * (I7[i] * nl[j] + nl[i] * I7[j]));
-            }
-            rotate_six(g, e, G);
-            for (int t = 0; t < 6; t++) acc_e[t] += G[t];
-        }
+    }
+    if (acc_e) {
+        const double nl[3] = {n0, n1, n2};
+        double e[6], G[6];
+        eig_six(m, e2, nl, I7, e);
+        rotate_six(g, e, G);
+        for (int t = 0; t < 6; t++) acc_e[t] += G[t];
     }
     double G[6];
     rotate_six(g, v, G);
@@ -1244,13 +1395,15 @@ __device__ __forceinline__ void pair_eig_contract(const NodalRec& g, const Nodal
     const NodalObs o = nodal_obs(g, x);
     double I7[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double, double, double y1, double y2, double R2, double w,
-                                                      double, double, double) {
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+            const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double c = w * iR * (iR2 * iR2) * iR2;
+            const double c = far_w(q) * iR * (iR2 * iR2) * iR2;
 #pragma unroll
             for (int j = 0; j < 3; j++) I7[j] += c * den_value<P>(D.f[j], y1, y2);
         });
+#pragma unroll
+        for (int j = 0; j < 3; j++) I7[j] *= g.area2;
     } else if (node_by_node<P>(g)) {
         NodeTab<P> W;
         node_tables<P, NF_E>(g, x, W);
@@ -1268,15 +1421,8 @@ __device__ __forceinline__ void pair_eig_contract(const NodalRec& g, const Nodal
             weight_moments<P, 0>(M.m7, C, &I7[j]);
         }
     }
-    const double phi = m.phi * g.eps2 * g.eps2;
-    const double un = g.nl[0] * I7[0] + g.nl[1] * I7[1] + g.nl[2] * I7[2];
-    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
     double e[6], G[6];
-#pragma unroll
-    for (int t = 0; t < 6; t++) {
-        const int i = ia[t], j = ib[t];
-        e[t] = phi * ((i == j ? m.lam * un : 0.0) + m.mu * (I7[i] * g.nl[j] + g.nl[i] * I7[j]));
-    }
+    eig_six(m, g.eps2, g.nl, I7, e);
     rotate_six(g, e, G);
 #pragma unroll
     for (int t = 0; t < 6; t++) acc[t] += G[t];
@@ -1293,10 +1439,10 @@ __device__ __forceinline__ void far_s_moments(const NodalRec& g, const NodalObs&
 #pragma unroll
         for (int t = 0; t < 10; t++) W5[j][t] = 0.0;
     }
-    far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double y1, double y2, double R2, double w,
-                                                  double, double, double) {
+    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
         const double iR = rsqrt(R2), iR2 = iR * iR;
-        const double a = w * iR * iR2, b = a * iR2;
+        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2;
         const double x11 = xi1 * xi1, x12 = xi1 * xi2, x22 = xi2 * xi2;
         const double p[10] = {1.0, xi1, xi2, x11, x12, x22, x11 * xi1, x11 * xi2, x22 * xi1, x22 * xi2};
 #pragma unroll
@@ -1411,12 +1557,9 @@ __device__ __forceinline__ void pair_traction_fam(const NodalRec& g, const doubl
 #pragma unroll
             for (int t = 0; t < 15; t++) W7[k][t] = 0.0;
         }
-        far_points(g, o, nd_far_n<P>(o.D2, g.L2), [&](double xi1, double xi2, double, double, double R2, double w,
-                                                      double l0, double l1, double l2) {
+        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q0) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double a = w * iR * iR2, b = a * iR2, c = b * iR2;
-            double N[K];
-            shape_values<P>(l0, l1, l2, N);
+            const double a = iR * iR2, b = a * iR2, c = b * iR2;
             double p[15];
             p[0] = 1.0; p[1] = xi1; p[2] = xi2;
 #pragma unroll
@@ -1427,7 +1570,8 @@ __device__ __forceinline__ void pair_traction_fam(const NodalRec& g, const doubl
             }
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                const double na = N[k] * a, nb = N[k] * b, nc = N[k] * c;
+                const double w = g.area2 * far_wn<P>(q0, k);
+                const double na = w * a, nb = w * b, nc = w * c;
                 if (F != NF_E) {
                     W3[k][0] += na;
 #pragma unroll
