@@ -2,7 +2,7 @@
 // independent Krylov iterations that share one tensor-core GEMM per step),
 // the BF16 copy of the operator that GEMM reads, and the FP64-accurate
 // residual R = B - A X of the mixed operator for a block of right-hand sides
-// (FP32 far field with double-float accumulation, FP64 near blocks).
+// (FP32 far field by exact digit products, tc_exact.cu; FP64 near blocks).
 //
 // Vectors of a block are RHS-major: (k, n) row-major, one row per right-hand
 // side, so a row is one solve's vector and the GEMM's K-major operand is a
@@ -198,87 +198,18 @@ batch_project_kernel(T* __restrict__ X, int64_t n, URanges ur) {
 }
 
 // ---------------------------------------------------------------------------
-// R = B - A X for a block: FP32 far field with double-float accumulation,
+// R = B - A X for a block: the exact far-field product (tc_exact.cu), then the
 // FP64 near blocks
 // ---------------------------------------------------------------------------
-constexpr int DF_ROWS = 64, DF_RHS = 64, DF_K = 16;
-
-__device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float p) {
-    const float t = __fadd_rn(hi, p);
-    const float bp = __fsub_rn(t, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, bp)), __fsub_rn(p, bp));
-    hi = t;
-    lo = __fadd_rn(lo, e);
-}
-
-// Y[r, row] = sum_j A32[row, j] X[r, j]: a block per (64 rows, 64 RHS), a
-// thread per (4 rows, 4 RHS); every product a x_hi exact (TwoProd), a x_lo
-// rounded, sums in hi/lo pairs
+// R[r, row] -= (near X[r])[row]; a thread per (r, row)
 __global__ void __launch_bounds__(BT)
-df_gemm_kernel(const float* __restrict__ A, int64_t lda, int64_t n_rows, int64_t n_cols,
-               const double* __restrict__ X, int64_t k, double* __restrict__ Y) {
-    __shared__ float As[DF_K][DF_ROWS + 4];
-    __shared__ float Xh[DF_K][DF_RHS + 4], Xl[DF_K][DF_RHS + 4];
-    const int64_t row0 = (int64_t)blockIdx.x * DF_ROWS, rhs0 = (int64_t)blockIdx.y * DF_RHS;
-    const int tr = threadIdx.x % 16, tc = threadIdx.x / 16;    // rows tr + 16a, RHS tc + 16b
-    float hi[4][4], lo[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) hi[a][b] = lo[a][b] = 0.0f;
-    for (int64_t j0 = 0; j0 < n_cols; j0 += DF_K) {
-        for (int e = threadIdx.x; e < DF_ROWS * DF_K; e += BT) {
-            const int i = e / DF_K, j = e % DF_K;      // i: row (and RHS) within the tile, j: column
-            const int64_t gr = row0 + i, gc = j0 + j;
-            As[j][i] = (gr < n_rows && gc < n_cols) ? A[gr * lda + gc] : 0.0f;
-            const int64_t rr = rhs0 + i;
-            const double xv = (rr < k && gc < n_cols) ? X[rr * n_cols + gc] : 0.0;
-            const float xh = (float)xv;
-            Xh[j][i] = xh;
-            Xl[j][i] = (float)(xv - (double)xh);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int j = 0; j < DF_K; j++) {
-            float av[4], xh[4], xl[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) av[a] = As[j][tr + 16 * a];
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                xh[b] = Xh[j][tc + 16 * b];
-                xl[b] = Xl[j][tc + 16 * b];
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const float p = __fmul_rn(av[a], xh[b]);
-                    const float err = __fmaf_rn(av[a], xh[b], -p);
-                    two_sum_acc(hi[a][b], lo[a][b], p);
-                    lo[a][b] = __fadd_rn(lo[a][b], __fmaf_rn(av[a], xl[b], err));
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int64_t gr = row0 + tr + 16 * a, rr = rhs0 + tc + 16 * b;
-            if (gr < n_rows && rr < k) Y[rr * n_rows + gr] = (double)hi[a][b] + (double)lo[a][b];
-        }
-}
-
-// R[r, row] = B[r, row] - Y[r, row] - (near X[r])[row]; a thread per (r, row)
-__global__ void __launch_bounds__(BT)
-residual_near_kernel(const double* __restrict__ B, const double* __restrict__ Yfar, const double* __restrict__ X,
-                     int64_t k, int64_t n, mbem_near_blocks nb, int first, double* __restrict__ R) {
+residual_near_kernel(const double* __restrict__ X, int64_t k, int64_t n, mbem_near_blocks nb, double* __restrict__ R) {
     const int64_t r = blockIdx.y;
     const int64_t row = (int64_t)blockIdx.x * BT + threadIdx.x;
     if (row >= n) return;
-    double v = first ? B[r * n + row] - Yfar[r * n + row] : R[r * n + row];
     const int64_t lr = row - nb.row0;
     if (lr >= 0 && lr < 3 * nb.n_field) {
+        double v = R[r * n + row];
         const int64_t f = lr / 3;
         const int a = (int)(lr % 3);
         const double* x = X + r * n;
@@ -287,8 +218,8 @@ residual_near_kernel(const double* __restrict__ B, const double* __restrict__ Yf
             const double* blk = nb.vals + 9 * q + 3 * a;
             v -= blk[0] * x[c0] + blk[1] * x[c0 + 1] + blk[2] * x[c0 + 2];
         }
+        R[r * n + row] = v;
     }
-    R[r * n + row] = v;
 }
 
 static int ranges_of(const int64_t* u_ranges, int n_u, URanges& ur) { return make_ranges(u_ranges, n_u, ur); }
@@ -414,7 +345,9 @@ int mbem_batch_project(void* X, int is_f64, int64_t k, int64_t n, const int64_t*
     return launch_status("batch_project_kernel");
 }
 
-size_t mbem_batch_residual_workspace_size(int64_t k, int64_t n) { return (size_t)k * n * sizeof(double); }
+size_t mbem_batch_residual_workspace_size(int64_t k, int64_t n) {
+    return k < 1 || n < 1 ? 0 : exact_residual_workspace(k, n);
+}
 
 int mbem_batch_residual_mixed(const mbem_mixed_operator* op, const double* B, const double* X, int64_t k, double* R,
                               void* work, size_t work_bytes, void* stream) {
@@ -423,21 +356,13 @@ int mbem_batch_residual_mixed(const mbem_mixed_operator* op, const double* B, co
     const int64_t n = op->n_rows;
     MBEM_REQUIRE(work && work_bytes >= mbem_batch_residual_workspace_size(k, n), MBEM_ERR_SIZE,
                  "batched residual workspace too small");
+    if (n == 0) return MBEM_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    double* Y = static_cast<double*>(work);
-    df_gemm_kernel<<<dim3((unsigned)ceil_div(n, DF_ROWS), (unsigned)ceil_div(k, DF_RHS)), BT, 0, st>>>(
-        op->A32, op->ld32, n, n, X, k, Y);
-    int e = launch_status("df_gemm_kernel");
+    int e = exact_residual(op->A32, op->ld32, n, B, X, k, R, work, work_bytes, st);
     if (e) return e;
     const dim3 grid((unsigned)ceil_div(n, BT), (unsigned)k);
-    if (op->n_near == 0) {
-        mbem_near_blocks none;
-        memset(&none, 0, sizeof(none));
-        residual_near_kernel<<<grid, BT, 0, st>>>(B, Y, X, k, n, none, 1, R);
-        return launch_status("residual_near_kernel");
-    }
     for (int t = 0; t < op->n_near; t++) {
-        residual_near_kernel<<<grid, BT, 0, st>>>(B, Y, X, k, n, op->near[t], t == 0, R);
+        residual_near_kernel<<<grid, BT, 0, st>>>(X, k, n, op->near[t], R);
         if ((e = launch_status("residual_near_kernel"))) return e;
     }
     return MBEM_OK;
