@@ -343,7 +343,9 @@ int tc_gemm_check(cudaStream_t st) {
 }
 
 static int gemm_bf16(const void* A, int64_t lda, const void* Xt, int64_t ldx, int64_t M, int64_t K, int n_rhs,
-                     float* Y, int64_t ldy, bool trans, float* work, size_t work_bytes, cudaStream_t st) {
+                     float* Y, int64_t ldy, bool trans, float* work, size_t work_bytes, cudaStream_t st,
+                     int* parts = nullptr) {
+    // parts: the partial sums stay in the workspace, their number goes there
     MBEM_REQUIRE(M >= 0 && K >= 1 && n_rhs >= 1 && n_rhs <= 256, MBEM_ERR_ARG,
                  "bad GEMM sizes (M=%lld, K=%lld, n_rhs=%d; n_rhs <= 256)", (long long)M, (long long)K, n_rhs);
     MBEM_REQUIRE(A && Xt && Y && lda >= K && ldx >= K && ldy >= (trans ? M : n_rhs), MBEM_ERR_ARG,
@@ -371,6 +373,10 @@ static int gemm_bf16(const void* A, int64_t lda, const void* Xt, int64_t ldx, in
     }
     const int kb_per = (int)ceil_div(kb_all, splits);
     splits = (int)ceil_div(kb_all, kb_per);                // every split non-empty
+    if (parts) {
+        *parts = splits;
+        return launch_bn<true>(bn, ma, mb, M, K, work, cols_out, n_rhs, splits, kb_per, slice, st);
+    }
     if (splits == 1)
         return trans ? launch_bn<true>(bn, ma, mb, M, K, Y, ldy, n_rhs, 1, kb_per, 0, st)
                      : launch_bn<false>(bn, ma, mb, M, K, Y, ldy, n_rhs, 1, kb_per, 0, st);
@@ -440,6 +446,14 @@ extern "C" int mbem_gemm_bf16_t_split(const void* A, int64_t lda, const void* Xt
                                       void* stream) {
     return gemm_bf16(A, lda, Xt, ldx, M, K, n_rhs, Yt, ldy, true, static_cast<float*>(work), work_bytes,
                      (cudaStream_t)stream);
+}
+
+extern "C" int mbem_gemm_bf16_t_parts(const void* A, int64_t lda, const void* Xt, int64_t ldx, int64_t M, int64_t K,
+                                      int n_rhs, float* work, size_t work_bytes, int* splits, void* stream) {
+    MBEM_REQUIRE(work && splits && work_bytes >= (size_t)M * n_rhs * sizeof(float), MBEM_ERR_SIZE,
+                 "GEMM workspace too small for one split");
+    *splits = 0;
+    return gemm_bf16(A, lda, Xt, ldx, M, K, n_rhs, work, M, true, work, work_bytes, (cudaStream_t)stream, splits);
 }
 
 extern "C" int mbem_gemm_bf16_check(void* stream) { return tc_gemm_check((cudaStream_t)stream); }

@@ -176,76 +176,46 @@ class BlockSolver:
         k, n = R.shape
         dev = self.device
         st = stream_handle()
+        ld, terms = self.ldp, self.terms
         V = torch.empty((m + 1, k, n), dtype=torch.float32, device=dev)
-        Vbf = torch.zeros((k, self.terms * self.ldp), dtype=torch.bfloat16, device=dev)
-        ld = self.ldp
-        terms = self.terms
-        W = torch.empty((k, n), dtype=torch.float32, device=dev)
-        norms = torch.empty(k, dtype=torch.float64, device=dev)
-        Hd = torch.empty((m + 1, k), dtype=torch.float64, device=dev)
-        H2d = torch.empty((m + 1, k), dtype=torch.float64, device=dev)
-
-        def normalize(src, is64, j):
-            # V[j] = src / |src|; the GEMM operand [V_hi | V_lo | V_hi] (or V_hi)
-            nat.call("mbem_batch_normalize", ptr(src), is64, k, n, ptr(norms), ptr(V[j]), None, st)
-            vh = V[j].to(torch.bfloat16)
-            Vbf[:, :n] = vh
-            if terms == 3:
-                Vbf[:, ld:ld + n] = (V[j] - vh.float()).to(torch.bfloat16)
-                Vbf[:, 2 * ld:2 * ld + n] = vh
-            return norms.cpu().numpy().copy()
-
-        beta = normalize(R, 1, 0)
-        live = beta > 0
-        H = np.zeros((m + 1, m, k))
-        cs = np.zeros((m, k))
-        sn = np.zeros((m, k))
-        g = np.zeros((m + 1, k))
+        # the GEMM operand [V_hi | V_lo | V_hi] (or V_hi); its padding stays zero
+        Vbf = torch.zeros((k, terms * ld), dtype=torch.bfloat16, device=dev)
+        beta = torch.empty(k, dtype=torch.float64, device=dev)
+        nat.call("mbem_batch_normalize", ptr(R), 1, k, n, ptr(beta), ptr(V[0]), None, st)
+        vh = V[0].to(torch.bfloat16)
+        Vbf[:, :n] = vh
+        if terms == 3:
+            Vbf[:, ld:ld + n] = (V[0] - vh.float()).to(torch.bfloat16)
+            Vbf[:, 2 * ld:2 * ld + n] = vh
+        H = torch.zeros((m, m, k), dtype=torch.float64, device=dev)
+        rot = torch.zeros((2, m, k), dtype=torch.float64, device=dev)
+        g = torch.zeros((m + 1, k), dtype=torch.float64, device=dev)
         g[0] = beta
-        ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        gemm_ms = 0.0
+        left = torch.zeros(m, dtype=torch.int32, device=dev)
+        need = nat.lib().mbem_gemm_bf16_workspace_size(n, k)
+        work = torch.empty(need // 4, dtype=torch.float32, device=dev)
+        parts = ctypes.c_int(0)
+        ranges = self._ranges.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+        events = []
         jdone = 0
         for j in range(m):
-            ev0.record()
-            gemm_bf16_t(self.A16, Vbf, terms * ld, W)
-            ev1.record()
-            self.project(W)
-            nat.call("mbem_batch_dots", ptr(V), j + 1, ptr(W), k, n, ptr(Hd), st)
-            nat.call("mbem_batch_axpy", ptr(W), ptr(V), j + 1, ptr(Hd), -1.0, k, n, st)
-            nat.call("mbem_batch_dots", ptr(V), j + 1, ptr(W), k, n, ptr(H2d), st)
-            nat.call("mbem_batch_axpy", ptr(W), ptr(V), j + 1, ptr(H2d), -1.0, k, n, st)
-            hn = normalize(W, 0, j + 1)
-            h = (Hd[:j + 1] + H2d[:j + 1]).cpu().numpy()
-            gemm_ms += ev0.elapsed_time(ev1)
-            col = np.vstack([h, hn[None, :]])            # (j + 2, k)
-            for i in range(j):                           # accumulated rotations
-                a, b = col[i].copy(), col[i + 1].copy()
-                col[i] = cs[i] * a + sn[i] * b
-                col[i + 1] = -sn[i] * a + cs[i] * b
-            den = np.hypot(col[j], col[j + 1])
-            ok = den > 0
-            cs[j] = np.where(ok, np.abs(col[j]) / np.where(ok, den, 1.0), 1.0)
-            sgn = np.where(col[j] >= 0, 1.0, -1.0)
-            sn[j] = np.where(ok, sgn * col[j + 1] / np.where(ok, den, 1.0), 0.0)
-            col[j] = cs[j] * col[j] + sn[j] * col[j + 1]
-            col[j + 1] = 0.0
-            H[:j + 2, j] = col
-            g[j + 1] = -sn[j] * g[j]
-            g[j] = cs[j] * g[j]
+            ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+            ev[0].record()
+            nat.call("mbem_gemm_bf16_t_parts", ptr(self.A16), self.A16.stride(0), ptr(Vbf), Vbf.stride(0), n,
+                     terms * ld, k, ptr(work), need, ctypes.byref(parts), st)
+            ev[1].record()
+            events.append(ev)
+            nat.call("mbem_batch_arnoldi", ptr(work), parts.value, n * k, ptr(V), j, m, k, n, ranges,
+                     len(self._ranges) // 2, ptr(Vbf), Vbf.stride(0), ld, terms, ptr(H), ptr(rot[0]), ptr(rot[1]),
+                     ptr(g), ptr(beta), float(rtol), ptr(left[j:]), st)
             jdone = j + 1
-            rel = np.where(live, np.abs(g[j + 1]) / np.where(live, beta, 1.0), 0.0)
-            if np.all(rel < rtol):
+            if int(left[j]) == 0:
                 break
-        # back substitution per right-hand side
-        Y = np.zeros((jdone, k))
-        for i in range(jdone - 1, -1, -1):
-            s = g[i] - (H[i, i + 1:jdone].T * Y[i + 1:jdone].T).sum(axis=1) if i + 1 < jdone else g[i].copy()
-            d = H[i, i]
-            Y[i] = np.where(d != 0, s / np.where(d != 0, d, 1.0), 0.0)
+        Y = torch.empty((jdone, k), dtype=torch.float64, device=dev)
+        nat.call("mbem_batch_backsolve", ptr(H), ptr(g), m, jdone, k, ptr(Y), st)
         D = torch.zeros((k, n), dtype=torch.float64, device=dev)
-        Yd = torch.from_numpy(np.ascontiguousarray(Y)).to(dev)
-        nat.call("mbem_batch_update", ptr(D), ptr(V), jdone, ptr(Yd), k, n, st)
-        return D, jdone, gemm_ms
+        nat.call("mbem_batch_update", ptr(D), ptr(V), jdone, ptr(Y), k, n, st)
+        return D, jdone, sum(a.elapsed_time(b) for a, b in events)
 
     # -- the solve ------------------------------------------------------
     def solve(self, B: torch.Tensor, rtol: float = 1e-8, max_outer: int = 12):
