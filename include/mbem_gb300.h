@@ -598,6 +598,13 @@ int mbem_gemm_bf16_t_split(const void* A, int64_t lda, const void* Xt, int64_t l
  * arrays (n_rhs, M), M * n_rhs floats apart, whose sum in order is Y^T. */
 int mbem_gemm_bf16_t_parts(const void* A, int64_t lda, const void* Xt, int64_t ldx, int64_t M, int64_t K, int n_rhs,
                            float* work, size_t work_bytes, int* splits, void* stream);
+/* The three-term product Y = A_hi X_hi + A_hi X_lo + A_lo X_hi, A_lo at column lo_a
+ * of A and X_lo at column lo_x of Xt, as partial sums in work (arrays (n_rhs, M)):
+ * the (128-row tile, K block) units, *kb a tile, are dealt out in runs of *per, and
+ * array i holds of each tile what the i-th run that meets it summed. work as above. */
+int mbem_gemm_bf16x3_t_parts(const void* A, int64_t lda, int64_t lo_a, const void* Xt, int64_t ldx, int64_t lo_x,
+                             int64_t M, int64_t K, int n_rhs, float* work, size_t work_bytes, int* kb, int* per,
+                             void* stream);
 int mbem_gemm_bf16_check(void* stream);
 /* C[M x N] -= A[M x K] Bt[N x K]^T on the tensor cores (BF16 row-major
  * operands, lda and ldb multiples of 8; FP32 C at ldc): the update of the
@@ -631,14 +638,15 @@ int mbem_batch_normalize(const void* W, int w_is_f64, int64_t k, int64_t n, doub
 /* X[r] += sum_i Y[i, r] V[i, r] (X FP64) */
 int mbem_batch_update(double* X, const float* V, int n_vec, const double* Y, int64_t k, int64_t n, void* stream);
 /* Step j (of m) of k Arnoldi iterations in one launch: W = the sum of the
- * `splits` GEMM partial sums P (split_stride floats apart, (k, n) each), the rigid
- * translations of the u-ranges removed, two passes of classical Gram-Schmidt
+ * `splits` GEMM partial sums P (split_stride floats apart, (k, n) each; with kb > 0
+ * mbem_gemm_bf16x3_t_parts' runs instead), the rigid translations of the u-ranges removed, two passes of classical Gram-Schmidt
  * against V[0 .. j] ((m + 1, k, n) FP32), the norm, V[j + 1], its BF16 operand in
  * Vbf (rows of ldbf; terms 3: [hi | lo | hi] at 0, ldp, 2 ldp, terms 1: [hi]), and
  * the right-hand side's Givens rotation: H[(i m + j) k + r], cs, sn, g[i k + r]
  * (g[0] = beta = |r_0| before step 0). *left is raised by the right-hand sides whose
  * residual estimate is not below rtol beta. */
-int mbem_batch_arnoldi(const float* P, int splits, int64_t split_stride, float* V, int j, int m, int64_t k, int64_t n,
+int mbem_batch_arnoldi(const float* P, int splits, int kb, int per, int64_t split_stride, float* V, int j, int m,
+                       int64_t k, int64_t n,
                        const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int terms,
                        double* H, double* cs, double* sn, double* g, const double* beta, double rtol, int* left,
                        void* stream);

@@ -185,7 +185,9 @@ _SIGNATURES = {
     "mbem_batch_normalize": (c_int, [_P, c_int, _I, _I, _P, _P, _P, _P]),
     "mbem_batch_update": (c_int, [_P, _P, c_int, _P, _I, _I, _P]),
     "mbem_gemm_bf16_t_parts": (c_int, [_P, _I, _P, _I, _I, _I, c_int, _P, c_size_t, POINTER(c_int), _P]),
-    "mbem_batch_arnoldi": (c_int, [_P, c_int, _I, _P, c_int, c_int, _I, _I, _P, c_int, _P, _I, _I, c_int, _P, _P, _P,
+    "mbem_gemm_bf16x3_t_parts": (c_int, [_P, _I, _I, _P, _I, _I, _I, _I, c_int, _P, c_size_t, POINTER(c_int),
+                                         POINTER(c_int), _P]),
+    "mbem_batch_arnoldi": (c_int, [_P, c_int, c_int, c_int, _I, _P, c_int, c_int, _I, _I, _P, c_int, _P, _I, _I, c_int, _P, _P, _P,
                                    _P, _P, _D, _P, _P]),
     "mbem_batch_backsolve": (c_int, [_P, _P, c_int, c_int, _I, _P, _P]),
     "mbem_batch_project": (c_int, [_P, c_int, _I, _I, _P, c_int, _P]),

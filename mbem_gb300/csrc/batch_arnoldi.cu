@@ -35,7 +35,8 @@ __host__ __device__ constexpr int ar_vectors(int m) { return m < 4 ? 4 : m; }
 
 struct ArnoldiArgs {
     const float* P;          // GEMM partial sums [split][k][n]
-    int splits;
+    int splits;              // their number, or with kb > 0 a row tile's own: the runs of `per` units that its
+    int kb, per;             // kb units (128 rows) meet (tc_block.cu)
     int64_t split_stride;
     float* V;                // basis [m + 1][k][n]
     int j, m;
@@ -144,6 +145,12 @@ __device__ __forceinline__ void ar_subtract(const float* __restrict__ V, int64_t
     }
 }
 
+__device__ __forceinline__ int ar_parts(const ArnoldiArgs& a, int64_t t) {
+    if (a.kb == 0) return a.splits;
+    const int tile = (int)(t >> 7);
+    return ((tile + 1) * a.kb - 1) / a.per - tile * a.kb / a.per + 1;
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
     extern __shared__ __align__(16) float ar_w[];
@@ -168,7 +175,8 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
     if (VEC) {
         for (int t = 4 * threadIdx.x; t < len; t += 4 * AR_T) {
             float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (int s = 0; s < a.splits; s++) {
+            const int parts = ar_parts(a, t0 + t);
+            for (int s = 0; s < parts; s++) {
                 const float4 q = *reinterpret_cast<const float4*>(p + s * a.split_stride + t);
                 x.x += q.x; x.y += q.y; x.z += q.z; x.w += q.w;
             }
@@ -177,7 +185,8 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
     } else {
         for (int t = threadIdx.x; t < len; t += AR_T) {
             float x = 0.0f;
-            for (int s = 0; s < a.splits; s++) x += p[s * a.split_stride + t];
+            const int parts = ar_parts(a, t0 + t);
+            for (int s = 0; s < parts; s++) x += p[s * a.split_stride + t];
             w[t] = x;
         }
     }
@@ -312,19 +321,20 @@ using namespace mbem;
 
 extern "C" {
 
-int mbem_batch_arnoldi(const float* P, int splits, int64_t split_stride, float* V, int j, int m, int64_t k, int64_t n,
+int mbem_batch_arnoldi(const float* P, int splits, int kb, int per, int64_t split_stride, float* V, int j, int m, int64_t k, int64_t n,
                        const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int terms,
                        double* H, double* cs, double* sn, double* g, const double* beta, double rtol, int* left,
                        void* stream) {
-    MBEM_REQUIRE(P && V && Vbf && H && cs && sn && g && beta && left && splits >= 1 && k >= 1 && n >= 1, MBEM_ERR_ARG,
+    MBEM_REQUIRE(P && V && Vbf && H && cs && sn && g && beta && left && k >= 1 && n >= 1, MBEM_ERR_ARG,
                  "bad batched Arnoldi arguments");
+    MBEM_REQUIRE(kb == 0 ? splits >= 1 : kb > 0 && per > 0, MBEM_ERR_ARG, "bad batched Arnoldi partial sums");
     MBEM_REQUIRE(j >= 0 && j < m, MBEM_ERR_ARG, "batched Arnoldi: step %d of %d", j, m);
-    MBEM_REQUIRE((terms == 1 || terms == 3) && ldp >= n && ldbf >= terms * ldp && split_stride >= (splits > 1 ? k * n : 0),
+    MBEM_REQUIRE((terms == 1 || terms == 3) && ldp >= n && ldbf >= terms * ldp && split_stride >= (kb > 0 || splits > 1 ? k * n : 0),
                  MBEM_ERR_ARG, "bad batched Arnoldi strides");
     ArnoldiArgs a;
     int e = make_ranges(u_ranges, n_u_ranges, a.ur);
     if (e) return e;
-    a.P = P; a.splits = splits; a.split_stride = split_stride; a.V = V; a.j = j; a.m = m; a.k = k; a.n = n;
+    a.P = P; a.splits = splits; a.kb = kb; a.per = per; a.split_stride = split_stride; a.V = V; a.j = j; a.m = m; a.k = k; a.n = n;
     a.Vbf = Vbf; a.ldbf = ldbf; a.ldp = ldp; a.terms = terms; a.H = H; a.cs = cs; a.sn = sn; a.g = g; a.beta = beta;
     a.rtol = rtol; a.left = left;
     // blocks a cluster: a slice fits twice an SM, and there are two blocks an SM

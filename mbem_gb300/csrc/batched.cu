@@ -201,7 +201,9 @@ batch_project_kernel(T* __restrict__ X, int64_t n, URanges ur) {
 // R = B - A X for a block: the exact far-field product (tc_exact.cu), then the
 // FP64 near blocks
 // ---------------------------------------------------------------------------
-// R[r, row] -= (near X[r])[row]; a thread per (r, row)
+// R[r, row] -= (near X[r])[row]; a thread per (r, row). Bound by the FP64 pipe
+// (three rows and four right-hand sides a thread, for a third of the loads,
+// measured 10 % slower).
 __global__ void __launch_bounds__(BT)
 residual_near_kernel(const double* __restrict__ X, int64_t k, int64_t n, mbem_near_blocks nb, double* __restrict__ R) {
     const int64_t r = blockIdx.y;

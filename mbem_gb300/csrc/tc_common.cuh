@@ -48,6 +48,8 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // BF16 row-major (rows x cols) at ld elements, box (64 cols x box_rows), 128B
 // swizzle (tc_gemm.cu; the encoder is looked up on first use)
 int tc_make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
+// the same with a box of 32 columns and the 64B swizzle
+int tc_make_map32(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
 // the device flag that a tensor-core wait that ran out sets (tc_gemm_check)
 int* tc_error_flag();
 

@@ -255,13 +255,15 @@ static int get_encode() {
 }
 
 // BF16 row-major (rows x cols) at ld elements, box (64 cols x box_rows), 128B swizzle
-static int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+static int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows,
+                    int box_cols = TC_BK) {
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(MBEM_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return MBEM_OK;
@@ -276,6 +278,12 @@ int tc_make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, 
     const int e0 = get_encode();
     if (e0) return e0;
     return make_map(map, base, rows, cols, ld, box_rows);
+}
+
+int tc_make_map32(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+    const int e0 = get_encode();
+    if (e0) return e0;
+    return make_map(map, base, rows, cols, ld, box_rows, 32);
 }
 
 template <int BN, bool TRANS>

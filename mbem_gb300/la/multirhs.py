@@ -194,19 +194,23 @@ class BlockSolver:
         left = torch.zeros(m, dtype=torch.int32, device=dev)
         need = nat.lib().mbem_gemm_bf16_workspace_size(n, k)
         work = torch.empty(need // 4, dtype=torch.float32, device=dev)
-        parts = ctypes.c_int(0)
+        parts, kb, per = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
         ranges = self._ranges.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
         events = []
         jdone = 0
         for j in range(m):
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record()
-            nat.call("mbem_gemm_bf16_t_parts", ptr(self.A16), self.A16.stride(0), ptr(Vbf), Vbf.stride(0), n,
-                     terms * ld, k, ptr(work), need, ctypes.byref(parts), st)
+            if terms == 3:
+                nat.call("mbem_gemm_bf16x3_t_parts", ptr(self.A16), self.A16.stride(0), 2 * ld, ptr(Vbf),
+                         Vbf.stride(0), ld, n, n, k, ptr(work), need, ctypes.byref(kb), ctypes.byref(per), st)
+            else:
+                nat.call("mbem_gemm_bf16_t_parts", ptr(self.A16), self.A16.stride(0), ptr(Vbf), Vbf.stride(0), n,
+                         terms * ld, k, ptr(work), need, ctypes.byref(parts), st)
             ev[1].record()
             events.append(ev)
-            nat.call("mbem_batch_arnoldi", ptr(work), parts.value, n * k, ptr(V), j, m, k, n, ranges,
-                     len(self._ranges) // 2, ptr(Vbf), Vbf.stride(0), ld, terms, ptr(H), ptr(rot[0]), ptr(rot[1]),
+            nat.call("mbem_batch_arnoldi", ptr(work), parts.value, kb.value, per.value, n * k, ptr(V), j, m, k, n,
+                     ranges, len(self._ranges) // 2, ptr(Vbf), Vbf.stride(0), ld, terms, ptr(H), ptr(rot[0]), ptr(rot[1]),
                      ptr(g), ptr(beta), float(rtol), ptr(left[j:]), st)
             jdone = j + 1
             if int(left[j]) == 0:

@@ -40,7 +40,7 @@ def test_steps(gpu, n, k, splits, terms, deflate):
     left = torch.zeros(m, dtype=torch.int32, device=dev)
     for j in range(steps):
         P = torch.randn((splits, k, n), generator=g, device=dev) * 10.0 ** (j - 2)
-        nat.call("mbem_batch_arnoldi", ptr(P), splits, n * k, ptr(V), j, m, k, n, rp, len(ranges) // 2, ptr(Vbf),
+        nat.call("mbem_batch_arnoldi", ptr(P), splits, 0, 0, n * k, ptr(V), j, m, k, n, rp, len(ranges) // 2, ptr(Vbf),
                  Vbf.stride(0), ldp, terms, ptr(H), ptr(cs), ptr(sn), ptr(gv), ptr(beta), 1e-3, ptr(left[j:]),
                  stream_handle())
         w = P.double().sum(dim=0)

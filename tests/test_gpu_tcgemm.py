@@ -75,3 +75,37 @@ def test_gemm_sub_update(gpu, M, N, K):
     err = float((C.double() - ref).abs().max() / P.abs().max())
     assert err < 1e-5, err
     assert torch.equal(C[M:], C0[M:]) and torch.equal(C[:, N:], C0[:, N:])
+
+
+@pytest.mark.parametrize("M,K,n", [(1, 1, 1), (127, 33, 16), (128, 32, 17), (129, 1000, 40), (700, 1001, 128),
+                                   (1025, 500, 256), (5000, 3001, 100)])
+def test_three_term_product_in_parts(gpu, M, K, n):
+    """The runs' partial sums, added tile by tile, against the FP32 products of
+    the same BF16 panels: FP32 accumulation in another order, 2^-24 times the sum
+    of magnitudes times the chains (K / 16 products, three terms)."""
+    import ctypes
+
+    from mbem_gb300 import _native as nat
+    from mbem_gb300._device import ptr, stream_handle
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    ld = (K + 7) // 8 * 8
+    A = torch.randn((M, 3 * ld), generator=g, device="cuda").to(torch.bfloat16)
+    X = torch.randn((n, 3 * ld), generator=g, device="cuda").to(torch.bfloat16)
+    need = nat.lib().mbem_gemm_bf16_workspace_size(M, n)
+    work = torch.full((need // 4,), float("nan"), device="cuda")
+    kb, per = ctypes.c_int(0), ctypes.c_int(0)
+    nat.call("mbem_gemm_bf16x3_t_parts", ptr(A), A.stride(0), 2 * ld, ptr(X), X.stride(0), ld, M, K, n, ptr(work),
+             need, ctypes.byref(kb), ctypes.byref(per), stream_handle())
+    nat.call("mbem_gemm_bf16_check", stream_handle())
+    kb, per = kb.value, per.value
+    P = work[:(work.numel() // (n * M)) * n * M].view(-1, n, M)
+    Y = torch.empty((n, M), device="cuda", dtype=torch.float64)
+    for t in range((M + 127) // 128):
+        parts = ((t + 1) * kb - 1) // per - t * kb // per + 1
+        rows = slice(128 * t, min(M, 128 * (t + 1)))
+        Y[:, rows] = P[:parts, :, rows].double().sum(dim=0)
+    ah, al = A[:, :K].double(), A[:, 2 * ld:2 * ld + K].double()
+    xh, xl = X[:, :K].double(), X[:, ld:ld + K].double()
+    ref = xh @ ah.T + xl @ ah.T + xh @ al.T
+    mag = xh.abs() @ ah.abs().T + xl.abs() @ ah.abs().T + xh.abs() @ al.abs().T
+    assert bool(((Y - ref).abs() <= 2.0 ** -24 * (3 * K / 16 + 16) * mag).all())
