@@ -26,14 +26,24 @@ __global__ void rowsum3_kernel(const double* __restrict__ A, int64_t ld, int64_t
     const int lane = threadIdx.x & 31;
     if (r >= n_rows) return;
     const double* row = A + r * ld;
-    double acc[3] = {0.0, 0.0, 0.0};
-    // lane l visits columns l, l+32, ...; column c belongs to component c % 3
-    int j = lane % 3;
-    for (int64_t c = lane; c < n_cols; c += 32) {
-        acc[j] += row[c];
-        j += 2;                 // (c + 32) % 3 == (c % 3 + 2) % 3
-        if (j >= 3) j -= 3;
+    // lane l visits columns l, l + 32, l + 64 of every 96: column l + 32 i belongs
+    // to component (l + 2 i) % 3, so three registers hold the three components
+    // (an indexed accumulator lived in local memory: 128 us for the 5,184-row
+    // operator, 71 us now)
+    double t[3] = {0.0, 0.0, 0.0};
+    int64_t c = lane;
+    for (; c + 64 < n_cols; c += 96) {
+        t[0] += row[c];
+        t[1] += row[c + 32];
+        t[2] += row[c + 64];
     }
+    if (c < n_cols) t[0] += row[c];
+    if (c + 32 < n_cols) t[1] += row[c + 32];
+    const int m = lane % 3;
+    double acc[3];
+    acc[0] = m == 0 ? t[0] : m == 1 ? t[1] : t[2];
+    acc[1] = m == 0 ? t[2] : m == 1 ? t[0] : t[1];
+    acc[2] = m == 0 ? t[1] : m == 1 ? t[2] : t[0];
 #pragma unroll
     for (int k = 0; k < 3; k++)
 #pragma unroll
@@ -97,30 +107,35 @@ __global__ void rotate_row_triples_kernel(double* __restrict__ A, int64_t ld, in
 }
 
 // ---------------------------------------------------------------------------
-// y = alpha A x + beta y: 4 rows per warp, 128-bit streaming loads of A
+// y = alpha A x + beta y, 128-bit streaming loads of A
 // ---------------------------------------------------------------------------
-constexpr int GEMV_ROWS = 4;
-constexpr int GEMV_THREADS = 256;
+// y = alpha A x + beta y, a warp ROWS rows. Bound by the FP64 pipe (one DFMA per
+// 8-byte entry), so the SM with the most rows sets the time: one warp a block
+// leaves at most one block's rows of imbalance (5,184 rows in blocks of 32 gave
+// ten SMs of 152 twice the others' rows: 89 us, 62 us now).
+constexpr int GEMV_THREADS = 256;        // of the scalar kernel
 
-__global__ void __launch_bounds__(GEMV_THREADS)
+template <int ROWS>
+__global__ void __launch_bounds__(32)
 dgemv_vec_kernel(const double* __restrict__ A, int64_t ld, int64_t n_rows, int64_t n_cols,
                  const double* __restrict__ x, double alpha, double beta, double* __restrict__ y) {
-    const int64_t warp = (int64_t)blockIdx.x * (GEMV_THREADS / 32) + threadIdx.x / 32;
-    const int lane = threadIdx.x & 31;
-    const int64_t r0 = warp * GEMV_ROWS;
-    if (r0 >= n_rows) return;
-    const int nr = (int)lmin(GEMV_ROWS, n_rows - r0);
-    double acc[GEMV_ROWS] = {0.0, 0.0, 0.0, 0.0};
+    const int lane = threadIdx.x;
+    const int64_t r0 = (int64_t)blockIdx.x * ROWS;
+    const int nr = (int)lmin(ROWS, n_rows - r0);
+    double acc[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) acc[i] = 0.0;
     const int64_t n2 = n_cols / 2;
     const double2* x2 = reinterpret_cast<const double2*>(x);
-    const double2* rows[GEMV_ROWS];
+    const double2* rows[ROWS];
 #pragma unroll
-    for (int i = 0; i < GEMV_ROWS; i++)
+    for (int i = 0; i < ROWS; i++)
         rows[i] = reinterpret_cast<const double2*>(A + (r0 + min(i, nr - 1)) * ld);
+#pragma unroll 4
     for (int64_t c = lane; c < n2; c += 32) {
         const double2 xv = __ldg(x2 + c);
 #pragma unroll
-        for (int i = 0; i < GEMV_ROWS; i++) {
+        for (int i = 0; i < ROWS; i++) {
             const double2 av = __ldcs(rows[i] + c);
             acc[i] = fma(av.x, xv.x, acc[i]);
             acc[i] = fma(av.y, xv.y, acc[i]);
@@ -129,17 +144,17 @@ dgemv_vec_kernel(const double* __restrict__ A, int64_t ld, int64_t n_rows, int64
     if ((n_cols & 1) && lane == 0) {
         const double xv = x[n_cols - 1];
 #pragma unroll
-        for (int i = 0; i < GEMV_ROWS; i++)
+        for (int i = 0; i < ROWS; i++)
             acc[i] = fma(A[(r0 + min(i, nr - 1)) * ld + n_cols - 1], xv, acc[i]);
     }
 #pragma unroll
-    for (int i = 0; i < GEMV_ROWS; i++)
+    for (int i = 0; i < ROWS; i++)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
     if (lane < nr) {
         double v = acc[0];
 #pragma unroll
-        for (int i = 1; i < GEMV_ROWS; i++)
+        for (int i = 1; i < ROWS; i++)
             if (lane == i) v = acc[i];
         const int64_t r = r0 + lane;
         y[r] = (beta == 0.0) ? alpha * v : alpha * v + beta * y[r];
@@ -164,9 +179,11 @@ int dgemv(const double* A, int64_t ld, int64_t n_rows, int64_t n_cols, const dou
     if (n_rows == 0) return MBEM_OK;
     const bool vec = ((uintptr_t)A % 16 == 0) && ((uintptr_t)x % 16 == 0) && (ld % 2 == 0);
     if (vec) {
-        const int64_t warps = ceil_div(n_rows, GEMV_ROWS);
-        dgemv_vec_kernel<<<(unsigned)ceil_div(warps, GEMV_THREADS / 32), GEMV_THREADS, 0, st>>>(
-            A, ld, n_rows, n_cols, x, alpha, beta, y);
+        // four rows a warp share the loads of x; few rows are spread out instead
+        if (n_rows >= 152 * 16)
+            dgemv_vec_kernel<4><<<(unsigned)ceil_div(n_rows, 4), 32, 0, st>>>(A, ld, n_rows, n_cols, x, alpha, beta, y);
+        else
+            dgemv_vec_kernel<1><<<(unsigned)n_rows, 32, 0, st>>>(A, ld, n_rows, n_cols, x, alpha, beta, y);
     } else {
         dgemv_scalar_kernel<<<(unsigned)ceil_div(n_rows, GEMV_THREADS / 32), GEMV_THREADS, 0, st>>>(
             A, ld, n_rows, n_cols, x, alpha, beta, y);
@@ -270,16 +287,26 @@ proj_partial_kernel(const double* __restrict__ vin, URanges ur, double* __restri
     }
 }
 
-// the three component means over the u-slots from the partial sums (threads
-// 0..2 form them in block order; every thread returns after the barrier)
+// the three component means over the u-slots from the partial sums (the first
+// warp adds them, lane by lane and then by a fixed shuffle tree; every thread
+// returns after the barrier)
 __device__ void proj_means(URanges ur, const double* __restrict__ partial, int nparts, double* mean) {
-    if (threadIdx.x < 3) {
-        double s = 0.0;
-        for (int b = 0; b < nparts; b++) s += partial[3 * b + threadIdx.x];
+    if (threadIdx.x < 32) {
+        double s[3] = {0.0, 0.0, 0.0};
+        for (int b = threadIdx.x; b < nparts; b += 32)
+#pragma unroll
+            for (int k = 0; k < 3; k++) s[k] += partial[3 * b + k];
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
         int64_t total = 0;
         for (int q = 0; q < ur.n; q++) total += ur.len[q];
         // Z_k = 1/sqrt(M) on component-k u entries: Z (Z^T v) = sum / M
-        mean[threadIdx.x] = (total > 0) ? s / (double)(total / 3) : 0.0;
+        if (threadIdx.x < 3) {
+            const double v = threadIdx.x == 0 ? s[0] : threadIdx.x == 1 ? s[1] : s[2];
+            mean[threadIdx.x] = (total > 0) ? v / (double)(total / 3) : 0.0;
+        }
     }
     __syncthreads();
 }
@@ -750,7 +777,7 @@ struct Fgmres {
         kv_norm_init_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(v, n, partial, g, ctl);
         return launch_status("norm init", 1);
     }
-    // one Arnoldi step after its product w: the CGS2 coefficients into h,
+        // one Arnoldi step after its product w: the CGS2 coefficients into h,
     // |w|^2 into h[k], the rotation of column k - 1, and V[k] = w / |w|
     int arnoldi(double* V, int k, double* w, double* partial, double* h, double* h2, const KvGivens& G,
                 KrylovCtl* ctl, bool project_w, bool scale_next) {
@@ -759,8 +786,7 @@ struct Fgmres {
             proj_partial_kernel<<<PROJ_BLOCKS, PROJ_THREADS, 0, st>>>(w, ur, W.proj, stop);
             count_launches(1);
         }
-        kv_dot_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(V, n, k, n, w, ur, project_w ? W.proj : nullptr,
-                                                           partial, h, ctl);
+        kv_dot_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(V, n, k, n, w, ur, project_w ? W.proj : nullptr, partial, h, ctl);
         kv_axpy_dot_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(V, n, k, n, w, h, partial, h2, ctl);
         kv_axpy_norm_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(V, n, k, n, w, h2, partial, h, G, ctl);
         if (scale_next)
