@@ -6,6 +6,7 @@
 // order (per-block partials, then one ordered pass), so results are
 // bit-reproducible run to run. The Arnoldi basis of an 83k-unknown system
 // at restart 50 is ~34 MB and stays L2-resident.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -16,6 +17,8 @@
 #include "common.cuh"
 
 namespace mbem {
+
+namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------
 // calibration row sums: out[r, j] (+)= alpha * sum_c A[r, 3c + j]
@@ -340,12 +343,12 @@ static int project(const double* vin, double* vout, int64_t n, const URanges& ur
 
 // ---------------------------------------------------------------------------
 // Device-side Arnoldi steps (la/solver.py:115-245, with classical
-// Gram-Schmidt applied twice). After its product a GMRES step is four
-// kernels: kv_dot (the projection's subtraction fused in, then the first
+// Gram-Schmidt applied twice). After its product a GMRES step is one kernel for
+// vectors up to KV_CLUSTER_N (kv_cluster) and four for longer ones: kv_dot (the projection's subtraction fused in, then the first
 // pass's dots), kv_axpy_dot (the first pass's subtraction, the second pass's
 // dots), kv_axpy_norm (the second subtraction, |w|^2 and the Givens rotation
 // of the new Hessenberg column) and the scaling of the next basis vector.
-// Each of the first three writes per-block partial sums; the last block to
+// Each of the first three of them writes per-block partial sums; the last block to
 // arrive adds them in block order, so the result does not depend on the
 // order in which blocks finish. The rotations, the rotated right-hand side g
 // and the triangular factor R stay on the device, next to a control block
@@ -453,21 +456,23 @@ __device__ void kv_block_sumsq(int64_t n, int64_t c0, double w0, double w1, doub
 }
 
 // The rotation of Hessenberg column j (la/solver.py:188-210): h[0..j] are
-// its Gram-Schmidt coefficients, h[j + 1] = |w|^2. The earlier rotations are
+// its Gram-Schmidt coefficients, w2 = |w|^2. The earlier rotations are
 // applied, a new one zeroes the subdiagonal, g is rotated and the column
 // stored in R. A zero pivot ends the basis before column j; on the inner
 // solve an invariant Krylov space (|w| = 0) or a residual estimate below
 // rtol beta ends it after.
-__device__ void kv_givens(KrylovCtl* ctl, const double* h, int j, const KvGivens& G) {
-    double* Rj = G.R + (int64_t)G.m * j;
-    for (int i = 0; i <= j; i++) Rj[i] = h[i];
-    const double sub = sqrt(fmax(h[j + 1], 0.0));
+// cs and sn are the earlier rotations (G's, or a copy nearer by).
+__device__ void kv_givens(KrylovCtl* ctl, const double* h, const double* cs, const double* sn, double w2, int j,
+                          const KvGivens& G) {
+    double* __restrict__ Rj = G.R + (int64_t)G.m * j;
+    const double sub = sqrt(fmax(w2, 0.0));
+    double hjj = h[0];
     for (int i = 0; i < j; i++) {
-        const double a = Rj[i], b = Rj[i + 1];
-        Rj[i] = G.cs[i] * a + G.sn[i] * b;
-        Rj[i + 1] = -G.sn[i] * a + G.cs[i] * b;
+        const double a = hjj, b = h[i + 1];
+        Rj[i] = cs[i] * a + sn[i] * b;
+        hjj = -sn[i] * a + cs[i] * b;
     }
-    const double hjj = Rj[j];
+    Rj[j] = hjj;
     const double den = sqrt(hjj * hjj + sub * sub);
     if (den == 0.0) {
         ctl->breakdown = 1;
@@ -573,9 +578,154 @@ kv_axpy_norm_kernel(const double* __restrict__ V, int64_t ldv, int k, int64_t n,
     if (!kv_last_block(&ctl->arrive[2])) return;
     if (threadIdx.x == 0) {
         h[k] = kv_sum_blocks(partial, gridDim.x, 1, 0);
-        kv_givens(ctl, h, k - 1, G);
+        kv_givens(ctl, h, G.cs, G.sn, h[k], k - 1, G);
         ctl->arrive[2] = 0;
     }
+}
+
+// ---------------------------------------------------------------------------
+// The whole Arnoldi step after the product in one launch, for vectors that a
+// cluster's shared memory holds: a slice of w a block, the sums over the blocks
+// through distributed shared memory in rank order. The projection, both
+// Gram-Schmidt passes, the norm, the rotation, V[k] = w / |w| and (outer solve)
+// the next product's input t = P V[k], the means taken from w's own.
+// The separate kernels are a chain of latencies, six launches of 5 to 17 us at 5,184
+// entries: 106 us a step beside its 89 us product (25 vectors), 63 us here beside a
+// product of 62. Their cost hardly grows with n, while here 16 SMs' FP64 pipes do
+// the 4 n k operations: at 32,000 entries a step takes 1,989 us here and 1,996 there
+// (25 vectors, the product included), which is where KV_CLUSTER_N lies.
+// ---------------------------------------------------------------------------
+constexpr int KC_THREADS = 512;
+constexpr int64_t KV_CLUSTER_N = 32768;
+
+struct KcArgs {
+    double* V;
+    int64_t n, slice;
+    int k;
+    double* w;
+    URanges ur;
+    int project, scale_next;
+    double* t;            // P V[k], or NULL
+    KvGivens G;
+    KrylovCtl* ctl;
+};
+
+__device__ __forceinline__ double kc_warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// full[i] = the sum over the cluster's blocks, in rank order, of their part[i]
+__device__ __forceinline__ void kc_cluster_sum(cg::cluster_group& cl, double* part, double* full, int cnt) {
+    cl.sync();
+    const int ranks = (int)cl.num_blocks();
+    for (int i = threadIdx.x; i < cnt; i += KC_THREADS) {
+        double s = 0.0;
+        for (int r = 0; r < ranks; r++) s += cl.map_shared_rank(part, r)[i];
+        full[i] = s;
+    }
+    cl.sync();      // part may be written again; full is seen by the block
+}
+
+// part[0..3) = the component sums of the slice over the u-ranges, part[3] = |slice|^2
+__device__ void kc_sums(const double* ws, int64_t t0, int len, const URanges& ur, bool comps, double* part) {
+    __shared__ double red[KC_THREADS / 32][4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (comps)
+        for (int q = 0; q < ur.n; q++) {
+            const int64_t lo = lmax(ur.off[q], t0), hi = lmin(ur.off[q] + ur.len[q], t0 + len);
+            for (int64_t t = lo + threadIdx.x; t < hi; t += KC_THREADS) {
+                const int c = (int)((t - ur.off[q]) % 3);
+                const double x = ws[t - t0];
+                if (c == 0) s[0] += x;
+                else if (c == 1) s[1] += x;
+                else s[2] += x;
+            }
+        }
+    for (int t = threadIdx.x; t < len; t += KC_THREADS) s[3] = fma(ws[t], ws[t], s[3]);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const double v = kc_warp_sum(s[c]);
+        if (lane == 0) red[warp][c] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.0;
+        for (int q = 0; q < KC_THREADS / 32; q++) v += red[q][threadIdx.x];
+        part[threadIdx.x] = v;
+    }
+}
+
+__global__ void __launch_bounds__(KC_THREADS) kv_cluster_kernel(KcArgs a) {
+    extern __shared__ __align__(16) double kc_smem[];
+    if (a.ctl->stop) return;          // written after the last cluster barrier only
+    const int mv = a.k < 4 ? 4 : a.k;
+    double* ws = kc_smem;             // the slice
+    double* part = ws + a.slice;
+    double* full = part + mv;
+    double* h1 = full + mv;
+    double* cs = h1 + mv;
+    double* sn = cs + mv;
+    cg::cluster_group cl = cg::this_cluster();
+    const int64_t n = a.n, t0 = (int64_t)cl.block_rank() * a.slice;
+    const int len = (int)lmax(0, lmin(a.slice, n - t0));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = a.k;
+    const double* V = a.V + t0;
+    int64_t total = 0;
+    for (int q = 0; q < a.ur.n; q++) total += a.ur.len[q];
+    const double inv_m = total > 0 ? 1.0 / (double)(total / 3) : 0.0;
+    for (int t = threadIdx.x; t < len; t += KC_THREADS) ws[t] = a.w[t0 + t];
+    for (int i = threadIdx.x; i < k - 1; i += KC_THREADS) {
+        cs[i] = a.G.cs[i];
+        sn[i] = a.G.sn[i];
+    }
+    __syncthreads();
+    if (a.project) {
+        kc_sums(ws, t0, len, a.ur, true, part);
+        kc_cluster_sum(cl, part, full, 3);
+        const double mean[3] = {full[0] * inv_m, full[1] * inv_m, full[2] * inv_m};
+        for (int t = threadIdx.x; t < len; t += KC_THREADS) ws[t] -= proj_mean_at(a.ur, mean, t0 + t);
+        __syncthreads();
+    }
+    for (int pass = 0; pass < 2; pass++) {
+        for (int i = warp; i < k; i += KC_THREADS / 32) {
+            const double* v = V + (int64_t)i * n;
+            double p[4] = {0.0, 0.0, 0.0, 0.0};
+            int t = lane;
+            for (; t + 96 < len; t += 128)
+#pragma unroll
+                for (int u = 0; u < 4; u++) p[u] = fma(v[t + 32 * u], ws[t + 32 * u], p[u]);
+            for (; t < len; t += 32) p[0] = fma(v[t], ws[t], p[0]);
+            const double s = kc_warp_sum((p[0] + p[1]) + (p[2] + p[3]));
+            if (lane == 0) part[i] = s;
+        }
+        kc_cluster_sum(cl, part, full, k);
+        for (int i = threadIdx.x; i < k; i += KC_THREADS) h1[i] = pass ? h1[i] + full[i] : full[i];
+        for (int t = threadIdx.x; t < len; t += KC_THREADS) {
+            double x = ws[t];
+#pragma unroll 8
+            for (int i = 0; i < k; i++) x = fma(V[(int64_t)i * n + t], -full[i], x);
+            ws[t] = x;
+        }
+        __syncthreads();
+    }
+    kc_sums(ws, t0, len, a.ur, a.t != nullptr, part);
+    kc_cluster_sum(cl, part, full, 4);
+    const double nrm2 = full[3];
+    const double inv = nrm2 > 0.0 ? 1.0 / sqrt(nrm2) : 0.0;
+    if (a.scale_next) {
+        const double mean[3] = {full[0] * inv_m * inv, full[1] * inv_m * inv, full[2] * inv_m * inv};
+        double* vn = a.V + (int64_t)k * n + t0;
+        for (int t = threadIdx.x; t < len; t += KC_THREADS) {
+            const double v = ws[t] * inv;
+            vn[t] = v;
+            if (a.t) a.t[t0 + t] = v - proj_mean_at(a.ur, mean, t0 + t);
+        }
+    }
+    if (cl.block_rank() == 0 && threadIdx.x == 0) kv_givens(a.ctl, h1, cs, sn, nrm2, k - 1, a.G);
 }
 
 // y = R^-1 g over the columns in use: one warp, rows from the bottom, each
@@ -727,21 +877,25 @@ struct Fgmres {
     // out = P A P in (uses W.t)
     int op(const double* in, double* out) {
         int e = proj(in, W.t);
-        if (e) return e;
+        if (e || (e = product(W.t, out))) return e;
+        return proj(out, out);
+    }
+    // out = A in
+    int product(const double* in, double* out) {
+        int e = MBEM_OK;
         cudaEvent_t ev[2] = {nullptr, nullptr};
         if (time_matvec) {
             cudaEventCreate(&ev[0]);
             cudaEventCreate(&ev[1]);
             cudaEventRecord(ev[0], st);
         }
-        e = mop ? mixed_matvec(mop, W.t, out, W.xh, W.xl, st) : dgemv(A, ld, n, n, W.t, 1.0, 0.0, out, st);
+        e = mop ? mixed_matvec(mop, in, out, W.xh, W.xl, st) : dgemv(A, ld, n, n, in, 1.0, 0.0, out, st);
         matvecs++;
         if (time_matvec) {
             cudaEventRecord(ev[1], st);
             pending.push_back({ev[0], ev[1]});
         }
-        if (e) return e;
-        return proj(out, out);
+        return e;
     }
     // accumulates the device time of the matvecs timed so far (after a sync)
     void collect_times() {
@@ -778,10 +932,22 @@ struct Fgmres {
         return launch_status("norm init", 1);
     }
         // one Arnoldi step after its product w: the CGS2 coefficients into h,
-    // |w|^2 into h[k], the rotation of column k - 1, and V[k] = w / |w|
+    // |w|^2 into h[k], the rotation of column k - 1, and V[k] = w / |w|; with
+    // t (and scale_next), t = P V[k]
     int arnoldi(double* V, int k, double* w, double* partial, double* h, double* h2, const KvGivens& G,
-                KrylovCtl* ctl, bool project_w, bool scale_next) {
+                KrylovCtl* ctl, bool project_w, bool scale_next, double* t = nullptr) {
         const int* stop = &ctl->stop;
+        const int ranks = cluster_ranks(k);
+        if (ranks > 0) {
+            KcArgs a;
+            a.V = V; a.n = n; a.slice = ceil_div(n, ranks); a.k = k; a.w = w; a.ur = ur; a.project = project_w;
+            a.scale_next = scale_next; a.t = scale_next ? t : nullptr; a.G = G; a.ctl = ctl;
+            cudaLaunchAttribute at;
+            cudaLaunchConfig_t cfg = cluster_config(ranks, k, &at);
+            const cudaError_t ce = cudaLaunchKernelEx(&cfg, kv_cluster_kernel, a);
+            if (ce != cudaSuccess) return set_error(MBEM_ERR_CUDA, "kv_cluster_kernel: %s", cudaGetErrorString(ce));
+            return launch_status("arnoldi step", 1);
+        }
         if (project_w) {
             proj_partial_kernel<<<PROJ_BLOCKS, PROJ_THREADS, 0, st>>>(w, ur, W.proj, stop);
             count_launches(1);
@@ -791,7 +957,41 @@ struct Fgmres {
         kv_axpy_norm_kernel<<<(unsigned)nb, KV_THREADS, 0, st>>>(V, n, k, n, w, h2, partial, h, G, ctl);
         if (scale_next)
             scale_by_rnorm_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(w, V + (int64_t)k * n, n, h + k, stop);
-        return launch_status("arnoldi step", 3 + (scale_next ? 1 : 0));
+        const int e = launch_status("arnoldi step", 3 + (scale_next ? 1 : 0));
+        if (e || !scale_next || !t) return e;
+        return proj(V + (int64_t)k * n, t);
+    }
+    cudaLaunchConfig_t cluster_config(int ranks, int k, cudaLaunchAttribute* at) const {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ranks);
+        cfg.blockDim = dim3(KC_THREADS);
+        cfg.dynamicSmemBytes = (size_t)(ceil_div(n, ranks) + 5 * max(k, 4)) * sizeof(double);
+        cfg.stream = st;
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = (unsigned)ranks;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cfg;
+    }
+    // blocks of kv_cluster_kernel's cluster, 0 for vectors that take the separate
+    // kernels; asked of the device once a solve
+    int cluster_max = -1;
+    int cluster_ranks(int k) {
+        if (n > KV_CLUSTER_N || k > 1001) return 0;
+        if (cluster_max < 0) {
+            cluster_max = 8;                       // the portable size: 32 KB + 40 KB a block
+            cudaFuncSetAttribute(kv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+            if (cudaFuncSetAttribute(kv_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+                cudaLaunchAttribute at;
+                cudaLaunchConfig_t cfg = cluster_config(16, 1001, &at);
+                int fit = 0;
+                if (cudaOccupancyMaxActiveClusters(&fit, kv_cluster_kernel, &cfg) == cudaSuccess && fit > 0)
+                    cluster_max = 16;
+            }
+            cudaGetLastError();
+        }
+        return cluster_max;
     }
 };
 
@@ -1157,6 +1357,7 @@ static int fgmres_run(const double* A, int64_t ld, const mbem_mixed_operator* mo
         int jdone = 0;
         for (int j = 0; j < mm; j++) {
             double* vj = W.V + (int64_t)j * n;
+            // w = A P v (the step below projects it)
             if (flexible) {
                 // z_j = M^-1 v_j, w = P A P z_j (right preconditioning, flexible: la/solver.py:160-170)
                 double* zj = W.Z + (int64_t)j * n;
@@ -1164,14 +1365,17 @@ static int fgmres_run(const double* A, int64_t ld, const mbem_mixed_operator* mo
                 // keep z_j in the deflated complement: the update x += Z y
                 // then never feeds the null space
                 if ((e = F.proj(zj, zj))) return e;
-                if ((e = F.op(zj, W.w))) return e;
-            } else if ((e = F.op(vj, W.w))) {               // w = P A P v_j
-                return e;
+                if ((e = F.proj(zj, W.t))) return e;
+            } else if (j == 0 && (e = F.proj(vj, W.t))) {
+                return e;                                   // later ones come from the step before
             }
+            if ((e = F.product(W.t, W.w))) return e;
             // CGS2, |w| and the rotation on the device; the host reads the
             // residual estimate for its stopping and stagnation tests (the
             // next step's preconditioner solve costs far more than this wait)
-            if ((e = F.arnoldi(W.V, j + 1, W.w, W.partial, W.h, W.h2, G, W.ctl, false, true))) return e;
+            if ((e = F.arnoldi(W.V, j + 1, W.w, W.partial, W.h, W.h2, G, W.ctl, F.deflate, true,
+                               flexible ? nullptr : W.t)))
+                return e;
             if ((e = S.post(W.ctl, j)) || (e = S.wait(j, &seen))) return e;
             if (seen.breakdown) {
                 // exact breakdown with a zero pivot: the Krylov space is
