@@ -456,24 +456,29 @@ __device__ void kv_block_sumsq(int64_t n, int64_t c0, double w0, double w1, doub
 }
 
 // The rotation of Hessenberg column j (la/solver.py:188-210): h[0..j] are
-// its Gram-Schmidt coefficients, w2 = |w|^2. The earlier rotations are
-// applied, a new one zeroes the subdiagonal, g is rotated and the column
-// stored in R. A zero pivot ends the basis before column j; on the inner
-// solve an invariant Krylov space (|w| = 0) or a residual estimate below
-// rtol beta ends it after.
-// cs and sn are the earlier rotations (G's, or a copy nearer by).
-__device__ void kv_givens(KrylovCtl* ctl, const double* h, const double* cs, const double* sn, double w2, int j,
-                          const KvGivens& G) {
+// its Gram-Schmidt coefficients. The earlier rotations are applied, a new one
+// zeroes the subdiagonal, g is rotated and the column stored in R. A zero
+// pivot ends the basis before column j; on the inner solve an invariant
+// Krylov space (|w| = 0) or a residual estimate below rtol beta ends it
+// after. kv_rotate does the earlier rotations (cs and sn: G's, or a copy nearer by)
+// and returns the column's entry j, kv_givens the new one; w2 = |w|^2.
+__device__ __forceinline__ double kv_rotate(const double* h, const double* cs, const double* sn, int j,
+                                            const KvGivens& G) {
     double* __restrict__ Rj = G.R + (int64_t)G.m * j;
-    const double sub = sqrt(fmax(w2, 0.0));
     double hjj = h[0];
     for (int i = 0; i < j; i++) {
-        const double a = hjj, b = h[i + 1];
-        Rj[i] = cs[i] * a + sn[i] * b;
-        hjj = -sn[i] * a + cs[i] * b;
+        const double b = h[i + 1];
+        Rj[i] = cs[i] * hjj + sn[i] * b;
+        hjj = -sn[i] * hjj + cs[i] * b;
     }
-    Rj[j] = hjj;
+    return hjj;
+}
+
+__device__ void kv_givens(KrylovCtl* ctl, double hjj, double w2, int j, const KvGivens& G) {
+    double* Rj = G.R + (int64_t)G.m * j;
+    const double sub = sqrt(fmax(w2, 0.0));
     const double den = sqrt(hjj * hjj + sub * sub);
+    Rj[j] = hjj;
     if (den == 0.0) {
         ctl->breakdown = 1;
         ctl->stop = 1;
@@ -578,7 +583,7 @@ kv_axpy_norm_kernel(const double* __restrict__ V, int64_t ldv, int k, int64_t n,
     if (!kv_last_block(&ctl->arrive[2])) return;
     if (threadIdx.x == 0) {
         h[k] = kv_sum_blocks(partial, gridDim.x, 1, 0);
-        kv_givens(ctl, h, G.cs, G.sn, h[k], k - 1, G);
+        kv_givens(ctl, kv_rotate(h, G.cs, G.sn, k - 1, G), h[k], k - 1, G);
         ctl->arrive[2] = 0;
     }
 }
@@ -590,21 +595,29 @@ kv_axpy_norm_kernel(const double* __restrict__ V, int64_t ldv, int k, int64_t n,
 // Gram-Schmidt passes, the norm, the rotation, V[k] = w / |w| and (outer solve)
 // the next product's input t = P V[k], the means taken from w's own.
 // The separate kernels are a chain of latencies, six launches of 5 to 17 us at 5,184
-// entries: 106 us a step beside its 89 us product (25 vectors), 63 us here beside a
+// entries: 106 us a step beside its 89 us product (25 vectors), 55 us here beside a
 // product of 62. Their cost hardly grows with n, while here 16 SMs' FP64 pipes do
-// the 4 n k operations: at 32,000 entries a step takes 1,989 us here and 1,996 there
+// the 4 n k operations: at 32,000 entries a step takes 1,994 us here and 1,996 there
 // (25 vectors, the product included), which is where KV_CLUSTER_N lies.
 // ---------------------------------------------------------------------------
 constexpr int KC_THREADS = 512;
+constexpr int KC_RANKS = 16;
+constexpr int KC_MAXV = 256;          // vectors: the exchange buffers hold every rank's sums
 constexpr int64_t KV_CLUSTER_N = 32768;
+
+__host__ __device__ constexpr int kc_vectors(int k) { return k < 4 ? 4 : k; }
+// the slice, part, full and h1, the rotations, and two buffers of the ranks' sums
+__host__ __device__ constexpr size_t kc_doubles(int64_t slice, int k) {
+    return (size_t)slice + (size_t)(5 + 2 * KC_RANKS) * kc_vectors(k);
+}
 
 struct KcArgs {
     double* V;
-    int64_t n, slice;
-    int k;
+    int n, slice, k;
     double* w;
     URanges ur;
     int project, scale_next;
+    double inv_m;         // 1 / nodes of the u-ranges, 0 without
     double* t;            // P V[k], or NULL
     KvGivens G;
     KrylovCtl* ctl;
@@ -616,116 +629,170 @@ __device__ __forceinline__ double kc_warp_sum(double v) {
     return v;
 }
 
-// full[i] = the sum over the cluster's blocks, in rank order, of their part[i]
-__device__ __forceinline__ void kc_cluster_sum(cg::cluster_group& cl, double* part, double* full, int cnt) {
-    cl.sync();
+// full[i] = the sum over the cluster's blocks, in rank order, of their part[i] (the
+// first three times `scale`): each
+// block stores its sums into the others' buffers and adds its own copy after one
+// barrier. Two buffers in turn: a block that writes one again has passed the
+// barrier that followed its last reads.
+__device__ __forceinline__ void kc_cluster_sum(cg::cluster_group& cl, const double* part, double* buf, double* full,
+                                               int cnt, double scale = 1.0) {
     const int ranks = (int)cl.num_blocks();
-    for (int i = threadIdx.x; i < cnt; i += KC_THREADS) {
-        double s = 0.0;
-        for (int r = 0; r < ranks; r++) s += cl.map_shared_rank(part, r)[i];
-        full[i] = s;
+    __syncthreads();
+    double* mine = buf + cl.block_rank() * cnt;
+    for (int q = threadIdx.x; q < ranks * cnt; q += KC_THREADS) {
+        const int r = q / cnt, i = q - r * cnt;
+        cl.map_shared_rank(mine, r)[i] = part[i];
     }
-    cl.sync();      // part may be written again; full is seen by the block
+    cl.sync();
+    for (int i = threadIdx.x; i < cnt; i += KC_THREADS) {
+        double v[KC_RANKS];
+#pragma unroll
+        for (int r = 0; r < KC_RANKS; r++) v[r] = r < ranks ? buf[r * cnt + i] : 0.0;
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < KC_RANKS; r++) s += v[r];
+        full[i] = scale != 1.0 && i < 3 ? s * scale : s;
+    }
+    __syncthreads();
 }
 
-// part[0..3) = the component sums of the slice over the u-ranges, part[3] = |slice|^2
-__device__ void kc_sums(const double* ws, int64_t t0, int len, const URanges& ur, bool comps, double* part) {
-    __shared__ double red[KC_THREADS / 32][4];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    if (comps)
-        for (int q = 0; q < ur.n; q++) {
-            const int64_t lo = lmax(ur.off[q], t0), hi = lmin(ur.off[q] + ur.len[q], t0 + len);
-            for (int64_t t = lo + threadIdx.x; t < hi; t += KC_THREADS) {
-                const int c = (int)((t - ur.off[q]) % 3);
-                const double x = ws[t - t0];
-                if (c == 0) s[0] += x;
-                else if (c == 1) s[1] += x;
-                else s[2] += x;
-            }
+// the component of entry c of the u-ranges, -1 outside
+__device__ __forceinline__ int kc_component(const URanges& ur, int c) {
+    int m = -1;
+    for (int q = 0; q < ur.n; q++) {
+        const int d = c - (int)ur.off[q];
+        if (d >= 0 && d < (int)ur.len[q]) m = d % 3;
+    }
+    return m;
+}
+
+// part[0..3) = the component sums of the slice over the u-ranges, part[3] = |slice|^2:
+// four warps a sum
+__device__ void kc_sums(const double* ws, int t0, int len, const URanges& ur, bool comps, double* part) {
+    __shared__ double red[16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = warp & 3;
+    if (c == 3 || comps) {
+        double s = 0.0;
+        for (int t = (warp >> 2) * 32 + lane; t < len; t += 128) {
+            const double x = ws[t];
+            if (c == 3) s = fma(x, x, s);
+            else if (kc_component(ur, t0 + t) == c) s += x;
         }
-    for (int t = threadIdx.x; t < len; t += KC_THREADS) s[3] = fma(ws[t], ws[t], s[3]);
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const double v = kc_warp_sum(s[c]);
-        if (lane == 0) red[warp][c] = v;
+        s = kc_warp_sum(s);
+        if (lane == 0) red[warp] = s;
     }
     __syncthreads();
     if (threadIdx.x < 4) {
-        double v = 0.0;
-        for (int q = 0; q < KC_THREADS / 32; q++) v += red[q][threadIdx.x];
-        part[threadIdx.x] = v;
+        const int i = threadIdx.x;
+        part[i] = i == 3 || comps ? (red[i] + red[4 + i]) + (red[8 + i] + red[12 + i]) : 0.0;
     }
 }
+static_assert(KC_THREADS == 512, "kc_sums adds four warps a sum");
 
+// The FP64 pipe issues a warp instruction every 16 cycles an SM, so whatever all 16
+// warps repeat costs 256 cycles an operation: scalars (the means, 1 / |w|) are formed
+// by one warp, and four vectors share a warp's shuffle tree.
 __global__ void __launch_bounds__(KC_THREADS) kv_cluster_kernel(KcArgs a) {
     extern __shared__ __align__(16) double kc_smem[];
-    if (a.ctl->stop) return;          // written after the last cluster barrier only
-    const int mv = a.k < 4 ? 4 : a.k;
+    const int mv = kc_vectors(a.k);
     double* ws = kc_smem;             // the slice
     double* part = ws + a.slice;
     double* full = part + mv;
     double* h1 = full + mv;
     double* cs = h1 + mv;
     double* sn = cs + mv;
+    double* buf[2] = {sn + mv, sn + mv + KC_RANKS * mv};
     cg::cluster_group cl = cg::this_cluster();
-    const int64_t n = a.n, t0 = (int64_t)cl.block_rank() * a.slice;
-    const int len = (int)lmax(0, lmin(a.slice, n - t0));
+    const int n = a.n, k = a.k, t0 = (int)cl.block_rank() * a.slice;
+    const int len = max(0, min(a.slice, n - t0));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k = a.k;
+    const bool rotates = cl.block_rank() == 0 && threadIdx.x == KC_THREADS - 32;
     const double* V = a.V + t0;
-    int64_t total = 0;
-    for (int q = 0; q < a.ur.n; q++) total += a.ur.len[q];
-    const double inv_m = total > 0 ? 1.0 / (double)(total / 3) : 0.0;
     for (int t = threadIdx.x; t < len; t += KC_THREADS) ws[t] = a.w[t0 + t];
     for (int i = threadIdx.x; i < k - 1; i += KC_THREADS) {
         cs[i] = a.G.cs[i];
         sn[i] = a.G.sn[i];
     }
-    __syncthreads();
+    if (a.ctl->stop) return;          // every block reads the same: written after the last cluster barrier
+    // other blocks of the cluster must have started before their buffers are written
+    cl.sync();
     if (a.project) {
         kc_sums(ws, t0, len, a.ur, true, part);
-        kc_cluster_sum(cl, part, full, 3);
-        const double mean[3] = {full[0] * inv_m, full[1] * inv_m, full[2] * inv_m};
-        for (int t = threadIdx.x; t < len; t += KC_THREADS) ws[t] -= proj_mean_at(a.ur, mean, t0 + t);
+        kc_cluster_sum(cl, part, buf[0], full, 3, a.inv_m);
+        for (int t = threadIdx.x; t < len; t += KC_THREADS) {
+            const int m = kc_component(a.ur, t0 + t);
+            if (m >= 0) ws[t] -= full[m];
+        }
         __syncthreads();
     }
     for (int pass = 0; pass < 2; pass++) {
-        for (int i = warp; i < k; i += KC_THREADS / 32) {
-            const double* v = V + (int64_t)i * n;
-            double p[4] = {0.0, 0.0, 0.0, 0.0};
-            int t = lane;
-            for (; t + 96 < len; t += 128)
+        for (int i = 4 * warp; i < k; i += 4 * (KC_THREADS / 32)) {
+            const double* v[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) p[u] = fma(v[t + 32 * u], ws[t + 32 * u], p[u]);
-            for (; t < len; t += 32) p[0] = fma(v[t], ws[t], p[0]);
-            const double s = kc_warp_sum((p[0] + p[1]) + (p[2] + p[3]));
-            if (lane == 0) part[i] = s;
+            for (int u = 0; u < 4; u++) v[u] = V + (int64_t)min(i + u, k - 1) * n;
+            double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+            for (int t = lane; t < len; t += 32) {
+                const double x = ws[t];
+#pragma unroll
+                for (int u = 0; u < 4; u++) p[u] = fma(v[u][t], x, p[u]);
+            }
+            // lanes' bits 4 and 3 choose the vector, the other three are summed
+            const bool b4 = lane & 16, b3 = lane & 8;
+            const double q0 = (b4 ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, b4 ? p[0] : p[2], 16);
+            const double q1 = (b4 ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, b4 ? p[1] : p[3], 16);
+            double s = (b3 ? q1 : q0) + __shfl_xor_sync(0xffffffffu, b3 ? q0 : q1, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const int u = (b4 ? 2 : 0) + (b3 ? 1 : 0);
+            if ((lane & 7) == 0 && i + u < k) part[i + u] = s;
         }
-        kc_cluster_sum(cl, part, full, k);
+        kc_cluster_sum(cl, part, buf[1 - pass], full, k);
         for (int i = threadIdx.x; i < k; i += KC_THREADS) h1[i] = pass ? h1[i] + full[i] : full[i];
         for (int t = threadIdx.x; t < len; t += KC_THREADS) {
             double x = ws[t];
-#pragma unroll 8
-            for (int i = 0; i < k; i++) x = fma(V[(int64_t)i * n + t], -full[i], x);
+            int i = 0;
+            for (; i + 8 <= k; i += 8) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = V[(int64_t)(i + u) * n + t];
+#pragma unroll
+                for (int u = 0; u < 8; u++) x = fma(v[u], -full[i + u], x);
+            }
+            if (i < k) {
+                double v[7];
+#pragma unroll
+                for (int u = 0; u < 7; u++) v[u] = i + u < k ? V[(int64_t)(i + u) * n + t] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 7; u++)
+                    if (i + u < k) x = fma(v[u], -full[i + u], x);
+            }
             ws[t] = x;
         }
         __syncthreads();
     }
     kc_sums(ws, t0, len, a.ur, a.t != nullptr, part);
-    kc_cluster_sum(cl, part, full, 4);
+    kc_cluster_sum(cl, part, buf[1], full, 4);
     const double nrm2 = full[3];
-    const double inv = nrm2 > 0.0 ? 1.0 / sqrt(nrm2) : 0.0;
     if (a.scale_next) {
-        const double mean[3] = {full[0] * inv_m * inv, full[1] * inv_m * inv, full[2] * inv_m * inv};
+        if (warp == 0) {
+            const double inv = nrm2 > 0.0 ? 1.0 / sqrt(nrm2) : 0.0;
+            if (lane == 0) part[3] = inv;
+            else if (lane <= 3) part[lane - 1] = full[lane - 1] * a.inv_m * inv;
+        }
+        __syncthreads();
+        const double inv = part[3];
         double* vn = a.V + (int64_t)k * n + t0;
         for (int t = threadIdx.x; t < len; t += KC_THREADS) {
             const double v = ws[t] * inv;
             vn[t] = v;
-            if (a.t) a.t[t0 + t] = v - proj_mean_at(a.ur, mean, t0 + t);
+            if (a.t) {
+                const int m = kc_component(a.ur, t0 + t);
+                a.t[t0 + t] = m < 0 ? v : v - part[m];
+            }
         }
     }
-    if (cl.block_rank() == 0 && threadIdx.x == 0) kv_givens(a.ctl, h1, cs, sn, nrm2, k - 1, a.G);
+    if (rotates) kv_givens(a.ctl, kv_rotate(h1, cs, sn, k - 1, a.G), nrm2, k - 1, a.G);
 }
 
 // y = R^-1 g over the columns in use: one warp, rows from the bottom, each
@@ -940,8 +1007,12 @@ struct Fgmres {
         const int ranks = cluster_ranks(k);
         if (ranks > 0) {
             KcArgs a;
-            a.V = V; a.n = n; a.slice = ceil_div(n, ranks); a.k = k; a.w = w; a.ur = ur; a.project = project_w;
-            a.scale_next = scale_next; a.t = scale_next ? t : nullptr; a.G = G; a.ctl = ctl;
+            a.V = V; a.n = (int)n; a.slice = (int)ceil_div(n, ranks); a.k = k; a.w = w; a.ur = ur; a.project = project_w;
+            a.scale_next = scale_next;
+            int64_t total = 0;
+            for (int q = 0; q < ur.n; q++) total += ur.len[q];
+            a.inv_m = total >= 3 ? 1.0 / (double)(total / 3) : 0.0;
+            a.t = scale_next ? t : nullptr; a.G = G; a.ctl = ctl;
             cudaLaunchAttribute at;
             cudaLaunchConfig_t cfg = cluster_config(ranks, k, &at);
             const cudaError_t ce = cudaLaunchKernelEx(&cfg, kv_cluster_kernel, a);
@@ -965,7 +1036,7 @@ struct Fgmres {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ranks);
         cfg.blockDim = dim3(KC_THREADS);
-        cfg.dynamicSmemBytes = (size_t)(ceil_div(n, ranks) + 5 * max(k, 4)) * sizeof(double);
+        cfg.dynamicSmemBytes = kc_doubles(ceil_div(n, ranks), k) * sizeof(double);
         cfg.stream = st;
         at->id = cudaLaunchAttributeClusterDimension;
         at->val.clusterDim.x = (unsigned)ranks;
@@ -978,16 +1049,17 @@ struct Fgmres {
     // kernels; asked of the device once a solve
     int cluster_max = -1;
     int cluster_ranks(int k) {
-        if (n > KV_CLUSTER_N || k > 1001) return 0;
+        if (n > KV_CLUSTER_N || k > KC_MAXV) return 0;
         if (cluster_max < 0) {
-            cluster_max = 8;                       // the portable size: 32 KB + 40 KB a block
-            cudaFuncSetAttribute(kv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+            cluster_max = 8;                       // the portable size
+            cudaFuncSetAttribute(kv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kc_doubles(ceil_div(KV_CLUSTER_N, 8), KC_MAXV) * sizeof(double)));
             if (cudaFuncSetAttribute(kv_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
                 cudaLaunchAttribute at;
-                cudaLaunchConfig_t cfg = cluster_config(16, 1001, &at);
+                cudaLaunchConfig_t cfg = cluster_config(KC_RANKS, KC_MAXV, &at);
                 int fit = 0;
                 if (cudaOccupancyMaxActiveClusters(&fit, kv_cluster_kernel, &cfg) == cudaSuccess && fit > 0)
-                    cluster_max = 16;
+                    cluster_max = KC_RANKS;
             }
             cudaGetLastError();
         }
