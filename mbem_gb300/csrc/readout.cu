@@ -16,6 +16,7 @@
 // Near pairs: D below near_factor * max(eps, L); listed per observer in
 // source order (a count pass, a scan, a fill), evaluated in FP64, and added
 // per observer in list order. Every sum runs in a fixed order.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <mutex>
@@ -25,13 +26,19 @@
 
 namespace mbem {
 
+namespace cg = cooperative_groups;
+
 constexpr int RO_Q0 = 9, RO_Q1 = 25, RO_Q2 = 64;
 constexpr int RO_Q = RO_Q0 + RO_Q1 + RO_Q2;
 constexpr int RO_HDR = 16;                    // c_hi[3], c_lo[3], n[3], eps, L, rnear2, pad
-constexpr int RO_REC = RO_HDR + 7 * RO_Q;     // + per point: offset[3], weight, slip[3]
-constexpr int RO_REC_PAD = (RO_REC + 3) / 4 * 4;
+constexpr int RO_REC = RO_HDR + 8 * RO_Q;     // + per point: offset[3], weight, slip[3], pad
 constexpr int RO_THREADS = 128;
-constexpr int RO_TILE = 16;                   // sources staged in shared memory at a time
+constexpr int RO_TILE = 4;                    // sources staged in shared memory at a time, two tiles in turn
+// Observers a block: halved down to 32 while there are fewer blocks than twelve rounds
+// of resident ones (whole readout, 128 | 64 | 32 observers a block: 5,000 observers 4.3 |
+// - | 3.2 ms, 20,000 7.5 | 6.7 | 6.3 ms, 100,000 22.8 | 22.1 | 22.3 ms).
+constexpr int64_t RO_BLOCKS = 12 * 5 * 152;
+constexpr int RO_RANKS = 8;                   // blocks of a cluster: they share the sources of their observers
 
 __constant__ double c_ro_lam[RO_Q][3];
 __constant__ double c_ro_w[RO_Q];
@@ -101,57 +108,62 @@ struct Lattice {
 // per-source record: centroid (double-float), normal, eps, L, near radius^2,
 // and the three rules' points (offset from the centroid, weight x 2 area,
 // interpolated slip)
+// A thread a (source, point), the header by point 0's: 98 points a thread took
+// 1.03 ms for 2,048 sources on 16 blocks, 0.12 ms now.
 __global__ void readout_prep_kernel(const double* __restrict__ tv, const double* __restrict__ normals,
                                     const double* __restrict__ eps, const double* __restrict__ density,
                                     int64_t n_src, Lattice lat, double near_factor, float* __restrict__ rec) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_src) return;
+    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= n_src * RO_Q) return;
+    const int64_t s = id / RO_Q;
+    const int q = (int)(id - s * RO_Q);
     const double* v = tv + 9 * s;
-    float* r = rec + s * RO_REC_PAD;
+    float* r = rec + s * RO_REC;
     double c[3];
-    for (int k = 0; k < 3; k++) {
-        c[k] = ((v[k] + v[3 + k]) + v[6 + k]) / 3.0;
-        const float hi = (float)c[k];
-        r[k] = hi;
-        r[3 + k] = (float)(c[k] - (double)hi);
-        r[6 + k] = (float)normals[3 * s + k];
-    }
-    double L = 0.0;
-    for (int e = 0; e < 3; e++) {
-        const int e2 = (e + 1) % 3;
-        const double dx = v[3 * e2] - v[3 * e], dy = v[3 * e2 + 1] - v[3 * e + 1], dz = v[3 * e2 + 2] - v[3 * e + 2];
-        L = fmax(L, sqrt(dx * dx + dy * dy + dz * dz));
+    for (int k = 0; k < 3; k++) c[k] = ((v[k] + v[3 + k]) + v[6 + k]) / 3.0;
+    if (q == 0) {
+        for (int k = 0; k < 3; k++) {
+            const float hi = (float)c[k];
+            r[k] = hi;
+            r[3 + k] = (float)(c[k] - (double)hi);
+            r[6 + k] = (float)normals[3 * s + k];
+        }
+        double L = 0.0;
+        for (int e = 0; e < 3; e++) {
+            const int e2 = (e + 1) % 3;
+            const double dx = v[3 * e2] - v[3 * e], dy = v[3 * e2 + 1] - v[3 * e + 1], dz = v[3 * e2 + 2] - v[3 * e + 2];
+            L = fmax(L, sqrt(dx * dx + dy * dy + dz * dz));
+        }
+        const double ep = eps[s];
+        const double rn = near_factor * fmax(ep, L);
+        r[9] = (float)ep;
+        r[10] = (float)L;
+        r[11] = (float)(rn * rn);
+        for (int k = 12; k < RO_HDR; k++) r[k] = 0.0f;
     }
     const double e1x = v[3] - v[0], e1y = v[4] - v[1], e1z = v[5] - v[2];
     const double e2x = v[6] - v[0], e2y = v[7] - v[1], e2z = v[8] - v[2];
     const double cx = e1y * e2z - e1z * e2y, cy = e1z * e2x - e1x * e2z, cz = e1x * e2y - e1y * e2x;
     const double area2 = sqrt(cx * cx + cy * cy + cz * cz);
-    const double ep = eps[s];
-    const double rn = near_factor * fmax(ep, L);
-    r[9] = (float)ep;
-    r[10] = (float)L;
-    r[11] = (float)(rn * rn);
-    for (int k = 12; k < RO_HDR; k++) r[k] = 0.0f;
-    for (int q = 0; q < RO_Q; q++) {
-        const double l0 = c_ro_lam[q][0], l1 = c_ro_lam[q][1], l2 = c_ro_lam[q][2];
-        const double lam3[3] = {l0, l1, l2};
-        float* pq = r + RO_HDR + 7 * q;
-        for (int k = 0; k < 3; k++) pq[k] = (float)(((l0 * v[k] + l1 * v[3 + k]) + l2 * v[6 + k]) - c[k]);
-        pq[3] = (float)(c_ro_w[q] * area2);
-        double sl[3] = {0.0, 0.0, 0.0};
-        for (int kk = 0; kk < lat.K; kk++) {
-            double N = 1.0;
-            for (int i = 0; i < 3; i++)
-                for (int j = 0; j < lat.a[kk][i]; j++) N *= (lat.order * lam3[i] - j) / (j + 1);
-            const double* d = density + 3 * (lat.K * s + kk);
-            sl[0] += N * d[0];
-            sl[1] += N * d[1];
-            sl[2] += N * d[2];
-        }
-        pq[4] = (float)sl[0];
-        pq[5] = (float)sl[1];
-        pq[6] = (float)sl[2];
+    const double l0 = c_ro_lam[q][0], l1 = c_ro_lam[q][1], l2 = c_ro_lam[q][2];
+    const double lam3[3] = {l0, l1, l2};
+    float* pq = r + RO_HDR + 8 * q;
+    for (int k = 0; k < 3; k++) pq[k] = (float)(((l0 * v[k] + l1 * v[3 + k]) + l2 * v[6 + k]) - c[k]);
+    pq[3] = (float)(c_ro_w[q] * area2);
+    double sl[3] = {0.0, 0.0, 0.0};
+    for (int kk = 0; kk < lat.K; kk++) {
+        double N = 1.0;
+        for (int i = 0; i < 3; i++)
+            for (int j = 0; j < lat.a[kk][i]; j++) N *= (lat.order * lam3[i] - j) / (j + 1);
+        const double* d = density + 3 * (lat.K * s + kk);
+        sl[0] += N * d[0];
+        sl[1] += N * d[1];
+        sl[2] += N * d[2];
     }
+    pq[4] = (float)sl[0];
+    pq[5] = (float)sl[1];
+    pq[6] = (float)sl[2];
+    pq[7] = 0.0f;
 }
 
 // |x - c| in double-float, as FP32 components
@@ -169,119 +181,228 @@ __device__ __forceinline__ float pair_d2(const float d[3], float eps) {
                      __fmul_rn(eps, eps));
 }
 
+// The near pairs of each observer: their number, or (FILL) the pairs themselves in
+// source order. Headers are staged in shared memory: read in place (one a source, all
+// lanes) the count took 0.59 ms for 100,000 observers x 2,048 sources, 0.18 ms now.
+constexpr int RO_HTILE = 128;
+template <bool FILL>
 __global__ void __launch_bounds__(RO_THREADS)
-readout_count_kernel(const double* __restrict__ x, int64_t n_obs, const float* __restrict__ rec, int64_t n_src,
-                     int64_t* __restrict__ counts) {
+readout_pairs_kernel(const double* __restrict__ x, int64_t n_obs, const float* __restrict__ rec, int64_t n_src,
+                     int64_t* __restrict__ counts, const int64_t* __restrict__ rowptr,
+                     int64_t* __restrict__ pair_obs, int32_t* __restrict__ pair_src) {
+    __shared__ __align__(16) float hdr[RO_HTILE][12];
     const int64_t f = (int64_t)blockIdx.x * RO_THREADS + threadIdx.x;
-    if (f >= n_obs) return;
-    int64_t cnt = 0;
-    for (int64_t s = 0; s < n_src; s++) {
-        const float* r = rec + s * RO_REC_PAD;
-        float d[3];
-        df_offset(x + 3 * f, r, d);
-        cnt += pair_d2(d, r[9]) <= r[11];
-    }
-    counts[f] = cnt;
-}
-
-__global__ void ro_scan_kernel(const int64_t* __restrict__ counts, int64_t n, int64_t* __restrict__ rowptr) {
-    __shared__ int64_t part[1024];
-    const int t = threadIdx.x;
-    const int64_t chunk = (n + 1023) / 1024;
-    const int64_t b0 = t * chunk, b1 = lmin(n, b0 + chunk);
-    int64_t s = 0;
-    for (int64_t i = b0; i < b1; i++) s += counts[i];
-    part[t] = s;
-    __syncthreads();
-    if (t == 0) {
-        int64_t run = 0;
-        for (int i = 0; i < 1024; i++) {
-            const int64_t v = part[i];
-            part[i] = run;
-            run += v;
+    const bool live = f < n_obs;
+    double xo[3] = {0.0, 0.0, 0.0};
+    if (live)
+        for (int k = 0; k < 3; k++) xo[k] = x[3 * f + k];
+    int64_t slot = FILL && live ? rowptr[f] : 0;
+    const int64_t slot_end = FILL && live ? rowptr[f + 1] : 0;
+    for (int64_t s0 = 0; s0 < n_src; s0 += RO_HTILE) {
+        const int ns = (int)lmin(RO_HTILE, n_src - s0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < 3 * ns; t += RO_THREADS)
+            *reinterpret_cast<float4*>(&hdr[t / 3][4 * (t % 3)]) =
+                *reinterpret_cast<const float4*>(rec + (s0 + t / 3) * RO_REC + 4 * (t % 3));
+        __syncthreads();
+        if (!live) continue;
+        for (int t = 0; t < ns; t++) {
+            float d[3];
+            df_offset(xo, hdr[t], d);
+            if (pair_d2(d, hdr[t][9]) <= hdr[t][11]) {
+                if (FILL && slot < slot_end) {
+                    pair_obs[slot] = f;
+                    pair_src[slot] = (int32_t)(s0 + t);
+                }
+                slot++;
+            }
         }
-        rowptr[n] = run;
     }
-    __syncthreads();
-    int64_t run = part[t];
-    for (int64_t i = b0; i < b1; i++) {
-        rowptr[i] = run;
-        run += counts[i];
-    }
+    if (!FILL && live) counts[f] = slot;
 }
 
-// far pairs by quadrature, near pairs listed; a thread per observer, sources
-// staged RO_TILE at a time in shared memory; with EIG the eigenstress of the
-// far pairs goes to eig_out as well
+// rowptr = the exclusive scan of counts, one block, four entries a thread at a time
+// (a strided run a thread took 110 us for 100,000 observers, 83 us now)
+__global__ void __launch_bounds__(1024) ro_scan_kernel(const int64_t* __restrict__ counts, int64_t n,
+                                                       int64_t* __restrict__ rowptr) {
+    __shared__ int64_t wsum[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int64_t base = 0, next[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) next[k] = 4 * t + k < n ? counts[4 * t + k] : 0;
+    for (int64_t i0 = 0; i0 < n; i0 += 4096) {
+        const int64_t i = i0 + 4 * t;
+        int64_t v[4], run = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[k] = run;
+            run += next[k];
+            next[k] = i + 4096 + k < n ? counts[i + 4096 + k] : 0;
+        }
+        int64_t s = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        if (lane == 31) wsum[warp] = s;
+        __syncthreads();
+        int64_t w = wsum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        const int64_t before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+        const int64_t all = __shfl_sync(0xffffffffu, w, 31);
+        const int64_t off = base + (warp > 0 ? before : 0) + (s - run);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (i + k < n) rowptr[i + k] = off + v[k];
+        base += all;
+        __syncthreads();
+    }
+    if (t == 0) rowptr[n] = base;
+}
+
+__device__ __forceinline__ void ro_cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// Far pairs by quadrature; sources staged RO_TILE at a time in shared memory; with
+// EIG the eigenstress of the far pairs goes to eig_out as well. Bound by the FP32 pipe
+// (some 150 operations a point, 9 to 64 points a pair). Neighbouring observers take
+// the same rule and so cost up to seven times others: a thread an observer for all
+// 2,048 sources left half of the SMs idle at the end (22.5 ms for 100,000 observers,
+// 17.1 ms now). A cluster's blocks take every RO_RANKS-th tile of their observers'
+// sources, and where the observers are few a block's threads share them too; the
+// FP64 sums are added in rank, then group order through distributed shared memory.
 template <bool EIG>
-__global__ void __launch_bounds__(RO_THREADS)
+__global__ void __launch_bounds__(RO_THREADS, 5)
 readout_far_kernel(const double* __restrict__ x, int64_t n_obs, const float* __restrict__ rec, int64_t n_src,
-                   RoMat mat, const int64_t* __restrict__ rowptr, int64_t* __restrict__ pair_obs,
-                   int32_t* __restrict__ pair_src, double alpha, int accumulate, double* __restrict__ out,
+                   RoMat mat, int ob, double alpha, int accumulate, double* __restrict__ out,
                    double* __restrict__ eig_out) {
-    extern __shared__ __align__(16) float tile[];
-    const int64_t f = (int64_t)blockIdx.x * RO_THREADS + threadIdx.x;
+    constexpr int NS = EIG ? 12 : 6;
+    __shared__ __align__(16) float tile[2][RO_TILE * RO_REC];
+    static_assert(sizeof(tile) >= NS * RO_THREADS * sizeof(double), "the sums reuse the tiles");
+    cg::cluster_group cl = cg::this_cluster();
+    const int ranks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    // ob observers a block: with fewer than its threads, groups share each tile
+    const int groups = RO_THREADS / ob, group = (int)threadIdx.x / ob;
+    const int64_t f0 = (int64_t)(blockIdx.x / ranks) * ob;
+    const int64_t f = f0 + (int)threadIdx.x % ob;
     const bool live = f < n_obs;
     double xo[3] = {0.0, 0.0, 0.0};
     if (live)
         for (int k = 0; k < 3; k++) xo[k] = x[3 * f + k];
     double acc[6] = {0, 0, 0, 0, 0, 0};
     double acc_e[6] = {0, 0, 0, 0, 0, 0};
-    int64_t slot = live ? rowptr[f] : 0;
-    const int64_t slot_end = live ? rowptr[f + 1] : 0;
-    for (int64_t s0 = 0; s0 < n_src; s0 += RO_TILE) {
+    const int64_t step = (int64_t)ranks * RO_TILE;
+    auto load = [&](int64_t s0, int b) {
+        const int n4 = (int)lmax(0, lmin(RO_TILE, n_src - s0)) * (RO_REC / 4);
+        const float4* src4 = reinterpret_cast<const float4*>(rec + s0 * RO_REC);
+        float4* dst4 = reinterpret_cast<float4*>(tile[b]);
+        for (int t = threadIdx.x; t < n4; t += RO_THREADS) ro_cp16(dst4 + t, src4 + t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load((int64_t)rank * RO_TILE, 0);
+    int b = 0;
+    for (int64_t s0 = (int64_t)rank * RO_TILE; s0 < n_src; s0 += step, b ^= 1) {
         const int ns = (int)lmin(RO_TILE, n_src - s0);
+        load(s0 + step, b ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-        const float4* src4 = reinterpret_cast<const float4*>(rec + s0 * RO_REC_PAD);
-        float4* dst4 = reinterpret_cast<float4*>(tile);
-        for (int t = threadIdx.x; t < ns * RO_REC_PAD / 4; t += RO_THREADS) dst4[t] = src4[t];
-        __syncthreads();
-        if (!live) continue;
-        for (int t = 0; t < ns; t++) {
-            const float* r = tile + t * RO_REC_PAD;
-            float dc[3];
-            df_offset(xo, r, dc);
-            const float eps2 = r[9] * r[9];
-            const float D2 = pair_d2(dc, r[9]);
-            if (D2 <= r[11]) {
-                if (slot < slot_end) {
-                    pair_obs[slot] = f;
-                    pair_src[slot] = (int32_t)(s0 + t);
+        if (live)
+            for (int t = group; t < ns; t += groups) {
+                const float* r = tile[b] + t * RO_REC;
+                float dc[3];
+                df_offset(xo, r, dc);
+                const float eps2 = r[9] * r[9];
+                const float D2 = pair_d2(dc, r[9]);
+                if (D2 <= r[11]) continue;                    // a near pair
+                const float L2 = r[10] * r[10];
+                int q0, q1;
+                if (D2 > 144.0f * L2) { q0 = 0; q1 = RO_Q0; }
+                else if (D2 > 36.0f * L2) { q0 = RO_Q0; q1 = RO_Q0 + RO_Q1; }
+                else { q0 = RO_Q0 + RO_Q1; q1 = RO_Q; }
+                const float nv[3] = {r[6], r[7], r[8]};
+                float sym[6] = {0, 0, 0, 0, 0, 0};
+                float sym_e[6] = {0, 0, 0, 0, 0, 0};
+                for (int q = q0; q < q1; q++) {
+                    const float4* pq = reinterpret_cast<const float4*>(r + RO_HDR + 8 * q);
+                    const float4 o = pq[0], p = pq[1];
+                    const float d[3] = {dc[0] - o.x, dc[1] - o.y, dc[2] - o.z};
+                    const float u[3] = {p.x, p.y, p.z};
+                    point_stress<EIG>(d, u, nv, o.w, eps2, mat, sym, sym_e);
                 }
-                slot++;
-                continue;
-            }
-            const float L2 = r[10] * r[10];
-            int q0, q1;
-            if (D2 > 144.0f * L2) { q0 = 0; q1 = RO_Q0; }
-            else if (D2 > 36.0f * L2) { q0 = RO_Q0; q1 = RO_Q0 + RO_Q1; }
-            else { q0 = RO_Q0 + RO_Q1; q1 = RO_Q; }
-            const float nv[3] = {r[6], r[7], r[8]};
-            float sym[6] = {0, 0, 0, 0, 0, 0};
-            float sym_e[6] = {0, 0, 0, 0, 0, 0};
-            for (int q = q0; q < q1; q++) {
-                const float* pq = r + RO_HDR + 7 * q;
-                const float d[3] = {dc[0] - pq[0], dc[1] - pq[1], dc[2] - pq[2]};
-                const float u[3] = {pq[4], pq[5], pq[6]};
-                point_stress<EIG>(d, u, nv, pq[3], eps2, mat, sym, sym_e);
-            }
 #pragma unroll
-            for (int k = 0; k < 6; k++) acc[k] += (double)sym[k];
-            if (EIG) {
+                for (int k = 0; k < 6; k++) acc[k] += (double)sym[k];
+                if (EIG) {
 #pragma unroll
-                for (int k = 0; k < 6; k++) acc_e[k] += (double)sym_e[k];
+                    for (int k = 0; k < 6; k++) acc_e[k] += (double)sym_e[k];
+                }
             }
+        __syncthreads();
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    double* sums = reinterpret_cast<double*>(&tile[0][0]);
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        sums[k * RO_THREADS + threadIdx.x] = acc[k];
+        if (EIG) sums[(6 + k) * RO_THREADS + threadIdx.x] = acc_e[k];
+    }
+    cl.sync();
+    // each block finishes its share of the observers
+    const int per = ob / ranks;
+    const int t = rank * per + (int)threadIdx.x;
+    if ((int)threadIdx.x < per && f0 + t < n_obs) {
+        double s[NS];
+#pragma unroll
+        for (int k = 0; k < NS; k++) s[k] = 0.0;
+        for (int r = 0; r < ranks; r++) {
+            const double* p = cl.map_shared_rank(sums, r) + t;
+            for (int g = 0; g < groups; g++, p += ob)
+#pragma unroll
+                for (int k = 0; k < NS; k++) s[k] += p[k * RO_THREADS];
+        }
+        constexpr int ix[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+        double* o = out + 9 * (f0 + t);
+#pragma unroll
+        for (int k = 0; k < 9; k++) o[k] = accumulate ? o[k] + alpha * s[ix[k]] : alpha * s[ix[k]];
+        if (EIG) {
+            double* oe = eig_out + 9 * (f0 + t);
+#pragma unroll
+            for (int k = 0; k < 9; k++) oe[k] = accumulate ? oe[k] + alpha * s[6 + ix[k]] : alpha * s[6 + ix[k]];
         }
     }
-    if (!live) return;
-    double* o = out + 9 * f;
-    const double v9[9] = {acc[0], acc[3], acc[4], acc[3], acc[1], acc[5], acc[4], acc[5], acc[2]};
-    for (int k = 0; k < 9; k++) o[k] = accumulate ? o[k] + alpha * v9[k] : alpha * v9[k];
-    if (EIG) {
-        double* oe = eig_out + 9 * f;
-        const double e9[9] = {acc_e[0], acc_e[3], acc_e[4], acc_e[3], acc_e[1], acc_e[5], acc_e[4], acc_e[5], acc_e[2]};
-        for (int k = 0; k < 9; k++) oe[k] = accumulate ? oe[k] + alpha * e9[k] : alpha * e9[k];
-    }
+    cl.sync();      // the others' sums stay until every block has read them
+}
+
+template <bool EIG>
+static int launch_far(const double* x, int64_t n_obs, const float* rec, int64_t n_src, const RoMat& m, double alpha,
+                      int accumulate, double* out, double* eig_out, cudaStream_t st) {
+    int ranks = RO_RANKS;
+    while (ranks > 1 && n_src <= (int64_t)(ranks / 2) * RO_TILE) ranks /= 2;
+    int ob = RO_THREADS;
+    while (ob > 32 && ceil_div(n_obs, ob) * ranks < RO_BLOCKS) ob /= 2;
+    const int64_t grid = ceil_div(n_obs, ob) * ranks;
+    MBEM_REQUIRE(grid < INT32_MAX, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)n_obs);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(RO_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ranks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t ce = cudaLaunchKernelEx(&cfg, readout_far_kernel<EIG>, x, n_obs, rec, n_src, m, ob, alpha,
+                                              accumulate, out, eig_out);
+    if (ce != cudaSuccess) return set_error(MBEM_ERR_CUDA, "readout_far_kernel: %s", cudaGetErrorString(ce));
+    return launch_status("readout_far_kernel");
 }
 
 // out[f] += alpha * sum of its near pairs' stresses, in list order
@@ -322,7 +443,7 @@ using namespace mbem;
 
 extern "C" {
 
-size_t mbem_readout_record_bytes(int64_t n_src) { return (size_t)n_src * RO_REC_PAD * sizeof(float); }
+size_t mbem_readout_record_bytes(int64_t n_src) { return (size_t)n_src * RO_REC * sizeof(float); }
 
 int mbem_readout_prepare(const double* x, int64_t n_obs, const double* tri_verts, const double* normals,
                          const double* eps, int64_t n_src, const double* density, int order, double near_factor,
@@ -337,8 +458,8 @@ int mbem_readout_prepare(const double* x, int64_t n_obs, const double* tri_verts
     if (e) return e;
     cudaStream_t st = (cudaStream_t)stream;
     if (n_src > 0) {
-        readout_prep_kernel<<<(unsigned)ceil_div(n_src, 128), 128, 0, st>>>(tri_verts, normals, eps, density, n_src,
-                                                                            lattice_of(order), near_factor, records);
+        readout_prep_kernel<<<(unsigned)ceil_div(n_src * RO_Q, 128), 128, 0, st>>>(
+            tri_verts, normals, eps, density, n_src, lattice_of(order), near_factor, records);
         if ((e = launch_status("readout_prep_kernel"))) return e;
     }
     if (n_obs == 0) {
@@ -347,9 +468,9 @@ int mbem_readout_prepare(const double* x, int64_t n_obs, const double* tri_verts
         return launch_status("readout memset", 0);
     }
     MBEM_REQUIRE(counts != nullptr, MBEM_ERR_ARG, "NULL counts");
-    readout_count_kernel<<<(unsigned)ceil_div(n_obs, RO_THREADS), RO_THREADS, 0, st>>>(x, n_obs, records, n_src,
-                                                                                       counts);
-    if ((e = launch_status("readout_count_kernel"))) return e;
+    readout_pairs_kernel<false><<<(unsigned)ceil_div(n_obs, RO_THREADS), RO_THREADS, 0, st>>>(
+        x, n_obs, records, n_src, counts, nullptr, nullptr, nullptr);
+    if ((e = launch_status("readout_pairs_kernel"))) return e;
     ro_scan_kernel<<<1, 1024, 0, st>>>(counts, n_obs, rowptr);
     if ((e = launch_status("ro_scan_kernel"))) return e;
     cudaMemcpyAsync(n_near, rowptr + n_obs, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
@@ -380,20 +501,13 @@ int mbem_readout_evaluate_parts(const double* x, int64_t n_obs, const double* tr
     if (n_obs == 0) return MBEM_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const RoMat m = make_romat(mu, lam);
-    const size_t smem = (size_t)RO_TILE * RO_REC_PAD * sizeof(float);
-    const unsigned grid = (unsigned)ceil_div(n_obs, RO_THREADS);
-    if (eig_out) {
-        cudaFuncSetAttribute(readout_far_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        readout_far_kernel<true><<<grid, RO_THREADS, smem, st>>>(x, n_obs, records, n_src, m, rowptr, pair_obs,
-                                                                 pair_src, alpha, accumulate, out, eig_out);
-    } else {
-        cudaFuncSetAttribute(readout_far_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        readout_far_kernel<false><<<grid, RO_THREADS, smem, st>>>(x, n_obs, records, n_src, m, rowptr, pair_obs,
-                                                                  pair_src, alpha, accumulate, out, nullptr);
-    }
-    int e = launch_status("readout_far_kernel");
+    int e = eig_out ? launch_far<true>(x, n_obs, records, n_src, m, alpha, accumulate, out, eig_out, st)
+                    : launch_far<false>(x, n_obs, records, n_src, m, alpha, accumulate, out, nullptr, st);
     if (e) return e;
     if (n_near == 0) return MBEM_OK;
+    readout_pairs_kernel<true><<<(unsigned)ceil_div(n_obs, RO_THREADS), RO_THREADS, 0, st>>>(
+        x, n_obs, records, n_src, nullptr, rowptr, pair_obs, pair_src);
+    if ((e = launch_status("readout_pairs_kernel"))) return e;
     if ((e = nodal_pairs_stress(x, tri_verts, normals, eps, density, mu, lam, order, pair_obs, pair_src, n_near,
                                 pair_out, st, eig_out ? pair_eig : nullptr)))
         return e;

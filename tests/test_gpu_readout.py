@@ -104,3 +104,20 @@ def test_evaluate_stress_mixed_parts_match_fp64(gpu, cube_small):
     assert np.abs(gs - rs).max() < 2e-5 * np.abs(rs).max()
     assert np.abs(ge - re).max() < 2e-5 * np.abs(re).max()
     assert np.abs(ge - g["stress_eigen"]).max() < 2e-5 * np.abs(g["stress_eigen"]).max()
+
+
+# observers a block of 32, 64 and 128 with remainders, and fewer source tiles than a
+# cluster has blocks: the far sums and the listed near pairs are those of the FP64 readout
+@pytest.mark.parametrize("n_fault, n_obs", [(1, 33), (2, 1), (3, 70001), (8, 36737), (8, 73001)])
+def test_mixed_readout_block_shapes(gpu, n_fault, n_obs):
+    from mbem_gb300.kernels import tri_nodal as tn
+    x, tv, n, e, d = _case(1, n_fault=n_fault, n_obs=n_obs, seed=n_obs)
+    x = torch.from_numpy(x).cuda()
+    got = tn.elastic_stress_readout(x, tv, n, e, d, 1.3, 1.95, order=1)
+    eig = torch.zeros((n_obs, 3, 3), dtype=torch.float64, device="cuda")
+    both = tn.elastic_stress_readout(x, tv, n, e, d, 1.3, 1.95, order=1, eig_out=eig)
+    ref = tn.elastic_stress_contract(x, tv, n, e, d, 1.3, 1.95, order=1)
+    scale = float(ref.abs().max())
+    # FP32 quadrature: the file's bound; the same sums with and without the eigenstress
+    assert float((got - ref).abs().max()) < 2e-5 * scale
+    assert float((both - got).abs().max()) < 2e-5 * scale
