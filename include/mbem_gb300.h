@@ -67,6 +67,9 @@ int mbem_fp64_fma_probe(double* out, int64_t iters, int blocks, int threads, voi
  * or out += alpha*M (accumulate=1), so a block lands directly inside a
  * larger system matrix. coeffs: 6 T coefficients (basis.py:58-72 t_coeffs)
  * or 3 U coefficients (basis.py:46-55 u_coeffs). ---------------------- */
+/* *suspect (host) = 1 if a triangle's height over its longest edge is not clearly
+ * above `limit` (or is NaN), else 0; waits for the stream (tri_nodal.py:1239-1254) */
+int mbem_shape_screen(const double* tri_verts, int64_t n, double limit, int* suspect, void* stream);
 int mbem_t_matrix_direct(const double* x_field, int64_t n_field, const double* tri_verts,
                          const double* normals, const double* eps, int64_t n_src,
                          const double* coeffs, int order, double alpha, int accumulate,

@@ -155,6 +155,7 @@ _SIGNATURES = {
     "mbem_launch_count": (ctypes.c_ulonglong, []),
     "mbem_fp32_fma_probe": (c_int, [_P, _I, c_int, c_int, c_int, _P]),
     "mbem_fp64_fma_probe": (c_int, [_P, _I, c_int, c_int, _P]),
+    "mbem_shape_screen": (c_int, [_P, _I, _D, POINTER(c_int), _P]),
     "mbem_t_matrix_direct": (c_int, [_P, _I, _P, _P, _P, _I, _P, c_int, _D, c_int, _P, _I, _P]),
     "mbem_u_matrix_direct": (c_int, [_P, _I, _P, _P, _I, _P, c_int, _D, c_int, _P, _I, _P]),
     "mbem_t_basis_matrices": (c_int, [_P, _I, _P, _P, _P, _I, c_int, _P, _P]),
@@ -313,7 +314,7 @@ def exported_symbols() -> list[str]:
 
 def call(name: str, *args) -> None:
     """Call an entry point and raise MbemError on a non-zero status."""
-    st = getattr(lib(), name)(*args)
+    st = getattr(_lib or lib(), name)(*args)
     if st != OK:
         msg = lib().mbem_last_error()
         msg = msg.decode(errors="replace") if msg else ""
@@ -322,6 +323,10 @@ def call(name: str, *args) -> None:
         raise MbemError(st, name, msg)
 
 
+# array types are made once: ctypes builds a new class for each `c_double * n`'s first use
+_dbl_types = [c_double * n for n in range(8)]
+
+
 def dbl_array(values) -> ctypes.Array:
     vals = [float(v) for v in values]
-    return (c_double * len(vals))(*vals)
+    return _dbl_types[len(vals)](*vals) if len(vals) < len(_dbl_types) else (c_double * len(vals))(*vals)

@@ -18,7 +18,7 @@ import torch
 
 from .. import _native as nat
 from .. import defaults
-from .._device import as_cuda, is_torch, out_like, ptr, stream_handle
+from .._device import as_cuda, is_torch, out_like, ptr, rows3, stream_handle
 
 
 def n_nodes(order: int) -> int:
@@ -30,7 +30,17 @@ def n_nodes(order: int) -> int:
 
 
 def _check_shape(tri_verts: np.ndarray) -> None:
-    """Refuse needles for a nodal density (tri_nodal.py:1239-1254)."""
+    """Refuse needles for a nodal density (tri_nodal.py:1239-1254). Vertices on
+    the device are screened there: only a mesh with a triangle at the limit is
+    copied back and judged here."""
+    if isinstance(tri_verts, torch.Tensor) and tri_verts.is_cuda and tri_verts.dtype is torch.float64 \
+            and tri_verts.get_device() == torch.cuda.current_device() and tri_verts.dim() == 3 \
+            and tri_verts.shape[1:] == (3, 3) and tri_verts.is_contiguous():
+        suspect = ctypes.c_int(0)
+        nat.call("mbem_shape_screen", ptr(tri_verts), tri_verts.shape[0], defaults.NODAL_MIN_HEIGHT_OVER_L,
+                 ctypes.byref(suspect), stream_handle())
+        if not suspect.value:
+            return
     tv = np.asarray(tri_verts.detach().cpu() if isinstance(tri_verts, torch.Tensor) else tri_verts,
                     float)
     if tv.shape[0] == 0:
@@ -48,12 +58,16 @@ def _check_shape(tri_verts: np.ndarray) -> None:
 
 
 def _geom(x_field, tri_verts, eps_arr, normals=None):
-    x = as_cuda(x_field).reshape(-1, 3)
-    tv = as_cuda(tri_verts).reshape(-1, 3, 3)
-    e = as_cuda(eps_arr).reshape(-1)
+    x = rows3(as_cuda(x_field))
+    tv = as_cuda(tri_verts)
+    if tv.dim() != 3 or tv.shape[1:] != (3, 3):
+        tv = tv.reshape(-1, 3, 3)
+    e = as_cuda(eps_arr)
+    if e.dim() != 1:
+        e = e.reshape(-1)
     if e.shape[0] != tv.shape[0]:
         raise ValueError(f"eps array shape ({e.shape[0]},) != ({tv.shape[0]},)")
-    n = None if normals is None else as_cuda(normals).reshape(-1, 3)
+    n = None if normals is None else rows3(as_cuda(normals))
     return x, tv, e, n
 
 
@@ -72,7 +86,7 @@ def t_matrix_direct(x_field, tri_verts, normals, eps_arr, c1, c2, c3, c4, c5, c6
     if order:
         _check_shape(tri_verts)
     x, tv, e, n = _geom(x_field, tri_verts, eps_arr, normals)
-    res = _out_matrix(out, 3 * x.shape[0], 3 * K * tv.shape[0])
+    res = _out_matrix(out, 3 * x.shape[0], 3 * K * tv.shape[0], x.device)
     nat.call("mbem_t_matrix_direct", ptr(x), x.shape[0], ptr(tv), ptr(n), ptr(e), tv.shape[0],
              _coeffs(c1, c2, c3, c4, c5, c6), order, float(alpha), int(bool(accumulate)), ptr(res),
              res.stride(0), stream_handle())
@@ -86,16 +100,16 @@ def u_matrix_direct(x_field, tri_verts, eps_arr, g1, g2, g3, order=0, out=None, 
     if order:
         _check_shape(tri_verts)
     x, tv, e, _ = _geom(x_field, tri_verts, eps_arr)
-    res = _out_matrix(out, 3 * x.shape[0], 3 * K * tv.shape[0])
+    res = _out_matrix(out, 3 * x.shape[0], 3 * K * tv.shape[0], x.device)
     nat.call("mbem_u_matrix_direct", ptr(x), x.shape[0], ptr(tv), ptr(e), tv.shape[0],
              _coeffs(g1, g2, g3), order, float(alpha), int(bool(accumulate)), ptr(res),
              res.stride(0), stream_handle())
     return res if out is not None else out_like(res, is_torch(x_field, tri_verts))
 
 
-def _out_matrix(out, rows, cols):
+def _out_matrix(out, rows, cols, device="cuda"):
     if out is None:
-        return torch.empty((rows, cols), dtype=torch.float64, device=torch.device("cuda"))
+        return torch.empty((rows, cols), dtype=torch.float64, device=device)
     if not isinstance(out, torch.Tensor) or out.dtype != torch.float64 or not out.is_cuda:
         raise ValueError("out must be a float64 CUDA tensor")
     if tuple(out.shape) != (rows, cols) or out.stride(1) != 1:
@@ -129,7 +143,7 @@ def u_basis_matrices(x_field, tri_verts, eps_arr, order=0):
 
 
 def _density(density, n_rows):
-    d = as_cuda(density).reshape(-1, 3)
+    d = rows3(as_cuda(density))
     if d.shape[0] != n_rows:
         raise ValueError(f"density has {d.shape[0]} rows, expected {n_rows}")
     return d
@@ -238,7 +252,7 @@ def traction_matrix(x_field, n_field, tri_verts, normals, eps_arr, ids, n_cols, 
         raise KeyError(which)
     K = n_nodes(order)
     x, tv, e, n = _geom(x_field, tri_verts, eps_arr, normals)
-    nf = as_cuda(n_field).reshape(-1, 3)
+    nf = rows3(as_cuda(n_field))
     ids_np = np.ascontiguousarray(np.asarray(ids.cpu() if isinstance(ids, torch.Tensor) else ids,
                                              dtype=np.int64))
     if ids_np.shape != (tv.shape[0], K):

@@ -93,3 +93,30 @@ def test_normal_branches(drivers, order):
         scale = np.abs(a).max()
         assert np.abs(a + b).max() <= 1e-12 * scale
         assert np.abs(a - c).max() <= 1e-12 * scale
+
+
+# the device's screen refuses what the host's test refuses, at both sides of the limit
+# and for triangles without a length
+@pytest.mark.parametrize("height, ok", [(0.5, True), (1.0000001, True), (1.0, True), (0.9999999, False), (0.0, False)])
+@pytest.mark.parametrize("n", [1, 129])
+def test_needles_refused_on_device(gpu, height, ok, n):
+    from mbem_gb300 import defaults
+    from mbem_gb300.kernels import tri_nodal as tn
+    h = height if height == 0.5 else height * defaults.NODAL_MIN_HEIGHT_OVER_L
+    tv = np.tile(np.array([[0.0, 0.0, 0.0], [1.0, 0.0, 0.0], [0.0, 0.8, 0.0]]), (n, 1, 1))
+    tv[-1] = [[0.0, 0.0, 0.0], [1.0, 0.0, 0.0], [0.5, h, 0.0]]
+    for v in (tv, torch.from_numpy(tv).cuda()):
+        try:
+            tn._check_shape(v)
+            accepted = True
+        except ValueError:
+            accepted = False
+        # at the limit itself the host's rounding decides for both
+        assert accepted == ok or height == 1.0
+    a = [True, True]
+    for i, v in enumerate((tv, torch.from_numpy(tv).cuda())):
+        try:
+            tn._check_shape(v)
+        except ValueError:
+            a[i] = False
+    assert a[0] == a[1]
