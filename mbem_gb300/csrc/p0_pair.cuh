@@ -22,6 +22,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "dp_math.cuh"
 
 namespace mbem {
 
@@ -316,7 +317,7 @@ __device__ __forceinline__ void pair_setup(const SrcP0& s, double ox, double oy,
     double d02 = p.px[0] * p.px[2] + p.py[0] * p.py[2] + p.h2;
     double numer = -p.h * s.area2;
     double denom = p.R[0] * p.R[1] * p.R[2] + p.R[2] * d01 + p.R[0] * d12 + p.R[1] * d02;
-    double omega = 2.0 * atan2(numer, denom);
+    double omega = 2.0 * angle64(numer, denom);
     p.I3 = -omega * ih;
 }
 
@@ -328,10 +329,8 @@ struct EdgeP0 {
 };
 
 // All three edges at once: dJ1 = log((u_b + R_b) / (u_a + R_a)) takes one
-// log per edge, and the three quotients and the three 1/rho^2 share one
-// division each through the product of their denominators.
+// log per edge.
 __device__ __forceinline__ void edges_setup(const SrcP0& s, const PairP0& p, EdgeP0 g[3]) {
-    double num[3], den[3];
 #pragma unroll
     for (int e = 0; e < 3; e++) {
         const int a = e, b = (e + 1) % 3;
@@ -341,28 +340,13 @@ __device__ __forceinline__ void edges_setup(const SrcP0& s, const PairP0& p, Edg
         g[e].ua = p.px[a] * g[e].tx + p.py[a] * g[e].ty;
         g[e].ub = p.px[b] * g[e].tx + p.py[b] * g[e].ty;
         g[e].rho2 = s.edge_ok[e] ? g[e].dp * g[e].dp + p.h2 : 1.0;
-        num[e] = s.edge_ok[e] ? g[e].ub + p.R[b] + 1e-300 : 1.0;
-        den[e] = s.edge_ok[e] ? g[e].ua + p.R[a] + 1e-300 : 1.0;
+        const double num = s.edge_ok[e] ? g[e].ub + p.R[b] + 1e-300 : 1.0;
+        const double den = s.edge_ok[e] ? g[e].ua + p.R[a] + 1e-300 : 1.0;
         g[e].dK1 = p.R[b] - p.R[a];
         g[e].dK3 = p.iR[a] - p.iR[b];
-    }
-    const double r01 = g[0].rho2 * g[1].rho2;
-    const double d01 = den[0] * den[1];
-    const bool tiny = fmin(fmin(g[0].rho2, g[1].rho2), g[2].rho2) < 1e-60;
-    const double ir = tiny ? 0.0 : 1.0 / (r01 * g[2].rho2);
-    const double id = 1.0 / (d01 * den[2]);
-    g[0].ir2 = g[1].rho2 * g[2].rho2 * ir;
-    g[1].ir2 = g[0].rho2 * g[2].rho2 * ir;
-    g[2].ir2 = r01 * ir;
-    if (tiny) {
-#pragma unroll
-        for (int e = 0; e < 3; e++) g[e].ir2 = (g[e].rho2 < 1e-60) ? 0.0 : 1.0 / g[e].rho2;
-    }
-    const double q[3] = {num[0] * den[1] * den[2] * id, num[1] * den[0] * den[2] * id, num[2] * d01 * id};
-#pragma unroll
-    for (int e = 0; e < 3; e++) {
-        const int a = e, b = (e + 1) % 3;
-        g[e].dJ1 = log(q[e]);
+        // rho2 < 1e-60, compared as integers off the FP64 pipe
+        g[e].ir2 = __double_as_longlong(g[e].rho2) < __double_as_longlong(1e-60) ? 0.0 : rcp64(g[e].rho2);
+        g[e].dJ1 = log64(num * rcp64(den));
         g[e].dJ3 = (g[e].ub * p.iR[b] - g[e].ua * p.iR[a]) * g[e].ir2;
         g[e].dL3 = g[e].dJ1 - g[e].rho2 * g[e].dJ3;
     }
