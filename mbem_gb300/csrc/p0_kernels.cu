@@ -10,10 +10,11 @@
 // blocks of a cluster, whose partial sums are added in slice, then rank order
 // through distributed shared memory (deterministic, no workspace).
 //
-// Measured: T block 128 x 128 347 -> 48 us (8 blocks of 16 observers a thread
-// before), 1,728 x 1,728 3.38 -> 2.41 ms (590 FP64 instructions a pair before);
-// T displacement of 6,912 sources at 48 stations 9.98 -> 0.60 ms (6 blocks
-// before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 9.9 ms.
+// Measured: T block 128 x 128 347 -> 24 us (8 blocks of 16 observers a thread
+// before), 1,728 x 1,728 3.38 -> 1.95 ms (590 FP64 instructions a pair before, some 340
+// now; 2.41 with the library's logarithm, atan2 and division);
+// T displacement of 6,912 sources at 48 stations 9.98 -> 0.37 ms (6 blocks
+// before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 9.7 ms.
 #include <cooperative_groups.h>
 #include <string.h>
 
@@ -27,8 +28,6 @@ namespace mbem {
 namespace cg = cooperative_groups;
 
 constexpr int MAT_THREADS = 64;
-constexpr int CON_THREADS = 64;
-constexpr int SRC_TILE = 32;
 constexpr int N_SM = 152;
 
 enum MatKind { MAT_T_DIRECT = 0, MAT_U_DIRECT = 1, MAT_T_BASIS = 2, MAT_U_BASIS = 3 };
@@ -191,7 +190,7 @@ struct ConArgs {
     double alpha;
     int accumulate;
     double* out;
-    int ob;          // observers a block; CON_THREADS / ob slices
+    int ob;          // observers a block; its threads / ob slices
 };
 
 struct SrcTile {
@@ -273,11 +272,11 @@ __device__ __forceinline__ void contract_pair(const SrcTile& T, const double x[3
     }
 }
 
-template <int KIND>
+template <int KIND, int CON_THREADS, int SRC_TILE>
 __global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
     constexpr int NO = KIND >= CON_DD_STRESS ? 6 : 3;
     __shared__ SrcTile tile[SRC_TILE];
-    __shared__ double red[CON_THREADS][NO];
+    __shared__ double red[CON_THREADS][NO], part[8][CON_THREADS / 16 * NO];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
     const int ob = a.ob, slices = CON_THREADS / ob;
@@ -298,9 +297,9 @@ __global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
     for (int64_t s0 = (int64_t)rank * SRC_TILE; s0 < a.n_src; s0 += (int64_t)ranks * SRC_TILE) {
         const int ns = (int)lmin(SRC_TILE, a.n_src - s0);
         __syncthreads();
-        for (int t = threadIdx.x; t < ns; t += CON_THREADS) {
-            const int64_t s = s0 + t;
-            SrcTile& T = tile[t];
+        if ((int)threadIdx.x < ns) {
+            const int64_t s = s0 + threadIdx.x;
+            SrcTile& T = tile[threadIdx.x];
             src_setup(a.tri_verts + 9 * s, a.eps[s], T.g);
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -321,15 +320,33 @@ __global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
 #pragma unroll
     for (int i = 0; i < NO; i++) red[threadIdx.x][i] = acc[i];
     __syncthreads();
-    if (slice == 0) {
-        for (int k = 1; k < slices; k++)
+    // the slices' sums, where there are many of them eight runs first
+    if (slices >= 16) {
+        const int items = ob * NO;
+        for (int it = threadIdx.x; it < 8 * items; it += CON_THREADS) {
+            const int g = it / items, r = it - g * items;
+            double v = 0.0;
+            for (int k = g; k < slices; k += 8) v += red[k * ob + r / NO][r % NO];
+            part[g][r] = v;
+        }
+        __syncthreads();
+        for (int r = threadIdx.x; r < items; r += CON_THREADS) {
+            double v = part[0][r];
 #pragma unroll
-            for (int i = 0; i < NO; i++) acc[i] += red[k * ob + lane][i];
-#pragma unroll
-        for (int i = 0; i < NO; i++) red[lane][i] = acc[i];
+            for (int g = 1; g < 8; g++) v += part[g][r];
+            red[r / NO][r % NO] = v;
+        }
+    } else {
+        for (int r = threadIdx.x; r < ob * NO; r += CON_THREADS) {
+            double v = red[r / NO][r % NO];
+            for (int k = 1; k < slices; k++) v += red[k * ob + r / NO][r % NO];
+            red[r / NO][r % NO] = v;
+        }
     }
     cluster.sync();
     if (rank == 0 && slice == 0 && active) {
+#pragma unroll
+        for (int i = 0; i < NO; i++) acc[i] = red[lane][i];
         for (int r = 1; r < ranks; r++) {
             const double* other = cluster.map_shared_rank(&red[lane][0], r);
 #pragma unroll
@@ -347,12 +364,20 @@ __global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
     cluster.sync();      // the partial sums stay until rank 0 has read them
 }
 
+// A warp alone takes some 5 us for a tile's records and 12 us for a pair, whatever the
+// tile's size, so few observers want large tiles: up to CON_FEW of them one observer a
+// block of 128 threads with 128 sources a tile (6,912 sources at 1 to 19 observers:
+// 480 us with 64 threads and tiles of 32, 150 with these; at 48 observers 507 and 370).
+// Above, contract_split's blocks of observers with 64 threads and tiles of 32 (at 200
+// observers 1,130 us, 1,145 with 128; at 1,000 4,960 and 5,070).
+constexpr int64_t CON_FEW = 76;
+
 template <int KIND>
-static cudaError_t launch_con(const ConArgs& a, int64_t grid, int ranks, cudaStream_t st) {
+static cudaError_t launch_con(const ConArgs& a, bool few, int64_t grid, int ranks, cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(CON_THREADS);
+    cfg.blockDim = dim3(few ? 128 : 64);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -360,7 +385,8 @@ static cudaError_t launch_con(const ConArgs& a, int64_t grid, int ranks, cudaStr
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, p0_contract_kernel<KIND>, a);
+    return few ? cudaLaunchKernelEx(&cfg, p0_contract_kernel<KIND, 128, 128>, a)
+               : cudaLaunchKernelEx(&cfg, p0_contract_kernel<KIND, 64, 32>, a);
 }
 
 static int check_common(const double* x, int64_t nf, const double* tv, const double* eps, int64_t ns,
@@ -402,18 +428,23 @@ int launch_contract(int kind, const double* x, int64_t nf, const double* tv, con
     for (int i = 0; i < 6; i++) a.c[i] = (c && i < nc) ? c[i] : 0.0;
     a.mu = mu; a.lam = lam; a.alpha = alpha; a.accumulate = accumulate; a.out = out;
     if (nf == 0) return MBEM_OK;
-    const ConSplit sp = contract_split(nf, ns, CON_THREADS, CON_THREADS, SRC_TILE, kind >= CON_DD_STRESS ? 500 : 400, 250);
+    const bool few = nf <= CON_FEW;
+    ConSplit sp = {1, 8};
+    if (few)
+        while (sp.ranks > 1 && (int64_t)128 * (sp.ranks / 2) >= ns) sp.ranks /= 2;      // no idle half
+    else
+        sp = contract_split(nf, ns, 64, 64, 32, kind >= CON_DD_STRESS ? 500 : 400, 250);
     a.ob = sp.ob;
     const int64_t grid = ceil_div(nf, sp.ob) * sp.ranks;
     MBEM_REQUIRE(grid < (int64_t)1 << 31, MBEM_ERR_SIZE, "too many observers (%lld)", (long long)nf);
     cudaError_t e;
     switch (kind) {
-        case CON_T_DISP: e = launch_con<CON_T_DISP>(a, grid, sp.ranks, st); break;
-        case CON_U_DISP: e = launch_con<CON_U_DISP>(a, grid, sp.ranks, st); break;
-        case CON_DD_STRESS: e = launch_con<CON_DD_STRESS>(a, grid, sp.ranks, st); break;
-        case CON_KELVIN_STRESS: e = launch_con<CON_KELVIN_STRESS>(a, grid, sp.ranks, st); break;
-        case CON_EIGENSTRESS: e = launch_con<CON_EIGENSTRESS>(a, grid, sp.ranks, st); break;
-        default: e = launch_con<CON_ELASTIC_STRESS>(a, grid, sp.ranks, st); break;
+        case CON_T_DISP: e = launch_con<CON_T_DISP>(a, few, grid, sp.ranks, st); break;
+        case CON_U_DISP: e = launch_con<CON_U_DISP>(a, few, grid, sp.ranks, st); break;
+        case CON_DD_STRESS: e = launch_con<CON_DD_STRESS>(a, few, grid, sp.ranks, st); break;
+        case CON_KELVIN_STRESS: e = launch_con<CON_KELVIN_STRESS>(a, few, grid, sp.ranks, st); break;
+        case CON_EIGENSTRESS: e = launch_con<CON_EIGENSTRESS>(a, few, grid, sp.ranks, st); break;
+        default: e = launch_con<CON_ELASTIC_STRESS>(a, few, grid, sp.ranks, st); break;
     }
     if (e != cudaSuccess) return set_error(MBEM_ERR_CUDA, "p0_contract_kernel: %s", cudaGetErrorString(e));
     return launch_status("p0_contract_kernel");

@@ -49,3 +49,33 @@ def test_against_the_oracle(gpu, oracle, nf, ns, branch):
                       ("kelvin", tk.kelvin_stress_contract(x, tv, e, d, mu, lam)),
                       ("eigen", tk.eigenstress_contract(x, tv, n, e, d, mu, lam))):
         assert _err(got, oracle.contract(name, x, tv, n, e, d, mu=mu, lam=lam)) < TOL
+
+
+# one observer a block and whole blocks of them, tiles of 128 sources with remainders
+# over one to eight blocks a cluster
+@pytest.mark.parametrize("nf,ns", [(1, 128), (3, 129), (19, 1025), (76, 513), (77, 513)])
+def test_few_observers(gpu, oracle, nf, ns):
+    from mbem_gb300.kernels import basis as kb
+    from mbem_gb300.kernels import tri_kernels as tk
+    x, tv, n, e, d = _case(ns, nf, seed=nf)
+    c = kb.t_coeffs(1.0, 1.3)
+    assert _err(tk.t_disp_contract(x, tv, n, e, d, *c), oracle.contract("t_disp", x, tv, n, e, d, c)) < TOL
+    assert _err(tk.dd_stress_contract(x, tv, n, e, d, 1.0, 1.3),
+                oracle.contract("dd", x, tv, n, e, d, mu=1.0, lam=1.3)) < TOL
+
+
+# The T block does not depend on the unit of length: by powers of two it is the same
+# numbers to a few ulps (the file's bound) wherever the element's frame exists. Areas
+# below 1e-30 count as degenerate, and areas whose squares overflow have no frame:
+# zero blocks for both.
+@pytest.mark.parametrize("k", [-60, 0, 60, 330])
+def test_block_in_any_unit(gpu, k):
+    from mbem_gb300.kernels import basis as kb
+    from mbem_gb300.kernels import tri_kernels as tk
+    x, tv, n, e, _ = _case(40, 60)
+    c, s = kb.t_coeffs(1.0, 1.3), 2.0 ** k
+    got = tk.t_matrix_direct(x * s, tv * s, n, e * s, *c)
+    if k in (-60, 330):
+        assert not got.any()
+    else:
+        assert _err(got, tk.t_matrix_direct(x, tv, n, e, *c)) < TOL
