@@ -5,14 +5,14 @@
 //
 // A cluster holds a right-hand side: its vector stays in shared memory from the
 // GEMM's output to the next basis vector, so a step reads the basis four times
-// and nothing else more than once (eleven launches before, the subtractions bound
+// (once from L1) and nothing else more than once (eleven launches before, the subtractions bound
 // by FP64 conversions and each vector through memory seven times). Sums over the
 // vector are FP32 products in eight chains a lane (at most n / (256 C) terms
 // each for C blocks a cluster, as few as one thread's before) added in FP64; the
 // subtractions carry a double-float (TwoProd, TwoSum) and round to FP32 once, as
 // the FP64 ones did.
-// 20,736 unknowns x 256 right-hand sides, 11 basis vectors on average: 300 us
-// a step (0.90 ms before, the GEMM's 0.56 ms apart).
+// 20,736 unknowns x 256 right-hand sides, 11 basis vectors on average: 223 us
+// a step (275 with four readings from L2, 0.90 ms before, the GEMM's 0.48 ms apart).
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -145,6 +145,55 @@ __device__ __forceinline__ void ar_subtract(const float* __restrict__ V, int64_t
     }
 }
 
+// w -= sum_i h_i V_i and part[i] = V_i . w, a piece of 4 AR_T entries after the other:
+// the second reading of a piece's basis entries finds them in L1 (the basis came from
+// L2 four times a step, three times now). The sums are ar_dots'. At most AR_FUSED vectors.
+constexpr int AR_FUSED = 3 * AR_T / 32;
+__device__ __forceinline__ void ar_subtract_dots(const float* __restrict__ V, int64_t stride, float* w, int len, int cnt,
+                                                 const F2* h, double* part) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float s[3][8];
+#pragma unroll
+    for (int v = 0; v < 3; v++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) s[v][c] = 0.0f;
+    for (int p = 0; p < len; p += 4 * AR_T) {
+        const int lim = min(4 * AR_T, len - p);
+        ar_subtract<true>(V + p, stride, w + p, lim, cnt, h);
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+            const int i = warp + v * (AR_T / 32);
+            if (i >= cnt) break;
+            const float* vi = V + i * stride + p;
+            int t = 4 * lane;
+            for (; t + 128 < lim; t += 256) {
+                const float4 a = *reinterpret_cast<const float4*>(vi + t), b = *reinterpret_cast<const float4*>(vi + t + 128);
+                const float4 x = *reinterpret_cast<const float4*>(w + p + t), y = *reinterpret_cast<const float4*>(w + p + t + 128);
+                s[v][0] = fmaf(a.x, x.x, s[v][0]); s[v][1] = fmaf(a.y, x.y, s[v][1]);
+                s[v][2] = fmaf(a.z, x.z, s[v][2]); s[v][3] = fmaf(a.w, x.w, s[v][3]);
+                s[v][4] = fmaf(b.x, y.x, s[v][4]); s[v][5] = fmaf(b.y, y.y, s[v][5]);
+                s[v][6] = fmaf(b.z, y.z, s[v][6]); s[v][7] = fmaf(b.w, y.w, s[v][7]);
+            }
+            if (t < lim) {
+                const float4 a = *reinterpret_cast<const float4*>(vi + t), x = *reinterpret_cast<const float4*>(w + p + t);
+                s[v][0] = fmaf(a.x, x.x, s[v][0]); s[v][1] = fmaf(a.y, x.y, s[v][1]);
+                s[v][2] = fmaf(a.z, x.z, s[v][2]); s[v][3] = fmaf(a.w, x.w, s[v][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+        const int i = warp + v * (AR_T / 32);
+        if (i >= cnt) break;
+        double d = 0.0;
+#pragma unroll
+        for (int c = 0; c < 8; c++) d += (double)s[v][c];
+        d = ar_warp_sum(d);
+        if (lane == 0) part[i] = d;
+    }
+}
+
 __device__ __forceinline__ int ar_parts(const ArnoldiArgs& a, int64_t t) {
     if (a.kb == 0) return a.splits;
     const int tile = (int)(t >> 7);
@@ -218,10 +267,10 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
             part[threadIdx.x] = s;
         }
         ar_cluster_sum(cl, part, full, 3);
+        // three threads divide: an FP64 instruction of all eight warps takes 128 cycles of the SM
+        if (threadIdx.x < 3) hc[threadIdx.x] = split_d(nodes > 0 ? full[threadIdx.x] / (double)nodes : 0.0);
         __syncthreads();
-        F2 mean[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) mean[c] = split_d(nodes > 0 ? full[c] / (double)nodes : 0.0);
+        const F2 mean[3] = {hc[0], hc[1], hc[2]};
         for (int q = 0; q < a.ur.n; q++) {
             const int64_t lo = lmax(a.ur.off[q], t0), hi = lmin(a.ur.off[q] + a.ur.len[q], t0 + len);
             for (int64_t t = lo + threadIdx.x; t < hi; t += AR_T) {
@@ -235,15 +284,17 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
         __syncthreads();
     }
     // classical Gram-Schmidt, twice
+    const bool fused = VEC && cnt <= AR_FUSED;
     for (int pass = 0; pass < 2; pass++) {
-        ar_dots<VEC>(V, stride, w, len, cnt, part);
+        if (pass == 0 || !fused) ar_dots<VEC>(V, stride, w, len, cnt, part);
         ar_cluster_sum(cl, part, full, cnt);
         for (int i = threadIdx.x; i < cnt; i += AR_T) {
             h1[i] = pass ? h1[i] + full[i] : full[i];
             hc[i] = split_d(-full[i]);
         }
         __syncthreads();
-        ar_subtract<VEC>(V, stride, w, len, cnt, hc);
+        if (pass == 0 && fused) ar_subtract_dots(V, stride, w, len, cnt, hc, part);
+        else ar_subtract<VEC>(V, stride, w, len, cnt, hc);
         __syncthreads();
     }
     // the norm
@@ -261,9 +312,14 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
         ar_cluster_sum(cl, part, full, 1);
         __syncthreads();
     }
-    const double nrm = sqrt(full[0]);
+    if (threadIdx.x == 0) {
+        const double nrm = sqrt(full[0]);
+        full[0] = nrm;
+        hc[0] = split_d(nrm > 0.0 ? 1.0 / nrm : 0.0);
+    }
+    __syncthreads();
     // the next basis vector and its operand
-    const F2 inv = split_d(nrm > 0.0 ? 1.0 / nrm : 0.0);
+    const F2 inv = hc[0];
     float* vn = a.V + ((int64_t)(a.j + 1) * a.k + r) * a.n + t0;
     uint16_t* vb = a.Vbf + r * a.ldbf + t0;
     for (int t = threadIdx.x; t < len; t += AR_T) {
@@ -280,6 +336,7 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
     // the column's rotations, by one thread of the right-hand side
     if (rank == 0 && threadIdx.x == 0) {
         const int j = a.j;
+        const double nrm = full[0];
         double col = h1[0];
         for (int i = 0; i < j; i++) {
             const double c = a.cs[i * a.k + r], s = a.sn[i * a.k + r], x = h1[i + 1];

@@ -81,3 +81,35 @@ def test_steps(gpu, n, k, splits, terms, deflate):
     nat.call("mbem_batch_backsolve", ptr(H), ptr(gv), m, steps, k, ptr(Y), stream_handle())
     back = torch.einsum("ilk,lk->ik", torch.triu(H[:steps, :steps].permute(2, 0, 1)).permute(1, 2, 0), Y)
     assert float((back - gv[:steps]).abs().max() / beta.max()) < 1e-10
+
+
+# one vector a warp, two, three, and more than the piecewise pass takes; whole and
+# partial pieces of 1,024 entries. The file's bound: 1e-5.
+@pytest.mark.parametrize("j", [7, 8, 23, 24])
+@pytest.mark.parametrize("n", [1024, 4100, 20736])
+def test_many_vectors(gpu, n, j):
+    from mbem_gb300 import _native as nat
+    from mbem_gb300._device import ptr, stream_handle
+    g = torch.Generator(device="cuda").manual_seed(n + j)
+    k, m, ldp, dev = 3, 30, (n + 7) // 8 * 8, "cuda"
+    V = torch.zeros((m + 1, k, n), device=dev)
+    for r in range(k):
+        q = torch.linalg.qr(torch.randn((n, j + 1), generator=g, device=dev, dtype=torch.float64))[0]
+        V[:j + 1, r] = q.T.float()
+    P = torch.randn((1, k, n), generator=g, device=dev)
+    Vbf = torch.zeros((k, ldp), dtype=torch.bfloat16, device=dev)
+    H = torch.zeros((m, m, k), dtype=torch.float64, device=dev)
+    cs, sn = torch.ones((m, k), dtype=torch.float64, device=dev), torch.zeros((m, k), dtype=torch.float64, device=dev)
+    gv, beta = torch.ones((m + 1, k), dtype=torch.float64, device=dev), torch.ones(k, dtype=torch.float64, device=dev)
+    left = torch.zeros(1, dtype=torch.int32, device=dev)
+    nat.call("mbem_batch_arnoldi", ptr(P), 1, 0, 0, n * k, ptr(V), j, m, k, n, None, 0, ptr(Vbf), Vbf.stride(0), ldp, 1,
+             ptr(H), ptr(cs), ptr(sn), ptr(gv), ptr(beta), 1e-3, ptr(left), stream_handle())
+    w, h = P[0].double(), 0.0
+    for _ in range(2):
+        d = torch.einsum("ikn,kn->ik", V[:j + 1].double(), w)
+        w, h = w - torch.einsum("ik,ikn->kn", d, V[:j + 1].double()), h + d
+    size = P[0].double().norm(dim=1)
+    v = V[j + 1].double()
+    assert float(((v * w.norm(dim=1)[:, None] - w).norm(dim=1) / size).max()) < 1e-5
+    assert float(torch.einsum("ikn,kn->ik", V[:j + 1].double(), v).abs().max()) < 1e-5
+    assert float(((H[:j, j] - h[:j]).abs() / size).max()) < 1e-5
