@@ -112,56 +112,31 @@ __global__ void rotate_row_triples_kernel(double* __restrict__ A, int64_t ld, in
 // ---------------------------------------------------------------------------
 // y = alpha A x + beta y, 128-bit streaming loads of A
 // ---------------------------------------------------------------------------
-// y = alpha A x + beta y, a warp ROWS rows. Bound by the FP64 pipe (one DFMA per
-// 8-byte entry), so the SM with the most rows sets the time: one warp a block
-// leaves at most one block's rows of imbalance (5,184 rows in blocks of 32 gave
-// ten SMs of 152 twice the others' rows: 89 us, 62 us now).
+// y = alpha A x + beta y, a warp a row. Bound by the FP64 pipe (one DFMA per 8-byte
+// entry), so the SM with the most rows sets the time: one warp a block leaves at
+// most a row of imbalance, and the many warps hide each other's loads (5,184 rows in
+// blocks of 32 gave ten SMs of 152 twice the others' rows, 89 us; four rows a warp 63,
+// one 59 us; 3,000 rows 37 and 21 us, 20,000 rows 749 and 681 us).
 constexpr int GEMV_THREADS = 256;        // of the scalar kernel
 
-template <int ROWS>
 __global__ void __launch_bounds__(32)
-dgemv_vec_kernel(const double* __restrict__ A, int64_t ld, int64_t n_rows, int64_t n_cols,
-                 const double* __restrict__ x, double alpha, double beta, double* __restrict__ y) {
+dgemv_vec_kernel(const double* __restrict__ A, int64_t ld, int64_t n_cols, const double* __restrict__ x, double alpha,
+                 double beta, double* __restrict__ y) {
     const int lane = threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * ROWS;
-    const int nr = (int)lmin(ROWS, n_rows - r0);
-    double acc[ROWS];
-#pragma unroll
-    for (int i = 0; i < ROWS; i++) acc[i] = 0.0;
-    const int64_t n2 = n_cols / 2;
+    const int64_t r = blockIdx.x, n2 = n_cols / 2;
     const double2* x2 = reinterpret_cast<const double2*>(x);
-    const double2* rows[ROWS];
-#pragma unroll
-    for (int i = 0; i < ROWS; i++)
-        rows[i] = reinterpret_cast<const double2*>(A + (r0 + min(i, nr - 1)) * ld);
+    const double2* row = reinterpret_cast<const double2*>(A + r * ld);
+    double acc = 0.0;
 #pragma unroll 4
     for (int64_t c = lane; c < n2; c += 32) {
-        const double2 xv = __ldg(x2 + c);
-#pragma unroll
-        for (int i = 0; i < ROWS; i++) {
-            const double2 av = __ldcs(rows[i] + c);
-            acc[i] = fma(av.x, xv.x, acc[i]);
-            acc[i] = fma(av.y, xv.y, acc[i]);
-        }
+        const double2 xv = __ldg(x2 + c), av = __ldcs(row + c);
+        acc = fma(av.x, xv.x, acc);
+        acc = fma(av.y, xv.y, acc);
     }
-    if ((n_cols & 1) && lane == 0) {
-        const double xv = x[n_cols - 1];
+    if ((n_cols & 1) && lane == 0) acc = fma(A[r * ld + n_cols - 1], x[n_cols - 1], acc);
 #pragma unroll
-        for (int i = 0; i < ROWS; i++)
-            acc[i] = fma(A[(r0 + min(i, nr - 1)) * ld + n_cols - 1], xv, acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < ROWS; i++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-    if (lane < nr) {
-        double v = acc[0];
-#pragma unroll
-        for (int i = 1; i < ROWS; i++)
-            if (lane == i) v = acc[i];
-        const int64_t r = r0 + lane;
-        y[r] = (beta == 0.0) ? alpha * v : alpha * v + beta * y[r];
-    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) y[r] = (beta == 0.0) ? alpha * acc : alpha * acc + beta * y[r];
 }
 
 __global__ void __launch_bounds__(GEMV_THREADS)
@@ -182,11 +157,8 @@ int dgemv(const double* A, int64_t ld, int64_t n_rows, int64_t n_cols, const dou
     if (n_rows == 0) return MBEM_OK;
     const bool vec = ((uintptr_t)A % 16 == 0) && ((uintptr_t)x % 16 == 0) && (ld % 2 == 0);
     if (vec) {
-        // four rows a warp share the loads of x; few rows are spread out instead
-        if (n_rows >= 152 * 16)
-            dgemv_vec_kernel<4><<<(unsigned)ceil_div(n_rows, 4), 32, 0, st>>>(A, ld, n_rows, n_cols, x, alpha, beta, y);
-        else
-            dgemv_vec_kernel<1><<<(unsigned)n_rows, 32, 0, st>>>(A, ld, n_rows, n_cols, x, alpha, beta, y);
+        MBEM_REQUIRE(n_rows < INT32_MAX, MBEM_ERR_SIZE, "too many rows (%lld)", (long long)n_rows);
+        dgemv_vec_kernel<<<(unsigned)n_rows, 32, 0, st>>>(A, ld, n_cols, x, alpha, beta, y);
     } else {
         dgemv_scalar_kernel<<<(unsigned)ceil_div(n_rows, GEMV_THREADS / 32), GEMV_THREADS, 0, st>>>(
             A, ld, n_rows, n_cols, x, alpha, beta, y);
@@ -596,7 +568,7 @@ kv_axpy_norm_kernel(const double* __restrict__ V, int64_t ldv, int k, int64_t n,
 // the next product's input t = P V[k], the means taken from w's own.
 // The separate kernels are a chain of latencies, six launches of 5 to 17 us at 5,184
 // entries: 106 us a step beside its 89 us product (25 vectors), 55 us here beside a
-// product of 62. Their cost hardly grows with n, while here 16 SMs' FP64 pipes do
+// product of 59. Their cost hardly grows with n, while here 16 SMs' FP64 pipes do
 // the 4 n k operations: at 32,000 entries a step takes 1,994 us here and 1,996 there
 // (25 vectors, the product included), which is where KV_CLUSTER_N lies.
 // ---------------------------------------------------------------------------
