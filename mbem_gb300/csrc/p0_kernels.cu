@@ -14,7 +14,7 @@
 // before), 1,728 x 1,728 3.38 -> 1.95 ms (590 FP64 instructions a pair before, some 340
 // now; 2.41 with the library's logarithm, atan2 and division);
 // T displacement of 6,912 sources at 48 stations 9.98 -> 0.37 ms (6 blocks
-// before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 9.7 ms.
+// before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 8.7 ms.
 #include <cooperative_groups.h>
 #include <string.h>
 
@@ -261,9 +261,8 @@ __device__ __forceinline__ void contract_pair(const SrcTile& T, const double x[3
                 v[5] = ph * sm.mu * T.dl[1];
             } else {
                 constexpr bool E = KIND == CON_ELASTIC_STRESS;
-                dd_unit<0>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[0], v);
-                dd_unit<1>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[1], v);
-                dd_unit<2>(m3, m5, m7, p.z, g.eps2, sm, E, g.sn * T.dl[2], v);
+                const double w[3] = {g.sn * T.dl[0], g.sn * T.dl[1], g.sn * T.dl[2]};
+                dd_slip(m3, m5, m7, p.z, g.eps2, sm, E, w, v);
             }
         }
         rotate_six(g, v, G);

@@ -281,6 +281,59 @@ __device__ __forceinline__ void dd_unit(const double* m3, const double* m5, cons
 #undef A7
 }
 
+// The same for a slip w (source frame) in one go: the in-plane components meet in
+// sums along the slip, and the normal one's T5 and T7 terms share their factors, some
+// 90 operations less than three dd_unit.
+__device__ __forceinline__ void dd_slip(const double* m3, const double* m5, const double* m7, double z, double eps2,
+                                        const SMat& m, bool eig, const double w[3], double out[6]) {
+#define A5(a, b) m5[nd_tri(a, b)]
+#define A7(a, b) m7[nd_tri(a, b)]
+    const double cb = m.blob * eps2, c15 = 15.0 * cb, z2 = z * z, mu = m.mu, lam = m.lam;
+    const double I3 = m3[0], I5 = A5(0, 0), I7 = A7(0, 0);
+    const double T02 = -z * A5(1, 0), T12 = -z * A5(0, 1), T22 = z2 * I5;
+    const double S02 = -z * A7(1, 0), S12 = -z * A7(0, 1), S22 = z2 * I7;
+    const double F02 = m.k3a * T02 + c15 * S02, F12 = m.k3a * T12 + c15 * S12, F22 = m.k3a * T22 + c15 * S22;
+    const double A = (1.0 - m.c34) * I3 - 3.0 * cb * I5;
+    const double gm = -m.C1 * mu;
+    // in-plane slip
+    const double Ts = w[0] * T02 + w[1] * T12, Ss = w[0] * S02 + w[1] * S12, Fs2 = 2.0 * (w[0] * F02 + w[1] * F12);
+    const double iso = lam * (Fs2 + 12.0 * Ts - 30.0 * eps2 * Ss) - 12.0 * mu * Ts;
+    const double z60 = 60.0 * z, zz = z60 * z, cz = c15 + zz;
+    const double g = 2.0 * A + F22, P = m.k3a * A5(1, 1) + cz * A7(1, 1);
+    const double s00 = iso + mu * (2.0 * w[0] * F02 - z60 * (w[0] * A7(3, 0) + w[1] * A7(2, 1)));
+    const double s11 = iso + mu * (2.0 * w[1] * F12 - z60 * (w[0] * A7(1, 2) + w[1] * A7(0, 3)));
+    const double s22 = iso + mu * (Fs2 + zz * Ss);
+    const double s01 = w[0] * F12 + w[1] * F02 - z60 * (w[0] * A7(2, 1) + w[1] * A7(1, 2));
+    const double s02 = w[0] * (g + m.k3a * A5(2, 0) + cz * A7(2, 0)) + w[1] * P;
+    const double s12 = w[1] * (g + m.k3a * A5(0, 2) + cz * A7(0, 2)) + w[0] * P;
+    // normal slip: l2 (xt T + xs S) + mu (60 z^2 S - 12 T) and the e3 terms
+    const double trT = I3 - eps2 * I5, trS = I5 - eps2 * I7, C22 = T22 - eps2 * S22;
+    const double xd = (4.0 - m.c34) * I3 - 3.0 * trT - 3.0 * cb * I5;
+    const double trX = 3.0 * xd + m.x1 * trT + 15.0 * (trT - eps2 * trS) + c15 * trS;
+    const double trY = 2.0 * A + 6.0 * I3 + 2.0 * F22 - 18.0 * T22 - 6.0 * trT + 30.0 * C22;
+    const double yd = 4.0 * I3 - 12.0 * T22, l2 = 2.0 * lam;
+    const double diag = lam * (lam * trX + mu * trY) + mu * (l2 * xd + mu * yd);
+    const double kt = l2 * (m.x1 + 15.0) - 12.0 * mu, ks = l2 * (c15 - 15.0 * eps2) + mu * zz;
+    const double gw = -m.C1 * w[2], gwm = gw * mu;
+    const double gm2 = gm * mu;
+    out[0] += gm * s00 + gw * diag + gwm * (kt * A5(2, 0) + ks * A7(2, 0));
+    out[1] += gm * s11 + gw * diag + gwm * (kt * A5(0, 2) + ks * A7(0, 2));
+    out[2] += gm * s22 + gw * diag + gwm * (kt * T22 + ks * S22 + 4.0 * mu * (F22 + A));
+    out[3] += gm2 * s01 + gwm * (kt * A5(1, 1) + ks * A7(1, 1));
+    out[4] += gm2 * s02 + gwm * (kt * T02 + ks * S02 + 2.0 * mu * F02);
+    out[5] += gm2 * s12 + gwm * (kt * T12 + ks * S12 + 2.0 * mu * F12);
+    if (eig) {
+        const double phi = m.phi * eps2 * eps2 * I7, pl = phi * lam * w[2], pm = phi * mu;
+        out[0] -= pl;
+        out[1] -= pl;
+        out[2] -= pl + 2.0 * pm * w[2];
+        out[4] -= pm * w[0];
+        out[5] -= pm * w[1];
+    }
+#undef A5
+#undef A7
+}
+
 // Pair geometry shared by all kernels: height, lift, projected vertices,
 // vertex distances and I3 = -Omega / h (tri_kernels.py:257-273).
 struct PairP0 {
@@ -743,13 +796,16 @@ __device__ __forceinline__ void dd_moments(const SrcP0& s, const PairP0& p, doub
     double d3 = 0, d5 = 0, x3[3] = {0, 0, 0}, y3[2] = {0, 0}, x5[6] = {0, 0, 0, 0, 0, 0}, y5[3] = {0, 0, 0};
     EdgeP0 G[3];
     edges_setup(s, p, G);
+    double i3[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) i3[k] = p.iR[k] * p.iR[k] * p.iR[k];
 #pragma unroll
     for (int e = 0; e < 3; e++) {
         if (!s.edge_ok[e]) continue;
         const EdgeP0& g = G[e];
         const int a = e, b = (e + 1) % 3;
         const double A = g.dp * g.nx, B = g.dp * g.ny;
-        const double ia3 = p.iR[a] * p.iR[a] * p.iR[a], ib3 = p.iR[b] * p.iR[b] * p.iR[b];
+        const double ia3 = i3[a], ib3 = i3[b];
         // J5 = u (3 rho^2 + 2 u^2) / (3 rho^4 R^3), K5 = -1 / (3 R^3)
         const double r3 = 3.0 * g.rho2;
         const double J = (g.ub * (r3 + 2.0 * g.ub * g.ub) * ib3 - g.ua * (r3 + 2.0 * g.ua * g.ua) * ia3) *
