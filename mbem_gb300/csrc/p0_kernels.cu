@@ -10,10 +10,10 @@
 // blocks of a cluster, whose partial sums are added in slice, then rank order
 // through distributed shared memory (deterministic, no workspace).
 //
-// Measured: T block 128 x 128 347 -> 24 us (8 blocks of 16 observers a thread
-// before), 1,728 x 1,728 3.38 -> 1.95 ms (590 FP64 instructions a pair before, some 340
+// Measured: T block 128 x 128 347 -> 22.5 us (8 blocks of 16 observers a thread
+// before), 1,728 x 1,728 3.38 -> 1.89 ms (590 FP64 instructions a pair before, some 330
 // now; 2.41 with the library's logarithm, atan2 and division);
-// T displacement of 6,912 sources at 48 stations 9.98 -> 0.37 ms (6 blocks
+// T displacement of 6,912 sources at 48 stations 9.98 -> 0.375 ms (6 blocks
 // before); elastic stress of 1,856 sources at 4,096 points 17.4 -> 8.7 ms.
 #include <cooperative_groups.h>
 #include <string.h>

@@ -381,6 +381,11 @@ struct EdgeP0 {
     double dJ1, dK1, dJ3, dK3, dL3;
 };
 
+// x, or 1e-300 for a zero, by integer operations
+__device__ __forceinline__ double not_zero(double x) {
+    return __double2hiint(x) == 0 ? 1e-300 : x;
+}
+
 // All three edges at once: dJ1 = log((u_b + R_b) / (u_a + R_a)) takes one
 // log per edge.
 __device__ __forceinline__ void edges_setup(const SrcP0& s, const PairP0& p, EdgeP0 g[3]) {
@@ -393,8 +398,8 @@ __device__ __forceinline__ void edges_setup(const SrcP0& s, const PairP0& p, Edg
         g[e].ua = p.px[a] * g[e].tx + p.py[a] * g[e].ty;
         g[e].ub = p.px[b] * g[e].tx + p.py[b] * g[e].ty;
         g[e].rho2 = s.edge_ok[e] ? g[e].dp * g[e].dp + p.h2 : 1.0;
-        const double num = s.edge_ok[e] ? g[e].ub + p.R[b] + 1e-300 : 1.0;
-        const double den = s.edge_ok[e] ? g[e].ua + p.R[a] + 1e-300 : 1.0;
+        const double num = s.edge_ok[e] ? not_zero(g[e].ub + p.R[b]) : 1.0;
+        const double den = s.edge_ok[e] ? not_zero(g[e].ua + p.R[a]) : 1.0;
         g[e].dK1 = p.R[b] - p.R[a];
         g[e].dK3 = p.iR[a] - p.iR[b];
         // rho2 < 1e-60, compared as integers off the FP64 pipe
@@ -534,8 +539,8 @@ __device__ __forceinline__ void t_block(const TMoments& m, const double* __restr
 
 // The T block of one pair (src_normal has been called). For the frame's normal
 // W = T3 . e3 needs n = 5 to degree 2 only and t follows from V3 and V5, so the
-// edges carry four sums less of degree 2 and no third row: about 400 FP64
-// instructions a pair where the general moments take 590.
+// edges carry four sums less of degree 2 and no third row: about 330 FP64
+// instructions a pair where the general moments take 520.
 static __device__ __noinline__ void t_pair_general(const SrcP0& s, const double* nrm, const PairP0& p, const TCoef& c,
                                                    double out[3][3]) {
     TMoments m;
@@ -550,19 +555,21 @@ __device__ __forceinline__ void t_pair(const SrcP0& s, const double* __restrict_
     }
     EdgeP0 G[3];
     edges_setup(s, p, G);
-    double x1 = 0, y1 = 0, d3 = 0, x3 = 0, y3 = 0, x10 = 0, x01 = 0, y01 = 0;
+    // (nx, ny) = (ty, -tx): with a = dp dJ3 the sums of nx v10 and ny v01 add up to that of a
+    double x1 = 0, y1 = 0, d3 = 0, x3 = 0, y3 = 0, x10 = 0, x01 = 0;
 #pragma unroll
     for (int e = 0; e < 3; e++) {
         if (!s.edge_ok[e]) continue;
         const EdgeP0& g = G[e];
-        const double A = g.dp * g.nx, B = g.dp * g.ny;
-        const double v10 = A * g.dJ3 + g.tx * g.dK3, v01 = B * g.dJ3 + g.ty * g.dK3;
+        const double a = g.dp * g.dJ3;
+        const double v10 = g.nx * a + g.tx * g.dK3, v01 = g.ny * a + g.ty * g.dK3;
         x1 += g.nx * g.dJ1; y1 += g.ny * g.dJ1;
-        d3 += g.dp * g.dJ3;
+        d3 += a;
         x3 += g.nx * g.dJ3; y3 += g.ny * g.dJ3;
         x10 += g.nx * v10;
-        x01 += g.nx * v01; y01 += g.ny * v01;
+        x01 += g.nx * v01;
     }
+    const double y01 = d3 - x10;
     const double th = 1.0 / 3.0, I3 = p.I3;
     double B[3][3];
     t_local(I3, -x1, -y1, (d3 + I3) * p.ih2 * th, -x3 * th, -y3 * th, (I3 - x10) * th, -x01 * th, (I3 - y01) * th, p.z,
