@@ -215,11 +215,17 @@ residual_near_kernel(const double* __restrict__ X, int64_t k, int64_t n, mbem_ne
         const int64_t f = lr / 3;
         const int a = (int)(lr % 3);
         const double* x = X + r * n;
+        // a sum a column of the blocks: three operations a block (four with the block's
+        // own sum taken off v, 3.2 ms for 20,736 unknowns x 256 against 2.25)
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
         for (int64_t q = nb.rowptr[f]; q < nb.rowptr[f + 1]; q++) {
             const int64_t c0 = nb.col0 + 3 * nb.cols[q];
             const double* blk = nb.vals + 9 * q + 3 * a;
-            v -= blk[0] * x[c0] + blk[1] * x[c0 + 1] + blk[2] * x[c0 + 2];
+            s0 = fma(blk[0], x[c0], s0);
+            s1 = fma(blk[1], x[c0 + 1], s1);
+            s2 = fma(blk[2], x[c0 + 2], s2);
         }
+        v -= (s0 + s1) + s2;
         R[r * n + row] = v;
     }
 }
