@@ -5,8 +5,8 @@
 //
 // Bound by the FP64 pipe. Against one thread per pair with run-time degrees and
 // tables in local memory (the 32-term series and about 12 KB a thread before),
-// the 8-per-face cube's P1 T block (1.77e6 pairs) went from 63.2 to 4.5 ms,
-// a ragged P2 U block (1,001 x 333) from 26.9 to 1.6 ms.
+// the 8-per-face cube's P1 T block (1.77e6 pairs) went from 63.2 to 4.1 ms,
+// a ragged P2 U block (1,001 x 333) from 26.9 to 1.4 ms.
 #include "nodal_launch.cuh"
 
 namespace mbem {

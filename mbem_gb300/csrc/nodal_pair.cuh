@@ -210,13 +210,9 @@ __device__ __forceinline__ void edge_gauss(double uc, double hl, double rho2, in
 #pragma unroll 2
     for (int q = q0; q < q1; q++) {
         const double u = uc + hl * MBEM_ND_RULES.ex[q];
-        const double iR = rsqrt(u * u + rho2);
-        double f = iR;
-        if (TOP >= 3) {
-            const double iR2 = iR * iR;
-            f *= iR2;
-            if (TOP >= 5) f *= iR2;
-        }
+        double f;
+        if constexpr (TOP == 1) f = rsqrt(u * u + rho2);
+        else f = inv_pow64<TOP>(u * u + rho2);
 #pragma unroll
         for (int k = 0; k <= KT; k++) s[k] += f * MBEM_ND_RULES.ew[q][k];
     }
@@ -437,8 +433,10 @@ __device__ __forceinline__ void nodal_moments(const NodalRec& g, const NodalObs&
     const double d01 = px[0] * px[1] + py[0] * py[1] + h2;
     const double d12 = px[1] * px[2] + py[1] * py[2] + h2;
     const double d02 = px[0] * px[2] + py[0] * py[2] + h2;
-    const double I3 =
-        -2.0 * atan2(-h * g.area2s, R[0] * R[1] * R[2] + R[2] * d01 + R[0] * d12 + R[1] * d02) * ih;
+    // (the P2 kernels keep the library's: the short one took their stress at 512 sources x
+    // 2,000 points from 4.9 to 5.6 ms, P1 matrices from 4.3 to 4.1 with the edges' powers)
+    const double num = -h * g.area2s, den = R[0] * R[1] * R[2] + R[2] * d01 + R[0] * d12 + R[1] * d02;
+    const double I3 = -2.0 * (P < 2 ? angle64(num, den) : atan2(num, den)) * ih;
 
     constexpr int e5 = G::e5, e3 = G::e3, e1 = G::e1, em1 = G::em1;
     double b5[nd_len(e5)], c5[nd_max(e5, 0) + 1], b3[nd_len(e3)], c3[nd_max(e3, 0) + 1], b1[nd_len(e1)],

@@ -6,7 +6,7 @@
 // does not depend on the order of the adds).
 //
 // Bound by the FP64 pipe. 288 points x 6,144 P0 sources ("slip"): 70.2 ms with
-// run-time tables in local memory and 144 / 64 far points, 4.05 ms now.
+// run-time tables in local memory and 144 / 64 far points, 3.97 ms now.
 #include "nodal_launch.cuh"
 
 namespace mbem {

@@ -120,3 +120,19 @@ def test_needles_refused_on_device(gpu, height, ok, n):
         except ValueError:
             a[i] = False
     assert a[0] == a[1]
+
+
+# The P1 T block does not depend on the unit of length: by powers of two the same numbers
+# to a few ulps of the largest (1e-11 as for the P0 blocks), also where the distances'
+# fifth powers leave the range of the short ones (lengths above 2^192).
+@pytest.mark.parametrize("k", [-40, 60, 195])
+def test_nodal_block_in_any_unit(gpu, k):
+    from mbem_gb300.kernels import basis as kb
+    from mbem_gb300.kernels import tri_nodal as tn
+    m = M.centre_fault(4)
+    x = np.random.default_rng(3).uniform(-1, 1, size=(50, 3))
+    tv, n, e = m.tri_verts(), m.normals_and_areas()[0], np.full(m.tri_verts().shape[0], 0.05)
+    c, s = kb.t_coeffs(1.0, 1.3), 2.0 ** k
+    ref = tn.t_matrix_direct(x, tv, n, e, *c, order=1)
+    got = tn.t_matrix_direct(x * s, tv * s, n, e * s, *c, order=1)
+    assert np.abs(got - ref).max() < 1e-11 * np.abs(ref).max()
