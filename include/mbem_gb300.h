@@ -659,10 +659,13 @@ int mbem_batch_backsolve(const double* H, const double* g, int m, int cnt, int64
 int mbem_batch_project(void* X, int is_f64, int64_t k, int64_t n, const int64_t* u_ranges, int n_u_ranges,
                        void* stream);
 /* R = B - A X for the mixed operator and k right-hand sides (k, n) FP64: the
- * far field (FP32 entries) by exact tensor-core products of six eight-bit
- * digits, right to 2^-48 of max|A_i| max|X_r| a term, the near blocks in FP64.
+ * far field (FP32 entries) by exact tensor-core products of eight-bit digits, the
+ * near blocks in FP64. A is scaled by powers of two by rows and by columns, X by
+ * the inverse column scales and by right-hand sides; a term is off by at most
+ * 7 x 2^-48 of the scaled largest entries, and by less where a right-hand side's scaled
+ * entries differ by many bits (more digits, as the device decides).
  * A row or right-hand side with an Inf or NaN gives NaN. The workspace holds the
- * digits of up to 6 GiB of rows at a time. */
+ * digits of up to 2 GiB of rows at a time. */
 size_t mbem_batch_residual_workspace_size(int64_t k, int64_t n);
 int mbem_batch_residual_mixed(const mbem_mixed_operator* op, const double* B, const double* X, int64_t k, double* R,
                               void* work, size_t work_bytes, void* stream);

@@ -74,8 +74,8 @@ int gj_block_update_tc(float* M, int64_t n, int64_t ld, int64_t k0, int b, uint1
 // C[M x N] -= A[M x K] B[N x K]^T on the tensor cores (BF16 operands, FP32 C).
 int gemm_bf16_sub(const void* A, int64_t lda, const void* Bt, int64_t ldb, int64_t M, int64_t N, int64_t K, float* C,
                   int64_t ldc, cudaStream_t st);
-// R = B - A X for k right-hand sides (rows of n), A n x n FP32, exact to about 2^-48
-// of |A| |X| on the tensor cores (tc_exact.cu).
+// R = B - A X for k right-hand sides (rows of n), A n x n FP32, on the tensor cores: a term
+// is off by at most 7 x 2^-48 of its row's, column's and right-hand side's scales (tc_exact.cu).
 size_t exact_residual_workspace(int64_t k, int64_t n);
 int exact_residual(const float* A, int64_t lda, int64_t n, const double* B, const double* X, int64_t k, double* R,
                    void* work, size_t work_bytes, cudaStream_t st);

@@ -2,21 +2,35 @@
 // tensor-core products of fixed-point digits (sm_103a).
 //
 // A refinement residual has to be right to about 2^-48 of |A| |X| while A X
-// cancels B, so no FP32 accumulation of rounded products will do. Every row of A
-// and every right-hand side is scaled by a power of two into [-1, 1] and cut into
-// six signed digits of eight bits, integers in [-128, 128], which BF16 holds
-// exactly (48 bits: every bit of an FP32 entry down to 2^-24 of its row's
-// largest). A product of two digits is at most 2^14 and 256 of them sum to at
+// cancels B, so no FP32 accumulation of rounded products will do. A is scaled by
+// powers of two, a row by r_i and then a column by c_j <= 1 (its largest entry of
+// the scaled rows), X by the inverse column scales and one a right-hand side, all into
+// [-1, 1]: systems with traction unknowns hold columns of 1 / mu beside unknowns of mu,
+// which one scale a row and one a right-hand side would cut away. Both are cut into
+// signed digits of eight bits, integers in [-128, 128], which BF16 holds exactly.
+// A product of two digits is at most 2^14 and 256 of them sum to at
 // most 2^22, so the tensor core's FP32 accumulator is exact over 256 columns; the
 // epilogue adds it to 32-bit integers (exact up to 131,072 columns) while the next
-// 256 run into a second accumulator. The 21 digit products of order p + q <= 5
-// are combined in FP64; what the cut leaves out is below 2^-48 of
-// max|A_i| max|X_r| a term. (Error-free splitting for matrix products: Ozaki,
+// 256 run into a second accumulator. The digit products of order p + q <= o
+// are combined; what is left out is below (o + 2) 2^(-8 (o + 1)) of the scales a term
+// (o + 1 products of the next order a bit over half a unit each, both last digits
+// rounded): 7 x 2^-48 for o = 5. (Error-free splitting for matrix products: Ozaki,
 // Ogita, Oishi, Rump, Numer. Algorithms 59, 2012.)
 //
+// The order is 5 (six digits, 21 products) where the entries of each scaled right-hand side lie
+// close to its largest one, and grows by one for every eight bits that they lie below
+// (ex_rhs_scale_kernel decides on the device): with o = 5 alone, one entry 10^4 times
+// the others cost the other rows a factor of 60 against the double-float product.
+// Against it (FP32 pairs, every entry with its own exponent) the errors are smaller
+// or equal for X of up to 14 decades, mu up to 3e10 and blocks of two materials
+// (emulated, 2,592 unknowns, largest and rms error relative to |A| |X|: balanced
+// random X 2e-16 | 4e-17 against 4e-13 | 4e-14; one entry 10^8 times the others
+// 3e-16 | 5e-17 against 7e-12 | 7e-13).
+//
 // Bound by the tensor pipe and the L2 traffic of its operands: 20,736 unknowns x
-// 256 right-hand sides 5.2 ms (splitting 1.5 ms, 21 products 3.5 ms at 1.33 PFLOP/s, 0.69 of the measured bf16 rate,
-// combination 0.1 ms), against 49 ms for a double-float product on the FP32
+// 256 right-hand sides 5.85 ms (row and column scales 0.53 ms, digits 1.4, 21 products
+// 3.6 ms at 1.29 PFLOP/s, 0.68 of the measured bf16 rate, combination 0.2 ms; 5.17 ms
+// with one scale a row), against 49 ms for a double-float product on the FP32
 // pipe (eleven instructions a term at 70 % of its issue slots).
 #include <limits.h>
 #include <math.h>
@@ -27,126 +41,226 @@
 
 namespace mbem {
 
-constexpr int EX_D = 6;                       // digits
-constexpr int EX_PAIRS = EX_D * (EX_D + 1) / 2;
+constexpr int EX_ORDER = 5, EX_ORDER_MAX = 11;     // least and largest order of the digit products
+constexpr int EX_DA = 8;                      // most digits of A: 64 bits, FP32 entries whole down to 2^-40 of the scales
+constexpr int EX_DX = EX_ORDER_MAX + 1;       // most digits of X
+// digits of A and digit products at order o
+__host__ __device__ constexpr int ex_digits_a(int o) { return o + 1 < EX_DA ? o + 1 : EX_DA; }
+__host__ __device__ constexpr int ex_pairs(int o) {
+    const int d = ex_digits_a(o);
+    return d * (o + 1) - d * (d - 1) / 2;
+}
 constexpr int EX_CHUNK = 4;                   // K blocks an accumulator takes: 256 columns, 2^22
 constexpr int EX_STAGES = 4;
 constexpr int EX_THREADS = 320;               // eight epilogue warps, producer, issuer
 constexpr int EX_NONFINITE = INT_MIN;         // exponent of a row that holds an Inf or NaN
+constexpr int EX_DEAD = -(1 << 20);           // exponent of a column without an entry
 
-// digits of v in [-1, 1] as BF16 bit patterns
-__device__ __forceinline__ void digits_f32(float v, uint16_t d[EX_D]) {
-    float r = v * 128.0f;
-#pragma unroll
-    for (int p = 0; p < EX_D; p++) {
-        const float t = rintf(r);
-        d[p] = (uint16_t)(__float_as_uint(t) >> 16);       // |t| <= 128: eight bits
-        r = (r - t) * 256.0f;                              // exact
-    }
-}
-__device__ __forceinline__ void digits_f64(double v, uint16_t d[EX_D]) {
-    double r = v * 128.0;
-#pragma unroll
-    for (int p = 0; p < EX_D; p++) {
-        const double t = rint(r);
-        d[p] = (uint16_t)(__float_as_uint((float)t) >> 16);
-        r = (r - t) * 256.0;
-    }
+// the exponent e of |v| = f 2^e, f in [1/2, 1), from the bits of a finite |v| > 0 (a subnormal
+// FP32 entry counts as 2^-127)
+__device__ __forceinline__ int ex_exp(int bits) { return (bits >> 23) - 126; }
+__device__ __forceinline__ int ex_exp(double v) {
+    const int e = (__double2hiint(v) >> 20) & 2047;
+    if (e > 0) return e - 1022;
+    int q;
+    frexp(v, &q);
+    return q;
 }
 
-__device__ __forceinline__ double ex_block_max(double v, double* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+// the exponents r_i of the rows of A (n columns at lda): EX_NONFINITE with an Inf or NaN,
+// 0 without an entry; a block a row
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+ex_row_scale_kernel(const float* __restrict__ A, int64_t lda, int64_t cols, int* __restrict__ ex) {
+    __shared__ int red[8];
+    const int64_t row = blockIdx.x;
+    const float* a = A + row * lda;
+    int m = 0;                                 // largest |a| as bits: an order on them, Inf and NaN above all
+    const int64_t c4 = VEC ? cols / 4 * 4 : 0;
+    for (int64_t c = 4 * threadIdx.x; c < c4; c += 1024) {
+        const float4 v = *reinterpret_cast<const float4*>(a + c);
+        m = max(max(m, __float_as_int(fabsf(v.x))), __float_as_int(fabsf(v.y)));
+        m = max(max(m, __float_as_int(fabsf(v.z))), __float_as_int(fabsf(v.w)));
+    }
+    for (int64_t c = c4 + threadIdx.x; c < cols; c += 256) m = max(m, __float_as_int(fabsf(a[c])));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
-    double m = red[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmax(m, red[w]);
-    return m;
-}
-// the exponent e with 2^e >= m, and 2^-e as two factors (either may be subnormal's)
-__device__ __forceinline__ int ex_exponent(double m, bool finite) {
-    if (!finite) return EX_NONFINITE;
-    if (!(m > 0.0)) return 0;
-    int e;
-    frexp(m, &e);
-    return e;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) m = max(m, red[w]);
+        ex[row] = m >= 0x7f800000 ? EX_NONFINITE : m == 0 ? 0 : ex_exp(m);
+    }
 }
 
-// Rows row0 .. row0 + n_rows of A (columns col0 .. col0 + cols) as digits
-// D[p][row][ld], zero from cols to ld; a block a row, its exponent in ex.
+// cmax[j] = the largest exponent of column j of the scaled rows as exponent - EX_DEAD (0: none),
+// by atomics: a block EX_CROWS rows of 1,024 columns, a thread four of them. The row that
+// has its largest entry in column j leaves it at 0, so a scaled row's largest entry stays
+// in [1/2, 1).
+constexpr int EX_CROWS = 64;
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+ex_col_scale_kernel(const float* __restrict__ A, int64_t lda, int64_t rows, int64_t cols, const int* __restrict__ ex,
+                    int* __restrict__ cmax) {
+    __shared__ int er[EX_CROWS];
+    const int64_t c = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4, r0 = (int64_t)blockIdx.y * EX_CROWS;
+    const int nr = (int)lmin(EX_CROWS, rows - r0);
+    if ((int)threadIdx.x < nr) er[threadIdx.x] = ex[r0 + threadIdx.x];
+    __syncthreads();
+    if (c >= cols) return;
+    const float* a = A + r0 * lda + c;
+    const int nc = (int)lmin(4, cols - c);
+    // an entry's bits less its row's exponent: their top is the scaled entry's exponent
+    constexpr int NONE = INT_MIN;
+    int m[4] = {NONE, NONE, NONE, NONE};
+#pragma unroll 8
+    for (int i = 0; i < nr; i++) {
+        float v[4];
+        if (VEC && nc == 4) {
+            const float4 q = *reinterpret_cast<const float4*>(a + i * lda);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = u < nc ? a[i * lda + u] : 0.0f;
+        }
+        const int e = er[i];
+        if (e == EX_NONFINITE) continue;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int b = __float_as_int(fabsf(v[u]));
+            m[u] = max(m[u], b ? b - (e << 23) : NONE);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (m[u] != NONE) atomicMax(&cmax[c + u], ex_exp(m[u]) - EX_DEAD);
+}
+
+// Exponents of the right-hand sides' largest entries under the column scales, and the order
+// that they need: an entry's error goes with the largest one, so the digits go on as
+// far as most entries lie below it (mean and standard deviation of their exponents;
+// 3 bits for smooth and 5 for random X), and half a bit
+// a factor of two in the columns that the double-float sum's error grows by. Six
+// digits are then no worse than it up to some 8 bits (a random X with one entry 10
+// times its largest: 7.3 bits, rms error 4e-14 against 3e-14; 10^3 times, 13 bits, 1e-12 against
+// 5e-14). A block a right-hand side; *extra is raised to the largest order - EX_ORDER.
+__global__ void __launch_bounds__(256)
+ex_rhs_scale_kernel(const double* __restrict__ X, int64_t ldx, int64_t cols, const int* __restrict__ cmax,
+                    float few, int* __restrict__ ex, int* __restrict__ extra) {
+    __shared__ int rm[8];
+    __shared__ long long rs[8][3];
+    const int64_t r = blockIdx.x;
+    const double* x = X + r * ldx;
+    int m = INT_MIN;
+    long long s[3] = {0, 0, 0};                // entries, their exponents' sum and sum of squares
+    bool ok = true;
+    for (int64_t c = threadIdx.x; c < cols; c += 256) {
+        const double v = x[c];
+        ok = ok && isfinite(v);
+        if (!isfinite(v) || v == 0.0 || cmax[c] == 0) continue;
+        const int e = ex_exp(v) + cmax[c] + EX_DEAD;
+        m = max(m, e);
+        s[0]++;
+        s[1] += e;
+        s[2] += (long long)e * e;
+    }
+    const bool finite = __syncthreads_and(ok);
+    m = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+    if ((threadIdx.x & 31) == 0) {
+        rm[threadIdx.x >> 5] = m;
+        for (int k = 0; k < 3; k++) rs[threadIdx.x >> 5][k] = s[k];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; w++) {
+        m = max(m, rm[w]);
+        for (int k = 0; k < 3; k++) s[k] += rs[w][k];
+    }
+    ex[r] = !finite ? EX_NONFINITE : s[0] == 0 ? 0 : m;
+    if (!finite || s[0] == 0) return;
+    const float mean = (float)((double)s[1] / (double)s[0]);
+    const float sd = sqrtf(fmaxf((float)((double)s[2] / (double)s[0] - (double)mean * mean), 0.0f));
+    const float need = ((float)m - mean + sd + few - 8.0f) / 8.0f;
+    const int o = need > 0.0f ? (int)ceilf(fminf(need, (float)(EX_ORDER_MAX - EX_ORDER))) : 0;
+    if (o > 0) atomicMax(extra, o);
+}
+
+// Rows of A under both scales as digits D[p][row][ld], p < ex_digits_a(order), zero from
+// cols to ld; a block a row
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 ex_split_rows_kernel(const float* __restrict__ A, int64_t lda, int64_t cols, int64_t rows_pad, int64_t ld,
-                     uint16_t* __restrict__ D, int* __restrict__ ex) {
-    __shared__ double red[8];
+                     const int* __restrict__ ex, const int* __restrict__ cmax, const int* __restrict__ extra,
+                     uint16_t* __restrict__ D) {
     const int64_t row = blockIdx.x;
     const float* a = A + row * lda;
-    float m = 0.0f;
-    bool ok = true;
-    if (VEC) {
-        for (int64_t c = 4 * threadIdx.x; c + 3 < cols; c += 1024) {
-            const float4 v = *reinterpret_cast<const float4*>(a + c);
-            m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-            ok = ok && isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
-        }
-        for (int64_t c = cols / 4 * 4 + threadIdx.x; c < cols; c += 256) {
-            m = fmaxf(m, fabsf(a[c]));
-            ok = ok && isfinite(a[c]);
-        }
-    } else {
-        for (int64_t c = threadIdx.x; c < cols; c += 256) {
-            m = fmaxf(m, fabsf(a[c]));
-            ok = ok && isfinite(a[c]);
-        }
-    }
-    const bool finite = __syncthreads_and(ok);
-    const int e = ex_exponent(ex_block_max((double)m, red), finite);
-    if (threadIdx.x == 0) ex[row] = e;
-    const int e1 = finite ? -(e / 2) : 0, e2 = finite ? -e - e1 : 0;
-    const float f1 = finite ? ldexpf(1.0f, e1) : 0.0f, f2 = finite ? ldexpf(1.0f, e2) : 0.0f;
+    const int e = ex[row], nd = ex_digits_a(EX_ORDER + *extra);
+    const bool finite = e != EX_NONFINITE;
     for (int64_t c = 4 * threadIdx.x; c < ld; c += 1024) {
         float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        int k[4] = {0, 0, 0, 0};
         if (finite) {
-            if (VEC && c + 3 < cols) {
-                const float4 q = *reinterpret_cast<const float4*>(a + c);
-                v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+            if (c + 3 < cols) {
+                if (VEC) {
+                    const float4 q = *reinterpret_cast<const float4*>(a + c);
+                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] = a[c + i];
+                }
+                const int4 q = *reinterpret_cast<const int4*>(cmax + c);
+                k[0] = q.x; k[1] = q.y; k[2] = q.z; k[3] = q.w;
             } else {
-                for (int i = 0; i < 4; i++) v[i] = c + i < cols ? a[c + i] : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (c + i < cols) {
+                        v[i] = a[c + i];
+                        k[i] = cmax[c + i];
+                    }
             }
         }
-        uint16_t d[4][EX_D];
+        float r[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) digits_f32(v[i] * f1 * f2, d[i]);
+        for (int i = 0; i < 4; i++) {
+            // 2^s as two factors: |v| 2^s <= 1, and what s below -250 leaves has no digit
+            const int s = min(max(-(k[i] + EX_DEAD) - e, -250), 250), h = s >> 1;
+            r[i] = k[i] ? v[i] * __int_as_float((127 + h) << 23) * __int_as_float((127 + s - h) << 23) * 128.0f : 0.0f;
+        }
 #pragma unroll
-        for (int p = 0; p < EX_D; p++)
-            *reinterpret_cast<ushort4*>(D + ((int64_t)p * rows_pad + row) * ld + c) =
-                make_ushort4(d[0][p], d[1][p], d[2][p], d[3][p]);
+        for (int p = 0; p < EX_DA; p++) {
+            if (p >= nd) break;
+            uint16_t d[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float t = rintf(r[i]);
+                d[i] = (uint16_t)(__float_as_uint(t) >> 16);       // |t| <= 128: eight bits
+                r[i] = (r[i] - t) * 256.0f;                        // exact
+            }
+            *reinterpret_cast<ushort4*>(D + ((int64_t)p * rows_pad + row) * ld + c) = make_ushort4(d[0], d[1], d[2], d[3]);
+        }
     }
 }
 
-// the right-hand sides, D[q][r][ld] for r < n_rhs (of rhs_pad); a block each
+// the right-hand sides, D[q][r][ld] for r < n_rhs (of rhs_pad), q <= order; a block each
 __global__ void __launch_bounds__(256)
 ex_split_rhs_kernel(const double* __restrict__ X, int64_t ldx, int64_t cols, int rhs_pad, int64_t ld,
-                    uint16_t* __restrict__ D, int* __restrict__ ex) {
-    __shared__ double red[8];
+                    const int* __restrict__ ex, const int* __restrict__ cmax, const int* __restrict__ extra,
+                    uint16_t* __restrict__ D) {
     const int64_t r = blockIdx.x;
     const double* x = X + r * ldx;
-    double m = 0.0;
-    bool ok = true;
-    for (int64_t c = threadIdx.x; c < cols; c += 256) {
-        m = fmax(m, fabs(x[c]));
-        ok = ok && isfinite(x[c]);
-    }
-    const bool finite = __syncthreads_and(ok);
-    const int e = ex_exponent(ex_block_max(m, red), finite);
-    if (threadIdx.x == 0) ex[r] = e;
-    const int e1 = finite ? -(e / 2) : 0, e2 = finite ? -e - e1 : 0;
-    const double f1 = finite ? ldexp(1.0, e1) : 0.0, f2 = finite ? ldexp(1.0, e2) : 0.0;
+    const int e = ex[r], nd = EX_ORDER + 1 + *extra;
+    const bool finite = e != EX_NONFINITE;
     for (int64_t c = threadIdx.x; c < ld; c += 256) {
-        uint16_t d[EX_D];
-        digits_f64(finite && c < cols ? x[c] * f1 * f2 : 0.0, d);
-#pragma unroll
-        for (int q = 0; q < EX_D; q++) D[((int64_t)q * rhs_pad + r) * ld + c] = d[q];
+        double v = finite && c < cols && cmax[c] ? x[c] : 0.0;
+        if (v != 0.0) v = scalbn(v, cmax[c] + EX_DEAD - e + 7);
+        for (int q = 0; q < nd; q++) {
+            const double t = rint(v);
+            D[((int64_t)q * rhs_pad + r) * ld + c] = (uint16_t)(__float_as_uint((float)t) >> 16);
+            v = (v - t) * 256.0;
+        }
     }
 }
 
@@ -178,7 +292,8 @@ __device__ __forceinline__ void ex_tmem_add(uint32_t ta, uint32_t* acc) {
 template <int BN>
 __global__ void __launch_bounds__(EX_THREADS, 1)
 tc_exact_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapX, int64_t rows,
-                int64_t rows_pad, int kb_total, int n_rhs, int items, int32_t* __restrict__ P, int* __restrict__ error) {
+                int64_t rows_pad, int kb_total, int n_rhs, const int* __restrict__ extra, int32_t* __restrict__ P,
+                int* __restrict__ error) {
     constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
     constexpr uint32_t TMEM_COLS = 2 * BN;      // BN in 32 .. 256: a power of two of at least 64
     constexpr int HALF = BN / 2;
@@ -209,9 +324,10 @@ tc_exact_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     const int chunks = (kb_total + EX_CHUNK - 1) / EX_CHUNK;
-    auto pair_of = [](int i, int& p, int& q) {
+    const int order = EX_ORDER + *extra, pairs = ex_pairs(order), items = (int)(rows_pad / TC_BM) * pairs;
+    auto pair_of = [order](int i, int& p, int& q) {
         p = 0;
-        while (i >= EX_D - p) i -= EX_D - p++;
+        while (i > order - p) i -= order + 1 - p++;
         q = i;
     };
 
@@ -219,8 +335,8 @@ tc_exact_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         uint32_t g = 0;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             int p, q;
-            pair_of(it % EX_PAIRS, p, q);
-            const int ya = (int)(p * rows_pad + (int64_t)(it / EX_PAIRS) * TC_BM), yx = q * BN;
+            pair_of(it % pairs, p, q);
+            const int ya = (int)(p * rows_pad + (int64_t)(it / pairs) * TC_BM), yx = q * BN;
             for (int kb = 0; kb < kb_total; kb++, g++) {
                 const int s = g % EX_STAGES;
                 if (!mbar_wait(&empty[s], ((g / EX_STAGES) & 1u) ^ 1u, TC_WAIT_LIMIT)) atomicExch(error, 1);
@@ -287,10 +403,10 @@ tc_exact_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[c & 1u]);
             }
-            const int64_t row = (int64_t)(it / EX_PAIRS) * TC_BM + 32 * (warp & 3) + lane;
+            const int64_t row = (int64_t)(it / pairs) * TC_BM + 32 * (warp & 3) + lane;
             const uint32_t off = (uint32_t)chunks * 0x4B400000u;
             if (row < rows) {
-                int32_t* out = P + ((int64_t)(it % EX_PAIRS) * n_rhs + col0) * rows_pad + row;
+                int32_t* out = P + ((int64_t)(it % pairs) * n_rhs + col0) * rows_pad + row;
 #pragma unroll
                 for (int i = 0; i < HALF; i++)
                     if ((int)col0 + i < n_rhs) out[(int64_t)i * rows_pad] = (int32_t)(acc[i] - off);
@@ -309,25 +425,34 @@ tc_exact_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 // R[r, row] = (first ? B : R)[r, row] - 2^(ea + ex - 14) sum_o 2^(-8 o) sum_{p + q = o} P
 __global__ void __launch_bounds__(256)
 ex_combine_kernel(const int32_t* __restrict__ P, int64_t rows, int64_t rows_pad, int n_rhs, const int* __restrict__ ea,
-                  const int* __restrict__ exr, const double* __restrict__ B, int64_t n, int64_t row0, int first,
-                  double* __restrict__ R) {
+                  const int* __restrict__ exr, const int* __restrict__ extra, const double* __restrict__ B, int64_t n,
+                  int64_t row0, int first, double* __restrict__ R) {
     const int64_t row = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int r = blockIdx.y;
     if (row >= rows) return;
-    int64_t s[EX_D];
+    const int order = EX_ORDER + *extra, nd = ex_digits_a(order);
+    int64_t s[EX_DX];
 #pragma unroll
-    for (int o = 0; o < EX_D; o++) s[o] = 0;
+    for (int o = 0; o < EX_DX; o++) s[o] = 0;
     const int32_t* p0 = P + (int64_t)r * rows_pad + row;
-    int i = 0;
+    const int64_t step = (int64_t)n_rhs * rows_pad;
 #pragma unroll
-    for (int p = 0; p < EX_D; p++)
+    for (int p = 0; p < EX_DA; p++) {
+        if (p >= nd) break;
 #pragma unroll
-        for (int q = 0; q < EX_D - p; q++, i++) s[p + q] += p0[(int64_t)i * n_rhs * rows_pad];
-    // pairs of orders are exact integers below 2^43
-    const double y = (double)(s[0] * 256 + s[1]) + (double)(s[2] * 256 + s[3]) * 0x1p-16 +
-                     (double)(s[4] * 256 + s[5]) * 0x1p-32;
+        for (int q = 0; q < EX_DX - p; q++)
+            if (p + q <= order) {
+                s[p + q] += *p0;
+                p0 += step;
+            }
+    }
+    // four orders are exact integers: at most eight products of 2^30 each, times 2^24
+    double y = 0.0;
+#pragma unroll
+    for (int o = EX_DX - 4; o >= 0; o -= 4)
+        y = y * 0x1p-32 + (double)(((s[o] * 256 + s[o + 1]) * 256 + s[o + 2]) * 256 + s[o + 3]);
     const int e1 = ea[row], e2 = exr[r];
-    const double v = (e1 == EX_NONFINITE || e2 == EX_NONFINITE) ? nan("") : scalbn(y, e1 + e2 - 14 - 8);
+    const double v = (e1 == EX_NONFINITE || e2 == EX_NONFINITE) ? nan("") : scalbn(y, e1 + e2 - 14 - 24);
     const int64_t o = (int64_t)r * n + row0 + row;
     R[o] = (first ? B[o] : R[o]) - v;
 }
@@ -336,35 +461,55 @@ ex_combine_kernel(const int32_t* __restrict__ P, int64_t rows, int64_t rows_pad,
 // host
 // ---------------------------------------------------------------------------
 constexpr int64_t EX_SEGMENT = 65536;             // columns at a time: the sums stay below 2^30
-constexpr int64_t EX_PIECE_BYTES = (int64_t)6 << 30;
+constexpr int64_t EX_PIECE_BYTES = (int64_t)2 << 30;
 
 struct ExPlan {
     int64_t ld, rows, rhs_pad, rhs;               // per column segment and row chunk
-    size_t digits_a, digits_x, products, total;
+    size_t digits_a, digits_x, products, exponents, total;
+    int sms;
 };
 static ExPlan ex_plan(int64_t k, int64_t n) {
     ExPlan p;
+    p.sms = 152;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
     p.ld = ceil_div(std::min(n, EX_SEGMENT), TC_BK) * TC_BK;
     p.rhs = std::min<int64_t>(k, 256);
     p.rhs_pad = p.rhs <= 32 ? 32 : p.rhs <= 64 ? 64 : p.rhs <= 128 ? 128 : 256;
-    const int64_t most = std::max<int64_t>(EX_PIECE_BYTES / (2 * EX_D * p.ld) / TC_BM * TC_BM, TC_BM);
-    p.rows = std::min(ceil_div(n, TC_BM) * TC_BM, most);
-    p.digits_a = (size_t)(2 * EX_D * p.rows * p.ld);
-    p.digits_x = (size_t)(2 * EX_D * p.rhs_pad * p.ld);
-    p.products = (size_t)(4 * EX_PAIRS * p.rhs * p.rows);
-    p.total = 1024 + p.digits_a + p.digits_x + p.products + 8 * (size_t)(p.rows + p.rhs_pad);
+    // The row tiles of a piece: of those whose digits fit EX_PIECE_BYTES the number with the
+    // fewest rounds of items over the SMs (a piece costs about half a round more)
+    const int64_t tiles = ceil_div(n, TC_BM), pairs = ex_pairs(EX_ORDER);
+    const int64_t most = std::max<int64_t>(1, std::min(tiles, EX_PIECE_BYTES / (2 * EX_DA * p.ld * TC_BM)));
+    double cost = 1e300;
+    int64_t best = most;
+    for (int64_t t = most; t > most / 2; t--) {
+        const int64_t whole = tiles / t, rest = tiles % t;
+        const double c = (double)(whole * ceil_div(t * pairs, p.sms) + ceil_div(rest * pairs, p.sms)) +
+                         0.5 * (double)(whole + (rest > 0));
+        if (c < cost) {
+            cost = c;
+            best = t;
+        }
+    }
+    p.rows = best * TC_BM;
+    p.digits_a = (size_t)(2 * EX_DA * p.rows * p.ld);
+    p.digits_x = (size_t)(2 * EX_DX * p.rhs_pad * p.ld);
+    p.products = (size_t)(4 * ex_pairs(EX_ORDER_MAX) * p.rhs * p.rows);
+    p.exponents = 4 * (size_t)(p.ld + 4 + n + p.rhs_pad);          // columns, the order, rows, right-hand sides
+    p.total = 1024 + p.digits_a + p.digits_x + p.products + p.exponents;
+    p.total = (p.total + 7) / 8 * 8;
     return p;
 }
 size_t exact_residual_workspace(int64_t k, int64_t n) { return ex_plan(k, n).total; }
 
 template <int BN>
 static void launch_exact(const CUtensorMap& ma, const CUtensorMap& mx, int64_t rows, int64_t rows_pad, int kb, int n_rhs,
-                         int sms, int32_t* P, int* err, cudaStream_t st) {
+                         int sms, const int* extra, int32_t* P, int* err, cudaStream_t st) {
     const size_t smem = (size_t)EX_STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024;
     cudaFuncSetAttribute(tc_exact_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int items = (int)(ceil_div(rows, TC_BM) * EX_PAIRS);
+    const int items = (int)(ceil_div(rows, TC_BM) * ex_pairs(EX_ORDER));       // at least
     tc_exact_kernel<BN><<<(unsigned)std::min(items, sms), EX_THREADS, smem, st>>>(ma, mx, rows, rows_pad, kb, n_rhs,
-                                                                                  items, P, err);
+                                                                                  extra, P, err);
 }
 
 // R = B - A X for k right-hand sides (rows of B, X, R, n each); A is n x n FP32 at lda
@@ -374,43 +519,51 @@ int exact_residual(const float* A, int64_t lda, int64_t n, const double* B, cons
     MBEM_REQUIRE(work && work_bytes >= pl.total, MBEM_ERR_SIZE, "batched residual workspace too small");
     int* err = tc_error_flag();
     MBEM_REQUIRE(err != nullptr, MBEM_ERR_CUDA, "no device error flag");
-    int sms = 152, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint8_t* w = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(work) + 1023) & ~(uintptr_t)1023);
     uint16_t* da = reinterpret_cast<uint16_t*>(w);
     uint16_t* dx = reinterpret_cast<uint16_t*>(w + pl.digits_a);
     int32_t* P = reinterpret_cast<int32_t*>(w + pl.digits_a + pl.digits_x);
-    int* ea = reinterpret_cast<int*>(w + pl.digits_a + pl.digits_x + pl.products);
-    int* exr = ea + pl.rows;
+    int* cmax = reinterpret_cast<int*>(w + pl.digits_a + pl.digits_x + pl.products);
+    int* extra = cmax + pl.ld;
+    int* ea = extra + 4;
+    int* exr = ea + n;
     const bool vec = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+    const float few = n < 32768 ? 0.5f * log2f(32768.0f / (float)n) : 0.0f;
     for (int64_t r0 = 0; r0 < k; r0 += 256) {
         const int nr = (int)std::min<int64_t>(256, k - r0);
         const int bn = nr <= 32 ? 32 : nr <= 64 ? 64 : nr <= 128 ? 128 : 256;
         for (int64_t c0 = 0; c0 < n; c0 += EX_SEGMENT) {
             const int64_t nc = std::min(EX_SEGMENT, n - c0), ld = ceil_div(nc, TC_BK) * TC_BK;
-            ex_split_rhs_kernel<<<(unsigned)nr, 256, 0, st>>>(X + r0 * n + c0, n, nc, bn, ld, dx, exr);
+            cudaMemsetAsync(cmax, 0, sizeof(int) * (size_t)(pl.ld + 4), st);
+            if (vec) ex_row_scale_kernel<true><<<(unsigned)n, 256, 0, st>>>(A + c0, lda, nc, ea);
+            else ex_row_scale_kernel<false><<<(unsigned)n, 256, 0, st>>>(A + c0, lda, nc, ea);
+            const dim3 cgrid((unsigned)ceil_div(nc, 1024), (unsigned)ceil_div(n, EX_CROWS));
+            if (vec) ex_col_scale_kernel<true><<<cgrid, 256, 0, st>>>(A + c0, lda, n, nc, ea, cmax);
+            else ex_col_scale_kernel<false><<<cgrid, 256, 0, st>>>(A + c0, lda, n, nc, ea, cmax);
+            ex_rhs_scale_kernel<<<(unsigned)nr, 256, 0, st>>>(X + r0 * n + c0, n, nc, cmax, few, exr, extra);
+            ex_split_rhs_kernel<<<(unsigned)nr, 256, 0, st>>>(X + r0 * n + c0, n, nc, bn, ld, exr, cmax, extra, dx);
             CUtensorMap ma, mx;
-            int e = tc_make_map(&mx, dx, (int64_t)EX_D * bn, ld, ld, bn);
+            int e = tc_make_map(&mx, dx, (int64_t)EX_DX * bn, ld, ld, bn);
             if (e) return e;
             for (int64_t row0 = 0; row0 < n; row0 += pl.rows) {
                 const int64_t rows = std::min(pl.rows, n - row0), pad = ceil_div(rows, TC_BM) * TC_BM;
                 const float* a = A + row0 * lda + c0;
-                if (vec) ex_split_rows_kernel<true><<<(unsigned)rows, 256, 0, st>>>(a, lda, nc, pad, ld, da, ea);
-                else ex_split_rows_kernel<false><<<(unsigned)rows, 256, 0, st>>>(a, lda, nc, pad, ld, da, ea);
-                if ((e = tc_make_map(&ma, da, (int64_t)EX_D * pad, ld, ld, TC_BM))) return e;
+                if (vec) ex_split_rows_kernel<true><<<(unsigned)rows, 256, 0, st>>>(a, lda, nc, pad, ld, ea + row0, cmax, extra, da);
+                else ex_split_rows_kernel<false><<<(unsigned)rows, 256, 0, st>>>(a, lda, nc, pad, ld, ea + row0, cmax, extra, da);
+                if ((e = tc_make_map(&ma, da, (int64_t)EX_DA * pad, ld, ld, TC_BM))) return e;
                 const int kb = (int)(ld / TC_BK);
                 switch (bn) {
-                    case 32: launch_exact<32>(ma, mx, rows, pad, kb, nr, sms, P, err, st); break;
-                    case 64: launch_exact<64>(ma, mx, rows, pad, kb, nr, sms, P, err, st); break;
-                    case 128: launch_exact<128>(ma, mx, rows, pad, kb, nr, sms, P, err, st); break;
-                    default: launch_exact<256>(ma, mx, rows, pad, kb, nr, sms, P, err, st); break;
+                    case 32: launch_exact<32>(ma, mx, rows, pad, kb, nr, pl.sms, extra, P, err, st); break;
+                    case 64: launch_exact<64>(ma, mx, rows, pad, kb, nr, pl.sms, extra, P, err, st); break;
+                    case 128: launch_exact<128>(ma, mx, rows, pad, kb, nr, pl.sms, extra, P, err, st); break;
+                    default: launch_exact<256>(ma, mx, rows, pad, kb, nr, pl.sms, extra, P, err, st); break;
                 }
                 ex_combine_kernel<<<dim3((unsigned)ceil_div(rows, 256), (unsigned)nr), 256, 0, st>>>(
-                    P, rows, pad, nr, ea, exr, B + r0 * n, n, row0, c0 == 0, R + r0 * n);
+                    P, rows, pad, nr, ea + row0, exr, extra, B + r0 * n, n, row0, c0 == 0, R + r0 * n);
                 count_launches(3);
                 if ((e = launch_status("exact_residual", 0))) return e;
             }
-            count_launches(1);
+            count_launches(4);
         }
     }
     return MBEM_OK;

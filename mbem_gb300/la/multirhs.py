@@ -98,8 +98,8 @@ class BlockSolver:
     """Solves A X = B for up to 256 right-hand sides at once.
 
     The refinement loop computes the residual R = P (B - A X) with the
-    accurate operator (the mixed operator's FP32 far field with double-float
-    accumulation and its FP64 near blocks, or the FP64 dense matrix), and
+    accurate operator (the mixed operator's FP32 far field by exact digit
+    products and its FP64 near blocks, or the FP64 dense matrix), and
     corrects X by batched GMRES on the BF16 copy of the operator, whose
     every step is one tensor-core GEMM over the whole block. P removes the
     rigid translations of the u-slots of a deflated system."""
