@@ -8,8 +8,8 @@
 // all four panels (48 KB) for six MMAs, two thirds of the traffic. The (row tile,
 // K block) units are dealt to the SMs in equal runs, so no SM waits for a last
 // wave; a run's pieces of a tile go to partial sums that the Arnoldi step adds in
-// order, and a second TMEM accumulator takes the next piece while the epilogue
-// reads the first. 20,736 x 20,736 x 256, three terms: 0.48 ms against 0.56.
+// order, and a second TMEM accumulator takes the next 16 units while the epilogue
+// adds the first in registers. 20,736 x 20,736 x 256, three terms: 0.47 ms against 0.56.
 #include <algorithm>
 
 #include "tc_common.cuh"
@@ -18,7 +18,13 @@ namespace mbem {
 
 constexpr int B3_BK = 32;                // 64-byte rows, 64-byte swizzle
 constexpr int B3_STAGES = 4;
-constexpr int B3_THREADS = 192;
+constexpr int B3_THREADS = 320;         // eight epilogue warps, producer, issuer
+// Units that an accumulator takes: 512 columns, 96 MMA steps. The tensor core's FP32 sums
+// come out low, so their error grows with the steps: over whole tiles (3,888 steps at
+// 20,736 columns) 1.8e-7 rms and -4.4e-5 of the sum on average for a block of slip
+// patterns, 0.57e-7 and -1.4e-5 with the K split of tc_gemm.cu, 0.07e-7 and -1.8e-6 with
+// the pieces' sums rounded to nearest (the three terms alone: 1.4e-8). No slower.
+constexpr int B3_CHUNK = 16;
 
 // as sw128_desc for 64-byte rows: 512 bytes between 8-row groups, swizzle mode 4 (64B)
 __device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
@@ -41,6 +47,7 @@ tc_block3_kernel(const __grid_constant__ B3Maps maps, int64_t M, int kb, int per
                  float* __restrict__ P, int* __restrict__ error) {
     constexpr int A_BYTES = TC_BM * B3_BK * 2, B_BYTES = BN * B3_BK * 2, STAGE = 2 * (A_BYTES + B_BYTES);
     constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
+    constexpr int COLS = BN < 32 ? BN : BN / 2, EPI = 4 * BN / COLS;     // columns an epilogue warp, epilogue warps
     extern __shared__ __align__(1024) uint8_t b3_smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)b3_smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t full[B3_STAGES], empty[B3_STAGES], acc_full[2], acc_empty[2];
@@ -54,11 +61,11 @@ tc_block3_kernel(const __grid_constant__ B3Maps maps, int64_t M, int kb, int per
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], EPI);
         }
         mbar_init_fence();
     }
-    if (warp == 5) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base)),
                      "r"(TMEM_COLS)
                      : "memory");
@@ -69,7 +76,7 @@ tc_block3_kernel(const __grid_constant__ B3Maps maps, int64_t M, int kb, int per
     tc_fence_after();
     const uint32_t tmem = tmem_base;
 
-    if (warp == 4 && lane == 0) {
+    if (warp == 8 && lane == 0) {
         for (int u = u0; u < u1; u++) {
             const uint32_t g = (uint32_t)(u - u0);
             const int s = g % B3_STAGES;
@@ -86,12 +93,16 @@ tc_block3_kernel(const __grid_constant__ B3Maps maps, int64_t M, int kb, int per
         const uint32_t n = (uint32_t)(u1 - u0);
         for (uint32_t h = n > B3_STAGES ? n - B3_STAGES : 0; h < n; h++)
             if (!mbar_wait(&full[h % B3_STAGES], (h / B3_STAGES) & 1u, TC_WAIT_LIMIT)) atomicExch(error, 1);
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 9 && lane == 0) {
         constexpr uint32_t idesc = f16_idesc(TC_BM, BN);
         uint32_t c = 0;
+        int in = 0;
         for (int u = u0; u < u1; u++) {
             const uint32_t g = (uint32_t)(u - u0);
-            const bool first = u == u0 || u % kb == 0, last = u == u1 - 1 || (u + 1) % kb == 0;
+            // an accumulator takes B3_CHUNK units from the run's first of the tile on
+            if (u % kb == 0) in = 0;
+            const bool first = in == 0, last = in == B3_CHUNK - 1 || u == u1 - 1 || (u + 1) % kb == 0;
+            in = last ? 0 : in + 1;
             const uint32_t d = tmem + (c & 1u) * BN;
             if (first) {
                 if (!mbar_wait(&acc_empty[c & 1u], ((c >> 1) & 1u) ^ 1u, TC_WAIT_LIMIT)) atomicExch(error, 1);
@@ -126,42 +137,52 @@ tc_block3_kernel(const __grid_constant__ B3Maps maps, int64_t M, int kb, int per
                 c++;
             }
         }
-    } else if (warp < 4) {
+    } else if (warp < EPI) {
+        // warp w: TMEM lanes 32 (w % 4) .., columns (w / 4) COLS ..
+        const int col0 = (warp >> 2) * COLS;
+        const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col0;
         uint32_t c = 0;
-        for (int u = u0; u < u1; c++) {
+        for (int u = u0; u < u1;) {
             const int tile = u / kb, end = min(u1, (tile + 1) * kb);
             const int part = (int)blockIdx.x - tile * kb / per;      // this run's place among the tile's
-            if (!mbar_wait(&acc_full[c & 1u], (c >> 1) & 1u, TC_WAIT_LIMIT)) atomicExch(error, 1);
-            tc_fence_after();
-            const int64_t row = (int64_t)tile * TC_BM + 32 * warp + lane;
-            float* out = P + (int64_t)part * n_rhs * M + row;
-            const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + (c & 1u) * BN;
-#pragma unroll 1
-            for (int q = 0; q < BN; q += 16) {
-                uint32_t v[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                    "%13, %14, %15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                      "=r"(v[15])
-                    : "r"(ta + (uint32_t)q));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < M) {
+            float acc[COLS];
 #pragma unroll
-                    for (int i = 0; i < 16; i++)
-                        if (q + i < n_rhs) out[(int64_t)(q + i) * M] = __uint_as_float(v[i]);
+            for (int i = 0; i < COLS; i++) acc[i] = 0.0f;
+#pragma unroll 1
+            for (; u < end; u += B3_CHUNK, c++) {
+                if (!mbar_wait(&acc_full[c & 1u], (c >> 1) & 1u, TC_WAIT_LIMIT)) atomicExch(error, 1);
+                tc_fence_after();
+#pragma unroll
+                for (int q = 0; q < COLS; q += 16) {
+                    uint32_t v[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                        "%12, %13, %14, %15}, [%16];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                          "=r"(v[14]), "=r"(v[15])
+                        : "r"(ta + (c & 1u) * BN + (uint32_t)q));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; i++) acc[q + i] += __uint_as_float(v[i]);
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[c & 1u]);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[c & 1u]);
             u = end;
+            const int64_t row = (int64_t)tile * TC_BM + 32 * (warp & 3) + lane;
+            if (row < M) {
+                float* out = P + ((int64_t)part * n_rhs + col0) * M + row;
+#pragma unroll
+                for (int i = 0; i < COLS; i++)
+                    if (col0 + i < n_rhs) out[(int64_t)i * M] = acc[i];
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 5) {
+    if (warp == 9) {
         // every MMA has completed: the epilogue has read each accumulator
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
