@@ -29,6 +29,7 @@ namespace cg = cooperative_groups;
 
 constexpr int AR_T = 256;
 constexpr int AR_SLICE = 27000;                // floats of a slice: two blocks an SM
+constexpr size_t AR_SMEM = 220 * 1024;         // most shared memory a block takes
 
 // sums a step takes: its basis vectors, or the projection's three means
 __host__ __device__ constexpr int ar_vectors(int m) { return m < 4 ? 4 : m; }
@@ -399,10 +400,11 @@ int mbem_batch_arnoldi(const float* P, int splits, int kb, int per, int64_t spli
     while (ranks < 8 && (ceil_div(n, ranks) > AR_SLICE || k * ranks < 2 * 152) && n / (2 * ranks) >= 1024) ranks *= 2;
     a.slice = ceil_div(ceil_div(n, ranks), 4) * 4;
     const size_t smem = (size_t)a.slice * sizeof(float) + (size_t)ar_vectors(m) * (3 * sizeof(double) + sizeof(F2));
-    MBEM_REQUIRE(smem <= 220 * 1024, MBEM_ERR_SIZE, "batched Arnoldi: %d vectors of %lld entries", m, (long long)n);
+    MBEM_REQUIRE(smem <= AR_SMEM, MBEM_ERR_SIZE, "batched Arnoldi: %d vectors of %lld entries", m, (long long)n);
     const bool vec = n % 4 == 0 && split_stride % 4 == 0 && ((uintptr_t)P | (uintptr_t)V) % 16 == 0;
     auto kernel = vec ? batch_arnoldi_kernel<true> : batch_arnoldi_kernel<false>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the kernel's, shared by all host threads: always its largest
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AR_SMEM);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(k * ranks));
     cfg.blockDim = dim3(AR_T);

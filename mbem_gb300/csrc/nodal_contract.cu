@@ -148,10 +148,17 @@ int nodal_pairs_stress(const double* x, const double* tv, const double* normals,
     return launch_status("nodal_pairs_stress_kernel");
 }
 
-template <typename Kernel>
-static cudaError_t launch_contract_kernel(const cudaLaunchConfig_t& cfg, Kernel k, const NodalArgs& a, int ob) {
-    // up to 47 KB of dynamic beside 3 KB of static shared memory (P2): four blocks an SM
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+template <int P>
+static constexpr size_t contract_smem(int kind, int ob) {
+    return NC_TILE * (sizeof(NodalTile<P>) + (size_t)ob * (kind <= NC_U ? 3 : 6) * sizeof(double));
+}
+
+template <int P, typename Kernel>
+static cudaError_t launch_contract_kernel(const cudaLaunchConfig_t& cfg, Kernel k, int kind, const NodalArgs& a, int ob) {
+    // up to 47 KB of dynamic beside 3 KB of static shared memory (P2): four blocks an SM.
+    // The limit is the kernel's, shared by all host threads: always its largest.
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)contract_smem<P>(kind, NC_OBS));
     return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, k, a, ob);
 }
 
@@ -162,7 +169,7 @@ static cudaError_t launch_nodal_contract(int kind, const NodalArgs& a, unsigned 
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(ND_THREADS);
-    cfg.dynamicSmemBytes = NC_TILE * (sizeof(NodalTile<P>) + (size_t)ob * (kind <= NC_U ? 3 : 6) * sizeof(double));
+    cfg.dynamicSmemBytes = contract_smem<P>(kind, ob);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -172,14 +179,14 @@ static cudaError_t launch_nodal_contract(int kind, const NodalArgs& a, unsigned 
     cfg.numAttrs = 1;
     static_assert(NC_TILE * NC_OBS <= ND_TILE_PAIRS, "a tile's pairs fit its queue");
     switch (kind) {
-        case NC_T: return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_T>, a, ob);
-        case NC_U: return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_U>, a, ob);
+        case NC_T: return launch_contract_kernel<P>(cfg, nodal_contract_kernel<P, NC_T>, kind, a, ob);
+        case NC_U: return launch_contract_kernel<P>(cfg, nodal_contract_kernel<P, NC_U>, kind, a, ob);
         case NC_STRESS + MBEM_STRESS_KELVIN:
-            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_KELVIN>, a, ob);
+            return launch_contract_kernel<P>(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_KELVIN>, kind, a, ob);
         case NC_STRESS + MBEM_STRESS_EIGEN:
-            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_EIGEN>, a, ob);
+            return launch_contract_kernel<P>(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_EIGEN>, kind, a, ob);
         default:
-            return launch_contract_kernel(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_DD>, a, ob);
+            return launch_contract_kernel<P>(cfg, nodal_contract_kernel<P, NC_STRESS + MBEM_STRESS_DD>, kind, a, ob);
     }
 }
 
