@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
     extern __shared__ __align__(16) unsigned char nd_smem[];
     __shared__ PairQueue queue;
     NodalRec* recs = reinterpret_cast<NodalRec*>(nd_smem);
-    constexpr int K = nd_nodes(P);
+    constexpr int K = nd_nodes(P), FAR = KIND == ND_T || KIND == ND_UBASIS ? NF_T : KIND == ND_U ? NF_U : NF_H;
     const int64_t s0 = (int64_t)blockIdx.x * sb;
     const int ns = (int)lmin(sb, a.n_src - s0);
     load_recs(a, s0, ns, recs);
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
         const int nf = (int)lmin(fb, a.n_field_pts - f0), total = ns * nf;
         queue_pairs(queue, total, [&](int p) {
             const int t = p / nf;
-            return pair_class<P>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
+            return pair_class<P, FAR>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
         });
         int p;
 #pragma unroll 1
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
                         }
                 };
                 const double zero[6] = {0, 0, 0, 0, 0, 0};
-                if (g.ok) pair_u<P>(g, x, a.c[2], put);
+                if (g.ok) pair_u<P, FAR>(g, x, a.c[2], put);
                 else
                     for (int k = 0; k < K; k++) put(k, 0.0, 0.0, zero);
             } else if (KIND == ND_TBASIS) {
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_matrix_kernel(NodalArgs a, i
                         }
                 };
                 const double zero[6] = {0, 0, 0, 0, 0, 0};
-                if (g.ok) pair_u<P>(g, x, 1.0, put);
+                if (g.ok) pair_u<P, FAR>(g, x, 1.0, put);
                 else
                     for (int k = 0; k < K; k++) put(k, 0.0, 0.0, zero);
             }
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_near_eval_kernel(NodalArgs a
                 for (int j = 0; j < 3; j++) o[9 * k + 3 * i + j] = a.alpha * G[i][j];
         });
     } else {
-        pair_u<P>(g, x, a.c[2], [&](int k, double I1, double I3, const double* G) {
+        pair_u<P, NF_U>(g, x, a.c[2], [&](int k, double I1, double I3, const double* G) {
             const double d = a.c[0] * I1 + a.c[1] * g.eps2 * I3;
             const int ix[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
 #pragma unroll

@@ -6,7 +6,8 @@
 // block: a few observers still fill the part, each partial sum has one owner
 // and the sums are added in slice, then rank order through distributed shared
 // memory (deterministic, no workspace). Bound by the FP64 pipe: the stress of a
-// 16 x 16 P2 fault at 2,000 observers went from 266 to 4.9 ms.
+// 16 x 16 P2 fault at 2,000 observers went from 266 to 5.85 ms (4.85 with far rules off by up
+// to 2e-14, nd_far_rule).
 #include <cooperative_groups.h>
 
 #include "contract_split.cuh"
@@ -42,6 +43,8 @@ template <int P, int KIND>
 __global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a, int ob) {
     extern __shared__ __align__(16) unsigned char nd_smem[];
     constexpr int NO = KIND <= NC_U ? 3 : 6;
+    constexpr int FAR = KIND == NC_T ? NF_T : KIND == NC_U ? NF_U : KIND == NC_STRESS + MBEM_STRESS_KELVIN ? NF_S
+                        : KIND == NC_STRESS + MBEM_STRESS_EIGEN ? NF_E : NF_H;
     __shared__ PairQueue queue;
     __shared__ double sum[NC_OBS * NO];
     __shared__ double xs[NC_OBS][3];
@@ -65,7 +68,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_contract_kernel(NodalArgs a,
             nodal_den<P>(tile[t].g, a.density + 3 * K * s, tile[t].d);
         }
         __syncthreads();
-        queue_pairs(queue, total, [&](int p) { return pair_class<P>(tile[p / nf].g, xs[p % nf]); });
+        queue_pairs(queue, total, [&](int p) { return pair_class<P, FAR>(tile[p / nf].g, xs[p % nf]); });
         int p;
 #pragma unroll 1
         while (queue_next(queue, total, p)) {

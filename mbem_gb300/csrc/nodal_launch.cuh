@@ -42,15 +42,15 @@ static inline void nd_gauss_legendre(int n, double* x, double* w) {
 }
 
 // Fully symmetric rules on the triangle, one line an orbit: points, weight (of a
-// unit sum), and two barycentric coordinates of a point of it. Degrees 6, 8, 9 and
-// 10 with 12, 16, 19 and 25 points, the orbit counts of Dunavant, Int. J. Numer.
+// unit sum), and two barycentric coordinates of a point of it. Degrees 6, 8, 9,
+// 10, 12 and 14 with 12, 16, 19, 25, 33 and 42 points, the orbit counts of Dunavant, Int. J. Numer.
 // Meth. Eng. 21 (1985); the values solve the moment equations (invariants
 // e2^i e3^j of the barycentric coordinates) by Newton's method in 50 digits.
 struct NdOrbit {
     int n;
     double w, a, b;
 };
-static const NdOrbit ND_ORBITS[4][6] = {
+static const NdOrbit ND_ORBITS[ND_FAR_RULES][10] = {
     {{3, 0.1167862757263793660252896, 0.2492867451709104212916386, 0.2492867451709104212916386},
      {3, 0.05084490637020681692093681, 0.0630890144915022283403316, 0.0630890144915022283403316},
      {6, 0.08285107561837357519355346, 0.6365024991213986472301426, 0.05314504984481694735324967}},
@@ -70,7 +70,25 @@ static const NdOrbit ND_ORBITS[4][6] = {
      {3, 0.01335296881314956627557298, 0.03205537321694351293098459, 0.03205537321694351293098459},
      {6, 0.06390490639642404543289873, 0.1481328857838205504978068, 0.5300541189273440282770957},
      {6, 0.03418464816295942862869158, 0.02961988948872976763383627, 0.3691467818278109869114208},
-     {6, 0.02529775770728838438904279, 0.8079306009228790650799499, 0.02836766533993843925043576}}};
+     {6, 0.02529775770728838438904279, 0.8079306009228790650799499, 0.02836766533993843925043576}},
+    {{3, 0.02573106644045533541779092, 0.4882173897738048825646621, 0.4882173897738048825646621},
+     {3, 0.04369254453803840213545726, 0.4397243922944602729797366, 0.4397243922944602729797366},
+     {3, 0.06285822421788510035427051, 0.2712103850121159223459513, 0.2712103850121159223459513},
+     {3, 0.0347961129307089429893284, 0.1275761455415859246738963, 0.1275761455415859246738963},
+     {3, 0.006166261051559017233866484, 0.02131735045321037024685698, 0.02131735045321037024685698},
+     {6, 0.0403715577663809295178287, 0.2757132696855141939747963, 0.6089432357797878068561924},
+     {6, 0.02235677320230344571183908, 0.2813255809899395482481307, 0.6958360867878034221416355},
+     {6, 0.0173162311086588923716421, 0.1162519159075971412413541, 0.8580140335440726305905366}},
+    {{3, 0.02188358136942889064084495, 0.488963910362178638677376, 0.488963910362178638677376},
+     {3, 0.03278835354412535064131098, 0.4176447193404539225094408, 0.4176447193404539225094408},
+     {3, 0.05177410450729158631478491, 0.2734775283088386597549443, 0.2734775283088386597549443},
+     {3, 0.04216258873699301753823044, 0.1772055324125434369566107, 0.1772055324125434369566107},
+     {3, 0.01443369966977666760170992, 0.06179988309087260126747883, 0.06179988309087260126747883},
+     {3, 0.004923403602400081681826024, 0.0193909612487010481782501, 0.0193909612487010481782501},
+     {6, 0.02466575321256367396287525, 0.1722666878213555783752896, 0.7706085547749964825890333},
+     {6, 0.03857151078706068322848903, 0.3368614597963450017440552, 0.5702222908466831734976962},
+     {6, 0.01443630811353384049608869, 0.2983728821362577529708315, 0.6869801678080878373586272},
+     {6, 0.005010228838500671769860093, 0.118974497696956845398182, 0.8797571713701711295145716}}};
 
 static inline NodalRules nd_make_rules() {
     NodalRules r;
@@ -86,7 +104,7 @@ static inline NodalRules nd_make_rules() {
         }
     }
     k = 0;
-    for (int d = 0; d < 4; d++)
+    for (int d = 0; d < ND_FAR_RULES; d++)
         for (const NdOrbit& o : ND_ORBITS[d]) {
             const double c = 1.0 - o.a - o.b;
             const double p[6][2] = {{o.a, o.b}, {c, o.a}, {o.b, c}, {o.b, o.a}, {o.a, c}, {c, o.b}};
@@ -176,18 +194,19 @@ __device__ __forceinline__ void load_recs(const NodalArgs& a, int64_t s0, int ns
 // far rules. A warp that mixes closed forms and quadratures runs both (45 to 69 %
 // of the lanes were at work in the P2 and traction kernels), so the block lists
 // its pairs by class and its warps take 32 at a time, whichever is free next.
-constexpr int ND_CLASSES = 6;
+constexpr int ND_CLASSES = 2 + ND_FAR_RULES;
 struct PairQueue {
     int count[ND_CLASSES], next;
     uint16_t list[ND_TILE_PAIRS];
 };
-template <int P>
+static_assert(ND_CLASSES <= 8, "queue_pairs keeps three bits a pair");
+template <int P, int F>
 __device__ __forceinline__ int pair_class(const NodalRec& g, const double* x) {
     const double dx = x[0] - g.c[0], dy = x[1] - g.c[1], dz = x[2] - g.c[2];
     const float q = (float)(dx * dx + dy * dy + dz * dz + g.eps2) / (float)g.L2;      // a hint: the pair decides again
     if (q <= 4.0f) return 0;
     if (q <= (float)(ND_D_STAR * ND_D_STAR)) return 1;
-    return 2 + nd_far_rule<P>(q, 1.0);
+    return 2 + nd_far_rule<P, F>(q, 1.0);
 }
 // queues `total` pairs (at most ND_TILE_PAIRS); cls(p) is called once a pair.
 // All threads of the block call it; it ends with a barrier.

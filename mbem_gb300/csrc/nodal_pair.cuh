@@ -26,9 +26,8 @@
 //    rule's own abscissa (tabulated with its weights), the edge's midpoint the
 //    origin of the chain below;
 //  * (A + t u)^a (B + t' u)^b integrates by a chain of two-term combinations;
-//  * the far quadratures are fully symmetric rules of 12 to 25 points (degrees 6,
-//    8, 9, 10), as accurate from 10 longest edges on as 49 to 16 collapsed
-//    Gauss-Legendre points;
+//  * the far quadratures are fully symmetric rules of 12 to 42 points (degrees 6,
+//    8, 9, 10, 12, 14), each from the distance on where it is off by less than 2e-16;
 //  * a nodal matrix block is assembled from the blocks of the shifted moments
 //    (one per monomial of the shape functions) instead of from one table per
 //    node, and a contraction folds the density's polynomial into the moments;
@@ -76,10 +75,10 @@ struct NDeg {
 
 // The edge rules (n = 7, 8, 9, 10, 12, 16): abscissae and weights times their
 // powers 0 .. 5; the last one's plain form also sums pieces. The far rules
-// (19, 16, 12 and 25 points): barycentric l1, l2, the weight (sum 1/2) and the
+// (12, 16, 19, 25, 33 and 42 points): barycentric l1, l2, the weight (sum 1/2) and the
 // weight times the shape functions of P1 (3) and P2 (6).
 constexpr int ND_EDGE_Q = 7 + 8 + 9 + 10 + 12 + 16;
-constexpr int ND_FAR_Q = 12 + 16 + 19 + 25;
+constexpr int ND_FAR_Q = 12 + 16 + 19 + 25 + 33 + 42;
 struct NodalRules {
     double ex[ND_EDGE_Q], ew[ND_EDGE_Q][6];
     double fl[ND_FAR_Q][3], fn[ND_FAR_Q][9];
@@ -89,19 +88,38 @@ static __constant__ NodalRules c_nd;       // one copy per translation unit (nod
 #define MBEM_ND_RULES c_nd
 #endif
 
-// The far rule, 0 .. 3 for 25, 19, 16, 12 points: its truncation is below 5e-16 of
-// the pair's largest entry (against 256 points over random triangles and
-// directions, T, U and stress kernels; 4e-15 for the P2 stress between 10 and 11
-// longest edges, where the closed form on the other side is off by 1e-13)
-template <int P>
+// The far rule, 0 .. 5 for 42, 33, 25, 19, 16, 12 points. Each is taken from the distance (in
+// longest edges) on where its truncation is below 2e-16 of the pair's largest entry, a tenth of
+// what the rounding of the sums leaves: against 196 points in 80-bit arithmetic over 1,200 random and slender triangles and
+// directions, along edges and medians among them, eps from 0 to D, and 4 % farther out. The
+// kernels differ by their highest power of 1 / R: U, T and Kelvin stress, DD stress, eigenstress.
+// (With one line for all of them the P2 stress was off by 2e-14 at 10 longest edges and the
+// P2 eigenstress by 8e-13; the lines for 5e-17 take another 12 % of the traction rows' time
+// and 7 % of the P2 stress's.)
+constexpr int ND_FAR_RULES = 6;
+__host__ __device__ constexpr double nd_far_at(int P, int F, int k) {
+    constexpr double never = 1e30;
+    constexpr double at[3][4][ND_FAR_RULES - 1] = {
+        {{0, 0, 0, 15.5, 33}, {0, 0, 13, 21.5, 49.5}, {0, 0, 16.5, 24.5, 69.5}, {0, 13.5, 22.5, 33, 94}},
+        {{0, 0, 13.5, 24, 70.5}, {0, 11, 18.5, 33, 115}, {0, 13.5, 24.5, 40, 149}, {10.7, 18.7, 34, 54.5, 215}},
+        {{0, 0, 20.2, 42.5, 187}, {0, 15, 30, 60.5, 315}, {0, 19.2, 40.7, 76, 435}, {13.8, 26.5, 53.5, 97, never}}};
+    const double d = at[P][F == NF_U ? 0 : F == NF_E ? 3 : F == NF_H || F == NF_HG ? 2 : 1][k];
+    return d * d;
+}
+template <int P, int F>
 __device__ __forceinline__ int nd_far_rule(double D2, double L2) {
-    if (P == 0) return D2 > (42.0 * 42.0) * L2 ? 3 : D2 > (18.0 * 18.0) * L2 ? 2 : D2 > (11.0 * 11.0) * L2 ? 1 : 0;
-    if (P == 1) return D2 > (90.0 * 90.0) * L2 ? 3 : D2 > (30.0 * 30.0) * L2 ? 2 : D2 > (17.0 * 17.0) * L2 ? 1 : 0;
-    return D2 > (55.0 * 55.0) * L2 ? 2 : D2 > (26.0 * 26.0) * L2 ? 1 : 0;
+    constexpr double a0 = nd_far_at(P, F, 0), a1 = nd_far_at(P, F, 1), a2 = nd_far_at(P, F, 2), a3 = nd_far_at(P, F, 3),
+                     a4 = nd_far_at(P, F, 4);
+    if (D2 > a2 * L2) return D2 > a4 * L2 ? 5 : D2 > a3 * L2 ? 4 : 3;
+    return a1 == 0.0 || D2 > a1 * L2 ? 2 : a0 == 0.0 || D2 > a0 * L2 ? 1 : 0;
 }
 // first and last + 1 point of rule r
-__device__ __forceinline__ int nd_far_first(int r) { return r == 0 ? 47 : r == 1 ? 28 : r == 2 ? 12 : 0; }
-__device__ __forceinline__ int nd_far_last(int r) { return r == 0 ? 72 : r == 1 ? 47 : r == 2 ? 28 : 12; }
+__device__ __forceinline__ int nd_far_first(int r) {
+    return r == 0 ? 105 : r == 1 ? 72 : r == 2 ? 47 : r == 3 ? 28 : r == 4 ? 12 : 0;
+}
+__device__ __forceinline__ int nd_far_last(int r) {
+    return r == 0 ? 147 : r == 1 ? 105 : r == 2 ? 72 : r == 3 ? 47 : r == 4 ? 28 : 12;
+}
 
 // ---------------------------------------------------------------------------
 // per-source record
@@ -741,7 +759,7 @@ __device__ __noinline__ void far_t_general(const NodalRec& g, const double* x, c
         for (int t = 0; t < 3; t++) W3[k][t] = 0.0;
         for (int t = 0; t < 10; t++) W5[k][t] = 0.0;
     }
-    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+    far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
         const double iR = rsqrt(R2), iR2 = iR * iR;
         const double a = iR * iR2, b = a * iR2;
         const double x11 = xi1 * xi1, x22 = xi2 * xi2;
@@ -776,7 +794,7 @@ __device__ __forceinline__ void pair_t_block(const NodalRec& g, const double* x,
         for (int k = 0; k < K; k++)
 #pragma unroll
             for (int t = 0; t < 8; t++) acc[k][t] = 0.0;
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = iR * iR2, b = a * iR2;
             const double b1 = b * xi1, b2 = b * xi2;
@@ -862,7 +880,7 @@ __device__ __forceinline__ void pair_t_basis(const NodalRec& g, const double* x,
             for (int t = 0; t < 3; t++) W3[k][t] = 0.0;
             for (int t = 0; t < 10; t++) W5[k][t] = 0.0;
         }
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        far_points(g, o, nd_far_rule<P, NF_H>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = iR * iR2, b = a * iR2;
             const double x11 = xi1 * xi1, x22 = xi2 * xi2;
@@ -903,8 +921,9 @@ __device__ __forceinline__ void pair_t_basis(const NodalRec& g, const double* x,
 }
 
 // U: put(k, I1, I3, T2) with T2 = int N_k d d / R^3 as 00 11 22 01 02 12
-// (global frame) times c2, I1 = int N_k / R and I3 = int N_k / R^3
-template <int P, class Put>
+// (global frame) times c2, I1 = int N_k / R and I3 = int N_k / R^3. F: the far rules' family
+// (the blocks by themselves: I3 falls off as the T kernel does)
+template <int P, int F, class Put>
 __device__ __forceinline__ void pair_u(const NodalRec& g, const double* x, double c2, Put&& put) {
     constexpr int K = nd_nodes(P);
     const NodalObs o = nodal_obs(g, x);
@@ -915,7 +934,7 @@ __device__ __forceinline__ void pair_u(const NodalRec& g, const double* x, doubl
         for (int k = 0; k < K; k++)
 #pragma unroll
             for (int t = 0; t < 8; t++) A[k][t] = 0.0;
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        far_points(g, o, nd_far_rule<P, F>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = iR * iR2;
             const double v0 = a * xi1, v1 = a * xi2;
@@ -1039,7 +1058,7 @@ __device__ __noinline__ void far_t_contract_general(const NodalRec& g, const Nod
     const NodalObs o = nodal_obs(g, x);
     const double z = o.z, c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
     const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
-    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+    far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
         const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
         const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
                      u2 = den_value<P>(D.f[2], e1, e2);
@@ -1071,7 +1090,7 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
             // normal s e3: s [ q d + pb z u + e3 sum pb (d.u) ], q = pa u3 + w6 z b (d.u)
             const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2, wz = c.w6 * z;
             double s0 = 0.0, s1 = 0.0, sq = 0.0, sd = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
-            far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+            far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
                 const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
                 const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
                              u2 = den_value<P>(D.f[2], e1, e2);
@@ -1140,7 +1159,7 @@ __device__ __forceinline__ void pair_u_contract(const NodalRec& g, const NodalDe
     const double ce = c[1] * g.eps2;
     double v[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        far_points(g, o, nd_far_rule<P, NF_U>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
             const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
                          u2 = den_value<P>(D.f[2], e1, e2);
@@ -1203,15 +1222,15 @@ __device__ __forceinline__ void eig_six(const SMat& m, double eps2, const double
 // f d d (f as below), G (z u + (d.u) e3) d, A u, and scalars in u3 and d.u, so the
 // sums are of those and the stress is formed once.
 template <int P>
-__device__ __forceinline__ void far_dd_frame(const NodalRec& g, const NodalDen<P>& D, const NodalObs& o, const SMat& m,
-                                             double v[6], double I7[3]) {
+__device__ __forceinline__ void far_dd_frame(const NodalRec& g, const NodalDen<P>& D, const NodalObs& o, int rule,
+                                             const SMat& m, double v[6], double I7[3]) {
     const double z = o.z, e = g.eps2, cb = m.blob * e, c15 = 15.0 * cb, ce = 15.0 * (cb - e);
     const double lam = m.lam, mu = m.mu, xt = m.x1 + 15.0;
     // f = u3 (kb b + kc c) + kd c (d.u)
     const double kb = 2.0 * lam * xt - 12.0 * mu, kc = 2.0 * lam * ce, kd = 60.0 * mu * z;
     double S00 = 0, S01 = 0, S11 = 0, f0s = 0, f1s = 0, fs = 0, au[3] = {0, 0, 0}, bu[3] = {0, 0, 0}, cu[3] = {0, 0, 0};
     double bd = 0, cd = 0, V0 = 0, V1 = 0, W0[3] = {0, 0, 0}, W1[3] = {0, 0, 0};
-    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+    far_points(g, o, rule, [&](double xi1, double xi2, double R2, int q) {
         const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
         const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
         const double iR = rsqrt(R2), iR2 = iR * iR;
@@ -1271,8 +1290,8 @@ __device__ __forceinline__ void far_dd_frame(const NodalRec& g, const NodalDen<P
 
 // the same for any normal
 template <int P>
-__device__ __noinline__ void far_dd_general(const NodalRec& g, const NodalDen<P>& D, const double* x, const SMat& m,
-                                            double v[6], double I7[3]) {
+__device__ __noinline__ void far_dd_general(const NodalRec& g, const NodalDen<P>& D, const double* x, int rule,
+                                            const SMat& m, double v[6], double I7[3]) {
     const NodalObs o = nodal_obs(g, x);
     const double z = o.z, e2 = g.eps2;
     const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
@@ -1281,7 +1300,7 @@ __device__ __noinline__ void far_dd_general(const NodalRec& g, const NodalDen<P>
     double S[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, V[3] = {0.0, 0.0, 0.0}, su = 0.0, Q[3] = {0.0, 0.0, 0.0};
     double W[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
     const double l2 = 2.0 * m.lam, mu2 = 2.0 * m.mu;
-    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+    far_points(g, o, rule, [&](double xi1, double xi2, double R2, int q) {
         const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
         const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
         const double iR = rsqrt(R2), iR2 = iR * iR;
@@ -1334,8 +1353,9 @@ __device__ __forceinline__ void pair_dd_contract(const NodalRec& g, const NodalD
     double I7[3] = {0.0, 0.0, 0.0};          // int u / R^7
     const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
     if (nodal_is_far(g, o)) {
-        if (g.aligned) far_dd_frame<P>(g, D, o, m, v, I7);
-        else far_dd_general<P>(g, D, x, m, v, I7);
+        const int rule = acc_e ? nd_far_rule<P, NF_E>(o.D2, g.L2) : nd_far_rule<P, NF_H>(o.D2, g.L2);
+        if (g.aligned) far_dd_frame<P>(g, D, o, rule, m, v, I7);
+        else far_dd_general<P>(g, D, x, rule, m, v, I7);
         if (eig) {
             const double nl[3] = {n0, n1, n2};
             double e[6];
@@ -1393,7 +1413,7 @@ __device__ __forceinline__ void pair_eig_contract(const NodalRec& g, const Nodal
     const NodalObs o = nodal_obs(g, x);
     double I7[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+        far_points(g, o, nd_far_rule<P, NF_E>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
             const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double c = far_w(q) * iR * (iR2 * iR2) * iR2;
@@ -1437,7 +1457,7 @@ __device__ __forceinline__ void far_s_moments(const NodalRec& g, const NodalObs&
 #pragma unroll
         for (int t = 0; t < 10; t++) W5[j][t] = 0.0;
     }
-    far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
+    far_points(g, o, nd_far_rule<P, NF_S>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
         const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
         const double iR = rsqrt(R2), iR2 = iR * iR;
         const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2;
@@ -1555,7 +1575,7 @@ __device__ __forceinline__ void pair_traction_fam(const NodalRec& g, const doubl
 #pragma unroll
             for (int t = 0; t < 15; t++) W7[k][t] = 0.0;
         }
-        far_points(g, o, nd_far_rule<P>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q0) {
+        far_points(g, o, nd_far_rule<P, F>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q0) {
             const double iR = rsqrt(R2), iR2 = iR * iR;
             const double a = iR * iR2, b = a * iR2, c = b * iR2;
             double p[15];

@@ -6,7 +6,7 @@
 // does not depend on the order of the adds).
 //
 // Bound by the FP64 pipe. 288 points x 6,144 P0 sources ("slip"): 70.2 ms with
-// run-time tables in local memory and 144 / 64 far points, 3.97 ms now.
+// run-time tables in local memory and 144 / 64 far points, 4.26 ms now.
 #include "nodal_launch.cuh"
 
 namespace mbem {
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(ND_THREADS) nodal_traction_kernel(NodalArgs a,
         const int nf = (int)lmin(fb, a.n_field_pts - f0), total = ns * nf;
         queue_pairs(queue, total, [&](int p) {
             const int t = p / nf;
-            return pair_class<P>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
+            return pair_class<P, F>(recs[t], a.x_field + 3 * (f0 + (p - t * nf)));
         });
         int p;
 #pragma unroll 1
