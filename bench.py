@@ -491,13 +491,13 @@ def _sync_time(fn):
 def multi_rhs_workload(peaks, n_face=24, n_fault=16, n_rhs=256):
     """Many right-hand sides (cube 24 x 24 per face, fault 16 x 16, 256 slip
     patterns from a Gaussian random field): the mixed operator, its
-    three-term BF16 copy and the block solver (batched GMRES on the tcgen05
-    GEMM inside FP64-accurate refinement), against the plain FP64 path
+    BF16 copy and the block solver (batched GMRES on the tcgen05 three-term
+    product inside FP64-accurate refinement), against the plain FP64 path
     solving the 256 systems one by one (FGMRES on the FP64 matrix)."""
     import torch
     from mbem_gb300.backends.dense import DenseBackend
     from mbem_gb300.cases import cube_fault_model, gaussian_slips
-    from mbem_gb300.la.multirhs import BlockSolver, gemm_bf16_t, slip_rhs
+    from mbem_gb300.la.multirhs import BlockSolver, slip_rhs
     from mbem_gb300.model import generate_system
     model, eps = cube_fault_model(n_face, n_fault)
     system = generate_system(model)
@@ -514,39 +514,31 @@ def multi_rhs_workload(peaks, n_face=24, n_fault=16, n_rhs=256):
         (X, rep), t_solve = _sync_time(lambda: bs.solve(B, rtol=RTOL))
         if timed:
             break
-        # after the warm-up pass: the GEMM's K split, tuned on the solver's own operator
-        from mbem_gb300 import autotune
-        Vt = torch.randn((n_rhs, bs.A16.shape[1]), device="cuda").to(torch.bfloat16)
-        Wt = torch.empty((n_rhs, bs.n), device="cuda")
-        out["autotune"] = autotune.Autotuner(cache_path="").tune(
-            "gemm_split", f"M={bs.n},K={bs.A16.shape[1]},k={n_rhs}",
-            lambda: gemm_bf16_t(bs.A16, Vt, bs.A16.shape[1], Wt)).summary()
-        del Vt, Wt, bs, asm
+        del bs, asm
         torch.cuda.empty_cache()
     total = t_asm + t_rhs + t_bf + t_solve
     n = bs.n
     Vbf = torch.randn((n_rhs, bs.A16.shape[1]), device="cuda").to(torch.bfloat16)
-    W = torch.empty((n_rhs, n), device="cuda")
-    K = bs.A16.shape[1]
+    work = bs.product_workspace(n_rhs)
     for _ in range(3):
-        gemm_bf16_t(bs.A16, Vbf, K, W)
+        bs.product_parts(Vbf, work)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
     for _ in range(10):
-        gemm_bf16_t(bs.A16, Vbf, K, W)
+        bs.product_parts(Vbf, work)
     e1.record()
     torch.cuda.synchronize()
     gemm_ms = e0.elapsed_time(e1) / 10
-    flops = 2.0 * n * K * n_rhs
+    flops = 2.0 * n * (3 * n) * n_rhs              # three terms
     bf16_peak = peaks.get("bf16_tflops") or 1900.0
     out["mixed_block"] = {"s": total, "assembly_s": t_asm, "rhs_s": t_rhs, "bf16_copy_s": t_bf, "solve_s": t_solve,
                           "refinement_steps": rep.outer, "inner_iterations": rep.inner_iterations,
                           "worst_true_relres": float(np.max(rep.true_relres)), "gemm_ms_in_solve": rep.gemm_ms,
                           "residual_ms_in_solve": rep.residual_ms}
-    out["roofline_gemm"] = {"kernel": "tc_gemm_kernel (tcgen05.mma kind::f16, TMA, TMEM)", "bound": "tensor",
+    out["roofline_gemm"] = {"kernel": "tc_block3_kernel (tcgen05.mma kind::f16, TMA, TMEM)", "bound": "tensor",
                             "achieved": flops / (gemm_ms / 1e3) / 1e12, "peak": bf16_peak, "unit": "TFLOP/s",
                             "frac": flops / (gemm_ms / 1e3) / 1e12 / bf16_peak, "launch_ms": gemm_ms,
-                            "flops_per_launch": flops, "hbm_gbs_of_A": 2.0 * n * K / (gemm_ms / 1e3) / 1e9,
+                            "flops_per_launch": flops, "hbm_gbs_of_A": 2.0 * n * bs.A16.shape[1] / (gemm_ms / 1e3) / 1e9,
                             "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)" if peaks.get("bf16_tflops")
                             else "fallback 1.9 PFLOP/s (of fallback)"}
     del bs, asm

@@ -644,13 +644,13 @@ int mbem_batch_update(double* X, const float* V, int n_vec, const double* Y, int
  * `splits` GEMM partial sums P (split_stride floats apart, (k, n) each; with kb > 0
  * mbem_gemm_bf16x3_t_parts' runs instead), the rigid translations of the u-ranges removed, two passes of classical Gram-Schmidt
  * against V[0 .. j] ((m + 1, k, n) FP32), the norm, V[j + 1], its BF16 operand in
- * Vbf (rows of ldbf; terms 3: [hi | lo | hi] at 0, ldp, 2 ldp, terms 1: [hi]), and
+ * Vbf (rows of ldbf; panels 1: [hi], 2: [hi | lo], 3: [hi | lo | hi] at 0, ldp, 2 ldp), and
  * the right-hand side's Givens rotation: H[(i m + j) k + r], cs, sn, g[i k + r]
  * (g[0] = beta = |r_0| before step 0). *left is raised by the right-hand sides whose
  * residual estimate is not below rtol beta. */
 int mbem_batch_arnoldi(const float* P, int splits, int kb, int per, int64_t split_stride, float* V, int j, int m,
                        int64_t k, int64_t n,
-                       const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int terms,
+                       const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int panels,
                        double* H, double* cs, double* sn, double* g, const double* beta, double rtol, int* left,
                        void* stream);
 /* Y[i k + r], i < cnt: the back substitution of the rotated systems */

@@ -43,9 +43,9 @@ struct ArnoldiArgs {
     int j, m;
     int64_t k, n, slice;
     URanges ur;
-    uint16_t* Vbf;           // next GEMM operand, row stride ldbf: [hi | lo | hi] at 0, ldp, 2 ldp (terms 3) or [hi]
-    int64_t ldbf, ldp;
-    int terms;
+    uint16_t* Vbf;           // next GEMM operand, row stride ldbf, panels at 0, ldp, 2 ldp: [hi], [hi | lo] (the
+    int64_t ldbf, ldp;       // three-term product's) or [hi | lo | hi] (of one GEMM over a three-fold K)
+    int panels;
     double *H, *cs, *sn, *g; // [(i m + j) k + r], [i k + r] x 3
     const double* beta;      // |r0|
     double rtol;
@@ -329,10 +329,8 @@ __global__ void __launch_bounds__(AR_T) batch_arnoldi_kernel(ArnoldiArgs a) {
         const __nv_bfloat16 h = __float2bfloat16_rn(v);
         const uint16_t hb = __bfloat16_as_ushort(h);
         vb[t] = hb;
-        if (a.terms == 3) {
-            vb[a.ldp + t] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(h)));
-            vb[2 * a.ldp + t] = hb;
-        }
+        if (a.panels > 1) vb[a.ldp + t] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(h)));
+        if (a.panels > 2) vb[2 * a.ldp + t] = hb;
     }
     // the column's rotations, by one thread of the right-hand side
     if (rank == 0 && threadIdx.x == 0) {
@@ -380,20 +378,20 @@ using namespace mbem;
 extern "C" {
 
 int mbem_batch_arnoldi(const float* P, int splits, int kb, int per, int64_t split_stride, float* V, int j, int m, int64_t k, int64_t n,
-                       const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int terms,
+                       const int64_t* u_ranges, int n_u_ranges, uint16_t* Vbf, int64_t ldbf, int64_t ldp, int panels,
                        double* H, double* cs, double* sn, double* g, const double* beta, double rtol, int* left,
                        void* stream) {
     MBEM_REQUIRE(P && V && Vbf && H && cs && sn && g && beta && left && k >= 1 && n >= 1, MBEM_ERR_ARG,
                  "bad batched Arnoldi arguments");
     MBEM_REQUIRE(kb == 0 ? splits >= 1 : kb > 0 && per > 0, MBEM_ERR_ARG, "bad batched Arnoldi partial sums");
     MBEM_REQUIRE(j >= 0 && j < m, MBEM_ERR_ARG, "batched Arnoldi: step %d of %d", j, m);
-    MBEM_REQUIRE((terms == 1 || terms == 3) && ldp >= n && ldbf >= terms * ldp && split_stride >= (kb > 0 || splits > 1 ? k * n : 0),
+    MBEM_REQUIRE(panels >= 1 && panels <= 3 && ldp >= n && ldbf >= panels * ldp && split_stride >= (kb > 0 || splits > 1 ? k * n : 0),
                  MBEM_ERR_ARG, "bad batched Arnoldi strides");
     ArnoldiArgs a;
     int e = make_ranges(u_ranges, n_u_ranges, a.ur);
     if (e) return e;
     a.P = P; a.splits = splits; a.kb = kb; a.per = per; a.split_stride = split_stride; a.V = V; a.j = j; a.m = m; a.k = k; a.n = n;
-    a.Vbf = Vbf; a.ldbf = ldbf; a.ldp = ldp; a.terms = terms; a.H = H; a.cs = cs; a.sn = sn; a.g = g; a.beta = beta;
+    a.Vbf = Vbf; a.ldbf = ldbf; a.ldp = ldp; a.panels = panels; a.H = H; a.cs = cs; a.sn = sn; a.g = g; a.beta = beta;
     a.rtol = rtol; a.left = left;
     // blocks a cluster: a slice fits twice an SM, and there are two blocks an SM
     int ranks = 1;

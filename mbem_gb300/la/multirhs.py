@@ -108,7 +108,7 @@ class BlockSolver:
         """``terms``: 1 = the operator in BF16 (relative error ~2^-9 per
         product: about five refinement steps to 1e-8); 3 = A and the Krylov
         vectors each split into BF16 high and low parts, A_hi V_hi + A_hi
-        V_lo + A_lo V_hi in one GEMM over a three-fold K (error ~2^-16: two
+        V_lo + A_lo V_hi in one product (error ~2^-16: two
         refinement steps)."""
         if terms not in (1, 3):
             raise ValueError("terms must be 1 or 3")
@@ -122,10 +122,11 @@ class BlockSolver:
         self.device = dev
         self.n = n = int(asm.b.shape[0])
         self.ldp = _pad8(n)
-        # A16 = [A_hi | A_hi | A_lo] (terms 3) or A_hi, each block ldp wide
-        self.A16 = torch.zeros((n, terms * self.ldp), dtype=torch.bfloat16, device=dev)
+        # A16 = [A_hi | A_lo] (terms 3) or A_hi, each panel ldp wide
+        self.panels = 2 if terms == 3 else 1
+        self.A16 = torch.zeros((n, self.panels * self.ldp), dtype=torch.bfloat16, device=dev)
         hi = self.A16[:, :self.ldp]
-        lo = self.A16[:, 2 * self.ldp:] if terms == 3 else None
+        lo = self.A16[:, self.ldp:] if terms == 3 else None
         st = stream_handle()
         ld16 = self.A16.stride(0)
         if self.op is not None:
@@ -135,8 +136,6 @@ class BlockSolver:
             nat.call("mbem_to_bf16x2", ptr(self.A), 1, self.A.stride(0), n, n, ptr(hi), ptr(lo), ld16, st)
         else:
             nat.call("mbem_to_bf16", ptr(self.A), 1, self.A.stride(0), n, n, ptr(hi), ld16, st)
-        if terms == 3:
-            self.A16[:, self.ldp:self.ldp + n] = hi[:, :n]
         rng = np.ascontiguousarray(np.asarray(asm.u_ranges(), dtype=np.int64).reshape(-1))
         self._ranges = rng
         self.inner_restart = inner_restart
@@ -170,47 +169,57 @@ class BlockSolver:
             R = B - Y.T
         return self.project(R)
 
+    def product_workspace(self, k: int) -> torch.Tensor:
+        return torch.empty(nat.lib().mbem_gemm_bf16_workspace_size(self.n, k) // 4, dtype=torch.float32,
+                           device=self.device)
+
+    def product_parts(self, Vbf: torch.Tensor, work: torch.Tensor):
+        """A16's product with the BF16 vectors of ``Vbf`` (k, panels ldp) as
+        partial sums in ``work``: (splits, kb, per), what
+        ``mbem_batch_arnoldi`` adds them up by."""
+        k, ld, st = Vbf.shape[0], self.ldp, stream_handle()
+        parts, kb, per = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+        if self.terms == 3:
+            nat.call("mbem_gemm_bf16x3_t_parts", ptr(self.A16), self.A16.stride(0), ld, ptr(Vbf), Vbf.stride(0), ld,
+                     self.n, self.n, k, ptr(work), 4 * work.numel(), ctypes.byref(kb), ctypes.byref(per), st)
+        else:
+            nat.call("mbem_gemm_bf16_t_parts", ptr(self.A16), self.A16.stride(0), ptr(Vbf), Vbf.stride(0), self.n, ld,
+                     k, ptr(work), 4 * work.numel(), ctypes.byref(parts), st)
+        return parts.value, kb.value, per.value
+
     def inner_gmres(self, R: torch.Tensor, m: int, rtol: float):
         """D (k, n) FP64 with |R - A16 D| small for every row, by batched
         GMRES(m) on the BF16 operator; returns (D, iterations, gemm_ms)."""
         k, n = R.shape
         dev = self.device
         st = stream_handle()
-        ld, terms = self.ldp, self.terms
+        ld = self.ldp
         V = torch.empty((m + 1, k, n), dtype=torch.float32, device=dev)
-        # the GEMM operand [V_hi | V_lo | V_hi] (or V_hi); its padding stays zero
-        Vbf = torch.zeros((k, terms * ld), dtype=torch.bfloat16, device=dev)
+        # the GEMM operand [V_hi | V_lo] (or V_hi); its padding stays zero
+        Vbf = torch.zeros((k, self.panels * ld), dtype=torch.bfloat16, device=dev)
         beta = torch.empty(k, dtype=torch.float64, device=dev)
         nat.call("mbem_batch_normalize", ptr(R), 1, k, n, ptr(beta), ptr(V[0]), None, st)
         vh = V[0].to(torch.bfloat16)
         Vbf[:, :n] = vh
-        if terms == 3:
+        if self.panels == 2:
             Vbf[:, ld:ld + n] = (V[0] - vh.float()).to(torch.bfloat16)
-            Vbf[:, 2 * ld:2 * ld + n] = vh
         H = torch.zeros((m, m, k), dtype=torch.float64, device=dev)
         rot = torch.zeros((2, m, k), dtype=torch.float64, device=dev)
         g = torch.zeros((m + 1, k), dtype=torch.float64, device=dev)
         g[0] = beta
         left = torch.zeros(m, dtype=torch.int32, device=dev)
-        need = nat.lib().mbem_gemm_bf16_workspace_size(n, k)
-        work = torch.empty(need // 4, dtype=torch.float32, device=dev)
-        parts, kb, per = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+        work = self.product_workspace(k)
         ranges = self._ranges.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
         events = []
         jdone = 0
         for j in range(m):
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record()
-            if terms == 3:
-                nat.call("mbem_gemm_bf16x3_t_parts", ptr(self.A16), self.A16.stride(0), 2 * ld, ptr(Vbf),
-                         Vbf.stride(0), ld, n, n, k, ptr(work), need, ctypes.byref(kb), ctypes.byref(per), st)
-            else:
-                nat.call("mbem_gemm_bf16_t_parts", ptr(self.A16), self.A16.stride(0), ptr(Vbf), Vbf.stride(0), n,
-                         terms * ld, k, ptr(work), need, ctypes.byref(parts), st)
+            parts, kb, per = self.product_parts(Vbf, work)
             ev[1].record()
             events.append(ev)
-            nat.call("mbem_batch_arnoldi", ptr(work), parts.value, kb.value, per.value, n * k, ptr(V), j, m, k, n,
-                     ranges, len(self._ranges) // 2, ptr(Vbf), Vbf.stride(0), ld, terms, ptr(H), ptr(rot[0]), ptr(rot[1]),
+            nat.call("mbem_batch_arnoldi", ptr(work), parts, kb, per, n * k, ptr(V), j, m, k, n, ranges,
+                     len(self._ranges) // 2, ptr(Vbf), Vbf.stride(0), ld, self.panels, ptr(H), ptr(rot[0]), ptr(rot[1]),
                      ptr(g), ptr(beta), float(rtol), ptr(left[j:]), st)
             jdone = j + 1
             if int(left[j]) == 0:

@@ -81,3 +81,48 @@ def test_one_term_solver(gpu):
         assert rep.converged and np.all(rep.true_relres < 1e-9)
         X.append(x)
     assert float((X[0] - X[1]).norm() / X[1].norm()) < 1e-6
+
+
+@pytest.mark.parametrize("n", [1003, 1024])
+def test_operand_panels(gpu, n):
+    """The next product's operand is [hi], [hi | lo] or [hi | lo | hi] of one and the same vector."""
+    from mbem_gb300 import _native as nat
+    from mbem_gb300._device import ptr, stream_handle
+    k, m, ldp, dev = 3, 2, (n + 7) // 8 * 8, "cuda"
+    P = torch.randn((1, k, n), device=dev)
+    V0 = torch.nn.functional.normalize(torch.randn((k, n), device=dev), dim=1)
+    seen = []
+    for panels in (1, 2, 3):
+        V = torch.zeros((m + 1, k, n), device=dev)
+        V[0] = V0
+        Vbf = torch.zeros((k, panels * ldp), dtype=torch.bfloat16, device=dev)
+        H = torch.zeros((m, m, k), dtype=torch.float64, device=dev)
+        cs, sn = (torch.zeros((m, k), dtype=torch.float64, device=dev) for _ in range(2))
+        g, beta = torch.ones((m + 1, k), dtype=torch.float64, device=dev), torch.ones(k, dtype=torch.float64, device=dev)
+        left = torch.zeros(1, dtype=torch.int32, device=dev)
+        nat.call("mbem_batch_arnoldi", ptr(P), 1, 0, 0, n * k, ptr(V), 0, m, k, n, None, 0, ptr(Vbf), Vbf.stride(0), ldp,
+                 panels, ptr(H), ptr(cs), ptr(sn), ptr(g), ptr(beta), 1e-3, ptr(left), stream_handle())
+        hi = V[1].to(torch.bfloat16)
+        lo = (V[1] - hi.float()).to(torch.bfloat16)
+        seen.append(V[1])
+        for p, want in enumerate((hi, lo, hi)[:panels]):
+            assert torch.equal(Vbf[:, p * ldp:p * ldp + n], want)
+    assert torch.equal(seen[0], seen[1]) and torch.equal(seen[0], seen[2])
+
+
+def test_two_panels_are_held(gpu):
+    from mbem_gb300.backends.dense import DenseBackend
+    from mbem_gb300.cases import cube_fault_model
+    from mbem_gb300.la.multirhs import BlockSolver
+    from mbem_gb300.model import generate_system
+    model, eps = cube_fault_model(4, 2)
+    asm = DenseBackend(jump="calibrated", deflate=True, precision="mixed").assemble(generate_system(model), eps)
+    for terms, panels in ((1, 1), (3, 2)):
+        bs = BlockSolver(asm, terms=terms)
+        assert bs.A16.shape == (bs.n, panels * bs.ldp)
+        if terms == 3:
+            A = asm.op.dense64()
+            A16 = bs.A16[:, :bs.n].double() + bs.A16[:, bs.ldp:bs.ldp + bs.n].double()
+            assert float((A16 - A).abs().max() / A.abs().max()) < 2.0 ** -16
+
+
