@@ -60,6 +60,9 @@ int mbem_fp32_fma_probe(float* out, int64_t iters, int blocks, int threads, int 
  * DFMA chains of `iters` steps (16*iters FLOP per thread); time it with
  * events for the FP64 roofline denominator. No reference counterpart. */
 int mbem_fp64_fma_probe(double* out, int64_t iters, int blocks, int threads, void* stream);
+/* The FP64 functions of the pair kernels (dp_math.cuh), one value a thread: fn 0: 1 / x,
+ * 1: log x, 2: the angle of (x, y), 3 and 4: x^(-3/2) and x^(-5/2). y is read by fn 2 only. */
+int mbem_dp_math_probe(int fn, const double* x, const double* y, int64_t n, double* out, void* stream);
 
 /* ---- kernel matrices: src/mbem/kernels/tri_nodal.py:1289-1306 (public
  * drivers) and src/mbem/kernels/tri_kernels.py:547-591 (P0 direct).

@@ -155,6 +155,7 @@ _SIGNATURES = {
     "mbem_launch_count": (ctypes.c_ulonglong, []),
     "mbem_fp32_fma_probe": (c_int, [_P, _I, c_int, c_int, c_int, _P]),
     "mbem_fp64_fma_probe": (c_int, [_P, _I, c_int, c_int, _P]),
+    "mbem_dp_math_probe": (c_int, [c_int, _P, _P, _I, _P, _P]),
     "mbem_shape_screen": (c_int, [_P, _I, _D, POINTER(c_int), _P]),
     "mbem_t_matrix_direct": (c_int, [_P, _I, _P, _P, _P, _I, _P, c_int, _D, c_int, _P, _I, _P]),
     "mbem_u_matrix_direct": (c_int, [_P, _I, _P, _P, _I, _P, c_int, _D, c_int, _P, _I, _P]),

@@ -5,6 +5,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "dp_math.cuh"
 
 namespace mbem {
 
@@ -47,6 +48,19 @@ __global__ void fp64_fma_probe_kernel(double* out, int64_t iters) {
 #pragma unroll
     for (int k = 0; k < 8; k++) s += a[k];
     if (s == 12345.678) out[0] = s;   // keeps the chains live; never true
+}
+
+// The pair kernels' FP64 functions, one value a thread.
+__global__ void dp_math_probe_kernel(int fn, const double* __restrict__ x, const double* __restrict__ y, int64_t n,
+                                     double* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double v = x[i];
+    out[i] = fn == 0   ? rcp64(v)
+             : fn == 1 ? log64(v)
+             : fn == 2 ? angle64(y[i], v)
+             : fn == 3 ? inv_pow64<3>(v)
+                       : inv_pow64<5>(v);
 }
 
 // Independent FP32 FMA chains for the FP32 pipe's throughput: 16 scalar
@@ -95,6 +109,15 @@ int mbem_fp32_fma_probe(float* out, int64_t iters, int blocks, int threads, int 
 }
 
 unsigned long long mbem_launch_count(void) { return mbem::g_launches.load(); }
+
+int mbem_dp_math_probe(int fn, const double* x, const double* y, int64_t n, double* out, void* stream) {
+    MBEM_REQUIRE(fn >= 0 && fn <= 4 && n >= 0 && (n == 0 || (x && out && (fn != 2 || y))), MBEM_ERR_ARG,
+                 "bad FP64 function probe");
+    MBEM_REQUIRE(mbem::ceil_div(n, 256) < INT32_MAX, MBEM_ERR_SIZE, "too many values");
+    if (n == 0) return MBEM_OK;
+    mbem::dp_math_probe_kernel<<<(unsigned)mbem::ceil_div(n, 256), 256, 0, (cudaStream_t)stream>>>(fn, x, y, n, out);
+    return mbem::launch_status("dp_math_probe_kernel");
+}
 
 int mbem_fp64_fma_probe(double* out, int64_t iters, int blocks, int threads, void* stream) {
     MBEM_REQUIRE(out && iters > 0 && blocks > 0 && threads > 0 && threads <= 1024, MBEM_ERR_ARG,
