@@ -145,8 +145,10 @@ __global__ void __launch_bounds__(MAT_THREADS) p0_matrix_kernel(MatArgs a) {
     }
 }
 
-// Observers a block: the FP64 pipe takes about 200 instructions for a source's
-// frame and 400 for a pair, so a tile of t costs 200 + 400 t a warp and the part
+// Observers a block: a tile of t costs a warp 200 + 400 t FP64 instructions (a source's frame
+// and its pairs; 250 and 330 with the short functions of dp_math.cuh, whose ratio
+// would take another tile, by one to three, in a fifth of the sizes from 40 to 30,000 and the
+// same one for blocks of 128, 1,728 and 5,184 squared, the sizes measured) and the part
 // the warps of its fullest SM; below about five warps an SM the pipe waits.
 static int matrix_tile(int64_t nf, int64_t ns) {
     int best = 16;
@@ -367,8 +369,12 @@ __global__ void __launch_bounds__(CON_THREADS) p0_contract_kernel(ConArgs a) {
 // tile's size, so few observers want large tiles: up to CON_FEW of them one observer a
 // block of 128 threads with 128 sources a tile (6,912 sources at 1 to 19 observers:
 // 480 us with 64 threads and tiles of 32, 150 with these; at 48 observers 507 and 370).
-// Above, contract_split's blocks of observers with 64 threads and tiles of 32 (at 200
-// observers 1,130 us, 1,145 with 128; at 1,000 4,960 and 5,070).
+// Above, contract_split's blocks of observers with 64 threads and tiles of 32. The two meet
+// at 76 observers, half an SM's share each (6,912 sources, T displacement | elastic
+// stress, one observer a block against contract_split's: 48: 375 | 530 and 517 | 687 us, 70: 500 | 687 and
+// 517 | 688, 76: 624 | 860 and 627 | 895, 80: 629 | 880 and 629 | 896, 90: 735 | 1,020 and
+// 629 | 896, 200: 1,425 | 2,045 and 1,100 | 1,654; 1,000 sources: 76: 98 | 140 and 99 | 141,
+// 90: 115 | 163 and 100 | 141).
 constexpr int64_t CON_FEW = 76;
 
 template <int KIND>
