@@ -1,7 +1,12 @@
 """One launch (or a few) of a hot kernel on a small case, for profilers
 (test tooling, not part of the package): ``python tests/kernel_cases.py <case>``.
 
-tcgemm    the block solver's GEMM: (20,736 x 62,208 BF16) x (62,208 x 256)
+tcgemm    the plain tensor-core GEMM: (20,736 x 62,208 BF16) x (62,208 x 256)
+block3    the block solver's three-term product (tc_block3_kernel) and Arnoldi
+          step (batch_arnoldi_kernel, 12th vector): 20,736 unknowns, 256
+          right-hand sides
+blockres  its residual's far field (tc_exact_kernel, ex_*) at the same sizes
+arnoldi   the FP64 solve of cube 12 (kv_cluster_kernel)
 traction  FAULT_TRACTION assembly, cube 16 x 16, fault 12 x 12, dip 60,
           with its block-Jacobi build (traction rows, bj_build_kernel)
 dfgemm    the block residual of the mixed operator, cube 24, 64 RHS
@@ -57,6 +62,45 @@ def run(which: str) -> None:
         W = torch.empty((k, n), device="cuda")
         for _ in range(3):
             gemm_bf16_t(A, X, 3 * n, W)
+    elif which == "block3":
+        import ctypes
+
+        from mbem_gb300 import _native as nat
+        from mbem_gb300._device import ptr, stream_handle
+        n, k, m, j, st = 20736, 256, 12, 11, stream_handle()
+        A = torch.randn((n, 2 * n), device="cuda").to(torch.bfloat16)
+        V = torch.randn((m + 1, k, n), device="cuda") / n ** 0.5
+        X = torch.zeros((k, 2 * n), dtype=torch.bfloat16, device="cuda")
+        X[:, :n] = V[j]
+        work = torch.empty(nat.lib().mbem_gemm_bf16_workspace_size(n, k) // 4, device="cuda")
+        H = torch.zeros((m, m, k), dtype=torch.float64, device="cuda")
+        cs, sn, g = (torch.ones((m + 1, k), dtype=torch.float64, device="cuda") for _ in range(3))
+        left = torch.zeros(1, dtype=torch.int32, device="cuda")
+        u = np.array([0, n], dtype=np.int64)
+        kb, per = ctypes.c_int(0), ctypes.c_int(0)
+        for _ in range(3):
+            nat.call("mbem_gemm_bf16x3_t_parts", ptr(A), A.stride(0), n, ptr(X), X.stride(0), n, n, n, k, ptr(work),
+                     4 * work.numel(), ctypes.byref(kb), ctypes.byref(per), st)
+            nat.call("mbem_batch_arnoldi", ptr(work), 0, kb.value, per.value, n * k, ptr(V), j, m, k, n,
+                     u.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), 1, ptr(X), X.stride(0), n, 2, ptr(H), ptr(cs),
+                     ptr(sn), ptr(g), ptr(g), 1e-3, ptr(left), st)
+    elif which == "blockres":
+        import ctypes
+
+        from mbem_gb300 import _native as nat
+        from mbem_gb300._device import ptr, stream_handle
+        from mbem_gb300.la.mixed import MixedOperator
+        n, k = 20736, 256
+        s = MixedOperator(torch.randn((n, n), device="cuda"), []).struct()
+        B, X = (torch.randn((k, n), dtype=torch.float64, device="cuda") for _ in range(2))
+        R, need = torch.empty_like(B), nat.lib().mbem_batch_residual_workspace_size(k, n)
+        work = torch.empty(need // 8, dtype=torch.float64, device="cuda")
+        for _ in range(2):
+            nat.call("mbem_batch_residual_mixed", ctypes.byref(s), ptr(B), ptr(X), k, ptr(R), ptr(work), need,
+                     stream_handle())
+    elif which == "arnoldi":
+        model, eps = cube_fault_model(12, 8)
+        DenseBackend(jump="calibrated", deflate=True, rtol=1e-10).assemble(generate_system(model), eps).solve()
     elif which == "traction":
         model, eps = fault_traction_model(16, 12, 60.0)
         asm = DenseBackend(jump="calibrated", deflate=True).assemble(generate_system(model), eps)
