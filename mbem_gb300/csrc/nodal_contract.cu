@@ -6,7 +6,7 @@
 // block: a few observers still fill the part, each partial sum has one owner
 // and the sums are added in slice, then rank order through distributed shared
 // memory (deterministic, no workspace). Bound by the FP64 pipe: the stress of a
-// 16 x 16 P2 fault at 2,000 observers went from 266 to 5.85 ms (4.85 with far rules off by up
+// 16 x 16 P2 fault at 2,000 observers went from 266 to 5.97 ms (4.85 with far rules off by up
 // to 2e-14, nd_far_rule).
 #include <cooperative_groups.h>
 

@@ -724,8 +724,7 @@ __device__ __forceinline__ void far_points(const NodalRec& g, const NodalObs& o,
         fn(xi1, xi2, xi1 * xi1 + xi2 * xi2 + o.h2, q);
     }
 }
-// weight of point q, and times the shape function of node k
-__device__ __forceinline__ double far_w(int q) { return MBEM_ND_RULES.fl[q][2]; }
+// weight of point q times the shape function of node k
 template <int P>
 __device__ __forceinline__ double far_wn(int q, int k) {
     return P == 0 ? MBEM_ND_RULES.fl[q][2] : MBEM_ND_RULES.fn[q][(P == 2 ? 3 : 0) + k];
@@ -1044,11 +1043,21 @@ __device__ __forceinline__ void den_at_foot(const double* f, double X1, double X
         q[5] = f[5];
     }
 }
+// Far pairs take the density from its nodal values and the rule's weighted shape functions:
+// u = w sum_k N_k d_k at point q. (From the polynomial about the centroid at the point's
+// coordinates, which lose D / L of their digits about the foot, the displacement of slender
+// triangles was off by 1e-12 at 30 longest edges.)
 template <int P>
-__device__ __forceinline__ double den_value(const double* f, double e1, double e2) {
-    if (P == 0) return f[0];
-    if (P == 1) return f[0] + f[1] * e1 + f[2] * e2;
-    return f[0] + e1 * (f[1] + f[3] * e1 + f[4] * e2) + e2 * (f[2] + f[5] * e2);
+__device__ __forceinline__ void far_density(const NodalDen<P>& D, int q, double u[3]) {
+    const double w0 = far_wn<P>(q, 0);
+#pragma unroll
+    for (int j = 0; j < 3; j++) u[j] = w0 * D.node[0][j];
+#pragma unroll
+    for (int k = 1; k < nd_nodes(P); k++) {
+        const double w = far_wn<P>(q, k);
+#pragma unroll
+        for (int j = 0; j < 3; j++) u[j] += w * D.node[k][j];
+    }
 }
 
 // far displacement of a slip density on a normal off the frame's (source frame)
@@ -1059,11 +1068,11 @@ __device__ __noinline__ void far_t_contract_general(const NodalRec& g, const Nod
     const double z = o.z, c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2;
     const double n0 = g.nl[0], n1 = g.nl[1], n2 = g.nl[2];
     far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
-        const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
-        const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
-                     u2 = den_value<P>(D.f[2], e1, e2);
+        double u[3];
+        far_density<P>(D, q, u);
+        const double u0 = u[0], u1 = u[1], u2 = u[2];
         const double iR = rsqrt(R2), iR2 = iR * iR;
-        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2;
+        const double a = g.area2 * iR * iR2, b = a * iR2;
         const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
         const double d0 = -xi1, d1 = -xi2;
         const double dn = d0 * n0 + d1 * n1 + z * n2, du = d0 * u0 + d1 * u1 + z * u2;
@@ -1091,11 +1100,11 @@ __device__ __forceinline__ void pair_t_contract(const NodalRec& g, const NodalDe
             const double c5 = c.c5 * g.eps2, ce6 = c.ce6 * g.eps2, wz = c.w6 * z;
             double s0 = 0.0, s1 = 0.0, sq = 0.0, sd = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
             far_points(g, o, nd_far_rule<P, NF_T>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
-                const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
-                const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
-                             u2 = den_value<P>(D.f[2], e1, e2);
+                double u[3];
+                far_density<P>(D, q, u);
+                const double u0 = u[0], u1 = u[1], u2 = u[2];
                 const double iR = rsqrt(R2), iR2 = iR * iR;
-                const double a = far_w(q) * iR * iR2, b = a * iR2;
+                const double a = iR * iR2, b = a * iR2;
                 const double pa = c.c3 * a + c5 * b, pb = c.cb * a + ce6 * b;
                 const double du = z * u2 - (xi1 * u0 + xi2 * u1);
                 const double r = pa * u2 + (wz * b) * du;
@@ -1160,12 +1169,12 @@ __device__ __forceinline__ void pair_u_contract(const NodalRec& g, const NodalDe
     double v[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
         far_points(g, o, nd_far_rule<P, NF_U>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
-            const double e1 = xi1 + o.X1, e2 = xi2 + o.X2;
-            const double u0 = den_value<P>(D.f[0], e1, e2), u1 = den_value<P>(D.f[1], e1, e2),
-                         u2 = den_value<P>(D.f[2], e1, e2);
+            double u[3];
+            far_density<P>(D, q, u);
+            const double u0 = u[0], u1 = u[1], u2 = u[2];
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double f = far_w(q) * iR, a = f * iR2;
-            const double dg = c[0] * f + ce * a, s = a * (z * u2 - (xi1 * u0 + xi2 * u1));
+            const double a = iR * iR2;
+            const double dg = c[0] * iR + ce * a, s = a * (z * u2 - (xi1 * u0 + xi2 * u1));
             v[0] += dg * u0 - (c[2] * s) * xi1;
             v[1] += dg * u1 - (c[2] * s) * xi2;
             v[2] += dg * u2 + (c[2] * s) * z;
@@ -1231,10 +1240,10 @@ __device__ __forceinline__ void far_dd_frame(const NodalRec& g, const NodalDen<P
     double S00 = 0, S01 = 0, S11 = 0, f0s = 0, f1s = 0, fs = 0, au[3] = {0, 0, 0}, bu[3] = {0, 0, 0}, cu[3] = {0, 0, 0};
     double bd = 0, cd = 0, V0 = 0, V1 = 0, W0[3] = {0, 0, 0}, W1[3] = {0, 0, 0};
     far_points(g, o, rule, [&](double xi1, double xi2, double R2, int q) {
-        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
-        const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
+        double u[3];
+        far_density<P>(D, q, u);
         const double iR = rsqrt(R2), iR2 = iR * iR;
-        const double a = far_w(q) * iR * iR2, b = a * iR2, c = b * iR2;
+        const double a = iR * iR2, b = a * iR2, c = b * iR2;
         const double du = z * u[2] - (xi1 * u[0] + xi2 * u[1]);
         const double bq = b * du, cq = c * du;
         const double f = u[2] * (kb * b + kc * c) + kd * cq;
@@ -1301,10 +1310,10 @@ __device__ __noinline__ void far_dd_general(const NodalRec& g, const NodalDen<P>
     double W[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
     const double l2 = 2.0 * m.lam, mu2 = 2.0 * m.mu;
     far_points(g, o, rule, [&](double xi1, double xi2, double R2, int q) {
-        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
-        const double u[3] = {den_value<P>(D.f[0], y1, y2), den_value<P>(D.f[1], y1, y2), den_value<P>(D.f[2], y1, y2)};
+        double u[3];
+        far_density<P>(D, q, u);
         const double iR = rsqrt(R2), iR2 = iR * iR;
-        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2, c = b * iR2;
+        const double a = g.area2 * iR * iR2, b = a * iR2, c = b * iR2;
         const double dd = R2 - e2;
         const double d[3] = {-xi1, -xi2, z};
         const double dn = d[0] * n0 + d[1] * n1 + z * n2, du = d[0] * u[0] + d[1] * u[1] + z * u[2];
@@ -1414,11 +1423,12 @@ __device__ __forceinline__ void pair_eig_contract(const NodalRec& g, const Nodal
     double I7[3] = {0.0, 0.0, 0.0};
     if (nodal_is_far(g, o)) {
         far_points(g, o, nd_far_rule<P, NF_E>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
-            const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
+            double u[3];
+            far_density<P>(D, q, u);
             const double iR = rsqrt(R2), iR2 = iR * iR;
-            const double c = far_w(q) * iR * (iR2 * iR2) * iR2;
+            const double c = iR * (iR2 * iR2) * iR2;
 #pragma unroll
-            for (int j = 0; j < 3; j++) I7[j] += c * den_value<P>(D.f[j], y1, y2);
+            for (int j = 0; j < 3; j++) I7[j] += c * u[j];
         });
 #pragma unroll
         for (int j = 0; j < 3; j++) I7[j] *= g.area2;
@@ -1448,7 +1458,7 @@ __device__ __forceinline__ void pair_eig_contract(const NodalRec& g, const Nodal
 
 // the moments m3 (degree 1) and m5 (degree 3) of a density component by quadrature
 template <int P>
-__device__ __forceinline__ void far_s_moments(const NodalRec& g, const NodalObs& o, const double (*f)[nd_nodes(P)],
+__device__ __forceinline__ void far_s_moments(const NodalRec& g, const NodalObs& o, const NodalDen<P>& D,
                                               double W3[3][3], double W5[3][10]) {
 #pragma unroll
     for (int j = 0; j < 3; j++) {
@@ -1458,15 +1468,15 @@ __device__ __forceinline__ void far_s_moments(const NodalRec& g, const NodalObs&
         for (int t = 0; t < 10; t++) W5[j][t] = 0.0;
     }
     far_points(g, o, nd_far_rule<P, NF_S>(o.D2, g.L2), [&](double xi1, double xi2, double R2, int q) {
-        const double y1 = xi1 + o.X1, y2 = xi2 + o.X2;
+        double u[3];
+        far_density<P>(D, q, u);
         const double iR = rsqrt(R2), iR2 = iR * iR;
-        const double a = g.area2 * far_w(q) * iR * iR2, b = a * iR2;
+        const double a = g.area2 * iR * iR2, b = a * iR2;
         const double x11 = xi1 * xi1, x12 = xi1 * xi2, x22 = xi2 * xi2;
         const double p[10] = {1.0, xi1, xi2, x11, x12, x22, x11 * xi1, x11 * xi2, x22 * xi1, x22 * xi2};
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const double u = den_value<P>(f[j], y1, y2);
-            const double ua = u * a, ub = u * b;
+            const double ua = u[j] * a, ub = u[j] * b;
 #pragma unroll
             for (int t = 0; t < 3; t++) W3[j][t] += ua * p[t];
 #pragma unroll
@@ -1483,7 +1493,7 @@ __device__ __forceinline__ void pair_kelvin_contract(const NodalRec& g, const No
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, G[6];
     if (nodal_is_far(g, o)) {
         double W3[3][3], W5[3][10];
-        far_s_moments<P>(g, o, D.f, W3, W5);
+        far_s_moments<P>(g, o, D, W3, W5);
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             const double fl[3] = {j == 0 ? 1.0 : 0.0, j == 1 ? 1.0 : 0.0, j == 2 ? 1.0 : 0.0};

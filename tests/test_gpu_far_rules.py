@@ -116,3 +116,36 @@ def test_far_pairs(gpu, order, dist):
                     g = got[kind][f].transpose(2, 3, 0, 1)
                 worst[kind] = max(worst.get(kind, 0.0), float(np.abs(g - v).max() / np.abs(v).max()))
     assert all(e < 5e-15 for e in worst.values()), worst
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("height", [0.01, 0.05, 0.5])
+@pytest.mark.parametrize("dist", [10.5, 14.0, 30.0, 200.0])
+def test_far_contractions(gpu, order, height, dist):
+    """A contraction of one far source against its matrix blocks times the density, slender
+    sources among them: both round some 40 times, 5e-15 of the sum of magnitudes each."""
+    from mbem_gb300.kernels import basis as kb
+    from mbem_gb300.kernels import tri_nodal as tn
+    rng = np.random.default_rng(int(1000 * height + dist) + order)
+    K = (order + 1) * (order + 2) // 2
+    tv = np.array([[0, 0, 0], [1, 0, 0], [0.3, height, 0]])
+    tv = ((tv - tv.mean(0)) @ np.linalg.qr(rng.normal(size=(3, 3)))[0])[None]
+    cr = np.cross(tv[0, 1] - tv[0, 0], tv[0, 2] - tv[0, 0])
+    n, eps = (cr / np.linalg.norm(cr))[None], np.array([0.2])
+    x = rng.normal(size=(40, 3))
+    x[:3] = tv[0] - np.roll(tv[0], 1, 0)
+    x *= dist / np.linalg.norm(x, axis=1, keepdims=True)
+    d = rng.normal(size=(K, 3))
+    t, u = kb.t_coeffs(1.0, 1.0), kb.u_coeffs(1.0, 1.0)
+    ids = np.arange(K).reshape(1, K)
+    rows = [(tn.t_disp_contract(x, tv, n, eps, d, *t, order), tn.t_matrix_direct(x, tv, n, eps, *t, order=order)),
+            (tn.u_disp_contract(x, tv, eps, d, *u, order), tn.u_matrix_direct(x, tv, eps, *u, order=order))]
+    for which, got in (("slip", tn.elastic_stress_contract(x, tv, n, eps, d, 1.0, 1.0, order)),
+                       ("eigen", tn.eigenstress_contract(x, tv, n, eps, d, 1.0, 1.0, order)),
+                       ("force", tn.kelvin_stress_contract(x, tv, eps, d, 1.0, 1.0, order))):
+        rows.append((got, tn.traction_matrix(np.repeat(x, 3, 0), np.tile(I3, (len(x), 1)), tv, n, eps, ids, K, 1.0, 1.0,
+                                             order, which)))
+    for got, M in rows:
+        err = np.abs(got.reshape(-1) - M @ d.reshape(-1))
+        size = (np.abs(M) @ np.abs(d.reshape(-1))).reshape(len(x), -1).max(1)       # of the observer
+        assert np.all(err.reshape(len(x), -1) <= 1e-14 * size[:, None]), float((err.reshape(len(x), -1) / size[:, None]).max())
