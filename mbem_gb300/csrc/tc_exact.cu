@@ -127,7 +127,7 @@ ex_col_scale_kernel(const float* __restrict__ A, int64_t lda, int64_t rows, int6
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int b = __float_as_int(fabsf(v[u]));
-            m[u] = max(m[u], b ? b - (e << 23) : NONE);
+            m[u] = max(m[u], b ? b - e * (1 << 23) : NONE);
         }
     }
 #pragma unroll
